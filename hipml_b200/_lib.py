@@ -6,9 +6,11 @@ if it cannot be loaded, importing the product path raises.
 from __future__ import annotations
 
 import ctypes as C
+import importlib.util
 import os
 
 HERE = os.path.dirname(os.path.abspath(__file__))
+CALLS_PATH = os.path.join(HERE, "lib", "_hipml_calls.so")
 LIB_PATH = os.path.join(HERE, "lib", "libhipml_cuda.so")
 
 ERR_BASE = 10000
@@ -145,6 +147,22 @@ def load() -> C.CDLL:
             fn.argtypes = args
         _lib = lib
     return _lib
+
+
+_calls = None
+
+
+def calls():
+    """The native module over the launchers that take the current torch stream."""
+    global _calls
+    if _calls is None:
+        load()
+        if not os.path.exists(CALLS_PATH):
+            raise ImportError(f"{CALLS_PATH} is missing: build it with `python hipml_b200/build.py`")
+        spec = importlib.util.spec_from_file_location("_hipml_calls", CALLS_PATH)
+        _calls = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(_calls)
+    return _calls
 
 
 def check(what: str, code: int) -> None:

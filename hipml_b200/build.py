@@ -4,11 +4,13 @@ from __future__ import annotations
 import os
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB_DIR = os.path.join(HERE, "lib")
 LIB = os.path.join(LIB_DIR, "libhipml_cuda.so")
+CALLS = os.path.join(LIB_DIR, "_hipml_calls.so")   # CPython view of the launchers
 
 SOURCES = [
     "device_api.cu",
@@ -39,16 +41,16 @@ def nvcc() -> str:
 
 
 def _stale() -> bool:
-    if not os.path.exists(LIB):
+    if not os.path.exists(LIB) or not os.path.exists(CALLS):
         return True
-    t = os.path.getmtime(LIB)
+    t = min(os.path.getmtime(LIB), os.path.getmtime(CALLS))
     deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC)]
     deps.append(os.path.join(os.path.dirname(HERE), "include", "hipml_cuda.h"))
     return any(os.path.getmtime(d) > t for d in deps)
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
-    """Compile every .cu into one shared library; returns its path."""
+    """Compile every .cu into one shared library and the Python call module; returns the library's path."""
     if not force and not _stale():
         return LIB
     os.makedirs(LIB_DIR, exist_ok=True)
@@ -62,6 +64,10 @@ def build(force: bool = False, verbose: bool = False) -> str:
         objs.append(obj)
     subprocess.check_call([nvcc(), "-shared", "-o", LIB, *objs, "-gencode",
                            "arch=compute_100a,code=sm_100a"])
+    # (links to the library beside it: the process holds one copy, whoever loads it first)
+    subprocess.check_call(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-Wall",
+                           "-I", sysconfig.get_paths()["include"], os.path.join(CSRC, "py_calls.cpp"),
+                           "-o", CALLS, "-L", LIB_DIR, "-l:libhipml_cuda.so", "-Wl,-rpath,$ORIGIN"])
     return LIB
 
 
