@@ -1268,7 +1268,7 @@ def profile_case(args):
     chunk  -- one 2048-token chunk at position 6144 of one layer (the largest chunk of the
               headline workload): kv_encode_bulk, stage, attn_chunk_tc, `--reps` times;
     decode -- one layer's decode at depth 100000 (217.6 MB of q8 K/V, larger than L2):
-              kv_encode_q8, attn_decode_kv_tc, attn_decode_kv_reduce, `--reps` times
+              kv_encode_q8, attn_decode_warps, `--reps` times
               (`--selector 1`: the same over a q4_0 cache, 115.2 MB);
     batched -- one layer of the 16-slot batched decode step (mixed depths 615..7824).
     Prints the CUDA-event time per repetition so the capture has an un-profiled number."""

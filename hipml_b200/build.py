@@ -17,6 +17,8 @@ SOURCES = [
     "kv_encode.cu",
     "attn_decode.cu",
     "attn_decode_tc.cu",
+    "attn_decode_warps.cu",
+    "attn_decode_cols.cu",
     "attn_decode_f32.cu",
     "decode_static.cu",
     "decode_exchange.cu",

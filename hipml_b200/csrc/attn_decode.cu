@@ -9,20 +9,9 @@
 // reference): part_acc[(h*splits + s)*D + d], part_ml[(h*splits + s)*2 + {0: max in
 // log2 units, 1: sum}]; slot b adds b*acc_slot / b*ml_slot.
 //
-// Two bodies:
-//  * attn_decode_kv_tc  -- head_dim 256. A CTA owns one (KV head, split[, slot]) and
-//    streams its rows through a double-buffered shared-memory ring with 16-byte
-//    asynchronous copies (rows are 272 B, 16-byte aligned, and consecutive positions
-//    of one head are contiguous, so a tile is one linear run). Both contractions run
-//    on the tensor cores with f16 operands built in registers: int8 codes are exact
-//    in f16, the query and the softmax weights are split into f16 high + low parts
-//    stacked along the M dimension of one m16n8k16 tile (rows 0..7 high, 8..15 low),
-//    and the per-block f16 scales are applied in f32 (K side: on the 32-wide partial
-//    dot products; V side: folded into the weight operand), so results agree with the
-//    f32 definition to ~1e-6. This keeps the CUDA cores for byte unpacking only: at
-//    12 f32 FMA per cache byte a scalar kernel cannot keep up with HBM3e.
-//  * attn_decode_kv_scalar -- any head_dim in 32..256 step 32, one warp per
-//    (query head, split), plain f32. Kept as the A/B kernel (selector 6).
+// attn_decode_kv_scalar: any head_dim in 32..256 step 32, one warp per (query head, split), plain
+// f32; what head sizes other than 256 take, and the A/B kernel at 256 (selector 6). The head_dim-256
+// bodies are in attn_decode_warps.cu and attn_decode_tc.cu.
 #include "params.cuh"
 #include "q8_pack.cuh"
 

@@ -1,0 +1,383 @@
+// Split-K flash-decode of several columns of one q8_0 stream (a speculative draft's columns, head_dim 256):
+// the body of attn_decode_warps.cu with the columns side by side. CPU definition per column:
+// crates/hipml-core/src/ops.rs:449-518; launcher replaced: launch_kv::launch_cols_ptrs.
+//
+// The columns see the same rows but for the last few, so a warp loads and converts a unit's codes once
+// and runs every column's MMAs on them: of the ~635 warp instructions that 16 rows cost a column, ~430
+// are the codes' and only ~205 the column's own. What does not fit is the accumulators (64 a lane and
+// column): they live in tensor memory, 128 of its columns per decode column, and come to the registers
+// 16 at a time for the pair of blocks at hand (tcgen05.ld / st, 2 x 64 words a lane per unit).
+// One launch per layer takes up to four columns in the time of about two; 4 columns of 8,192 rows took
+// 36 us a layer as four grids of the single-column body.
+//
+// Each column's arithmetic is that of its own launch, operation for operation -- the plan, the order of
+// every sum, the movements of the references -- so its result is the same bits.
+#include <mutex>
+
+#include "decode_warp_body.cuh"
+
+namespace hipml {
+
+namespace {
+
+using namespace warp_body;
+
+constexpr int kCols = 4;          // columns side by side
+constexpr int kC = 2;             // CTAs per cluster, as the single-column form
+constexpr int kUnitRows = 32;
+constexpr unsigned kTmemCols = 512;
+
+struct Cfg {
+    static constexpr int kSlot = kUnitRows * kRowBytes;
+    static constexpr int kRing = 2 * kSlot;                        // per warp: a unit of K and one of V; later a partial
+    static_assert(kRing >= 8 * kHeadPitch * 4, "a warp's partial fits its ring");
+    static constexpr int kQBytes = 16 * 32 * 16;                   // a column's query fragments, later its partial of the CTA
+    static constexpr int kBiasBytes = 8 * 4 * 16;
+    static constexpr int kOffQ = kWarps * kRing;
+    static constexpr int kOffBias = kOffQ + kCols * kQBytes;
+    static constexpr int kOffMl = kOffBias + kCols * kBiasBytes;   // [8 heads][warps] {reference, sum}
+    static constexpr int kOffCml = kOffMl + kWarps * 8 * 8;        // per column [8 heads]
+    static constexpr int kOffBar = kOffCml + kCols * 8 * 8;
+    static constexpr int kSmem = kOffBar + kWarps * 2 * 8;
+    static_assert(kSmem + 1024 <= 227 * 1024, "one CTA per SM");
+};
+
+__device__ int g_arrive_cols[kArriveRegions * kArriveRegionInts];
+
+// grid (n_kv * runs * kC, ceil(columns / kCols)), clusters of kC.
+__global__ void __launch_bounds__(kThreads, 1) attn_decode_cols(DecodeParams p, int *status) {
+    using C = Cfg;
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ int s_last;
+    __shared__ unsigned s_tmem;
+    griddep_launch();
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int g = lane >> 2, t = lane & 3;
+    const int group = p.n_heads / p.n_kv;
+    const int rank = (int)cluster_rank();
+    unsigned char *const ring = smem + warp * C::kRing;
+    const unsigned ring_addr = smem_u32(ring), bar = smem_u32(smem + C::kOffBar) + warp * 16;
+    if (lane == 0) {
+        mbar_init(bar, 1);
+        mbar_init(bar + 8, 1);
+        mbar_init_fence();
+    }
+    if (warp == 0) tmem_alloc<1>(smem_u32(&s_tmem), kTmemCols);
+    const int col0 = blockIdx.y * kCols, col_end = min(p.n_slots, col0 + kCols);
+    const int *const len_at = p.len + p.len_offset;
+    {
+        // Nothing that the grids ahead may write can be relied on yet, but the lengths as they stand are a
+        // good guess: enough to ask L2 for the first rows (the cache rows themselves are read later).
+        const Work w = plan_stream<kC, kUnitRows>(p, col0, rank, min(max(__ldcg(len_at + col0 * p.len_stride), 0), p.stride));
+        const int first = w.row0 + w.unit * warp;
+        if (lane == 0 && first < w.row1) {
+            const size_t at = ((size_t)w.kvh * p.stride + first) * kRowBytes;
+            const unsigned bytes = (unsigned)(min(w.unit, w.row1 - first) * kRowBytes);
+            prefetch_l2(p.k + at, bytes);
+            prefetch_l2(p.v + at, bytes);
+        }
+    }
+    griddep_wait();
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    // this warp's accumulators of column c: lanes 32 * (warp % 4), columns 128 c + 64 * (warp / 4)
+    const unsigned tmem = s_tmem + ((unsigned)(warp & 3) << 21) + 64u * (warp >> 2);
+    unsigned phase = 0;
+    bool landed = true;
+    auto wait = [&](int slot) {
+        unsigned spin = 0;
+        while (!mbar_try_wait(bar + 8 * slot, phase)) {
+            if (++spin > kSpinLimit) {   // the copy never landed: flag it and carry on
+                landed = false;
+                break;
+            }
+        }
+    };
+
+    for (int base = col0; base < col_end;) {
+        // Columns base .. base + n - 1 share a plan: the same units for every warp. (Ascending lengths leave it
+        // only where they cross a multiple of the unit; then the rest is a second round.)
+        Work w[kCols];
+        int n = 0, units = 0;
+#pragma unroll
+        for (int c = 0; c < kCols; c++) {
+            w[c] = plan_stream<kC, kUnitRows>(p, base + c, rank, base + c < col_end ? __ldcg(len_at + (base + c) * p.len_stride) : 0);
+            const int u = div_up(w[c].len, w[c].unit);
+            if (c == 0) {
+                n = 1;
+                units = u;
+            } else if (n == c && base + c < col_end && u == units && w[c].unit == w[0].unit && w[c].runs == w[0].runs) {
+                n = c + 1;
+            }
+        }
+        const int kvh = w[0].kvh, unit = w[0].unit;
+        int row1 = w[0].row1;
+#pragma unroll
+        for (int c = 1; c < kCols; c++)
+            if (c < n) row1 = max(row1, w[c].row1);
+        auto neutral = [&](int col, int r) {
+            float *const pa = p.part_acc + (size_t)col * p.acc_slot + (size_t)kvh * group * p.splits * 256;
+            float *const pm = p.part_ml + (size_t)col * p.ml_slot + (size_t)kvh * group * p.splits * 2;
+            for (int i = rank * kThreads + tid; i < group * 256; i += kC * kThreads)
+                pa[((size_t)(i >> 8) * p.splits + r) * 256 + (i & 255)] = 0.0f;
+            if (rank == 0 && tid < group)
+                *reinterpret_cast<float2 *>(pm + ((size_t)tid * p.splits + r) * 2) = make_float2(-INFINITY, 0.0f);
+        };
+        for (int c = 0; c < n; c++) {
+            for (int r = w[0].run + p.run_cap; r < min(p.splits, kNeutralSlots); r += p.run_cap) neutral(base + c, r);
+            if (w[0].run >= w[0].runs) neutral(base + c, w[0].run);
+        }
+        if (w[0].run < w[0].runs) {
+        const size_t head_byte = (size_t)kvh * p.stride * kRowBytes;   // (the columns share the cache)
+        const int first = w[0].row0 + unit * warp;
+        const int nw = first < row1 ? div_up(row1 - first, unit * kWarps) : 0;
+        const size_t step = (size_t)unit * kWarps * kRowBytes;
+        const unsigned char *kp = p.k + head_byte + (size_t)first * kRowBytes;
+        const unsigned char *vp = p.v + head_byte + (size_t)first * kRowBytes;
+        auto fetch = [&](int i, const unsigned char *src, int slot) {   // unit i: one lane
+            const unsigned bytes = (unsigned)(min(unit, row1 - (first + i * unit * kWarps)) * kRowBytes);
+            mbar_arrive_expect_tx(bar + 8 * slot, bytes);
+            bulk_load(ring_addr + slot * C::kSlot, src, bytes, bar + 8 * slot);
+        };
+        // Query fragments of every column, warp b makes block b's (as in the single-column body).
+        {
+            float2 x[kCols][2][2];
+#pragma unroll
+            for (int c = 0; c < kCols; c++) {
+                const float *const qh = p.q + (size_t)(base + c) * p.q_slot + (size_t)(kvh * group + g) * 256;
+#pragma unroll
+                for (int k = 0; k < 2; k++)
+#pragma unroll
+                    for (int i = 0; i < 2; i++) {
+                        x[c][k][i] = make_float2(0.0f, 0.0f);
+                        if (g < group && c < n)
+                            x[c][k][i] = *reinterpret_cast<const float2 *>(qh + k_word_dim(warp, 4 * k + t, 2 * i));
+                    }
+            }
+            if (lane == 0 && nw > 0) {
+                fetch(0, kp, 0);
+                fetch(0, vp, 1);
+            }
+#pragma unroll
+            for (int c = 0; c < kCols; c++) {
+                if (c >= n) break;
+                store_query<false>(x[c], p.scale_log2, warp, lane, reinterpret_cast<uint4 *>(smem + C::kOffQ + c * C::kQBytes),
+                                   reinterpret_cast<float *>(smem + C::kOffBias + c * C::kBiasBytes));
+            }
+        }
+        __syncthreads();
+
+        Running run[kCols];
+#pragma unroll
+        for (int c = 0; c < kCols; c++) start(run[c]);
+        auto work = [&](auto tiles, int i, int rows) __attribute__((always_inline)) {
+            constexpr int kT = decltype(tiles)::value;
+            const int r0 = first + i * unit * kWarps;
+            // ---- scores of all columns
+            wait(0);
+            float s[kCols][kT][4];
+#pragma unroll
+            for (int c = 0; c < kCols; c++)
+#pragma unroll
+                for (int j = 0; j < kT; j++)
+#pragma unroll
+                    for (int e = 0; e < 4; e++) s[c][j][e] = 0.0f;
+            const unsigned *const krow = reinterpret_cast<const unsigned *>(ring) + g * Row<false>::kPitch;
+            auto score = [&](auto m) __attribute__((always_inline)) {
+                constexpr int M = decltype(m)::value;
+                KFrag<kT> f;
+                load_k<M, false, kT>(krow, t, f);
+#pragma unroll
+                for (int c = 0; c < kCols; c++)
+                    if (c < n)
+                        add_scores<M, kT>(f, reinterpret_cast<const uint4 *>(smem + C::kOffQ + c * C::kQBytes) + lane,
+                                          reinterpret_cast<const float4 *>(smem + C::kOffBias + c * C::kBiasBytes) + t, s[c]);
+            };
+            score(Int<0>{});
+            score(Int<1>{});
+            score(Int<2>{});
+            score(Int<3>{});
+            __syncwarp();
+            kp += step;
+            if (lane == 0 && i + 1 < nw) fetch(i + 1, kp, 0);
+            // ---- softmax
+            __half2 ph[kCols][kT][2], pl[kCols][kT][2];
+#pragma unroll
+            for (int c = 0; c < kCols; c++) {
+                if (c >= n) break;
+                float corr[2];
+                if (softmax<kT>(s[c], min(unit, w[c].row1 - r0), g, run[c], ph[c], pl[c], corr) && i > 0) {
+#pragma unroll 1
+                    for (int m = 0; m < 4; m++) {
+                        float a[16];
+                        tmem_ld16(tmem + 128 * c + 16 * m, a);
+                        tmem_wait_ld();
+#pragma unroll
+                        for (int e = 0; e < 16; e++) a[e] *= corr[e & 1];
+                        tmem_st16(tmem + 128 * c + 16 * m, a);
+                    }
+                    tmem_wait_st();
+                }
+            }
+            // ---- values
+            wait(1);
+            unsigned char *const vt = ring + C::kSlot;
+            if (rows < 16 * kT) {
+                // stale rows have weight 0, but their scales must not be NaN or infinite
+                for (int j = lane; j < (16 * kT - rows) * (kRowBytes / 16); j += 32)
+                    reinterpret_cast<uint4 *>(vt + rows * kRowBytes)[j] = make_uint4(0, 0, 0, 0);
+                __syncwarp();
+            }
+            const unsigned *const vrow = reinterpret_cast<const unsigned *>(vt) + 2 * t * Row<false>::kPitch;
+            auto value = [&](auto m) __attribute__((always_inline)) {
+                constexpr int M = decltype(m)::value;
+                VFrag f[kT];
+#pragma unroll
+                for (int j = 0; j < kT; j++) load_v<M, false>(vrow + j * 16 * Row<false>::kPitch, g, f[j]);
+#pragma unroll
+                for (int c = 0; c < kCols; c++) {
+                    if (c >= n) break;
+                    float a[16];
+#pragma unroll
+                    for (int e = 0; e < 16; e++) a[e] = 0.0f;
+                    if (i > 0) {
+                        tmem_ld16(tmem + 128 * c + 16 * M, a);
+                        tmem_wait_ld();
+                    }
+                    float ae[2][4], ao[2][4];
+#pragma unroll
+                    for (int e = 0; e < 8; e++) {
+                        ae[e >> 2][e & 3] = a[e];
+                        ao[e >> 2][e & 3] = a[8 + e];
+                    }
+#pragma unroll
+                    for (int j = 0; j < kT; j++) add_values(f[j], ph[c][j], pl[c][j], ae, ao);
+#pragma unroll
+                    for (int e = 0; e < 8; e++) {
+                        a[e] = ae[e >> 2][e & 3];
+                        a[8 + e] = ao[e >> 2][e & 3];
+                    }
+                    tmem_st16(tmem + 128 * c + 16 * M, a);
+                }
+            };
+            value(Int<0>{});
+            value(Int<1>{});
+            value(Int<2>{});
+            value(Int<3>{});
+            tmem_wait_st();
+            __syncwarp();
+            vp += step;
+            if (lane == 0 && i + 1 < nw) fetch(i + 1, vp, 1);
+            phase ^= 1;
+        };
+        for (int i = 0; i < nw; i++) {
+            const int rows = min(unit, row1 - (first + i * unit * kWarps));
+            if (rows > 16)
+                work(Int<2>{}, i, rows);
+            else
+                work(Int<1>{}, i, rows);
+        }
+
+        // ---- merge: the warps of the CTA column by column, then the cluster, then the runs
+        const int items = group * 64;
+        const bool one_run = w[0].runs == 1 && p.out != nullptr;
+        float2 *const wml = reinterpret_cast<float2 *>(smem + C::kOffMl);
+        auto cpart = [&](int c) { return reinterpret_cast<float4 *>(smem + C::kOffQ + c * C::kQBytes); };
+        auto cml = [&](int c) { return reinterpret_cast<float2 *>(smem + C::kOffCml) + 8 * c; };
+#pragma unroll
+        for (int c = 0; c < kCols; c++) {
+            if (c >= n) break;
+            sum_rows(run[c]);
+            if (g == 0) {
+                wml[(2 * t) * kWarps + warp] = make_float2(run[c].m[0], run[c].l[0]);
+                wml[(2 * t + 1) * kWarps + warp] = make_float2(run[c].m[1], run[c].l[1]);
+            }
+            float acc[8][2][4];
+#pragma unroll
+            for (int m = 0; m < 4; m++) {
+                float a[16];
+#pragma unroll
+                for (int e = 0; e < 16; e++) a[e] = 0.0f;
+                if (nw > 0) {
+                    tmem_ld16(tmem + 128 * c + 16 * m, a);
+                    tmem_wait_ld();
+                }
+#pragma unroll
+                for (int e = 0; e < 16; e++) acc[2 * m + (e >> 3)][(e >> 2) & 1][e & 3] = a[e];
+            }
+            store_warp_partial<false>(reinterpret_cast<float *>(ring), acc, group, g, t);
+            __syncthreads();
+            fold_warps(smem, C::kRing, wml, items, [&](int item, const Part &r) {
+                cpart(c)[item] = r.a;
+                if ((item & 63) == 0) cml(c)[item >> 6] = make_float2(r.m, r.l);
+            });
+            __syncthreads();
+        }
+        cluster_sync_all();
+        for (int c = 0; c < n; c++) {
+            const int col = base + c;
+            fold_cluster<kC>(cpart(c), cml(c), items, rank, [&](int item, const Part &r) {
+                if (one_run) emit_item(p, col, kvh, group, item, r);
+                const size_t row = (size_t)(kvh * group + (item >> 6)) * p.splits + w[0].run;
+                reinterpret_cast<float4 *>(p.part_acc + (size_t)col * p.acc_slot + row * 256)[item & 63] = r.a;
+                if ((item & 63) == 0)
+                    *reinterpret_cast<float2 *>(p.part_ml + (size_t)col * p.ml_slot + row * 2) = make_float2(r.m, r.l);
+            });
+        }
+        cluster_arrive();   // no CTA may leave, or start over, while another still reads its partials
+        if (p.out != nullptr && !one_run) {
+            int *const ctr = g_arrive_cols + (size_t)p.arrive_region * kArriveRegionInts +
+                             (size_t)(base * p.n_kv + kvh) * p.arrive_stride + rank;
+            __syncthreads();
+            if (tid == 0) {
+                const int last = arrive_acq_rel(ctr) == w[0].runs - 1;
+                if (last) *ctr = 0;
+                s_last = last;
+            }
+            __syncthreads();
+            if (s_last)
+                for (int c = 0; c < n; c++) fold_runs<kC>(p, base + c, kvh, group, w[0].runs, rank, nullptr);
+        }
+        cluster_wait();
+        __syncthreads();
+        if (lane == 0) fence_async_shared();   // partials were written over the rings; a next round's copies follow
+        }   // run with rows
+        base += n;
+    }
+    if (!landed && status) atomicCAS(status, 0, 21);
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) {
+        tc_fence_after();
+        tmem_dealloc<1>(s_tmem, kTmemCols);
+    }
+}
+
+int setup(int **status) {
+    static std::mutex mu;
+    static int *status_word[64] = {};   // nullptr: device not set up yet
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64) dev = 0;
+    std::lock_guard<std::mutex> lock(mu);
+    if (status_word[dev] == nullptr) {
+        const cudaError_t e = cudaFuncSetAttribute(attn_decode_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem);
+        if (e != cudaSuccess) return (int)e;
+        status_word[dev] = device_status_word();
+        if (status_word[dev] == nullptr) return launch_status();
+    }
+    *status = status_word[dev];
+    return 0;
+}
+
+}  // namespace
+
+int launch_decode_cols(cudaStream_t stream, const DecodeParams &p, int cols) {
+    int *status = nullptr;
+    if (int e = setup(&status)) return e;
+    const dim3 grid(p.n_kv * min(p.splits, p.run_cap) * kC, (cols + kCols - 1) / kCols);
+    return launch_pdl(attn_decode_cols, grid, dim3(kThreads), (size_t)Cfg::kSmem, stream, kC, p, status);
+}
+
+}  // namespace hipml

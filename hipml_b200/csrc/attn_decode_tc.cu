@@ -1,80 +1,48 @@
-// Split-K flash-decode over the q8_0 cache, tensor-core body (head_dim 256).
+// Split-K flash-decode over the q8_0 cache (head_dim 256) with the value side on the 5th-generation
+// tensor cores (tcgen05.mma kind::i8, accumulators in TMEM), and the dispatch between this body and
+// the default one (attn_decode_warps.cu). CPU definition: crates/hipml-core/src/ops.rs:449-518.
 //
-// A CTA of 8 warps owns one (KV head, split[, slot]) and streams its rows through a
-// three-stage shared-memory ring filled by bulk asynchronous copies (cp.async.bulk, one per
-// tensor and tile, completion on an mbarrier): rows are 272 B, 16-byte aligned, and
-// consecutive positions of one head are contiguous, so a 64-key tile of K (or V) is one
-// linear 17 KB run. One thread issues the copy of tile i+2 as soon as tile i-1 has been
-// consumed, so two tiles (70 KB per CTA, two CTAs per SM) are always in flight while the
-// third is being computed on. Both contractions run on the tensor cores
-// (mma.sync m16n8k16, f16 operands, f32 accumulate) with operands built in registers:
-//   * int8 codes are exact in f16. Scores: one byte permute per two codes -- the byte
-//     code + 128 under a zero high byte is the f16 subnormal (code + 128) * 2^-24; the offset
-//     leaves through the accumulators, which start at -2^-17 * (sum of the query over the
-//     block), and the factor 2^-24 when the scores are read. Values: 0x6400 | (code + 128) is
-//     1152 + code, minus 1152 (the weights are all positive, so an offset left in the
-//     accumulators would cost precision there);
-//   * scores: the codes are the A operand (16 keys x 16 dims), the query the B operand as an
-//     f16 high and a low part in two chained MMAs, so the block scale multiplies whole
-//     accumulator rows; values: the softmax weights are split into f16 high + low parts
-//     stacked along M (rows 0..7 high, rows 8..15 low of the same head);
-//   * the per-block f16 scales are applied in f32: on the K side to the 32-wide partial dot
-//     products, on the V side folded into the weight operand (weight * scale kept as an
-//     exact f16 high + low pair).
-// Results agree with the f32 definition to ~1e-6. The CUDA cores only unpack bytes: at 12
-// f32 FMA per cache byte a scalar kernel cannot keep up with HBM3e.
-//
-// Per tile: (1) scores -- warp (kg, dh) computes the partial scores of keys [16kg, 16kg+16)
-// over blocks [4dh, 4dh+4); (2) softmax -- warp g owns query head g of the group: running
-// max / sum, weights written once to shared memory as f16 high/low; (3) values -- warp w
-// owns block w (32 dims) for all 64 keys. CPU definition: crates/hipml-core/src/ops.rs:
-// 449-518; kernel replaced: crates/hipml-kernels/kernels/attn_decode_kv_w.hip:92-285 and
-// attn_decode_kv.hip:251-374,427-484.
+// A CTA of 8 warps owns one (KV head, run[, slot]) and streams it in tiles of 64 rows through rings
+// filled by asynchronous copies, completion on mbarriers. Per tile: (1) scores -- warp (kg, dh)
+// computes the partial scores of keys [16kg, 16kg+16) over blocks [4dh, 4dh+4) with mma.sync, the codes
+// as the A operand, the query as an f16 high and low part as the B operand; (2) softmax -- warp g owns
+// query head g; (3) values:
+//   * the V tile is brought in by 17 tensor (TMA) copies of {16 bytes, 64 rows}, one per
+//     16-byte column chunk of the 272-byte rows, so it lands as [chunk][key][16 B]: exactly the
+//     canonical MN-major operand of the MMA (8 keys x 16 bytes contiguous per core matrix).
+//     The int8 codes are the A operand as they are: M = byte of the row (three M tiles of 128
+//     cover the 272 bytes; the two scale bytes of each block are rows whose results are never
+//     read), K = key. No conversion of a single code on the CUDA cores;
+//   * the B operand is built per tile: column (block b, head h, digit) holds the weight
+//     exp2(score - ref_h) * scale(key, b) as a 23-bit fixed-point number in three unsigned
+//     bytes, taken straight out of the mantissa of weight * F + 2^23. A block's results only
+//     need that block's columns, so an M tile multiplies a window of 32 .. 96 columns;
+//   * products accumulate as int32 in TMEM (exact); per head the reference `ref_h` of the
+//     exponentials and the unit of the value scales stay fixed while the running maximum stays
+//     within 2^5.5 of it, so the accumulators are read out only when a reference moves (a few
+//     times per run) and at the end: digits are combined and scaled in f32 there.
+// Weights carry 17 bits below the reference (error 2^-18 of the largest weight), the int32
+// sums are exact, scores are as before: results agree with the f32 definition to ~1e-6.
 #include <atomic>
 #include <map>
 #include <mutex>
 #include <tuple>
 
+#include "decode_fold.cuh"
+#include "decode_rows.cuh"
 #include "params.cuh"
 #include "q8_pack.cuh"
 #include "sm100_ptx.cuh"
-#include "decode_fold.cuh"
 
 namespace hipml {
 
 namespace {
 
-constexpr int kTile = 64;                        // keys per shared-memory tile
-constexpr int kRowBytes = 8 * kQ8BlockBytes;     // 272
 constexpr int kTileBytes = kTile * kRowBytes;    // 17408
 constexpr int kThreads = 256;
 constexpr int kSsStride = 68;                    // padded row of the score tile (floats)
-constexpr int kPStride = 72;                     // padded row of the weight tile (halves)
-constexpr float kPScale = 1024.0f;               // keeps weight*scale in f16's normal range
-
-constexpr int kStages = 3;                       // ring depth (tiles of K and V)
-constexpr unsigned kSpinLimit = 1u << 24;        // polls of a full barrier before giving up
-
-// Dynamic shared memory: stage[3] = (K tile | V tile) | scores [2][8][72] f32 | weights hi,
-// lo [8][72] f16 | corr[8] f32 | full barriers [3].
-constexpr int kOffSs = 2 * kStages * kTileBytes;
-constexpr int kOffPh = kOffSs + 2 * 8 * kSsStride * 4;
-constexpr int kOffPl = kOffPh + 8 * kPStride * 2;
-constexpr int kOffCorr = kOffPl + 8 * kPStride * 2;
-constexpr int kOffBar = kOffCorr + 8 * 4;
-constexpr int kSmemBytes = kOffBar + kStages * 8;
-static_assert(2 * (kSmemBytes + 1024) <= 227 * 1024, "two CTAs per SM");
 
 using namespace ptx;
-
-__device__ __forceinline__ void mma_16816(float (&c)[4], const unsigned (&a)[4], unsigned b0,
-                                          unsigned b1) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, "
-        "{%8,%9}, {%0,%1,%2,%3};\n"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
 
 // K side: the eight "logical words" (four codes each) of block blk, all 4-byte aligned loads.
 // Odd blocks start 2 bytes past a word boundary, so word j holds codes 4j..4j+3. Even blocks
@@ -95,46 +63,6 @@ __device__ __forceinline__ unsigned k_word(const unsigned *row, int t) {
         const unsigned b = row[last ? 17 * m + 8 : 17 * m + 5 + t];
         return __byte_perm(a, b, last ? 0x5432 : 0x3210);
     }
-}
-
-// head_dim index of byte i of logical word j of block blk, in k_word's order.
-__device__ __forceinline__ int k_word_dim(int blk, int j, int i) {
-    if (blk & 1) return blk * 32 + 4 * j + i;
-    if (j < 7) return blk * 32 + 4 * j + 2 + i;
-    return blk * 32 + (i < 2 ? i : 28 + i);
-}
-
-// V side: codes 4j..4j+3 of a block in natural order; `blk_row` points at the block's first
-// aligned word (odd blocks: its first code word; even blocks: the word that starts with the
-// scale, so the codes straddle word boundaries: two loads and a permute).
-template <bool kOdd>
-__device__ __forceinline__ unsigned v_word(const unsigned *blk_row, int j) {
-    if constexpr (kOdd) return blk_row[j];
-    return __byte_perm(blk_row[j], blk_row[j + 1], 0x5432);
-}
-
-// Two bytes of `biased` (code ^ 0x80 = code + 128) as a half2 of f16 subnormals: 0x00xx is
-// xx * 2^-24 exactly, so one permute converts two codes. The offset of 128 is taken out
-// again through the accumulators (see score_block and the values phase), the factor 2^-24
-// when the scores / partials are written.
-__device__ __forceinline__ unsigned codes_to_half2(unsigned biased, unsigned selector) {
-    return __byte_perm(biased, 0u, selector);
-}
-// Value side: bytes of `biased` as an exact half2 through 0x64xx = 1024 + xx, minus 1152. The
-// weights are all positive there, so an offset carried in the accumulators would cost
-// several bits (measured: 4e-5 relative on a flat 256-key run); this form is exact.
-__device__ __forceinline__ unsigned codes_to_half2_exact(unsigned biased, unsigned selector) {
-    const unsigned h = __byte_perm(biased, 0x64646464u, selector);
-    const __half2 r =
-        __hsub2(*reinterpret_cast<const __half2 *>(&h), __half2half2(__ushort_as_half(0x6480)));
-    return *reinterpret_cast<const unsigned *>(&r);
-}
-constexpr float kCodeUnit = 16777216.0f;          // 2^24
-constexpr float kCodeBias = 128.0f / 16777216.0f; // the offset in the operand's units: 2^-17
-
-__device__ __forceinline__ unsigned pack_half2(__half lo, __half hi) {
-    const __half2 r = __halves2half2(lo, hi);
-    return *reinterpret_cast<const unsigned *>(&r);
 }
 
 // Rows [lo, hi) of run `split` of a slot. The partials are scratch (only their fold is
@@ -207,223 +135,9 @@ __device__ __forceinline__ void score_block(const unsigned char *ktile, int key_
     s[3] += d1 * c[3];
 }
 
-// Values of one tile for block `blk` (32 dims): acc = acc * corr + weights * scale * codes over
-// the 64 keys. A = weight * block scale as an exact f16 high + low pair (rows 0..7 high part of
-// head g, rows 8..15 low part), B = the block's codes, four n-tiles: output column n of MMA i
-// is dim 32*blk + 4n + i. All shared-memory offsets inside the unrolled loop are immediates
-// off three per-thread base pointers.
-template <bool kOdd>
-__device__ __forceinline__ void values_block(const unsigned char *vtile, int blk, int g, int t,
-                                             const __half *ph, const __half *pl, float corr,
-                                             float (&acc)[4][4]) {
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int c = 0; c < 4; c++) acc[i][c] *= corr;
-    // keys k0 = 16*ks + 2t, k0 + 1, k0 + 8, k0 + 9 of every 16-key step
-    const unsigned char *scale0 = vtile + 2 * t * kRowBytes + blk * kQ8BlockBytes;
-    const unsigned *code0 =
-        reinterpret_cast<const unsigned *>(scale0 + (kOdd ? 2 : 0)) + g;
-    const __half *ph0 = ph + g * kPStride + 2 * t, *pl0 = pl + g * kPStride + 2 * t;
-    constexpr int kRowWords = kRowBytes / 4;
-#pragma unroll
-    for (int ks = 0; ks < 4; ks++) {
-        constexpr int kOff[4] = {0, 1, 8, 9};
-        __half dv[4];
-        unsigned w[4];
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-            dv[e] = __ushort_as_half(*reinterpret_cast<const unsigned short *>(
-                scale0 + (ks * 16 + kOff[e]) * kRowBytes));
-            w[e] = v_word<kOdd>(code0 + (ks * 16 + kOff[e]) * kRowWords, 0) ^ 0x80808080u;
-        }
-        const __half2 d01 = __halves2half2(dv[0], dv[1]), d23 = __halves2half2(dv[2], dv[3]);
-        const __half2 ph01 = *reinterpret_cast<const __half2 *>(ph0 + ks * 16);
-        const __half2 ph23 = *reinterpret_cast<const __half2 *>(ph0 + ks * 16 + 8);
-        const __half2 pl01 = *reinterpret_cast<const __half2 *>(pl0 + ks * 16);
-        const __half2 pl23 = *reinterpret_cast<const __half2 *>(pl0 + ks * 16 + 8);
-        const __half2 h01 = __hmul2(ph01, d01), h23 = __hmul2(ph23, d23);
-        const __half2 l01 = __hfma2(pl01, d01, __hfma2(ph01, d01, __hneg2(h01)));
-        const __half2 l23 = __hfma2(pl23, d23, __hfma2(ph23, d23, __hneg2(h23)));
-        unsigned afrag[4];
-        afrag[0] = *reinterpret_cast<const unsigned *>(&h01);
-        afrag[1] = *reinterpret_cast<const unsigned *>(&l01);
-        afrag[2] = *reinterpret_cast<const unsigned *>(&h23);
-        afrag[3] = *reinterpret_cast<const unsigned *>(&l23);
-        const unsigned ab01 = __byte_perm(w[0], w[1], 0x5140);  // [a0 b0 a1 b1]
-        const unsigned ab23 = __byte_perm(w[0], w[1], 0x7362);  // [a2 b2 a3 b3]
-        const unsigned cd01 = __byte_perm(w[2], w[3], 0x5140);
-        const unsigned cd23 = __byte_perm(w[2], w[3], 0x7362);
-        mma_16816(acc[0], afrag, codes_to_half2_exact(ab01, 0x4140), codes_to_half2_exact(cd01, 0x4140));
-        mma_16816(acc[1], afrag, codes_to_half2_exact(ab01, 0x4342), codes_to_half2_exact(cd01, 0x4342));
-        mma_16816(acc[2], afrag, codes_to_half2_exact(ab23, 0x4140), codes_to_half2_exact(cd23, 0x4140));
-        mma_16816(acc[3], afrag, codes_to_half2_exact(ab23, 0x4342), codes_to_half2_exact(cd23, 0x4342));
-    }
-}
-
-// ---- q4_0 rows read in place (144-byte rows of 18-byte blocks: f16 scale, then 16 bytes
-// whose low nibbles are values 0..15 and high nibbles values 16..31, each value + 8).
-constexpr int kQ4RowBytes = 8 * kQ4BlockBytes;   // 144 = 36 words; a block pair is 9 words
-
-// K side: the four "logical words" of block BLK (four code bytes each), aligned loads only.
-// Odd blocks start on a word boundary after their scale's half word; even blocks hold bytes
-// 2..13 in three aligned words and bytes 0, 1, 14, 15 in the two words they share with the
-// scales, stitched into the fourth. The contraction order is free (the query follows it).
-template <int BLK>
-__device__ __forceinline__ unsigned k_word_q4(const unsigned *row, int t) {
-    constexpr int m = BLK >> 1;
-    if constexpr (BLK & 1) {
-        return row[9 * m + 5 + t];
-    } else {
-        const bool last = t == 3;
-        const unsigned a = row[last ? 9 * m : 9 * m + 1 + t];
-        const unsigned b = row[last ? 9 * m + 4 : 9 * m + 1 + t];
-        return __byte_perm(a, b, last ? 0x5432 : 0x3210);
-    }
-}
-// head_dim index of byte i of logical word j (low nibble; the high nibble is 16 further).
-__device__ __forceinline__ int k_word_dim_q4(int blk, int j, int i) {
-    if (blk & 1) return blk * 32 + 4 * j + i;
-    if (j < 3) return blk * 32 + 4 * j + 2 + i;
-    return blk * 32 + (i < 2 ? i : 12 + i);
-}
-
-// Scores of one q4_0 block for this warp's 16 keys: as score_block, with step 0 of the
-// contraction over the low nibbles (values 0..15 of the block) and step 1 over the high ones.
-// A nibble is value + 8, an f16 subnormal as it stands: no XOR, offset 8.
-template <int BLK>
-__device__ __forceinline__ void score_block_q4(const unsigned char *ktile, int key_base, int g, int t,
-                                               const unsigned (&qb0)[4], const unsigned (&qb1)[4],
-                                               const float (&bias)[2], float (&s)[4]) {
-    const unsigned *row0 = reinterpret_cast<const unsigned *>(ktile + (key_base + g) * kQ4RowBytes);
-    const unsigned *row1 = row0 + 8 * (kQ4RowBytes / 4);
-    float c[4] = {bias[0], bias[1], bias[0], bias[1]};
-    const unsigned w0 = k_word_q4<BLK>(row0, t), w1 = k_word_q4<BLK>(row1, t);
-    {
-        const unsigned x0 = w0 & 0x0f0f0f0fu, x1 = w1 & 0x0f0f0f0fu;
-        const unsigned a[4] = {codes_to_half2(x0, 0x4140), codes_to_half2(x1, 0x4140),
-                               codes_to_half2(x0, 0x4342), codes_to_half2(x1, 0x4342)};
-        mma_16816(c, a, qb0[0], qb0[1]);
-        mma_16816(c, a, qb0[2], qb0[3]);
-    }
-    {
-        const unsigned x0 = (w0 >> 4) & 0x0f0f0f0fu, x1 = (w1 >> 4) & 0x0f0f0f0fu;
-        const unsigned a[4] = {codes_to_half2(x0, 0x4140), codes_to_half2(x1, 0x4140),
-                               codes_to_half2(x0, 0x4342), codes_to_half2(x1, 0x4342)};
-        mma_16816(c, a, qb1[0], qb1[1]);
-        mma_16816(c, a, qb1[2], qb1[3]);
-    }
-    const unsigned char *sc = ktile + (key_base + g) * kQ4RowBytes + BLK * kQ4BlockBytes;
-    const float d0 = half_bits_to_float(*reinterpret_cast<const unsigned short *>(sc));
-    const float d1 = half_bits_to_float(*reinterpret_cast<const unsigned short *>(sc + 8 * kQ4RowBytes));
-    s[0] += d0 * c[0];
-    s[1] += d0 * c[1];
-    s[2] += d1 * c[2];
-    s[3] += d1 * c[3];
-}
-
-// Values of one tile for q4_0 block `blk`: as values_block. Lane group g takes code word g & 3
-// (natural order: values 4(g&3) .. +3 in the low nibbles, 16 further in the high ones) and the
-// nibble half g >> 2, so output column n of MMA i is dim 32*blk + 4n + i as for q8_0.
-// 0x6400 | nibble is 1024 + value + 8, minus 1032: exact.
-template <bool kOdd>
-__device__ __forceinline__ void values_block_q4(const unsigned char *vtile, int blk, int g, int t,
-                                                const __half *ph, const __half *pl, float corr,
-                                                float (&acc)[4][4]) {
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int c = 0; c < 4; c++) acc[i][c] *= corr;
-    const unsigned char *scale0 = vtile + 2 * t * kQ4RowBytes + blk * kQ4BlockBytes;
-    const unsigned *code0 = reinterpret_cast<const unsigned *>(scale0 + (kOdd ? 2 : 0)) + (g & 3);
-    const int shift = (g >> 2) * 4;
-    const __half *ph0 = ph + g * kPStride + 2 * t, *pl0 = pl + g * kPStride + 2 * t;
-    constexpr int kRowWords = kQ4RowBytes / 4;
-    const __half2 off = __half2half2(__ushort_as_half(0x6408));   // 1032
-#pragma unroll
-    for (int ks = 0; ks < 4; ks++) {
-        constexpr int kOff[4] = {0, 1, 8, 9};
-        __half dv[4];
-        unsigned w[4];
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-            dv[e] = __ushort_as_half(*reinterpret_cast<const unsigned short *>(
-                scale0 + (ks * 16 + kOff[e]) * kQ4RowBytes));
-            w[e] = (v_word<kOdd>(code0 + (ks * 16 + kOff[e]) * kRowWords, 0) >> shift) & 0x0f0f0f0fu;
-        }
-        const __half2 d01 = __halves2half2(dv[0], dv[1]), d23 = __halves2half2(dv[2], dv[3]);
-        const __half2 ph01 = *reinterpret_cast<const __half2 *>(ph0 + ks * 16);
-        const __half2 ph23 = *reinterpret_cast<const __half2 *>(ph0 + ks * 16 + 8);
-        const __half2 pl01 = *reinterpret_cast<const __half2 *>(pl0 + ks * 16);
-        const __half2 pl23 = *reinterpret_cast<const __half2 *>(pl0 + ks * 16 + 8);
-        const __half2 h01 = __hmul2(ph01, d01), h23 = __hmul2(ph23, d23);
-        const __half2 l01 = __hfma2(pl01, d01, __hfma2(ph01, d01, __hneg2(h01)));
-        const __half2 l23 = __hfma2(pl23, d23, __hfma2(ph23, d23, __hneg2(h23)));
-        unsigned afrag[4];
-        afrag[0] = *reinterpret_cast<const unsigned *>(&h01);
-        afrag[1] = *reinterpret_cast<const unsigned *>(&l01);
-        afrag[2] = *reinterpret_cast<const unsigned *>(&h23);
-        afrag[3] = *reinterpret_cast<const unsigned *>(&l23);
-        const unsigned ab01 = __byte_perm(w[0], w[1], 0x5140);  // [a0 b0 a1 b1]
-        const unsigned ab23 = __byte_perm(w[0], w[1], 0x7362);  // [a2 b2 a3 b3]
-        const unsigned cd01 = __byte_perm(w[2], w[3], 0x5140);
-        const unsigned cd23 = __byte_perm(w[2], w[3], 0x7362);
-        auto conv = [&](unsigned x, unsigned sel) {
-            const unsigned h = __byte_perm(x, 0x64646464u, sel);
-            const __half2 r = __hsub2(*reinterpret_cast<const __half2 *>(&h), off);
-            return *reinterpret_cast<const unsigned *>(&r);
-        };
-        mma_16816(acc[0], afrag, conv(ab01, 0x4140), conv(cd01, 0x4140));
-        mma_16816(acc[1], afrag, conv(ab01, 0x4342), conv(cd01, 0x4342));
-        mma_16816(acc[2], afrag, conv(ab23, 0x4140), conv(cd23, 0x4140));
-        mma_16816(acc[3], afrag, conv(ab23, 0x4342), conv(cd23, 0x4342));
-    }
-}
-
 // Arrival counters of the fold inside the split pass: kArriveRegions regions of
 // kArriveRegionInts counters, zero at load and zero again after every launch that used them.
-constexpr int kArriveRegions = 128;
 __device__ int g_arrive[kArriveRegions * kArriveRegionInts];
-
-// What the CTA that holds the final fold of a (slot, KV head) does with it: write the output
-// rows, or (sequence-split decode across GPUs) publish the triples to every rank's table
-// and / or collect all ranks' triples and fold those. All threads of the CTA call it; warp w
-// holds head w of the group in f.
-__device__ __forceinline__ void fold_finish(const DecodeParams &p, int *status, int slot, int kvh,
-                                            int group, FoldAcc &f) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int h = kvh * group + warp;
-    if (p.xch.phases == 0) {
-        if (warp < group) fold_emit(p, slot, h, f, lane, p.normalize != 0);
-        return;
-    }
-    __shared__ int s_epoch;
-    int *hdr = reinterpret_cast<int *>(p.xch.ws[p.xch.rank]);
-    // Every folding CTA of the call reads the epoch before it adds itself to the counter, and
-    // the epoch advances only after the last of them has: all of them see the same value.
-    if (threadIdx.x == 0) s_epoch = *reinterpret_cast<volatile int *>(hdr) + ((p.xch.phases & 1) ? 1 : 0);
-    __syncthreads();
-    const int e = s_epoch;
-    if (p.xch.phases & 1) {
-        if (warp < group) exchange_publish_warp(p.xch, p.n_heads, h, e, f, lane);
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            if (atomicAdd(hdr + 1, 1) == p.n_kv - 1) {
-                hdr[1] = 0;
-                *reinterpret_cast<volatile int *>(hdr) = e;
-            }
-        }
-    }
-    if (p.xch.phases & 2) {
-        if (warp < group && (!p.xch.by_head || exchange_owner(p.xch, p.n_heads, h) == p.xch.rank)) {
-            const unsigned long long deadline = global_timer_ns() + 1000ull * p.xch.wait_us;
-            if (exchange_collect_warp(p.xch, p.n_heads, h, e, deadline, lane, f))
-                fold_emit(p, slot, h, f, lane, true);
-            else if (lane == 0 && status)
-                atomicCAS(status, 0, 31);
-        }
-    }
-}
 
 // The end of a split-pass CTA whose partial is live: arrive at the group's counter; the last
 // of a group folds it into the group's first slot and arrives at the head group's counter;
@@ -470,364 +184,6 @@ __device__ __forceinline__ void fold_tail(const DecodeParams &p, int *status, in
     fold_finish(p, status, slot, kvh, group, f);
 }
 
-// kQ4: the cache is q4_0; the phases read the 144-byte rows as they were copied.
-template <bool kQ4>
-__global__ void __launch_bounds__(kThreads, 2) attn_decode_kv_tc(DecodeParams p, int *status) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    griddep_launch();
-    // Everything this kernel reads -- the live lengths, the query, the cache rows with this
-    // step's append -- may come from the grids before it, and a dependent launch can start
-    // while the grid before its predecessor is still running: nothing is read before this.
-    griddep_wait();
-    auto ktile_at = [&](int stage) { return smem + 2 * stage * kTileBytes; };
-    auto vtile_at = [&](int stage) { return smem + (2 * stage + 1) * kTileBytes; };
-    float *ss = reinterpret_cast<float *>(smem + kOffSs);            // [2][8][kSsStride]
-    __half *ph = reinterpret_cast<__half *>(smem + kOffPh);          // [8][kPStride]
-    __half *pl = reinterpret_cast<__half *>(smem + kOffPl);
-    float *corr_s = reinterpret_cast<float *>(smem + kOffCorr);      // [8]
-
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int g = lane >> 2, t = lane & 3;
-    const int group = p.n_heads / p.n_kv;
-    const int kg = warp & 3, dh = warp >> 2;
-
-    // Which (slot, KV head, run) this CTA owns. Plain form: grid (n_kv * splits, slots).
-    // Shared form (several slots, share_slots > 0): a one-dimensional grid of exactly the
-    // device's CTA slots; CTA b takes the b-th live run in (slot, head, run) order, found by a
-    // scan over the slots' run counts, and CTAs past the last live run have nothing to do (no
-    // dead run is ever launched, so no live run waits behind them).
-    __shared__ int s_plan[4];   // slot (-1: none), kvh, split, quota
-    // (single stream with balanced runs: only the first min(splits, run_cap) runs of a head
-    // can hold rows, and only those are launched)
-    const int grid_splits = (p.by_stride || p.run_cap <= 0) ? p.splits : min(p.splits, p.run_cap);
-    int slot = blockIdx.y, kvh = blockIdx.x / grid_splits, split = blockIdx.x - kvh * grid_splits;
-    if (p.share_slots > 0) {
-        if (warp == 0) {
-            const int quota = shared_quota_warp(p.len, p.len_stride, p.len_offset, p.n_slots, p.splits,
-                                                p.share_slots, p.n_kv);
-            const int b = blockIdx.x;
-            int base = 0;
-            if (lane == 0) {
-                s_plan[0] = -1;
-                s_plan[3] = quota;
-            }
-            __syncwarp();
-            for (int s0 = 0; s0 < p.n_slots; s0 += 32) {
-                const int s = s0 + lane;
-                const int per = s < p.n_slots
-                    ? shared_runs_of((p.len[s * p.len_stride + p.len_offset] + 63) >> 6, quota) : 0;
-                const int runs = per * p.n_kv;
-                int incl = runs;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int up = __shfl_up_sync(0xffffffffu, incl, o);
-                    if (lane >= o) incl += up;
-                }
-                const int first = base + incl - runs;
-                if (runs > 0 && b >= first && b < first + runs) {
-                    const int r = b - first;
-                    s_plan[0] = s;
-                    s_plan[1] = r / per;
-                    s_plan[2] = r - (r / per) * per;
-                }
-                base += __shfl_sync(0xffffffffu, incl, 31);
-            }
-        }
-        __syncthreads();
-        slot = s_plan[0];
-        kvh = s_plan[1];
-        split = s_plan[2];
-        if (slot < 0) return;
-    }
-    // The query values this lane feeds to the tensor cores, loaded straight into registers
-    // before anything that depends on the live length, so that the two round trips overlap.
-    float qv[8][4];
-    {
-        const float *qh = p.q + (size_t)slot * p.q_slot + (size_t)(kvh * group + g) * 256;
-#pragma unroll
-        for (int ks = 0; ks < 8; ks++) {
-            const int blk = dh * 4 + (ks >> 1), j = (ks & 1) * 4 + t;
-#pragma unroll
-            for (int i = 0; i < 4; i += 2) {
-                const int d = kQ4 ? k_word_dim_q4(blk, t, i) + 16 * (ks & 1) : k_word_dim(blk, j, i);
-                float2 x = make_float2(0.0f, 0.0f);
-                if (g < group) x = *reinterpret_cast<const float2 *>(qh + d);
-                qv[ks][i] = x.x;
-                qv[ks][i + 1] = x.y;
-            }
-        }
-    }
-    int lo, hi;
-    split_range(p, slot, split, p.share_slots > 0 ? s_plan[3] : 0, lo, hi);
-    const int ntiles = (hi - lo + kTile - 1) / kTile;
-    if (ntiles == 0) {
-        // A split without rows: neutral partials (zero sum, -inf maximum), nothing else.
-        for (int i = tid; i < group * 256; i += kThreads) {
-            const int h = kvh * group + (i >> 8);
-            p.part_acc[(size_t)slot * p.acc_slot + ((size_t)h * p.splits + split) * 256 + (i & 255)] = 0.0f;
-        }
-        if (tid < group) {
-            float *pm = p.part_ml + (size_t)slot * p.ml_slot +
-                        ((size_t)(kvh * group + tid) * p.splits + split) * 2;
-            pm[0] = -INFINITY;
-            pm[1] = 0.0f;
-        }
-    }
-
-    if (ntiles > 0) {
-    constexpr int kSrcRow = kQ4 ? kQ4RowBytes : kRowBytes;   // bytes of a cache row
-    const size_t head_byte = (size_t)slot * p.kv_slot_bytes + (size_t)kvh * p.stride * kSrcRow;
-    const unsigned char *kbase = p.k + head_byte;
-    const unsigned char *vbase = p.v + head_byte;
-    int append_pos = -1;
-    if (p.k_row != nullptr) {
-        append_pos = p.len[slot * p.len_stride + p.len_offset - 1];
-        // the fused form appends the last live row; anything else is the caller's error
-        if (split == 0 && kvh == 0 && tid == 0 &&
-            append_pos != p.len[slot * p.len_stride + p.len_offset] - 1 && status)
-            atomicCAS(status, 0, 22);
-    }
-
-    // Ring: stage tile % 3; thread 0 arms the stage's barrier with the byte count and issues
-    // the two copies. A stage is re-filled only after the __syncthreads that ends the tile
-    // which last read it.
-    const unsigned bar_full = smem_u32(smem + kOffBar);
-    auto fetch = [&](int tile) {
-        const int stage = tile % kStages;
-        const int r0 = lo + tile * kTile;
-        const unsigned bytes = (unsigned)(min(kTile, hi - r0) * kSrcRow);
-        const size_t off = (size_t)r0 * kSrcRow;
-        constexpr int kDst = 0;
-        // earlier generic-proxy writes to the stage (the zero fill of a short tile) come first
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        mbar_arrive_expect_tx(bar_full + 8 * stage, 2 * bytes);
-        bulk_load(smem_u32(ktile_at(stage)) + kDst, kbase + off, bytes, bar_full + 8 * stage);
-        bulk_load(smem_u32(vtile_at(stage)) + kDst, vbase + off, bytes, bar_full + 8 * stage);
-    };
-    if (tid == 0) {
-#pragma unroll
-        for (int s = 0; s < kStages; s++) mbar_init(bar_full + 8 * s, 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        fetch(0);
-        if (ntiles > 1) fetch(1);
-    }
-
-    // B fragments of the query for this warp's four blocks and both 16-slot steps of each:
-    // column g = head g, as an f16 high and low part ({hi b0, hi b1, lo b0, lo b1}); the
-    // contraction slots follow k_word's order (slots 2t, 2t+1 = bytes 0, 1 of word t, slots
-    // 2t+8, 2t+9 = bytes 2, 3). The 32 values a lane needs arrived in registers (qv, loaded
-    // straight from memory in that order while the first tiles were being fetched); rows past
-    // the group are zero. Scores are kept in log2 units.
-    unsigned qb[8][4];
-    float qbias[4][2];
-#pragma unroll
-    for (int b = 0; b < 4; b++) {
-        float sum = 0.0f;   // of the block's query values as the tensor cores see them
-#pragma unroll
-        for (int half = 0; half < 2; half++) {
-            const int ks = 2 * b + half;
-            __half xh[4], xl[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const float x = qv[ks][i] * p.scale_log2;
-                xh[i] = __float2half_rn(x);
-                xl[i] = __float2half_rn(x - __half2float(xh[i]));
-                sum += __half2float(xh[i]) + __half2float(xl[i]);
-            }
-            qb[ks][0] = pack_half2(xh[0], xh[1]);
-            qb[ks][1] = pack_half2(xh[2], xh[3]);
-            qb[ks][2] = pack_half2(xl[0], xl[1]);
-            qb[ks][3] = pack_half2(xl[2], xl[3]);
-        }
-        // the four lanes of a head hold a quarter of the block each; the score accumulators of
-        // lane (g, t) are heads 2t and 2t + 1 and start at -2^-17 * (sum over the block), which
-        // takes the codes' offset of 128 out again (nibbles carry an offset of 8)
-        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-        const float bias = -(kQ4 ? kCodeBias / 16.0f : kCodeBias) * sum;
-        qbias[b][0] = __shfl_sync(0xffffffffu, bias, (2 * t) * 4);
-        qbias[b][1] = __shfl_sync(0xffffffffu, bias, (2 * t + 1) * 4);
-    }
-    // (set-up wrote the barriers; the first tiles are on their way)
-    __syncthreads();
-
-    float acc[4][4];  // block `warp`: [byte i of the code word][c0..c3]
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int c = 0; c < 4; c++) acc[i][c] = 0.0f;
-    float m_run = -INFINITY, l_run = 0.0f;  // meaningful in warp g' = head of the group
-
-    bool landed = true;
-    for (int tile = 0; tile < ntiles; tile++) {
-        const int buf = tile % kStages;
-        // the stage of tile + 2 was read last by tile - 1, which every warp has left
-        if (tid == 0 && tile + 2 < ntiles) fetch(tile + 2);
-        {
-            const unsigned bar = bar_full + 8 * buf, parity = (unsigned)(tile / kStages) & 1u;
-            unsigned spin = 0;
-            while (!mbar_try_wait(bar, parity)) {
-                if (++spin > kSpinLimit) {  // the copy never landed: flag it and carry on
-                    landed = false;
-                    break;
-                }
-            }
-        }
-        const int nvalid = min(kTile, hi - (lo + tile * kTile));
-        unsigned char *const ktile_b = ktile_at(buf), *const vtile_b = vtile_at(buf);
-        // (no barrier here: every thread has seen the copy land for itself)
-        if (p.k_row != nullptr) {
-            // Fused append: the row at the append position was copied as it was before this
-            // step. Warp 0 (K) and warp 1 (V) quantise the new row into the tile, with the
-            // encoder's own arithmetic, and store its bytes to the cache.
-            const int prow = append_pos - (lo + tile * kTile);
-            if (prow >= 0 && prow < nvalid) {
-                if (warp < 2) {
-                    const float *src = (warp == 0 ? p.k_row : p.v_row) + (size_t)slot * p.row_slot +
-                                       (size_t)kvh * 256 + lane * 8;
-                    unsigned char *row = (warp == 0 ? ktile_b : vtile_b) + prow * kSrcRow;
-                    const float4 a = __ldg(reinterpret_cast<const float4 *>(src));
-                    const float4 b = __ldg(reinterpret_cast<const float4 *>(src) + 1);
-                    if constexpr (kQ4)
-                        q4_put8(a, b, lane, row);
-                    else
-                        q8_put8(a, b, lane, row);
-                    __syncwarp();
-                    row_store((warp == 0 ? p.kw : p.vw) + head_byte + (size_t)append_pos * kSrcRow, row,
-                              kSrcRow, lane, 32);
-                }
-                __syncthreads();
-            }
-        }
-        if (nvalid < kTile) {
-            // Rows past the split's end hold stale bytes; their V scales must read as zero.
-            for (int i = tid; i < (kTile - nvalid) * (kSrcRow / 16); i += kThreads)
-                reinterpret_cast<uint4 *>(vtile_b + nvalid * kSrcRow)[i] = make_uint4(0, 0, 0, 0);
-        }
-
-        // ---- (1) scores
-        {
-            float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-            if constexpr (kQ4) {
-                if (dh == 0) {
-                    score_block_q4<0>(ktile_b, kg * 16, g, t, qb[0], qb[1], qbias[0], s);
-                    score_block_q4<1>(ktile_b, kg * 16, g, t, qb[2], qb[3], qbias[1], s);
-                    score_block_q4<2>(ktile_b, kg * 16, g, t, qb[4], qb[5], qbias[2], s);
-                    score_block_q4<3>(ktile_b, kg * 16, g, t, qb[6], qb[7], qbias[3], s);
-                } else {
-                    score_block_q4<4>(ktile_b, kg * 16, g, t, qb[0], qb[1], qbias[0], s);
-                    score_block_q4<5>(ktile_b, kg * 16, g, t, qb[2], qb[3], qbias[1], s);
-                    score_block_q4<6>(ktile_b, kg * 16, g, t, qb[4], qb[5], qbias[2], s);
-                    score_block_q4<7>(ktile_b, kg * 16, g, t, qb[6], qb[7], qbias[3], s);
-                }
-            } else if (dh == 0) {
-                score_block<0>(ktile_b, kg * 16, g, t, qb[0], qb[1], qbias[0], s);
-                score_block<1>(ktile_b, kg * 16, g, t, qb[2], qb[3], qbias[1], s);
-                score_block<2>(ktile_b, kg * 16, g, t, qb[4], qb[5], qbias[2], s);
-                score_block<3>(ktile_b, kg * 16, g, t, qb[6], qb[7], qbias[3], s);
-            } else {
-                score_block<4>(ktile_b, kg * 16, g, t, qb[0], qb[1], qbias[0], s);
-                score_block<5>(ktile_b, kg * 16, g, t, qb[2], qb[3], qbias[1], s);
-                score_block<6>(ktile_b, kg * 16, g, t, qb[4], qb[5], qbias[2], s);
-                score_block<7>(ktile_b, kg * 16, g, t, qb[6], qb[7], qbias[3], s);
-            }
-            float *dst = ss + (dh * 8 + 2 * t) * kSsStride + kg * 16 + g;
-            dst[0] = s[0];
-            dst[kSsStride] = s[1];
-            dst[8] = s[2];
-            dst[kSsStride + 8] = s[3];
-        }
-        __syncthreads();
-
-        // ---- (2) softmax: warp = head of the group, lane = keys 2*lane, 2*lane+1
-        {
-            const float2 a = *reinterpret_cast<const float2 *>(ss + warp * kSsStride + 2 * lane);
-            const float2 b = *reinterpret_cast<const float2 *>(ss + (8 + warp) * kSsStride + 2 * lane);
-            const float s0 = 2 * lane < nvalid ? (a.x + b.x) * kCodeUnit : -INFINITY;
-            const float s1 = 2 * lane + 1 < nvalid ? (a.y + b.y) * kCodeUnit : -INFINITY;
-            const float m_new = fmaxf(m_run, warp_max(fmaxf(s0, s1)));
-            // m_new is -inf only while every key so far was masked: nothing to scale then.
-            const float corr = (m_new == -INFINITY) ? 1.0f : exp2f(m_run - m_new);
-            const float p0 = (s0 == -INFINITY) ? 0.0f : exp2f(s0 - m_new);
-            const float p1 = (s1 == -INFINITY) ? 0.0f : exp2f(s1 - m_new);
-            l_run = l_run * corr + warp_sum(p0 + p1);
-            m_run = m_new;
-            const float w0 = p0 * kPScale, w1 = p1 * kPScale;
-            const __half h0 = __float2half_rn(w0), h1 = __float2half_rn(w1);
-            const __half l0 = __float2half_rn(w0 - __half2float(h0));
-            const __half l1 = __float2half_rn(w1 - __half2float(h1));
-            *reinterpret_cast<unsigned *>(ph + warp * kPStride + 2 * lane) = pack_half2(h0, h1);
-            *reinterpret_cast<unsigned *>(pl + warp * kPStride + 2 * lane) = pack_half2(l0, l1);
-            if (lane == 0) corr_s[warp] = corr;
-        }
-        __syncthreads();
-
-        // ---- (3) values: warp = block (32 dims), all 64 keys
-        if constexpr (kQ4) {
-            if (warp & 1)
-                values_block_q4<true>(vtile_b, warp, g, t, ph, pl, corr_s[g], acc);
-            else
-                values_block_q4<false>(vtile_b, warp, g, t, ph, pl, corr_s[g], acc);
-        } else if (warp & 1) {
-            values_block<true>(vtile_b, warp, g, t, ph, pl, corr_s[g], acc);
-        } else {
-            values_block<false>(vtile_b, warp, g, t, ph, pl, corr_s[g], acc);
-        }
-        __syncthreads();  // tile buffers, ss and the weight tile are reused by the next tile
-    }
-
-    if (!landed && status) atomicCAS(status, 0, 21);
-
-    // ---- partials. Output column n of MMA i is dim 32*blk + 4n + i; this thread holds
-    // columns 2t, 2t+1, i.e. dims 32*blk + 8t + i and 32*blk + 8t + 4 + i of head g
-    // (c0/c1: high-part row, c2/c3: low-part row).
-    if (g < group) {
-        const int h = kvh * group + g;
-        float *pa = p.part_acc + (size_t)slot * p.acc_slot + ((size_t)h * p.splits + split) * 256 +
-                    warp * 32 + 8 * t;
-        const float inv = 1.0f / kPScale;
-        *reinterpret_cast<float4 *>(pa) =
-            make_float4((acc[0][0] + acc[0][2]) * inv, (acc[1][0] + acc[1][2]) * inv,
-                        (acc[2][0] + acc[2][2]) * inv, (acc[3][0] + acc[3][2]) * inv);
-        *reinterpret_cast<float4 *>(pa + 4) =
-            make_float4((acc[0][1] + acc[0][3]) * inv, (acc[1][1] + acc[1][3]) * inv,
-                        (acc[2][1] + acc[2][3]) * inv, (acc[3][1] + acc[3][3]) * inv);
-    }
-    if (warp < group && lane == 0) {
-        const int h = kvh * group + warp;
-        float *pm = p.part_ml + (size_t)slot * p.ml_slot + ((size_t)h * p.splits + split) * 2;
-        pm[0] = m_run;
-        pm[1] = l_run;
-    }
-    }   // ntiles > 0
-
-    // ---- fold inside the split pass
-    if (p.out == nullptr) return;
-    const int runs = live_runs(p, slot, p.share_slots > 0 ? s_plan[3] : 0);
-    if (split >= runs) return;   // a launched run past the live ones: its neutral partial is not read
-    fold_tail(p, status, slot, kvh, split, runs, group, tid);
-}
-
-// ------------------------------------------------------------------------------------------
-// The q8_0 body with the value side on the 5th-generation tensor cores (tcgen05.mma kind::i8,
-// accumulators in TMEM). Scores, tiles, run plan, fused append and fold are those of
-// attn_decode_kv_tc; what changes is phase (3):
-//   * the V tile is brought in by 17 tensor (TMA) copies of {16 bytes, 64 rows}, one per
-//     16-byte column chunk of the 272-byte rows, so it lands as [chunk][key][16 B]: exactly the
-//     canonical MN-major operand of the MMA (8 keys x 16 bytes contiguous per core matrix).
-//     The int8 codes are the A operand as they are: M = byte of the row (three M tiles of 128
-//     cover the 272 bytes; the two scale bytes of each block are rows whose results are never
-//     read), K = key. No conversion of a single code on the CUDA cores;
-//   * the B operand is built per tile: column (block b, head h, digit) holds the weight
-//     exp2(score - ref_h) * scale(key, b) as a 23-bit fixed-point number in three unsigned
-//     bytes, taken straight out of the mantissa of weight * F + 2^23. A block's results only
-//     need that block's columns, so an M tile multiplies a window of 32 .. 96 columns;
-//   * products accumulate as int32 in TMEM (exact); per head the reference `ref_h` of the
-//     exponentials and the unit of the value scales stay fixed while the running maximum stays
-//     within 2^5.5 of it, so the accumulators are read out only when a reference moves (a few
-//     times per run) and at the end: digits are combined and scaled in f32 there.
-// Weights carry 17 bits below the reference (error 2^-18 of the largest weight), the int32
-// sums are exact, scores are as before: results agree with the f32 definition to ~1e-6.
 namespace i8 {
 
 constexpr float kMagicLimit = 8388608.0f;
@@ -992,7 +348,7 @@ attn_decode_kv_i8(const __grid_constant__ CUtensorMap vmap, int v3d, DecodeParam
     }
     const bool idle = slot < 0;   // (the shared grid is one round of CTAs; the tail of it may be spare)
 
-    // query values of this lane (see attn_decode_kv_tc), before anything that depends on the length
+    // query values of this lane (as the MMA wants them), before anything that depends on the length
     float qv[8][4];
     if (!idle) {
         const float *qh = p.q + (size_t)slot * p.q_slot + (size_t)(kvh * group + g) * 256;
@@ -1098,10 +454,10 @@ attn_decode_kv_i8(const __grid_constant__ CUtensorMap vmap, int v3d, DecodeParam
                 xl[i] = __float2half_rn(x - __half2float(xh[i]));
                 sum += __half2float(xh[i]) + __half2float(xl[i]);
             }
-            qb[ks][0] = pack_half2(xh[0], xh[1]);
-            qb[ks][1] = pack_half2(xh[2], xh[3]);
-            qb[ks][2] = pack_half2(xl[0], xl[1]);
-            qb[ks][3] = pack_half2(xl[2], xl[3]);
+            qb[ks][0] = pack2(xh[0], xh[1]);
+            qb[ks][1] = pack2(xh[2], xh[3]);
+            qb[ks][2] = pack2(xl[0], xl[1]);
+            qb[ks][3] = pack2(xl[2], xl[3]);
         }
         sum += __shfl_xor_sync(0xffffffffu, sum, 1);
         sum += __shfl_xor_sync(0xffffffffu, sum, 2);
@@ -1409,7 +765,7 @@ __global__ void __launch_bounds__(kThreads) attn_decode_fold_tree(DecodeParams p
 
 namespace {
 
-// Per-device set-up of the two kernels (dynamic shared memory limit, status word), done once.
+// Per-device set-up of the kernel (dynamic shared memory limit, status word), done once.
 int *decode_tc_setup(int *rc) {
     static std::mutex mu;
     static int *status_word[64] = {};   // nullptr = device not set up yet
@@ -1419,11 +775,8 @@ int *decode_tc_setup(int *rc) {
     if (dev < 0 || dev >= 64) dev = 0;
     std::lock_guard<std::mutex> lock(mu);
     if (status_word[dev] == nullptr) {
-        cudaError_t e = cudaFuncSetAttribute(attn_decode_kv_tc<false>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(attn_decode_kv_tc<true>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+        const cudaError_t e = cudaFuncSetAttribute(i8::attn_decode_kv_i8,
+                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, i8::kSmem);
         if (e != cudaSuccess) {
             *rc = (int)e;
             return nullptr;
@@ -1436,22 +789,6 @@ int *decode_tc_setup(int *rc) {
 
 std::atomic<int> g_two_launch_fold{0};
 std::atomic<int> g_decode_body{1};   // 1: values on mma.sync, 2: values on tcgen05 kind::i8
-
-int i8_setup() {
-    static std::mutex mu;
-    static bool done[64] = {};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64) dev = 0;
-    std::lock_guard<std::mutex> lock(mu);
-    if (!done[dev]) {
-        const cudaError_t e = cudaFuncSetAttribute(i8::attn_decode_kv_i8,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, i8::kSmem);
-        if (e != cudaSuccess) return (int)e;
-        done[dev] = true;
-    }
-    return 0;
-}
 
 }  // namespace
 
@@ -1499,18 +836,15 @@ int decode_arrive_region(cudaStream_t stream, long long counters) {
     return region;
 }
 
-int launch_decode_fold_tree(cudaStream_t stream, const DecodeParams &p, int slots) {
-    int rc = 0;
-    int *status = decode_tc_setup(&rc);
-    if (!status) return rc;
-    DecodeParams q = p;
-    q.n_slots = slots;
-    return launch_pdl(attn_decode_fold_tree, dim3(q.n_kv, slots), dim3(kThreads), 0, stream, 1, q, status);
-}
-
 // Split pass; with p.out set also the fold: inside the same launch when an arrival-counter
 // region is to be had, as a second launch otherwise.
+// (selector 7 asks for the mma.sync values, selector 8 for the tcgen05 values; otherwise the
+// process-wide choice of hipml_set_decode_body, whose default is the faster of the two. The tcgen05
+// body takes q8_0, a GQA group of at most 6, slots a whole number of 272-byte rows apart.)
 int launch_decode_tc(cudaStream_t stream, const DecodeParams &p, int slots) {
+    const int want = p.legacy_body == 1 ? 1 : (p.legacy_body == 2 ? 2 : g_decode_body.load());
+    if (!(want == 2 && !p.q4 && p.n_heads / p.n_kv <= 6 && p.kv_slot_bytes % kRowBytes == 0))
+        return launch_decode_warps(stream, p, slots);
     int rc = 0;
     int *status = decode_tc_setup(&rc);
     if (!status) return rc;
@@ -1521,46 +855,37 @@ int launch_decode_tc(cudaStream_t stream, const DecodeParams &p, int slots) {
         grid = dim3(q.share_slots, 1);
     else if (!q.by_stride && q.run_cap > 0 && q.run_cap < q.splits)
         grid = dim3(q.n_kv * q.run_cap, slots);
-    // The body with the value side on tcgen05 (int8 operands): q8_0, a GQA group of at most 6,
-    // slots a whole number of 272-byte rows apart.
-    // (selector 7 asks for the mma.sync values, selector 8 for the tcgen05 values; otherwise the
-    // process-wide choice of hipml_set_decode_body, whose default is the faster of the two)
-    const int want = q.legacy_body == 1 ? 1 : (q.legacy_body == 2 ? 2 : g_decode_body.load());
-    const bool i8_body = want == 2 && !q.q4 && q.n_heads / q.n_kv <= 6 && q.kv_slot_bytes % kRowBytes == 0;
     CUtensorMap vmap;
     int v3d = 0;
-    if (i8_body) {
-        if (int e = i8_setup()) return e;
-        EncodeTiledFn fn = encode_tiled_fn();
-        if (!fn) return fail(HIPML_ERR_INVALID_ARGUMENT, "cuTensorMapEncodeTiled is not available");
-        const cuuint64_t rows = (cuuint64_t)(slots > 1 ? (slots - 1) * (q.kv_slot_bytes / kRowBytes) : 0) +
-                                (cuuint64_t)q.n_kv * q.stride;
-        // the tile in chunk order with one copy: {16 bytes, rows (272 apart), 17 chunks (16 apart)}
-        const cuuint64_t dims3[3] = {16, rows, 17};
-        const cuuint64_t strides3[2] = {(cuuint64_t)kRowBytes, 16};
-        const cuuint32_t box3[3] = {16, (cuuint32_t)kTile, 17};
-        const cuuint32_t elem3[3] = {1, 1, 1};
-        CUresult r = fn(&vmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<unsigned char *>(q.v), dims3,
-                        strides3, box3, elem3, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        v3d = r == CUDA_SUCCESS;
-        static const bool verbose = getenv("HIPML_VERBOSE") != nullptr;
-        if (verbose)
-            fprintf(stderr, "hipml: decode V tiles land with %s\n",
-                    v3d ? "one 3-D tensor copy" : "17 2-D tensor copies (3-D view refused)");
-        if (!v3d) {
-            // the driver refuses the overlapping view: one copy per chunk from the plain 2-D view
-            const cuuint64_t dims[2] = {(cuuint64_t)kRowBytes, rows};
-            const cuuint64_t strides[1] = {(cuuint64_t)kRowBytes};
-            const cuuint32_t box[2] = {16, (cuuint32_t)kTile};
-            const cuuint32_t elem[2] = {1, 1};
-            r = fn(&vmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<unsigned char *>(q.v), dims, strides,
-                   box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        }
-        if (r != CUDA_SUCCESS)
-            return fail(HIPML_ERR_INVALID_ARGUMENT, "cuTensorMapEncodeTiled (V cache) failed: %d", (int)r);
+    EncodeTiledFn fn = encode_tiled_fn();
+    if (!fn) return fail(HIPML_ERR_INVALID_ARGUMENT, "cuTensorMapEncodeTiled is not available");
+    const cuuint64_t rows = (cuuint64_t)(slots > 1 ? (slots - 1) * (q.kv_slot_bytes / kRowBytes) : 0) +
+                            (cuuint64_t)q.n_kv * q.stride;
+    // the tile in chunk order with one copy: {16 bytes, rows (272 apart), 17 chunks (16 apart)}
+    const cuuint64_t dims3[3] = {16, rows, 17};
+    const cuuint64_t strides3[2] = {(cuuint64_t)kRowBytes, 16};
+    const cuuint32_t box3[3] = {16, (cuuint32_t)kTile, 17};
+    const cuuint32_t elem3[3] = {1, 1, 1};
+    CUresult r = fn(&vmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<unsigned char *>(q.v), dims3,
+                    strides3, box3, elem3, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    v3d = r == CUDA_SUCCESS;
+    static const bool verbose = getenv("HIPML_VERBOSE") != nullptr;
+    if (verbose)
+        fprintf(stderr, "hipml: decode V tiles land with %s\n",
+                v3d ? "one 3-D tensor copy" : "17 2-D tensor copies (3-D view refused)");
+    if (!v3d) {
+        // the driver refuses the overlapping view: one copy per chunk from the plain 2-D view
+        const cuuint64_t dims[2] = {(cuuint64_t)kRowBytes, rows};
+        const cuuint64_t strides[1] = {(cuuint64_t)kRowBytes};
+        const cuuint32_t box[2] = {16, (cuuint32_t)kTile};
+        const cuuint32_t elem[2] = {1, 1};
+        r = fn(&vmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<unsigned char *>(q.v), dims, strides,
+               box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     }
+    if (r != CUDA_SUCCESS)
+        return fail(HIPML_ERR_INVALID_ARGUMENT, "cuTensorMapEncodeTiled (V cache) failed: %d", (int)r);
     bool second_launch = false;
     if (q.out != nullptr) {
         // most runs a (slot, KV head) can have under the plan in force
@@ -1574,14 +899,7 @@ int launch_decode_tc(cudaStream_t stream, const DecodeParams &p, int slots) {
             q.out = nullptr;
         }
     }
-    if (i8_body)
-        rc = launch_pdl(i8::attn_decode_kv_i8, grid, dim3(kThreads), (size_t)i8::kSmem, stream, 1, vmap, v3d, q,
-                        status);
-    else
-        rc = q.q4 ? launch_pdl(attn_decode_kv_tc<true>, grid, dim3(kThreads), (size_t)kSmemBytes, stream, 1,
-                               q, status)
-                  : launch_pdl(attn_decode_kv_tc<false>, grid, dim3(kThreads), (size_t)kSmemBytes, stream, 1,
-                               q, status);
+    rc = launch_pdl(i8::attn_decode_kv_i8, grid, dim3(kThreads), (size_t)i8::kSmem, stream, 1, vmap, v3d, q, status);
     if (rc != 0 || !second_launch) return rc;
     q.out = p.out;
     return launch_pdl(attn_decode_fold_tree, dim3(q.n_kv, slots), dim3(kThreads), 0, stream, 1, q, status);

@@ -283,4 +283,44 @@ __device__ __forceinline__ void fold_emit(const DecodeParams &p, int slot, int h
     }
 }
 
+// What the CTA that holds the final fold of a (slot, KV head) does with it: write the output
+// rows, or (sequence-split decode across GPUs) publish the triples to every rank's table
+// and / or collect all ranks' triples and fold those. All threads of the CTA call it; warp w
+// holds head w of the group in f.
+__device__ __forceinline__ void fold_finish(const DecodeParams &p, int *status, int slot, int kvh,
+                                            int group, FoldAcc &f) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int h = kvh * group + warp;
+    if (p.xch.phases == 0) {
+        if (warp < group) fold_emit(p, slot, h, f, lane, p.normalize != 0);
+        return;
+    }
+    __shared__ int s_epoch;
+    int *hdr = reinterpret_cast<int *>(p.xch.ws[p.xch.rank]);
+    // Every folding CTA of the call reads the epoch before it adds itself to the counter, and
+    // the epoch advances only after the last of them has: all of them see the same value.
+    if (threadIdx.x == 0) s_epoch = *reinterpret_cast<volatile int *>(hdr) + ((p.xch.phases & 1) ? 1 : 0);
+    __syncthreads();
+    const int e = s_epoch;
+    if (p.xch.phases & 1) {
+        if (warp < group) exchange_publish_warp(p.xch, p.n_heads, h, e, f, lane);
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            if (atomicAdd(hdr + 1, 1) == p.n_kv - 1) {
+                hdr[1] = 0;
+                *reinterpret_cast<volatile int *>(hdr) = e;
+            }
+        }
+    }
+    if (p.xch.phases & 2) {
+        if (warp < group && (!p.xch.by_head || exchange_owner(p.xch, p.n_heads, h) == p.xch.rank)) {
+            const unsigned long long deadline = global_timer_ns() + 1000ull * p.xch.wait_us;
+            if (exchange_collect_warp(p.xch, p.n_heads, h, e, deadline, lane, f))
+                fold_emit(p, slot, h, f, lane, true);
+            else if (lane == 0 && status)
+                atomicCAS(status, 0, 31);
+        }
+    }
+}
+
 }  // namespace hipml

@@ -1,0 +1,596 @@
+// The pieces of the decode body whose warps work alone (attn_decode_warps.cu) that its form for several
+// columns of one stream (attn_decode_cols.cu) shares, operation for operation: a column's result does
+// not depend on which of the two computed it.
+#pragma once
+
+#include <type_traits>
+
+#include "decode_fold.cuh"
+#include "decode_rows.cuh"
+#include "params.cuh"
+#include "sm100_ptx.cuh"
+
+namespace hipml {
+namespace warp_body {
+
+using namespace ptx;
+
+template <int N>
+using Int = std::integral_constant<int, N>;
+
+constexpr int kWarps = 8;                        // per CTA
+constexpr int kThreads = 32 * kWarps;
+constexpr int kHeadPitch = 260;                  // floats per head of a warp's partial (bank spread)
+// A reference is set this far (log2) above the maximum seen, so that the few units a warp takes
+// rarely move it again: with the exact maximum 75 % of the units of a 100,000-row step rescaled 64
+// accumulators.
+constexpr float kMargin = 1.5f;
+constexpr int kNeutralSlots = 32;   // partial slots that are written whether or not a run of rows has them
+constexpr int kPrefetch = 2;   // units of K and of V a warp asks L2 for ahead of the grid dependency
+
+__device__ __forceinline__ float ex2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+// Transpose of an 8 x 8 tile of f16 held one 32-bit pair per lane (row = lane / 4).
+__device__ __forceinline__ unsigned transpose8(unsigned x) {
+    unsigned y;
+    asm("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(y) : "r"(x));
+    return y;
+}
+__device__ __forceinline__ void split2(float a, float b, unsigned &hi, unsigned &lo) {
+    const __half2 h = __floats2half2_rn(a, b);
+    const float2 f = __half22float2(h);
+    const __half2 l = __floats2half2_rn(a - f.x, b - f.y);
+    hi = *reinterpret_cast<const unsigned *>(&h);
+    lo = *reinterpret_cast<const unsigned *>(&l);
+}
+
+// A pair of blocks (2M, 2M + 1) of a row is a whole number of words from a word boundary: W[0] =
+// {scale of the even block, its codes 0, 1}, W[kHalf] = {its last two code bytes, scale of the odd
+// block}, then the odd block's code words. So every code word but one is an aligned word of the
+// row: the even block's word j holds code bytes 4j + 2 .. 4j + 5, and its last one is stitched from
+// the outer two words, whose other halves are the scales.
+template <bool kQ4>
+struct Row {
+    static constexpr int kWords = kQ4 ? 4 : 8;         // code words of a block
+    static constexpr int kHalf = kWords;               // the word with the odd block's scale
+    static constexpr int kPair = 2 * kWords + 1;       // words of a pair
+    static constexpr int kPitch = kQ4 ? kQ4RowBytes / 4 : kRowBytes / 4;
+};
+__device__ __forceinline__ unsigned stitch(unsigned w0, unsigned wh) { return __byte_perm(w0, wh, 0x5432); }
+__device__ __forceinline__ float low_half(unsigned w) { return half_bits_to_float((unsigned short)w); }
+__device__ __forceinline__ float high_half(unsigned w) { return half_bits_to_float((unsigned short)(w >> 16)); }
+
+// Query fragments of one block (the warp's) into `frag`: for each of its two 16-slot steps the B
+// operand's {hi b0, hi b1, lo b0, lo b1} of column g (head g; heads past the group are zero), slots in the
+// order of k_word_dim (2t, 2t + 1 = bytes 0, 1 of word t; 2t + 8, 2t + 9 = bytes 2, 3); x holds the lane's values
+// in that order. And the C operand that takes the codes' offset of 128 (nibbles: 8) out: -2^-17 * their
+// sum, as {head 2t, 2t + 1, 2t, 2t + 1}.
+template <bool kQ4>
+__device__ __forceinline__ void store_query(const float2 (&x)[2][2], float scale_log2, int blk, int lane, uint4 *frag,
+                                            float *bias) {
+    const int g = lane >> 2, t = lane & 3;
+    float sum = 0.0f;   // of the block's query values as the tensor cores see them
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        uint4 f;
+        split2(x[k][0].x * scale_log2, x[k][0].y * scale_log2, f.x, f.z);
+        split2(x[k][1].x * scale_log2, x[k][1].y * scale_log2, f.y, f.w);
+        const unsigned v[4] = {f.x, f.y, f.z, f.w};
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const float2 y = __half22float2(*reinterpret_cast<const __half2 *>(&v[i]));
+            sum += y.x + y.y;
+        }
+        frag[(2 * blk + k) * 32 + lane] = f;
+    }
+    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+    if (t == 0) {
+        float *const dst = bias + blk * 16 + (g >> 1) * 4 + (g & 1);
+        dst[0] = dst[2] = -(kQ4 ? kCodeBias / 16.0f : kCodeBias) * sum;
+    }
+}
+
+// ---- scores. A warp's K operands of blocks 2M, 2M + 1 for kT tiles of 16 rows.
+template <int kT>
+struct KFrag {
+    unsigned e[2][kT][4], o[2][kT][4];   // [16-slot step][tile]: A fragment of the even / odd block
+    float de[kT][2], dd[kT][2];          // their scales, rows g and g + 8
+};
+template <int M, bool kQ4, int kT>
+__device__ __forceinline__ void load_k(const unsigned *row, int t, KFrag<kT> &f) {
+    using R = Row<kQ4>;
+#pragma unroll
+    for (int i = 0; i < kT; i++) {
+        unsigned e[2][2], o[2][2];       // [step][row g, g + 8]: biased codes
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            const unsigned *w = row + (i * 16 + r * 8) * R::kPitch + M * R::kPair;
+            const unsigned w0 = w[0], wh = w[R::kHalf];
+            f.de[i][r] = low_half(w0);
+            f.dd[i][r] = high_half(wh);
+            if constexpr (kQ4) {
+                const unsigned x = w[1 + t], y = w[5 + t];
+                const unsigned ev = t == 3 ? stitch(w0, wh) : x;
+                e[0][r] = ev & 0x0f0f0f0fu;
+                e[1][r] = (ev >> 4) & 0x0f0f0f0fu;
+                o[0][r] = y & 0x0f0f0f0fu;
+                o[1][r] = (y >> 4) & 0x0f0f0f0fu;
+            } else {
+                const unsigned x0 = w[1 + t], x1 = w[5 + t];
+                e[0][r] = x0 ^ 0x80808080u;
+                e[1][r] = (t == 3 ? stitch(w0, wh) : x1) ^ 0x80808080u;
+                o[0][r] = w[9 + t] ^ 0x80808080u;
+                o[1][r] = w[13 + t] ^ 0x80808080u;
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 2; k++)
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                f.e[k][i][c] = codes_to_half2(e[k][c & 1], c < 2 ? 0x4140 : 0x4342);
+                f.o[k][i][c] = codes_to_half2(o[k][c & 1], c < 2 ? 0x4140 : 0x4342);
+            }
+    }
+}
+// Adds the two blocks' scores into s: s[i][0], s[i][1] = row g of tile i, heads 2t and 2t + 1; s[i][2],
+// s[i][3] = row g + 8. A query fragment serves all tiles; the MMA chains of tiles and blocks interleave.
+template <int M, int kT>
+__device__ __forceinline__ void add_scores(const KFrag<kT> &f, const uint4 *qf, const float4 *bias, float (&s)[kT][4]) {
+    const float4 be = bias[2 * M * 4], bo = bias[(2 * M + 1) * 4];
+    const float c0e[4] = {be.x, be.y, be.z, be.w}, c0o[4] = {bo.x, bo.y, bo.z, bo.w};
+    float ce[kT][4], co[kT][4];
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const uint4 qe = qf[(4 * M + k) * 32], qo = qf[(4 * M + 2 + k) * 32];
+#pragma unroll
+        for (int i = 0; i < kT; i++) {
+            if (k == 0) {
+                mma_16816(ce[i], f.e[k][i], qe.x, qe.y, c0e);
+                mma_16816(co[i], f.o[k][i], qo.x, qo.y, c0o);
+            } else {
+                mma_16816(ce[i], f.e[k][i], qe.x, qe.y);
+                mma_16816(co[i], f.o[k][i], qo.x, qo.y);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < kT; i++) {
+            mma_16816(ce[i], f.e[k][i], qe.z, qe.w);
+            mma_16816(co[i], f.o[k][i], qo.z, qo.w);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < kT; i++)
+#pragma unroll
+        for (int c = 0; c < 4; c++) s[i][c] = fmaf(f.dd[i][c >> 1], co[i][c], fmaf(f.de[i][c >> 1], ce[i][c], s[i][c]));
+}
+
+// ---- softmax of a unit: running reference and sum of a lane's heads 2t, 2t + 1.
+struct Running {
+    float m[2], nm[2], l[2];   // reference, 10 - reference, sum (of this lane's rows)
+};
+__device__ __forceinline__ void start(Running &r) {
+    r.m[0] = r.m[1] = -INFINITY;
+    r.nm[0] = r.nm[1] = INFINITY;
+    r.l[0] = r.l[1] = 0.0f;
+}
+__device__ __forceinline__ void sum_rows(Running &r) {   // over the lanes of a head
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        r.l[h] += __shfl_xor_sync(0xffffffffu, r.l[h], 4);
+        r.l[h] += __shfl_xor_sync(0xffffffffu, r.l[h], 8);
+        r.l[h] += __shfl_xor_sync(0xffffffffu, r.l[h], 16);
+    }
+}
+// The weights 2^(score - reference + 10) of kT tiles, as f16 high and low pairs in the B operand's
+// layout: ph[j][0] = rows 2t, 2t + 1 of tile j for head g, ph[j][1] = rows 2t + 8, 2t + 9. Rows from `rows` on
+// get weight 0. True when the references moved: what was accumulated must be multiplied by corr.
+template <int kT>
+__device__ __forceinline__ bool softmax(float (&s)[kT][4], int rows, int g, Running &r, __half2 (&ph)[kT][2],
+                                        __half2 (&pl)[kT][2], float (&corr)[2]) {
+    if (rows < 16 * kT) {   // rows past the end hold stale bytes
+#pragma unroll
+        for (int j = 0; j < kT; j++) {
+            if (16 * j + g >= rows) s[j][0] = s[j][1] = -INFINITY;
+            if (16 * j + g + 8 >= rows) s[j][2] = s[j][3] = -INFINITY;
+        }
+    }
+    float x[kT][4], xm = -INFINITY;
+#pragma unroll
+    for (int j = 0; j < kT; j++)
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            x[j][c] = fmaf(s[j][c], kCodeUnit, r.nm[c & 1]);
+            xm = fmaxf(xm, x[j][c]);
+        }
+    const bool moved = __any_sync(0xffffffffu, xm > kPScaleLog2);
+    if (moved) {
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            float mx = -INFINITY;
+#pragma unroll
+            for (int j = 0; j < kT; j++) mx = fmaxf(mx, fmaxf(s[j][h], s[j][h + 2]));
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+            // (rounded up to 1/16, so that the shift by 10 is exact)
+            const float top = ceilf(mx * (kCodeUnit * 16.0f)) * 0.0625f;
+            const float mn = top > r.m[h] ? top + kMargin : r.m[h];
+            corr[h] = ex2(r.m[h] - mn);
+            r.m[h] = mn;
+            r.nm[h] = kPScaleLog2 - mn;
+            r.l[h] *= corr[h];
+        }
+#pragma unroll
+        for (int j = 0; j < kT; j++)
+#pragma unroll
+            for (int c = 0; c < 4; c++) x[j][c] = fmaf(s[j][c], kCodeUnit, r.nm[c & 1]);
+    }
+#pragma unroll
+    for (int j = 0; j < kT; j++) {
+        float pw[4];
+#pragma unroll
+        for (int c = 0; c < 4; c++) pw[c] = ex2(x[j][c]);
+        r.l[0] += pw[0] + pw[2];
+        r.l[1] += pw[1] + pw[3];
+#pragma unroll
+        for (int c = 0; c < 2; c++) {
+            unsigned hi, lo;
+            split2(pw[2 * c], pw[2 * c + 1], hi, lo);
+            hi = transpose8(hi);
+            lo = transpose8(lo);
+            ph[j][c] = *reinterpret_cast<const __half2 *>(&hi);
+            pl[j][c] = *reinterpret_cast<const __half2 *>(&lo);
+        }
+    }
+    return moved;
+}
+
+// ---- values. A warp's V operands of blocks 2M, 2M + 1 for one tile of 16 rows (`row`: its row 2t).
+struct VFrag {
+    unsigned e[2][4], o[2][4];         // A fragments: code bytes {0, 1} and {2, 3} of the lane's word of each row
+    __half2 de01, de23, do01, do23;    // scales of rows 2t, 2t + 1 / 2t + 8, 2t + 9
+};
+template <int M, bool kQ4>
+__device__ __forceinline__ void load_v(const unsigned *row, int g, VFrag &f) {
+    using R = Row<kQ4>;
+    constexpr int kRowOf[4] = {0, 1, 8, 9};
+    const int j = kQ4 ? (g & 3) : g;
+    unsigned w0[4], wh[4], we[4], wo[4];
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+        const unsigned *w = row + kRowOf[e] * R::kPitch + M * R::kPair;
+        w0[e] = w[0];
+        wh[e] = w[R::kHalf];
+        we[e] = w[1 + j];
+        wo[e] = w[R::kHalf + 1 + j];
+    }
+    auto half2_of = [](unsigned x) { return *reinterpret_cast<const __half2 *>(&x); };
+    auto convert = [&](unsigned (&x)[4], unsigned (&a)[2][4]) {
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            if constexpr (kQ4)
+                x[e] = (x[e] >> ((g >> 2) * 4)) & 0x0f0f0f0fu;
+            else
+                x[e] ^= 0x80808080u;
+        }
+        // 0x64xx = 1024 + xx, minus 1152 (nibbles: 1032): exact. (The weights are all positive, an offset
+        // left to the accumulators would cost several bits: 4e-5 relative on a flat 256-key run.)
+        auto conv = [&](unsigned y, unsigned sel) {
+            const __half2 r = __hsub2(half2_of(__byte_perm(y, 0x64646464u, sel)),
+                                      __half2half2(__ushort_as_half(kQ4 ? 0x6408 : 0x6480)));
+            return *reinterpret_cast<const unsigned *>(&r);
+        };
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const unsigned ab = __byte_perm(x[0], x[1], i ? 0x7362 : 0x5140);   // [a0 b0 a1 b1] / [a2 b2 a3 b3]
+            const unsigned cd = __byte_perm(x[2], x[3], i ? 0x7362 : 0x5140);
+            a[i][0] = conv(ab, 0x4140);
+            a[i][1] = conv(ab, 0x4342);
+            a[i][2] = conv(cd, 0x4140);
+            a[i][3] = conv(cd, 0x4342);
+        }
+    };
+#pragma unroll
+    for (int e = 0; e < 4; e++) we[e] = j == R::kWords - 1 ? stitch(w0[e], wh[e]) : we[e];
+    f.de01 = half2_of(__byte_perm(w0[0], w0[1], 0x5410));
+    f.de23 = half2_of(__byte_perm(w0[2], w0[3], 0x5410));
+    f.do01 = half2_of(__byte_perm(wh[0], wh[1], 0x7632));
+    f.do23 = half2_of(__byte_perm(wh[2], wh[3], 0x7632));
+    convert(we, f.e);
+    convert(wo, f.o);
+}
+// acc[block][i][c] += weights * values: code bytes {0, 1} (i = 0) and {2, 3} of the lane's word of the even /
+// odd block, c = {byte 0, 1} x {head 2t, 2t + 1} (value_dim).
+__device__ __forceinline__ void add_values(const VFrag &f, const __half2 (&ph)[2], const __half2 (&pl)[2],
+                                           float (&acc_e)[2][4], float (&acc_o)[2][4]) {
+    auto bits = [](const __half2 &h) { return *reinterpret_cast<const unsigned *>(&h); };
+    auto block = [&](const __half2 d01, const __half2 d23, const unsigned (&a)[2][4], float (&acc)[2][4]) {
+        const __half2 h01 = __hmul2(ph[0], d01), h23 = __hmul2(ph[1], d23);
+        const __half2 l01 = __hfma2(pl[0], d01, __hfma2(ph[0], d01, __hneg2(h01)));
+        const __half2 l23 = __hfma2(pl[1], d23, __hfma2(ph[1], d23, __hneg2(h23)));
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            mma_16816(acc[i], a[i], bits(h01), bits(h23));
+            mma_16816(acc[i], a[i], bits(l01), bits(l23));
+        }
+    };
+    block(f.de01, f.de23, f.e, acc_e);
+    block(f.do01, f.do23, f.o, acc_o);
+}
+// First dim (within the block) of code bytes {0, 1} (half 0) and {2, 3} (half 1) of lane group g's word.
+template <bool kQ4>
+__device__ __forceinline__ int value_dim(int blk, int g, int half) {
+    const int j = kQ4 ? (g & 3) : g, base = kQ4 ? 16 * (g >> 2) : 0, words = Row<kQ4>::kWords;
+    if (blk & 1) return base + 4 * j + 2 * half;
+    if (j == words - 1) return base + (half ? 4 * words - 2 : 0);
+    return base + 4 * j + 2 + 2 * half;
+}
+
+// ---- folds. A partial of a head is (acc, m, l) with weights relative to 2^m; folding partials is
+// associative up to rounding, and always runs in one order with explicit operations.
+struct Part {
+    float4 a;
+    float m, l;
+};
+__device__ __forceinline__ void rescale(Part &r, float big) {
+    const float c = r.m == -INFINITY ? 0.0f : ex2(r.m - big);
+    r.a.x = __fmul_rn(r.a.x, c);
+    r.a.y = __fmul_rn(r.a.y, c);
+    r.a.z = __fmul_rn(r.a.z, c);
+    r.a.w = __fmul_rn(r.a.w, c);
+    r.l = __fmul_rn(r.l, c);
+    r.m = big;
+}
+__device__ __forceinline__ void add(Part &r, const float4 &x, const float2 &ml) {   // r.m >= ml.x
+    const float w = ml.x == -INFINITY ? 0.0f : ex2(ml.x - r.m);
+    r.a.x = fmaf(x.x, w, r.a.x);
+    r.a.y = fmaf(x.y, w, r.a.y);
+    r.a.z = fmaf(x.z, w, r.a.z);
+    r.a.w = fmaf(x.w, w, r.a.w);
+    r.l = fmaf(ml.y, w, r.l);
+}
+
+// Folds sources [i0, i1) of kPer items each: load(i, j, x, ml) fetches source i of item j. The loads of
+// kBatch sources are issued together: a batch costs one round trip.
+template <int kPer, int kBatch, class Load>
+__device__ __forceinline__ void fold_sources(int i0, int i1, Load load, Part (&r)[kPer]) {
+#pragma unroll
+    for (int j = 0; j < kPer; j++) {
+        r[j].a = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        r[j].m = -INFINITY;
+        r[j].l = 0.0f;
+    }
+    for (int s0 = i0; s0 < i1; s0 += kBatch) {
+        float4 x[kPer][kBatch];
+        float2 ml[kPer][kBatch];
+#pragma unroll
+        for (int i = 0; i < kBatch; i++)
+#pragma unroll
+            for (int j = 0; j < kPer; j++) {
+                x[j][i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                ml[j][i] = make_float2(-INFINITY, 0.0f);
+                if (s0 + i < i1) load(s0 + i, j, x[j][i], ml[j][i]);
+            }
+#pragma unroll
+        for (int j = 0; j < kPer; j++) {
+            float big = r[j].m;
+#pragma unroll
+            for (int i = 0; i < kBatch; i++) big = fmaxf(big, ml[j][i].x);
+            rescale(r[j], big);
+#pragma unroll
+            for (int i = 0; i < kBatch; i++) add(r[j], x[j][i], ml[j][i]);
+        }
+    }
+}
+
+// How the threads of a CTA divide a slice of 1 / kC of a head group's items (at most 512): kShare
+// neighbouring threads per item, each with a contiguous share of the sources, joined by shuffles; or
+// kPer items per thread.
+template <int kC>
+struct Split {
+    static constexpr int kShare = kC > 2 ? kC / 2 : 1;
+    static constexpr int kPer = kC == 1 ? 2 : 1;
+};
+template <int kShare>
+__device__ __forceinline__ void join(Part &r) {
+#pragma unroll
+    for (int o = 1; o < kShare; o <<= 1) {
+        float4 x;
+        float2 ml;
+        x.x = __shfl_xor_sync(0xffffffffu, r.a.x, o);
+        x.y = __shfl_xor_sync(0xffffffffu, r.a.y, o);
+        x.z = __shfl_xor_sync(0xffffffffu, r.a.z, o);
+        x.w = __shfl_xor_sync(0xffffffffu, r.a.w, o);
+        ml.x = __shfl_xor_sync(0xffffffffu, r.m, o);
+        ml.y = __shfl_xor_sync(0xffffffffu, r.l, o);
+        rescale(r, fmaxf(r.m, ml.x));
+        add(r, x, ml);
+    }
+}
+
+// A warp's accumulators as a partial [head][dims] with kHeadPitch floats per head.
+template <bool kQ4>
+__device__ __forceinline__ void store_warp_partial(float *dst, const float (&acc)[8][2][4], int group, int g, int t) {
+#pragma unroll
+    for (int h = 0; h < 2; h++)
+        if (2 * t + h < group) {
+#pragma unroll
+            for (int b = 0; b < 8; b++)
+#pragma unroll
+                for (int i = 0; i < 2; i++)
+                    *reinterpret_cast<float2 *>(dst + (2 * t + h) * kHeadPitch + 32 * b + value_dim<kQ4>(b, g, i)) =
+                        make_float2(acc[b][i][h], acc[b][i][2 + h]);
+        }
+}
+// Folds the partials of a CTA's warps (`pitch` bytes apart; ml: [8 heads][warp]); done(item, part).
+template <class Done>
+__device__ __forceinline__ void fold_warps(const unsigned char *partials, int pitch, const float2 *ml_at, int items,
+                                           Done done) {
+    using S = Split<1>;
+    Part r[S::kPer];
+    fold_sources<S::kPer, kWarps>(
+        0, kWarps,
+        [&](int i, int j, float4 &x, float2 &ml) {
+            const int item = min((int)threadIdx.x + j * kThreads, items - 1);
+            x = *reinterpret_cast<const float4 *>(partials + i * pitch + ((item >> 6) * kHeadPitch + 4 * (item & 63)) * 4);
+            ml = ml_at[(item >> 6) * kWarps + i];
+        },
+        r);
+#pragma unroll
+    for (int j = 0; j < S::kPer; j++)
+        if ((int)threadIdx.x + j * kThreads < items) done(threadIdx.x + j * kThreads, r[j]);
+}
+// Folds slice `rank` of the items of the kC CTAs of a cluster (cpart: [item], cml: [8 heads], at the same
+// place in each of them).
+template <int kC, class Done>
+__device__ __forceinline__ void fold_cluster(const float4 *cpart, const float2 *cml, int items, int rank, Done done) {
+    using S = Split<kC>;
+    static_assert(S::kPer == 1 && kC % S::kShare == 0, "slices");
+    const int first = items * rank / kC, count = items * (rank + 1) / kC - first;
+    const int at = threadIdx.x / S::kShare, part = threadIdx.x % S::kShare, item = first + min(at, count - 1);
+    const unsigned area = smem_u32(cpart + item), ml_area = smem_u32(cml + (item >> 6));
+    Part r[1];
+    fold_sources<1, kC / S::kShare>(
+        part * (kC / S::kShare), (part + 1) * (kC / S::kShare),
+        [&](int i, int, float4 &x, float2 &ml) {
+            x = ld_cluster_f4(map_to_cta(area, i));
+            ml = ld_cluster_f2(map_to_cta(ml_area, i));
+        },
+        r);
+    join<S::kShare>(r[0]);
+    if (at < count && part == 0) done(item, r[0]);
+}
+
+// One float4 (item = head of the group * 64 + dims / 4) of the output: normalised (and gated), or
+// the raw triple of a shard, whose reference maximum leaves the weights' scale of 2^10 out.
+__device__ __forceinline__ void emit_item(const DecodeParams &p, int slot, int kvh, int group, int item,
+                                          const Part &r) {
+    const int h = kvh * group + (item >> 6), j = item & 63;
+    const size_t at = (size_t)slot * p.out_slot + (size_t)h * p.out_head_stride + 4 * j;
+    float *o = p.out + at;
+    if (p.normalize) {
+        float4 y;
+        y.x = r.l > 0.0f ? __fdiv_rn(r.a.x, r.l) : 0.0f;
+        y.y = r.l > 0.0f ? __fdiv_rn(r.a.y, r.l) : 0.0f;
+        y.z = r.l > 0.0f ? __fdiv_rn(r.a.z, r.l) : 0.0f;
+        y.w = r.l > 0.0f ? __fdiv_rn(r.a.w, r.l) : 0.0f;
+        if (p.gate) {
+            const float4 g = *reinterpret_cast<const float4 *>(p.gate + at);
+            y.x *= 1.0f / (1.0f + expf(-g.x));
+            y.y *= 1.0f / (1.0f + expf(-g.y));
+            y.z *= 1.0f / (1.0f + expf(-g.z));
+            y.w *= 1.0f / (1.0f + expf(-g.w));
+        }
+        *reinterpret_cast<float4 *>(o) = y;
+    } else {
+        // rows of head_dim + 2 floats are only 8-byte aligned
+        constexpr float kInv = 1.0f / kPScale;
+        reinterpret_cast<float2 *>(o)[0] = make_float2(r.a.x * kInv, r.a.y * kInv);
+        reinterpret_cast<float2 *>(o)[1] = make_float2(r.a.z * kInv, r.a.w * kInv);
+        if (j == 0) {
+            o[256] = r.m + kPScaleLog2;
+            o[257] = r.l * kInv;
+        }
+    }
+}
+
+// Folds the `runs` partials of slice `rank` of a head group from memory and emits it (or, staged !=
+// nullptr, leaves it there: [8 heads][256] sums, then [8 heads]{max, sum}).
+template <int kC>
+__device__ __forceinline__ void fold_runs(const DecodeParams &p, int slot, int kvh, int group, int runs, int rank,
+                                          float *staged) {
+    using S = Split<kC>;
+    const float *pa = p.part_acc + (size_t)slot * p.acc_slot + (size_t)kvh * group * p.splits * 256;
+    const float *pm = p.part_ml + (size_t)slot * p.ml_slot + (size_t)kvh * group * p.splits * 2;
+    const int items = group * 64, first = items * rank / kC, count = items * (rank + 1) / kC - first;
+    const int at0 = threadIdx.x / S::kShare, part = threadIdx.x % S::kShare;
+    Part r[S::kPer];
+    fold_sources<S::kPer, S::kPer == 1 ? 10 : 8>(
+        runs * part / S::kShare, runs * (part + 1) / S::kShare,
+        [&](int i, int j, float4 &x, float2 &ml) {
+            const int item = first + min(at0 + j * kThreads, count - 1);
+            const size_t row = (size_t)(item >> 6) * p.splits + i;
+            x = __ldcg(reinterpret_cast<const float4 *>(pa + row * 256) + (item & 63));
+            ml = __ldcg(reinterpret_cast<const float2 *>(pm + row * 2));
+        },
+        r);
+#pragma unroll
+    for (int j = 0; j < S::kPer; j++) {
+        join<S::kShare>(r[j]);
+        const int item = first + at0 + j * kThreads;
+        if (at0 + j * kThreads >= count || part != 0) continue;
+        if (staged) {
+            reinterpret_cast<float4 *>(staged)[item] = r[j].a;
+            if ((item & 63) == 0) reinterpret_cast<float2 *>(staged + 8 * 256)[item >> 6] = make_float2(r[j].m, r[j].l);
+        } else {
+            emit_item(p, slot, kvh, group, item, r[j]);
+        }
+    }
+}
+
+// Which rows a CTA works on.
+struct Work {
+    int slot, kvh, run;   // slot < 0: none; run: index of the partial (a cluster of kC CTAs shares one)
+    int runs;             // live runs of the head (what its fold reads); run >= runs: a run without rows
+    int row0, row1;       // this CTA's rows; row0 a multiple of 16
+    int unit;             // rows per unit of a warp: 16 while that gives every warp at most one, else 32
+    int len;              // live rows of the slot
+};
+
+__device__ __forceinline__ int div_up(int a, int b) { return (a + b - 1) / b; }
+
+// The balanced plan of one stream: every warp of every run gets a unit before any gets two, and units
+// are 16 rows as long as one each is enough (half the latency of a short step), then 32 (an eighth
+// fewer instructions per row).
+struct Balance {
+    int unit, runs;
+};
+__device__ __forceinline__ Balance balance(const DecodeParams &p, int len, int ctas, int most) {
+    const int cap = min(p.splits, p.run_cap), warps = kWarps * ctas;
+    Balance b;
+    b.unit = div_up(len, 16) <= cap * warps ? 16 : most;
+    b.runs = max(1, min(div_up(div_up(len, b.unit), warps), cap));
+    return b;
+}
+
+// One stream, or a column of one, of `len` live rows.
+template <int kC, int kUnitRows>
+__device__ __forceinline__ Work plan_stream(const DecodeParams &p, int slot, int rank, int len) {
+    Work w;
+    w.slot = slot;
+    w.len = len;
+    const int cluster = (int)blockIdx.x / kC;
+    if (!p.by_stride && p.run_cap > 0) {
+        const int cap = min(p.splits, p.run_cap);
+        const Balance b = balance(p, len, kC, kUnitRows);
+        w.kvh = cluster / cap;
+        w.run = cluster - w.kvh * cap;
+        w.runs = b.runs;
+        w.unit = b.unit;
+        w.row0 = w.row1 = 0;
+        if (w.run < w.runs) {
+            const int units = div_up(len, b.unit);
+            const int c0 = (int)((long long)w.run * units / w.runs), c1 = (int)((long long)(w.run + 1) * units / w.runs);
+            w.row0 = min((c0 + (c1 - c0) * rank / kC) * b.unit, len);
+            w.row1 = min((c0 + (c1 - c0) * (rank + 1) / kC) * b.unit, len);
+        }
+        return w;
+    }
+    // fixed runs of ceil(span / splits) rows, rounded up to 64
+    w.kvh = cluster / p.splits;
+    w.run = cluster - w.kvh * p.splits;
+    w.runs = p.splits;
+    const int span = p.by_stride ? p.stride : len;
+    const int per = div_up(div_up(span, p.splits), kTile) * kTile;
+    w.row0 = min(w.run * per, len);
+    w.row1 = min(w.row0 + per, len);
+    w.unit = w.row1 - w.row0 <= 16 * kWarps ? 16 : kUnitRows;
+    return w;
+}
+
+}  // namespace warp_body
+}  // namespace hipml

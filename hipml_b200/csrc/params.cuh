@@ -23,10 +23,10 @@ struct DecodeParams {
     int q4;               // 1: the cache is q4_0 (18-byte blocks), 0: q8_0
     int legacy_body = 0;  // q8_0 value side: 0 the process-wide default, 1 mma.sync (selector 7),
                           // 2 tcgen05 kind::i8 (selector 8)
-    int run_cap;          // tensor-core body, by_stride == 0: at most this many live runs per
-                          // KV head, balanced to within one 64-key tile (0: the reference's runs)
-    int share_slots;      // tensor-core body, several slots: the device's CTA slots, shared by
-                          // all slots in proportion to their live lengths (0: off)
+    int run_cap;          // tensor-core bodies, by_stride == 0: the device's CTA slots (two per SM) per
+                          // KV head: at most so many live runs, balanced (0: the reference's runs)
+    int share_slots;      // tensor-core bodies, several slots: the device's CTA slots (two per SM),
+                          // shared by all slots in proportion to their live lengths (0: off)
     int n_slots;          // set by launch_decode_tc
     // Optional fused append (tensor-core body, q8_0): the new K/V rows of every slot, f32
     // [n_kv][256] at k_row + slot * row_slot. The CTA whose run holds the append position
@@ -36,12 +36,12 @@ struct DecodeParams {
     unsigned char *kw = nullptr, *vw = nullptr;
     long long row_slot = 0;
     long long kv_slot_bytes, acc_slot, ml_slot, q_slot;
-    // Fold inside the split pass (tensor-core body). The CTA that completes a group of eight
-    // runs of a (slot, KV head) folds them into the group's first slot, and the CTA that
-    // completes the last group folds the groups and writes the output rows of the head group,
-    // so a decode step of a layer is one launch (a head with at most 30 runs is one group). The arrival counters live in library-owned
-    // device memory (region `arrive_region`, `arrive_stride` counters per (slot, KV head):
-    // one for the groups, then one per group) and return to zero by themselves.
+    // Fold inside the split pass (tensor-core bodies), so that a decode step of a layer is one launch:
+    // the CTA that arrives last at a counter folds the partials it stands for and writes their output.
+    // The counters live in library-owned device memory (region `arrive_region`, `arrive_stride` per
+    // (slot, KV head)) and return to zero by themselves. Default body: one counter per slice of the
+    // head group's outputs (a CTA of the cluster each). tcgen05 body: one for the groups of eight
+    // runs, then one per group (a head with at most 30 runs is one group).
     float *out = nullptr;            // nullptr: partials only, the caller launches the fold
     long long out_slot = 0, out_head_stride = 0;
     int normalize = 1;               // 0: out row = [acc (unnormalised) | max | sum]
@@ -143,9 +143,10 @@ int decode_plan_quota_host(const int *lens, int slots, int splits, int share_slo
 // Launches the split pass (the caller launches the reduce).
 int launch_decode_split(cudaStream_t stream, const DecodeParams &p, int slots, bool tensor_core);
 int launch_decode_tc(cudaStream_t stream, const DecodeParams &p, int slots);
-// The fold of the tensor-core split pass as a launch of its own (the same arithmetic, bit for
-// bit, as the fold inside the split pass): p.out and the fields after it say where it goes.
-int launch_decode_fold_tree(cudaStream_t stream, const DecodeParams &p, int slots);
+// The default body of the split pass (attn_decode_warps.cu); launch_decode_tc calls it.
+int launch_decode_warps(cudaStream_t stream, const DecodeParams &p, int slots);
+// The same for several columns of one cache; p as launch_decode_warps set it up for its own launch.
+int launch_decode_cols(cudaStream_t stream, const DecodeParams &p, int cols);
 // Arrival-counter region for a launch on `stream` (-1: none free, use the two-launch form);
 // `counters` = slots * n_kv * arrive_stride must fit a region.
 int decode_arrive_region(cudaStream_t stream, long long counters);
@@ -156,6 +157,7 @@ constexpr int kFoldFlat = 30;          // up to this many runs a head is folded 
 __host__ __device__ __forceinline__ int fold_group_of(int runs) {
     return runs <= kFoldFlat ? 32 : kFoldGroup;
 }
+constexpr int kArriveRegions = 128;
 constexpr int kArriveRegionInts = 4096;
 // Fold of (acc, max, sum) triples over the split axis; all strides in floats.
 struct FoldParams {

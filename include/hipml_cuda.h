@@ -172,11 +172,10 @@ int hipml_kv_append_chunk_f32(hipml_stream_t stream, float *k_cache, float *v_ca
  * attn_decode_kv_reduce, launch_kv.rs:232-279) with split s over positions [s*per, (s+1)*per),
  * per = ceil(seq/splits). The scalar kernel (selector 6, or any head_dim other than 256) keeps
  * exactly that and fills every slot. The tensor-core kernel is ONE launch and deals the rows
- * out for this device instead: R = max(1, min(splits, ceil(seq/64), CTA slots / n_kv)) runs
- * per KV head, balanced to within one 64-row tile, partial of run r in slot r; slots from R up
- * to min(splits, CTA slots / n_kv) receive neutral partials (max -inf, sum 0), slots past that
- * are not written at all; the CTA that completes a group of eight runs folds it into the
- * group's first slot, and the last CTA of a KV head folds the groups and writes `out`. A
+ * out for this device instead: at most R = min(splits, the device's pairs of SMs / n_kv) runs per
+ * KV head, only as many as the live rows can occupy, partial of run r in slot r; of the other slots
+ * those below R and the first 32 receive neutral partials (max -inf, sum 0), the rest are not
+ * written. The last CTA to finish a part of a KV head's outputs folds the runs into `out`. A
  * caller must therefore not point the by-name attn_decode_kv_reduce kernel at these partials.
  * The tensor-core kernel needs out, part_acc (16 bytes) and part_ml (8 bytes) aligned. Two
  * calls that may overlap on the device must not share scratch (as in the reference); the
@@ -236,8 +235,8 @@ int hipml_attn_decode_kv_gated(hipml_stream_t stream, const int *step, int selec
  * step[0], then hipml_attn_decode_kv over the step[1] live rows (the reference makes the two
  * launches kv_encode_ptr_on + launch_ptrs, crates/hipml-model/src/gpu/attn_tile.rs:150-224).
  * step[0] must be step[1] - 1 (device status 22 otherwise). With selector 0 / 1 / 4, head_dim 256
- * and 16-byte aligned rows and caches the append happens inside the split pass -- the CTA
- * whose run ends the sequence quantises the row into its tile and stores it to the cache,
+ * and 16-byte aligned rows and caches the append happens inside the split pass -- the warp
+ * whose rows end the sequence quantises the row for itself and stores it to the cache,
  * bit-identical to hipml_kv_encode -- otherwise the two launches are made here. `gate` is
  * optional (NULL: none) and applied as in hipml_attn_decode_kv_gated. */
 int hipml_attn_decode_kv_append(hipml_stream_t stream, const int *step, int selector,
@@ -459,7 +458,8 @@ int hipml_attn_chunk_staged_gated(hipml_stream_t stream, const float *q, float *
  * small caches. hipml_set_decode_fold_mode: 0 (default) folds inside the split pass, 1 makes
  * the fold a second launch with the same arithmetic (bit-identical output).
  * hipml_decode_plan_quota: host restatement of the multi-slot plan, for tests -- the 64-row
- * tiles per run that the kernel derives from the live lengths `lens[slots]`; the plan's runs,
+ * tiles per run that a kernel with `cta_slots` CTAs derives from the live lengths `lens[slots]`
+ * (cta_slots, or half of it where the kernel runs one CTA per SM); the plan's runs,
  * sum over slots of max(1, ceil(ceil(len/64) / quota)) * n_kv, never exceed cta_slots.
  * Returns -1 for arguments outside the plan's domain (cta_slots < 2 * slots * n_kv). */
 int hipml_set_decode_cta_slots(int slots);
