@@ -6,9 +6,16 @@
 // (split pass + reduce) and kv_append_cols_f32.hip:11-31; launcher
 // crates/hipml-kernels/src/attn_gpu/imp/attn_cols.rs:15-173. The key axis is cut into
 // `splits` runs of `per = ceil(n_ctx / splits)` rows fixed in cache positions, so a column's
-// arithmetic does not depend on how many columns share the launch. This is the `--kv f32`
-// path of the reference: plain f32, one warp per (query head, run, column).
-#include "params.cuh"
+// arithmetic does not depend on how many columns share the launch. This is the `--kv f32` path of the
+// reference: plain f32 products and sums on the CUDA cores.
+//
+// head_dim 256: attn_decode_rows_f32, a CTA per (run, KV head, column). Bound by the HBM stream of the
+// rows (16.8 MB per layer at 2,048 rows) once latency is hidden; the arithmetic is 1.5 FMA per byte. So a
+// warp reads a row once for all heads of the group (one warp per head read it six times), four rows at
+// a time with all loads in flight; the four rows' dot products are summed over the lanes by one
+// reduce-scatter (25 shuffles for 24 sums, where a butterfly each took 120). Other head sizes:
+// attn_decode_cols_f32, one warp per (query head, run, column).
+#include "decode_warp_body.cuh"
 
 namespace hipml {
 
@@ -26,6 +33,198 @@ struct ColsParams {
 
 namespace {
 
+using namespace warp_body;
+
+constexpr int kF32Cluster = 8;     // CTAs (runs) per cluster, folded through distributed shared memory
+constexpr int kRowsAtOnce = 4;
+constexpr int kOffMlF32 = kWarps * 8 * kHeadPitch * 4;             // after the warps' partials: [8 heads][warp]
+constexpr int kOffPartF32 = kOffMlF32 + kWarps * 8 * 8;            // the CTA's partial [8 heads][256]
+constexpr int kOffCmlF32 = kOffPartF32 + 8 * 256 * 4;              // [8 heads]
+constexpr int kSmemF32 = kOffCmlF32 + 8 * 8;
+
+__device__ int g_arrive_f32[kArriveRegions * kArriveRegionInts];
+
+// Sums v[row][head] over the 32 lanes; lane 8 * row + head returns its own sum.
+template <int kHeads>
+__device__ __forceinline__ float reduce_scatter(const float (&v)[kRowsAtOnce][kHeads], int lane) {
+    float a[2][kHeads], b[8];
+#pragma unroll
+    for (int h = 0; h < kHeads; h++) {
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            const float keep = (lane & 16) ? v[2 + r][h] : v[r][h], give = (lane & 16) ? v[r][h] : v[2 + r][h];
+            a[r][h] = keep + __shfl_xor_sync(0xffffffffu, give, 16);
+        }
+        const float keep = (lane & 8) ? a[1][h] : a[0][h], give = (lane & 8) ? a[0][h] : a[1][h];
+        b[h] = keep + __shfl_xor_sync(0xffffffffu, give, 8);
+    }
+#pragma unroll
+    for (int h = kHeads; h < 8; h++) b[h] = 0.0f;
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+        for (int h = 0; h < o; h++) {
+            const float keep = (lane & o) ? b[o + h] : b[h], give = (lane & o) ? b[h] : b[o + h];
+            b[h] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+    return b[0];
+}
+
+// grid (n_kv * clusters * 8, columns), clusters of 8. d: out, scratch and counters (as the quantised body's).
+template <int kHeads>
+__global__ void __launch_bounds__(kThreads, 2) attn_decode_rows_f32(ColsParams p, DecodeParams d, int clusters) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ __align__(16) float s_q[8 * 256];
+    __shared__ __align__(16) float s_w[kWarps][8][kRowsAtOnce];
+    __shared__ int s_last;
+    griddep_launch();
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int rank = (int)cluster_rank(), cluster = (int)blockIdx.x / kF32Cluster;
+    const int kvh = cluster / clusters, in_head = cluster - kvh * clusters, col = blockIdx.y;
+    const int group = p.n_heads / p.n_kv, width = p.n_kv * 256, seq = p.pos0 + col + 1;
+    // this warp's share of the run, fixed in cache positions, cut at the column's last row
+    const int run = in_head * kF32Cluster + rank;
+    const int run0 = run * p.per, run_rows = run < p.splits ? p.per : 0;
+    const int lo = min(run0 + run_rows * warp / kWarps, seq), hi = min(run0 + run_rows * (warp + 1) / kWarps, seq);
+    const float *const kb = p.k + (size_t)kvh * 256, *const vb = p.v + (size_t)kvh * 256;
+    // (asks L2 only; the rows are read once the grids ahead are done)
+    for (int i = lane; i < 2 * (hi - lo); i += 32)
+        prefetch_l2(((i & 1) ? vb : kb) + (size_t)(lo + (i >> 1)) * width, 1024);
+    griddep_wait();
+    for (int i = tid; i < 8 * 64; i += kThreads) {
+        float4 x = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (i < group * 64)
+            x = reinterpret_cast<const float4 *>(p.q + ((size_t)col * p.n_heads + kvh * group) * 256)[i];
+        x.x *= p.scale_log2;
+        x.y *= p.scale_log2;
+        x.z *= p.scale_log2;
+        x.w *= p.scale_log2;
+        reinterpret_cast<float4 *>(s_q)[i] = x;
+    }
+    __syncthreads();
+
+    // lane: dims 4 * lane .. + 3 and 128 + 4 * lane .. + 3
+    float acc[kHeads][8];
+#pragma unroll
+    for (int h = 0; h < kHeads; h++)
+#pragma unroll
+        for (int e = 0; e < 8; e++) acc[h][e] = 0.0f;
+    float m = -INFINITY, l = 0.0f;   // lane 8 * row + head: the head's maximum, the sum over rows = row (mod 4)
+    for (int r0 = lo; r0 < hi; r0 += kRowsAtOnce) {
+        float4 k[kRowsAtOnce][2], v[kRowsAtOnce][2];
+#pragma unroll
+        for (int r = 0; r < kRowsAtOnce; r++) {
+            const size_t at = (size_t)min(r0 + r, hi - 1) * width + 4 * lane;
+            k[r][0] = *reinterpret_cast<const float4 *>(kb + at);
+            k[r][1] = *reinterpret_cast<const float4 *>(kb + at + 128);
+            v[r][0] = *reinterpret_cast<const float4 *>(vb + at);
+            v[r][1] = *reinterpret_cast<const float4 *>(vb + at + 128);
+        }
+        float s[kRowsAtOnce][kHeads];
+#pragma unroll
+        for (int h = 0; h < kHeads; h++) {
+            const float4 q0 = *reinterpret_cast<const float4 *>(s_q + h * 256 + 4 * lane);
+            const float4 q1 = *reinterpret_cast<const float4 *>(s_q + h * 256 + 128 + 4 * lane);
+#pragma unroll
+            for (int r = 0; r < kRowsAtOnce; r++) {
+                float x = q0.x * k[r][0].x;
+                x = fmaf(q0.y, k[r][0].y, x);
+                x = fmaf(q0.z, k[r][0].z, x);
+                x = fmaf(q0.w, k[r][0].w, x);
+                x = fmaf(q1.x, k[r][1].x, x);
+                x = fmaf(q1.y, k[r][1].y, x);
+                x = fmaf(q1.z, k[r][1].z, x);
+                s[r][h] = fmaf(q1.w, k[r][1].w, x);
+            }
+        }
+        float score = reduce_scatter<kHeads>(s, lane);
+        if (r0 + (lane >> 3) >= hi) score = -INFINITY;
+        float top = fmaxf(score, __shfl_xor_sync(0xffffffffu, score, 8));
+        top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 16));
+        const float m_new = fmaxf(m, top);
+        if (__any_sync(0xffffffffu, m_new > m)) {
+            const float corr = ex2(m - m_new);
+            l *= corr;
+            m = m_new;
+#pragma unroll
+            for (int h = 0; h < kHeads; h++) {
+                const float c = __shfl_sync(0xffffffffu, corr, h);
+#pragma unroll
+                for (int e = 0; e < 8; e++) acc[h][e] *= c;
+            }
+        }
+        const float w = ex2(score - m);
+        l += w;
+        s_w[warp][lane & 7][lane >> 3] = w;
+        __syncwarp();
+#pragma unroll
+        for (int h = 0; h < kHeads; h++) {
+            const float4 wh = *reinterpret_cast<const float4 *>(s_w[warp][h]);
+            const float wr[4] = {wh.x, wh.y, wh.z, wh.w};
+#pragma unroll
+            for (int r = 0; r < kRowsAtOnce; r++) {
+                acc[h][0] = fmaf(wr[r], v[r][0].x, acc[h][0]);
+                acc[h][1] = fmaf(wr[r], v[r][0].y, acc[h][1]);
+                acc[h][2] = fmaf(wr[r], v[r][0].z, acc[h][2]);
+                acc[h][3] = fmaf(wr[r], v[r][0].w, acc[h][3]);
+                acc[h][4] = fmaf(wr[r], v[r][1].x, acc[h][4]);
+                acc[h][5] = fmaf(wr[r], v[r][1].y, acc[h][5]);
+                acc[h][6] = fmaf(wr[r], v[r][1].z, acc[h][6]);
+                acc[h][7] = fmaf(wr[r], v[r][1].w, acc[h][7]);
+            }
+        }
+        __syncwarp();
+    }
+
+    // ---- merge: the warps, the cluster, then the head's clusters (the last to arrive)
+    l += __shfl_xor_sync(0xffffffffu, l, 8);
+    l += __shfl_xor_sync(0xffffffffu, l, 16);
+    float2 *const wml = reinterpret_cast<float2 *>(smem + kOffMlF32);
+    if (lane < 8) wml[lane * kWarps + warp] = make_float2(m, l);
+    float *const mine = reinterpret_cast<float *>(smem) + warp * 8 * kHeadPitch;
+#pragma unroll
+    for (int h = 0; h < kHeads; h++) {
+        *reinterpret_cast<float4 *>(mine + h * kHeadPitch + 4 * lane) = make_float4(acc[h][0], acc[h][1], acc[h][2], acc[h][3]);
+        *reinterpret_cast<float4 *>(mine + h * kHeadPitch + 128 + 4 * lane) =
+            make_float4(acc[h][4], acc[h][5], acc[h][6], acc[h][7]);
+    }
+    __syncthreads();
+    const int items = group * 64;
+    float4 *const cpart = reinterpret_cast<float4 *>(smem + kOffPartF32);
+    float2 *const cml = reinterpret_cast<float2 *>(smem + kOffCmlF32);
+    fold_warps(smem, 8 * kHeadPitch * 4, wml, items, [&](int item, const Part &r) {
+        cpart[item] = r.a;
+        if ((item & 63) == 0) cml[item >> 6] = make_float2(r.m, r.l);
+    });
+    cluster_sync_all();
+    const bool one = clusters == 1 && d.out != nullptr;
+    fold_cluster<kF32Cluster>(cpart, cml, items, rank, [&](int item, const Part &r) {
+        if (one) {
+            emit_item(d, col, kvh, group, item, r);
+            return;
+        }
+        const size_t row = (size_t)(kvh * group + (item >> 6)) * d.splits + in_head;
+        reinterpret_cast<float4 *>(d.part_acc + (size_t)col * d.acc_slot + row * 256)[item & 63] = r.a;
+        if ((item & 63) == 0)
+            *reinterpret_cast<float2 *>(d.part_ml + (size_t)col * d.ml_slot + row * 2) = make_float2(r.m, r.l);
+    });
+    cluster_arrive();   // no CTA may leave while another still reads its partial
+    if (d.out != nullptr && !one) {
+        int *const ctr = g_arrive_f32 + (size_t)d.arrive_region * kArriveRegionInts +
+                         (size_t)(col * p.n_kv + kvh) * kF32Cluster + rank;
+        __syncthreads();
+        if (tid == 0) {
+            const int last = arrive_acq_rel(ctr) == clusters - 1;
+            if (last) *ctr = 0;
+            s_last = last;
+        }
+        __syncthreads();
+        if (s_last) fold_runs<kF32Cluster>(d, col, kvh, group, clusters, rank, nullptr);
+    }
+    cluster_wait();
+}
+
+// One warp per (query head, run, column), any head size.
 __global__ void __launch_bounds__(128) attn_decode_cols_f32(ColsParams p) {
     griddep_launch();
     griddep_wait();
@@ -103,6 +302,65 @@ const void *lookup_cols_kernel(const char *name) {
     return nullptr;
 }
 
+namespace {
+
+template <int kHeads>
+int launch_rows_f32_heads(cudaStream_t stream, const ColsParams &p, const DecodeParams &d, int clusters) {
+    static bool configured[64] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64 || !configured[dev]) {
+        const cudaError_t e =
+            cudaFuncSetAttribute(attn_decode_rows_f32<kHeads>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemF32);
+        if (e != cudaSuccess) return (int)e;
+        if (dev >= 0 && dev < 64) configured[dev] = true;
+    }
+    return launch_pdl(attn_decode_rows_f32<kHeads>, dim3(p.n_kv * clusters * kF32Cluster, p.rows), dim3(kThreads),
+                      (size_t)kSmemF32, stream, kF32Cluster, p, d, clusters);
+}
+
+int launch_rows_f32(cudaStream_t stream, const ColsParams &p, float *out, long long acc_slot, long long ml_slot,
+                    long long out_slot) {
+    const int clusters = (p.splits + kF32Cluster - 1) / kF32Cluster;
+    DecodeParams d = {};
+    d.part_acc = p.part_acc;
+    d.part_ml = p.part_ml;
+    d.n_heads = p.n_heads;
+    d.n_kv = p.n_kv;
+    d.head_dim = 256;
+    d.splits = p.splits;
+    d.acc_slot = acc_slot;
+    d.ml_slot = ml_slot;
+    d.out = out;
+    d.out_slot = out_slot;
+    d.out_head_stride = 256;
+    d.normalize = 1;
+    d.arrive_region = decode_arrive_region(stream, (long long)p.rows * p.n_kv * kF32Cluster);
+    const bool second_launch = d.arrive_region < 0;
+    if (second_launch) d.out = nullptr;
+    const int rc = p.n_heads / p.n_kv <= 6 ? launch_rows_f32_heads<6>(stream, p, d, clusters)
+                                           : launch_rows_f32_heads<8>(stream, p, d, clusters);
+    if (rc != 0 || !second_launch) return rc;
+    FoldParams f = {};
+    f.acc = p.part_acc;
+    f.ml = p.part_ml;
+    f.out = out;
+    f.head_dim = 256;
+    f.splits = clusters;
+    f.acc_head_stride = (long long)p.splits * 256;
+    f.acc_split_stride = 256;
+    f.ml_head_stride = (long long)p.splits * 2;
+    f.ml_split_stride = 2;
+    f.acc_slot = acc_slot;
+    f.ml_slot = ml_slot;
+    f.out_slot = out_slot;
+    f.out_head_stride = 256;
+    f.normalize = 1;
+    return launch_decode_fold(stream, f, p.n_heads, p.rows);
+}
+
+}  // namespace
+
 int launch_decode_cols_f32(cudaStream_t stream, const float *q, const float *k, const float *v,
                            float *part_acc, float *part_ml, float *out, int n_heads, int n_kv,
                            int head_dim, int n_ctx, int pos0, int rows, int splits) {
@@ -120,12 +378,17 @@ int launch_decode_cols_f32(cudaStream_t stream, const float *q, const float *k, 
     p.scale_log2 = (1.0f / sqrtf((float)head_dim)) * 1.4426950408889634f;
     p.splits = splits;
     p.per = (n_ctx + splits - 1) / splits;
+    const long long acc_slot = (long long)n_heads * splits * head_dim, ml_slot = (long long)n_heads * splits * 2;
+    const long long out_slot = (long long)n_heads * head_dim;
+    const size_t align = reinterpret_cast<size_t>(q) | reinterpret_cast<size_t>(k) | reinterpret_cast<size_t>(v) |
+                         reinterpret_cast<size_t>(part_acc) | reinterpret_cast<size_t>(out);
+    if (head_dim == 256 && (align & 15) == 0 && (reinterpret_cast<size_t>(part_ml) & 7) == 0)
+        return launch_rows_f32(stream, p, out, acc_slot, ml_slot, out_slot);
     dim3 grid((n_heads * splits + 3) / 4, rows);
     if (int e = launch_pdl(attn_decode_cols_f32, grid, dim3(128), 0, stream, 1, p)) return e;
     if (int e = launch_status()) return e;
-    return launch_decode_reduce(stream, part_acc, part_ml, out, n_heads, head_dim, splits, rows,
-                                (long long)n_heads * splits * head_dim,
-                                (long long)n_heads * splits * 2, (long long)n_heads * head_dim);
+    return launch_decode_reduce(stream, part_acc, part_ml, out, n_heads, head_dim, splits, rows, acc_slot, ml_slot,
+                                out_slot);
 }
 
 }  // namespace hipml

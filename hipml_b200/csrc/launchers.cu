@@ -115,8 +115,8 @@ int hipml_kv_append_f32(hipml_stream_t stream, const int *step, float *k_cache, 
                         const float *k_row, const float *v_row, int width) {
     if (width <= 0) return fail(HIPML_ERR_INVALID_ARGUMENT, "width %d must be positive", width);
     void *args[] = {&k_cache, &v_cache, &k_row, &v_row, &step, &width};
-    return (int)cudaLaunchKernel(lookup_kv_kernel("kv_append_f32"), dim3((2 * width + 255) / 256),
-                                 dim3(256), args, 0, as_stream(stream));
+    return launch_pdl_args(lookup_kv_kernel("kv_append_f32"), dim3((2 * width + 255) / 256), dim3(256), args, 0,
+                           as_stream(stream));
 }
 
 int hipml_kv_append_chunk_f32(hipml_stream_t stream, float *k_cache, float *v_cache,
@@ -129,8 +129,8 @@ int hipml_kv_append_chunk_f32(hipml_stream_t stream, float *k_cache, float *v_ca
     if (blocks < 1) blocks = 1;
     if (blocks > 148 * 16) blocks = 148 * 16;
     void *args[] = {&k_cache, &v_cache, &k, &v, &pos0, &width, &tokens};
-    return (int)cudaLaunchKernel(lookup_kv_kernel("kv_append_chunk_f32"), dim3((unsigned)blocks),
-                                 dim3(256), args, 0, as_stream(stream));
+    return launch_pdl_args(lookup_kv_kernel("kv_append_chunk_f32"), dim3((unsigned)blocks), dim3(256), args, 0,
+                           as_stream(stream));
 }
 
 // Peer-memory exchange that replaces the plain fold (hipml_attn_decode_kv_shard_exchange).
@@ -755,9 +755,8 @@ int hipml_kv_append_cols_f32(hipml_stream_t stream, float *k_cache, float *v_cac
     if (rows == 0) return 0;
     const long long n = 2LL * width * rows;
     void *args[] = {&k_cache, &v_cache, &k, &v, &pos0, &rows, &width};
-    return (int)cudaLaunchKernel(lookup_cols_kernel("kv_append_cols_f32"),
-                                 dim3((unsigned)((n + 255) / 256)), dim3(256), args, 0,
-                                 as_stream(stream));
+    return launch_pdl_args(lookup_cols_kernel("kv_append_cols_f32"), dim3((unsigned)((n + 255) / 256)), dim3(256), args,
+                           0, as_stream(stream));
 }
 
 // ---- attention front end and tail --------------------------------------------------------

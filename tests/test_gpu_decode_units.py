@@ -95,3 +95,28 @@ def test_columns_side_by_side_give_each_columns_own_bits(pos0, cols):
         api.attn_decode_kv(step, q[c], kc, vc, acc, ml, one, heads, n_kv, hd, stride, scale, splits)
         assert torch.equal(one, out[c]), f"column {c}"
     assert api.check_device_status() == 0
+
+
+@pytest.mark.parametrize("heads,n_kv", [(24, 4), (8, 1), (2, 2)])
+@pytest.mark.parametrize("n_ctx,pos0,rows", [(1, 0, 1), (33, 31, 2), (260, 250, 3), (2100, 2090, 8), (8200, 8199, 1),
+                                             (8200, 3, 2)])
+def test_f32_cache_decode_at_the_edges_of_runs(heads, n_kv, n_ctx, pos0, rows):
+    """head_dim 256: runs of ceil(n_ctx / splits) rows, eight warps per run, eight runs per cluster."""
+    from hipml_b200 import api
+    hd = 256
+    gen = torch.Generator(device="cuda").manual_seed(n_ctx + rows)
+    k, v = (torch.full((n_ctx, n_kv * hd), float("nan"), device="cuda") for _ in range(2))
+    live = pos0 + rows
+    k[:live] = torch.randn(live, n_kv * hd, device="cuda", generator=gen)
+    v[:live] = torch.randn(live, n_kv * hd, device="cuda", generator=gen)
+    q = torch.randn(rows, heads * hd, device="cuda", generator=gen)
+    splits = api.cols_splits(n_ctx)
+    acc, ml = (torch.full((rows * heads * splits * n,), float("nan"), device="cuda") for n in (hd, 2))
+    out = torch.full((rows, heads * hd), float("nan"), device="cuda")
+    for _ in range(2):
+        api.attn_decode_cols_f32(q, k, v, acc, ml, out, heads, n_kv, hd, n_ctx, pos0, rows)
+    kn, vn, qn = k.cpu().numpy(), v.cpu().numpy(), q.cpu().numpy()
+    for c in range(rows):
+        seq = pos0 + c + 1
+        want = O.attn_causal_f32(qn[c], kn[:seq], vn[:seq], heads, n_kv, hd, seq, 0.0625)
+        assert O.max_abs(want, out[c].cpu().numpy()) <= 5e-6 and O.rel_l2(want, out[c].cpu().numpy()) <= 5e-6
