@@ -8,9 +8,10 @@
 // launch shapes (a launch by name with the reference's argument array works unchanged) around
 // bodies of this file's own; attn_front_rows_q8 is the form this library's own launchers use.
 //
-// attn_front_rows_q8: one CTA of 8 warps per token. The rotation angles depend on the
+// attn_front_rows_q8: a CTA of 8 warps per token, or several where tokens are few. The rotation angles depend on the
 // position and the channel pair only, so the CTA computes the n_rot/2 (cos, sin) pairs once
-// (f64 pow and sincos, as the definition does) and all heads share them. A warp owns a
+// (f64 sincos over f64 frequencies, as the definition does) and all its heads share them; where the
+// launch carries the positions it does so before the grid dependency resolves. A warp owns a
 // whole 256-wide head row: 8 values per lane (two 16-byte loads), the sum of squares by
 // shuffles, the rotation partner (channel +- n_rot/2) in the lane n_rot/16 away. The K row
 // leaves as a q8_0 cache row straight from the normalised, rotated registers and the V row
@@ -206,6 +207,7 @@ struct FrontRowsParams {
     int n_heads, n_kv, stride, pos0, tokens;
     RopeSpec rope;
     float eps;
+    double freq[kMaxHeadDim / 2];   // theta^(-2c / n_rot) of every channel pair
 };
 
 __device__ __forceinline__ void load8(const float *p, float (&x)[8]) {
@@ -243,39 +245,57 @@ __device__ __forceinline__ void norm_rope_lane8(float (&x)[8], const float *w, i
     }
 }
 
-// grid (tokens), block 256.
-__global__ void __launch_bounds__(256) attn_front_rows_q8(FrontRowsParams p) {
+// grid (tokens, row groups), block 256: CTA (t, y) takes head rows y * 8 + warp, + 8 * groups, ... of token t.
+__global__ void __launch_bounds__(256) attn_front_rows_q8(const __grid_constant__ FrontRowsParams p) {
     __shared__ float cs[kMaxHeadDim / 2], sn[kMaxHeadDim / 2];
     __shared__ __align__(16) unsigned char img[8][kMaxRowBytes];
     griddep_launch();
-    griddep_wait();   // positions and rows may come from a grid that is still running
     const int t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    int p4[4];
-    if (p.pos4) {
-        p4[0] = p.pos4[0]; p4[1] = p.pos4[1]; p4[2] = p.pos4[2]; p4[3] = p.pos4[3];
-    } else {
-        p4[0] = p4[1] = p4[2] = p4[3] = p.pos0 + t;
+    auto angles = [&](const int (&p4)[4]) {
+        for (int c = threadIdx.x; c < p.rope.n_rot >> 1; c += blockDim.x) {
+            double s, co;
+            sincos((double)rope_pos(p.rope, c, p4) * p.freq[c], &s, &co);
+            cs[c] = (float)co;
+            sn[c] = (float)s;
+        }
+    };
+    if (!p.pos4) {
+        // positions that the launch carries: the angles need not wait for the grids ahead
+        const int p4[4] = {p.pos0 + t, p.pos0 + t, p.pos0 + t, p.pos0 + t};
+        angles(p4);
     }
-    const int half = p.rope.n_rot >> 1;
-    for (int c = threadIdx.x; c < half; c += blockDim.x) rope_angle(p.rope, c, p4, cs[c], sn[c]);
-    __syncthreads();
-    const int cache_row = p.step ? p.step[0] : p.pos0 + t;
-    const int rows = p.n_heads + 2 * p.n_kv;
-    for (int r = warp; r < rows; r += 8) {
-        float x[8];
+    griddep_wait();   // positions and rows may come from a grid that is still running
+    const int rows = p.n_heads + 2 * p.n_kv, hop = 8 * gridDim.y;
+    float x[8], g[8];   // the row at hand (and the gate half of a query row)
+    auto load_row = [&](int r) {
         if (r < p.n_heads) {
             const float *src = p.qg + ((size_t)t * p.n_heads + r) * 512;
-            float g[8];
             load8(src + 8 * lane, x);
             load8(src + 256 + 8 * lane, g);
+        } else if (r < rows) {
+            const bool is_k = r < p.n_heads + p.n_kv;
+            const int h = is_k ? r - p.n_heads : r - p.n_heads - p.n_kv;
+            load8((is_k ? p.k : p.v) + ((size_t)t * p.n_kv + h) * 256 + 8 * lane, x);
+        }
+    };
+    int r = blockIdx.y * 8 + warp;
+    load_row(r);
+    const int cache_row = p.step ? p.step[0] : p.pos0 + t;
+    if (p.pos4) {
+        const int p4[4] = {p.pos4[0], p.pos4[1], p.pos4[2], p.pos4[3]};
+        angles(p4);
+    }
+    __syncthreads();
+    for (; r < rows; r += hop) {
+        if (r < p.n_heads) {
             store8(p.gate + ((size_t)t * p.n_heads + r) * 256 + 8 * lane, g);
             norm_rope_lane8(x, p.q_norm, lane, p.rope.n_rot, p.eps, cs, sn);
             store8(p.q + ((size_t)t * p.n_heads + r) * 256 + 8 * lane, x);
+            load_row(r + hop);
             continue;
         }
         const bool is_k = r < p.n_heads + p.n_kv;
         const int h = is_k ? r - p.n_heads : r - p.n_heads - p.n_kv;
-        load8((is_k ? p.k : p.v) + ((size_t)t * p.n_kv + h) * 256 + 8 * lane, x);
         if (is_k) {
             norm_rope_lane8(x, p.k_norm, lane, p.rope.n_rot, p.eps, cs, sn);
             if (p.k_out) store8(p.k_out + ((size_t)t * p.n_kv + h) * 256 + 8 * lane, x);
@@ -289,7 +309,22 @@ __global__ void __launch_bounds__(256) attn_front_rows_q8(FrontRowsParams p) {
                       32);
             __syncwarp();
         }
+        load_row(r + hop);
     }
+}
+
+// The pairs' frequencies, in f64 as the definition computes them; they depend on the model only, so a
+// thread keeps the last model's (32 pow calls are ~2 us of host time, and were ~3 us of every kernel).
+void rope_freqs(float theta_base, int n_rot, double (&freq)[kMaxHeadDim / 2]) {
+    thread_local float last_theta = 0.0f;
+    thread_local int last_rot = -1;
+    thread_local double table[kMaxHeadDim / 2];
+    if (last_rot != n_rot || !(last_theta == theta_base)) {
+        for (int c = 0; c < n_rot / 2; c++) table[c] = pow((double)theta_base, -2.0 * (double)c / (double)n_rot);
+        last_theta = theta_base;
+        last_rot = n_rot;
+    }
+    for (int c = 0; c < n_rot / 2; c++) freq[c] = table[c];
 }
 
 }  // namespace
@@ -349,7 +384,13 @@ int launch_front_rows_q8(cudaStream_t stream, const float *qg, const float *k, c
     p.rope.s3 = sections ? sections[3] : 0;
     p.rope.theta_base = theta_base;
     p.eps = eps;
-    return launch_pdl(attn_front_rows_q8, dim3(tokens), dim3(256), 0, stream, 1, p);
+    rope_freqs(theta_base, n_rot, p.freq);
+    // A head row per warp while that leaves SMs free (one token of 24 + 8 rows took 9.0 us in one CTA, 4 in
+    // four); two CTAs per token beyond, where the angles' cost shows (2,048 tokens: 41.3 us with two, 45.1
+    // with four; 700 tokens: 17.1 us with two, 19.8 with one).
+    const int all = (n_heads + 2 * n_kv + 7) / 8;
+    const int groups = tokens <= 2 * 148 ? all : (all < 2 ? all : 2);
+    return launch_pdl(attn_front_rows_q8, dim3(tokens, groups), dim3(256), 0, stream, 1, p);
 }
 
 }  // namespace hipml
