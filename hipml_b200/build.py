@@ -24,6 +24,7 @@ SOURCES = [
     "decode_exchange.cu",
     "attn_front.cu",
     "attn_chunk_scalar.cu",
+    "attn_chunk_small.cu",
     "attn_chunk_tc.cu",
     "launchers.cu",
 ]

@@ -188,22 +188,45 @@ __global__ void __launch_bounds__(256) attn_chunk_combine_256(const float *__res
     if (pair >= (long long)tokens * n_heads) return;
     const int t = (int)(pair / n_heads), h = (int)(pair - (long long)t * n_heads);
     const int d4 = threadIdx.x & 63;
-    float big = -INFINITY;
-    for (int s = 0; s < splits; s++) {
-        const float2 ml = *reinterpret_cast<const float2 *>(
-            part_ml + (((size_t)s * qslots + t) * n_heads + h) * 2);
-        if (ml.y > 0.0f) big = fmaxf(big, ml.x);
-    }
+    // eight slices at a time with all their loads in flight (one dependent load after the other, 8 slices
+    // of a 2,048-token chunk took 281 us = 1.6 TB/s); an empty slice carries sum 0 and weighs nothing
+    constexpr int kBatch = 8;
+    float big = -INFINITY, den = 0.0f;
     float4 num = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    float den = 0.0f;
-    for (int s = 0; s < splits; s++) {
-        const size_t slot = ((size_t)s * qslots + t) * n_heads + h;
-        const float2 ml = *reinterpret_cast<const float2 *>(part_ml + slot * 2);
-        if (!(ml.y > 0.0f)) continue;
-        const float w = exp2f(ml.x - big);
-        const float4 a = __ldg(reinterpret_cast<const float4 *>(part_acc + slot * 256) + d4);
-        num.x += a.x * w; num.y += a.y * w; num.z += a.z * w; num.w += a.w * w;
-        den += ml.y * w;
+    for (int s0 = 0; s0 < splits; s0 += kBatch) {
+        float2 ml[kBatch];
+        float4 a[kBatch];
+#pragma unroll
+        for (int i = 0; i < kBatch; i++) {
+            ml[i] = make_float2(0.0f, 0.0f);
+            a[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (s0 + i < splits) {
+                const size_t slot = ((size_t)(s0 + i) * qslots + t) * n_heads + h;
+                ml[i] = __ldg(reinterpret_cast<const float2 *>(part_ml + slot * 2));
+                a[i] = __ldcs(reinterpret_cast<const float4 *>(part_acc + slot * 256) + d4);
+            }
+        }
+        float top = big;
+#pragma unroll
+        for (int i = 0; i < kBatch; i++)
+            if (ml[i].y > 0.0f) top = fmaxf(top, ml[i].x);
+        const float corr = big == -INFINITY ? 0.0f : exp2f(big - top);
+        num.x *= corr;
+        num.y *= corr;
+        num.z *= corr;
+        num.w *= corr;
+        den *= corr;
+        big = top;
+#pragma unroll
+        for (int i = 0; i < kBatch; i++) {
+            if (!(ml[i].y > 0.0f)) continue;
+            const float w = exp2f(ml[i].x - big);
+            num.x = fmaf(a[i].x, w, num.x);
+            num.y = fmaf(a[i].y, w, num.y);
+            num.z = fmaf(a[i].z, w, num.z);
+            num.w = fmaf(a[i].w, w, num.w);
+            den = fmaf(ml[i].y, w, den);
+        }
     }
     const bool ok = den > 0.0f;
     float4 o = make_float4(ok ? num.x / den : 0.0f, ok ? num.y / den : 0.0f,

@@ -53,6 +53,8 @@
 // wait observes, and the CTA falls through to its teardown (TMEM is always released).
 #include <cuda.h>
 
+#include <atomic>
+
 #include "params.cuh"
 #include "q8_pack.cuh"
 #include "sm100_ptx.cuh"
@@ -72,7 +74,8 @@ struct ChunkTcParams {
     float scale_log2;
     int splits, qslots;
     int single_pass;   // 1: hi*hi only
-    const float *gate; // optional [tokens][n_heads*256]: out *= sigmoid(gate) (one-pass form only)
+    const float *gate; // optional [tokens][n_heads*256]: out *= sigmoid(gate) (not with splits >= 2)
+    int fold;          // >= 2: key slices of a tile, folded inside their cluster (splits < 2 then)
 };
 
 namespace {
@@ -96,6 +99,7 @@ constexpr float kRescaleThreshold = 8.0f;        // log2 units: P stays <= 256
 // in f32 by the CUDA cores) and the next PV product starts a fresh accumulator, which bounds
 // the chain at 8,192 keys whatever the depth. Rows that see at most 8,192 keys never flush.
 constexpr int kFlushTiles = 64;
+constexpr int kMaxFold = 8;   // most key slices of a query tile that one cluster folds (16 CTAs)
 
 // ------------------------------------------------------------------ PTX helpers
 
@@ -272,7 +276,9 @@ attn_chunk_tc(const __grid_constant__ CUtensorMap map_k_hi, const __grid_constan
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // The launch order is heaviest first: x = 0 holds the last query tiles, which walk the
     // most keys, so the tail of the grid is made of the short tiles.
-    const unsigned rank = kCtas == 2 ? cluster_rank() : 0;
+    // (a cluster holds one pair, or the pairs of all key slices of a query tile: ranks 2 sp, 2 sp + 1)
+    const unsigned in_cluster = kCtas == 2 ? cluster_rank() : 0, leader = in_cluster & ~1u, rank = in_cluster & 1u;
+    const unsigned short both = (unsigned short)(3u << leader);
     const int unit = (int)(gridDim.x / kCtas) - 1 - (int)(blockIdx.x / kCtas);  // tile or pair
     const int qt = unit * kCtas + (int)rank, kvh = blockIdx.y, sp = blockIdx.z;
     const int t0 = qt * p.qtile;
@@ -284,15 +290,16 @@ attn_chunk_tc(const __grid_constant__ CUtensorMap map_k_hi, const __grid_constan
     const unsigned bar_s = smem_u32(bars + 6), bar_p = smem_u32(bars + 8), bar_o = smem_u32(bars + 10);
     const unsigned bar_x = smem_u32(bars + 12);
     // Barriers of the leader CTA that this CTA signals (its own when there is no pair).
-    const unsigned lead_full = kCtas == 2 ? map_to_cta(bar_full, 0) : bar_full;
-    const unsigned lead_p = kCtas == 2 ? map_to_cta(bar_p, 0) : bar_p;
+    const unsigned lead_full = kCtas == 2 ? map_to_cta(bar_full, leader) : bar_full;
+    const unsigned lead_p = kCtas == 2 ? map_to_cta(bar_p, leader) : bar_p;
     const unsigned peer_abort =
-        kCtas == 2 ? map_to_cta(smem_u32(const_cast<int *>(abort_flag)), rank ^ 1) : 0;
+        kCtas == 2 ? map_to_cta(smem_u32(const_cast<int *>(abort_flag)), in_cluster ^ 1) : 0;
 
     // Key tiles the CTA (pair) walks: its rows see cache rows < pos0 + (last live query + 1).
     const int t_end = min(p.tokens, (unit + 1) * kCtas * p.qtile);
     const int n_tiles_all = (p.pos0 + t_end + kKeyTile - 1) / kKeyTile;
-    const int nsp = p.splits < 2 ? 1 : p.splits;
+    const bool fold = kCtas == 2 && p.fold > 1;
+    const int nsp = fold ? p.fold : (p.splits < 2 ? 1 : p.splits);
     const int kt_lo = (int)((long long)n_tiles_all * sp / nsp);
     const int kt_hi = (int)((long long)n_tiles_all * (sp + 1) / nsp);
     const int n_tiles = kt_hi - kt_lo;
@@ -468,7 +475,7 @@ attn_chunk_tc(const __grid_constant__ CUtensorMap map_k_hi, const __grid_constan
                 return smem_u32(ring + stage * kStageBytes);
             };
             auto release = [&]() {  // the slot is free once the MMAs issued so far are done
-                tc_commit<kCtas>(bar_empty + 8 * (n % kStages));
+                tc_commit<kCtas>(bar_empty + 8 * (n % kStages), both);
                 n++;
             };
             // The issuing thread is a serial instruction stream: an MMA of N = 128 keeps the
@@ -515,7 +522,7 @@ attn_chunk_tc(const __grid_constant__ CUtensorMap map_k_hi, const __grid_constan
                         release();
                     }
                 }
-                if (ok) tc_commit<kCtas>(bar_s + 8 * (i & 1));
+                if (ok) tc_commit<kCtas>(bar_s + 8 * (i & 1), both);
             };
             auto pv = [&](int i) {
                 const unsigned a_base = tmem_s[i & 1];
@@ -548,7 +555,7 @@ attn_chunk_tc(const __grid_constant__ CUtensorMap map_k_hi, const __grid_constan
                         }
                         release();
                     }
-                if (ok) tc_commit<kCtas>(bar_o + 8 * (i & 1));
+                if (ok) tc_commit<kCtas>(bar_o + 8 * (i & 1), both);
             };
             qk(0);
             for (int i = 0; i < n_tiles && ok; i++) {
@@ -577,7 +584,7 @@ attn_chunk_tc(const __grid_constant__ CUtensorMap map_k_hi, const __grid_constan
         const bool live = r < rows_live;
         const int rq = r / p.group, rh = r - rq * p.group;
         const int h = kvh * p.group + rh;
-        const bool norm = p.splits < 2;
+        const bool norm = p.splits < 2 && !fold;
         const size_t slot = ((size_t)sp * p.qslots + (t0 + rq)) * p.n_heads + h;
         float *const dst = (norm ? p.out + ((size_t)(t0 + rq) * p.n_heads + h) * kD : p.part_acc + slot * kD) +
                            128 * half;
@@ -736,12 +743,12 @@ attn_chunk_tc(const __grid_constant__ CUtensorMap map_k_hi, const __grid_constan
                                         __uint_as_float(v[e + 2]) * pre, __uint_as_float(v[e + 3]) * pre);
                 }
             }
-            if (bulk_rows) fence_async_shared();   // these rows are read by the bulk copies below
+            if (bulk_rows && !fold) fence_async_shared();   // these rows are read by the bulk copies below
             if (live && half == 0) {
                 const bool flushed = m_glob != -INFINITY;   // part of O is in memory already
-                row_scale[2 * r] = flushed ? exp2f(m_glob - m_used) : -1.0f;
-                row_scale[2 * r + 1] = inv;
-                if (!norm) {
+                row_scale[2 * r] = fold ? m_used : (flushed ? exp2f(m_glob - m_used) : -1.0f);
+                row_scale[2 * r + 1] = fold ? l : inv;
+                if (!norm && !fold) {
                     p.part_ml[slot * 2] = m_used;
                     p.part_ml[slot * 2 + 1] = l;
                 }
@@ -749,7 +756,9 @@ attn_chunk_tc(const __grid_constant__ CUtensorMap map_k_hi, const __grid_constan
         }
         // (the eight softmax warps; a warp that gave up still arrives, and nothing is written then)
         asm volatile("bar.sync 1, 256;" ::: "memory");
-        if (*abort_flag == 0 && bulk_rows) {
+        if (fold) {
+            // (the slices meet below)
+        } else if (*abort_flag == 0 && bulk_rows) {
             if (lane == 0) {
                 for (int rr = warp; rr < rows_live; rr += 8) {
                     const int q2 = rr / p.group, h2 = kvh * p.group + (rr - q2 * p.group);
@@ -790,6 +799,64 @@ attn_chunk_tc(const __grid_constant__ CUtensorMap map_k_hi, const __grid_constan
                         w.w *= 1.0f / (1.0f + expf(-g.w));
                     }
                     *reinterpret_cast<float4 *>(drow + col) = w;
+                }
+            }
+        }
+    }
+
+    // Slices of a tile in one cluster: every CTA folds its share of the rows of all slices' staged
+    // partials through distributed shared memory and writes the output.
+    if constexpr (kCtas == 2) {
+        if (fold) {
+            cluster_sync_all();
+            if (warp < 8 && *abort_flag == 0) {
+                constexpr int kPitch = kD + 4;
+                const float *const stage = reinterpret_cast<const float *>(smem);
+                const unsigned stage_addr = smem_u32(stage), ml_addr = smem_u32(stage + 128 * kPitch);
+                const int r_lo = rows_live * sp / nsp, r_hi = rows_live * (sp + 1) / nsp;
+                for (int r = r_lo + warp; r < r_hi; r += 8) {
+                    // lane s holds slice s's {maximum, sum}
+                    float2 ml = make_float2(-INFINITY, 0.0f);
+                    if (lane < nsp) ml = ld_cluster_f2(map_to_cta(ml_addr + 8 * r, 2 * lane + rank));
+                    const float big = warp_max(ml.x);
+                    const float wt = ml.x == -INFINITY ? 0.0f : exp2f(ml.x - big);
+                    const float den = warp_sum(ml.y * wt), inv = den > 0.0f ? 1.0f / den : 0.0f;
+                    float4 x[kMaxFold][2];
+#pragma unroll
+                    for (int s = 0; s < kMaxFold; s++)
+                        if (s < nsp) {
+                            const unsigned src = map_to_cta(stage_addr + (r * kPitch + 4 * lane) * 4, 2 * s + rank);
+                            x[s][0] = ld_cluster_f4(src);
+                            x[s][1] = ld_cluster_f4(src + 512);
+                        }
+                    float4 y[2] = {make_float4(0.0f, 0.0f, 0.0f, 0.0f), make_float4(0.0f, 0.0f, 0.0f, 0.0f)};
+#pragma unroll
+                    for (int s = 0; s < kMaxFold; s++)
+                        if (s < nsp) {
+                            const float ws = __shfl_sync(0xffffffffu, wt, s);
+#pragma unroll
+                            for (int c = 0; c < 2; c++) {
+                                y[c].x = fmaf(x[s][c].x, ws, y[c].x);
+                                y[c].y = fmaf(x[s][c].y, ws, y[c].y);
+                                y[c].z = fmaf(x[s][c].z, ws, y[c].z);
+                                y[c].w = fmaf(x[s][c].w, ws, y[c].w);
+                            }
+                        }
+                    const int rq = r / p.group;
+                    const size_t row = (size_t)(t0 + rq) * p.n_heads + kvh * p.group + (r - rq * p.group);
+#pragma unroll
+                    for (int c = 0; c < 2; c++) {
+                        const int col = 128 * c + 4 * lane;
+                        float4 w = make_float4(y[c].x * inv, y[c].y * inv, y[c].z * inv, y[c].w * inv);
+                        if (p.gate) {
+                            const float4 g = *reinterpret_cast<const float4 *>(p.gate + row * kD + col);
+                            w.x *= 1.0f / (1.0f + expf(-g.x));
+                            w.y *= 1.0f / (1.0f + expf(-g.y));
+                            w.z *= 1.0f / (1.0f + expf(-g.z));
+                            w.w *= 1.0f / (1.0f + expf(-g.w));
+                        }
+                        *reinterpret_cast<float4 *>(p.out + row * kD + col) = w;
+                    }
                 }
             }
         }
@@ -854,6 +921,46 @@ int launch_chunk_stage(cudaStream_t stream, const void *k_cache, const void *v_c
     return launch_pdl(attn_chunk_stage, dim3(tile_end - sp.tile0, n_kv, 3), dim3(256), 0, stream, 1, sp);
 }
 
+// How many clusters of `slices` CTA pairs fit the device at once (one CTA per SM; cached per device).
+static int fold_capacity(int slices) {
+    static std::atomic<int> cached[64][kMaxFold + 1];
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64) dev = 0;
+    int n = cached[dev][slices].load();
+    if (n == 0) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(2, 64, slices);
+        cfg.blockDim = dim3(kTcThreads);
+        cfg.dynamicSmemBytes = kSmemBytes;
+        cudaLaunchAttribute attr;
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = 2;
+        attr.val.clusterDim.y = 1;
+        attr.val.clusterDim.z = slices;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        if (cudaOccupancyMaxActiveClusters(&n, attn_chunk_tc<2>, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            n = 0;
+        }
+        n = n > 0 ? n : -1;
+        cached[dev][slices].store(n);
+    }
+    return n;
+}
+
+// Key slices per query tile of a one-pass launch of `pairs` CTA pairs. A launch with fewer pairs than the
+// device has SM pairs leaves the rest idle, and every pair walks its keys alone at ~4.4 us per 128-key tile
+// behind ~13 us of its own (301 tokens at 3,001: 32 pairs, 26 tiles, 127 us). So: as many slices as still
+// start together, at least two key tiles each (the fold costs ~4 us), none past the 64 tiles where a
+// pair would move its sums to memory. (B200: 33 clusters of 2 slices, 15 of 4, 7 of 8.)
+static int fold_slices(int pairs, int key_tiles) {
+    for (int s = kMaxFold; s >= 2; s--)
+        if (key_tiles >= 2 * s && (key_tiles + s - 1) / s <= kFlushTiles && pairs <= fold_capacity(s)) return s;
+    return 1;
+}
+
 // Launches the tensor-core kernel over a workspace staged for `cap` keys per head.
 // variant bit 0: single-pass precision (hi*hi only); bit 1: the single-CTA form instead of
 // CTA pairs. Shapes are validated by the caller.
@@ -881,6 +988,8 @@ int launch_chunk_tc(cudaStream_t stream, const float *q, float *out, float *part
         if (e == cudaSuccess)
             e = cudaFuncSetAttribute(attn_chunk_tc<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      kSmemBytes);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(attn_chunk_tc<2>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         if (e != cudaSuccess) return (int)e;
         configured[dev] = true;
     }
@@ -903,16 +1012,21 @@ int launch_chunk_tc(cudaStream_t stream, const float *q, float *out, float *part
     p.qslots = (tokens + 31) / 32 * 32;
     p.single_pass = single_pass;
     p.gate = gate;
+    p.fold = 1;
     const int nsp = splits < 2 ? 1 : splits;
     const int qtiles = (tokens + p.qtile - 1) / p.qtile;
     if (!pair) {
         return launch_pdl(attn_chunk_tc<1>, dim3(qtiles, n_kv, nsp), dim3(kTcThreads), (size_t)kSmemBytes,
                           stream, 1, mk_hi, mk_lo, mv_hi, mv_lo, p);
     }
-    // Clusters of two CTAs along x: consecutive query tiles of one KV head (an odd tile
-    // count leaves the last pair's second CTA without live queries).
-    return launch_pdl(attn_chunk_tc<2>, dim3((qtiles + 1) / 2 * 2, n_kv, nsp), dim3(kTcThreads),
-                      (size_t)kSmemBytes, stream, 2, mk_hi, mk_lo, mv_hi, mv_lo, p);
+    // Clusters of two CTAs along x: consecutive query tiles of one KV head (an odd tile count leaves the
+    // last pair's second CTA without live queries), and along z the key slices that fold in the cluster.
+    const int pairs = (qtiles + 1) / 2;
+    const int key_tiles = (pos0 + tokens + kKeyTile - 1) / kKeyTile;
+    p.fold = splits < 2 ? fold_slices(pairs * n_kv, key_tiles) : 1;
+    const dim3 grid(pairs * 2, n_kv, p.fold > 1 ? p.fold : nsp);
+    return launch_pdl(attn_chunk_tc<2>, grid, dim3(kTcThreads), (size_t)kSmemBytes, stream,
+                      dim3(2, 1, p.fold > 1 ? p.fold : 1), mk_hi, mk_lo, mv_hi, mv_lo, p);
 }
 
 }  // namespace hipml

@@ -15,7 +15,7 @@
 // a time with all loads in flight; the four rows' dot products are summed over the lanes by one
 // reduce-scatter (25 shuffles for 24 sums, where a butterfly each took 120). Other head sizes:
 // attn_decode_cols_f32, one warp per (query head, run, column).
-#include "decode_warp_body.cuh"
+#include "decode_rows_f32.cuh"
 
 namespace hipml {
 
@@ -36,39 +36,12 @@ namespace {
 using namespace warp_body;
 
 constexpr int kF32Cluster = 8;     // CTAs (runs) per cluster, folded through distributed shared memory
-constexpr int kRowsAtOnce = 4;
 constexpr int kOffMlF32 = kWarps * 8 * kHeadPitch * 4;             // after the warps' partials: [8 heads][warp]
 constexpr int kOffPartF32 = kOffMlF32 + kWarps * 8 * 8;            // the CTA's partial [8 heads][256]
 constexpr int kOffCmlF32 = kOffPartF32 + 8 * 256 * 4;              // [8 heads]
 constexpr int kSmemF32 = kOffCmlF32 + 8 * 8;
 
 __device__ int g_arrive_f32[kArriveRegions * kArriveRegionInts];
-
-// Sums v[row][head] over the 32 lanes; lane 8 * row + head returns its own sum.
-template <int kHeads>
-__device__ __forceinline__ float reduce_scatter(const float (&v)[kRowsAtOnce][kHeads], int lane) {
-    float a[2][kHeads], b[8];
-#pragma unroll
-    for (int h = 0; h < kHeads; h++) {
-#pragma unroll
-        for (int r = 0; r < 2; r++) {
-            const float keep = (lane & 16) ? v[2 + r][h] : v[r][h], give = (lane & 16) ? v[r][h] : v[2 + r][h];
-            a[r][h] = keep + __shfl_xor_sync(0xffffffffu, give, 16);
-        }
-        const float keep = (lane & 8) ? a[1][h] : a[0][h], give = (lane & 8) ? a[0][h] : a[1][h];
-        b[h] = keep + __shfl_xor_sync(0xffffffffu, give, 8);
-    }
-#pragma unroll
-    for (int h = kHeads; h < 8; h++) b[h] = 0.0f;
-#pragma unroll
-    for (int o = 4; o > 0; o >>= 1)
-#pragma unroll
-        for (int h = 0; h < o; h++) {
-            const float keep = (lane & o) ? b[o + h] : b[h], give = (lane & o) ? b[h] : b[o + h];
-            b[h] = keep + __shfl_xor_sync(0xffffffffu, give, o);
-        }
-    return b[0];
-}
 
 // grid (n_kv * clusters * 8, columns), clusters of 8. d: out, scratch and counters (as the quantised body's).
 template <int kHeads>
@@ -104,89 +77,33 @@ __global__ void __launch_bounds__(kThreads, 2) attn_decode_rows_f32(ColsParams p
     __syncthreads();
 
     // lane: dims 4 * lane .. + 3 and 128 + 4 * lane .. + 3
-    float acc[kHeads][8];
-#pragma unroll
-    for (int h = 0; h < kHeads; h++)
-#pragma unroll
-        for (int e = 0; e < 8; e++) acc[h][e] = 0.0f;
-    float m = -INFINITY, l = 0.0f;   // lane 8 * row + head: the head's maximum, the sum over rows = row (mod 4)
+    RowsF32<kHeads> st;
+    st.start();
     for (int r0 = lo; r0 < hi; r0 += kRowsAtOnce) {
-        float4 k[kRowsAtOnce][2], v[kRowsAtOnce][2];
+        float k[kRowsAtOnce][8], v[kRowsAtOnce][8];
 #pragma unroll
         for (int r = 0; r < kRowsAtOnce; r++) {
             const size_t at = (size_t)min(r0 + r, hi - 1) * width + 4 * lane;
-            k[r][0] = *reinterpret_cast<const float4 *>(kb + at);
-            k[r][1] = *reinterpret_cast<const float4 *>(kb + at + 128);
-            v[r][0] = *reinterpret_cast<const float4 *>(vb + at);
-            v[r][1] = *reinterpret_cast<const float4 *>(vb + at + 128);
-        }
-        float s[kRowsAtOnce][kHeads];
 #pragma unroll
-        for (int h = 0; h < kHeads; h++) {
-            const float4 q0 = *reinterpret_cast<const float4 *>(s_q + h * 256 + 4 * lane);
-            const float4 q1 = *reinterpret_cast<const float4 *>(s_q + h * 256 + 128 + 4 * lane);
-#pragma unroll
-            for (int r = 0; r < kRowsAtOnce; r++) {
-                float x = q0.x * k[r][0].x;
-                x = fmaf(q0.y, k[r][0].y, x);
-                x = fmaf(q0.z, k[r][0].z, x);
-                x = fmaf(q0.w, k[r][0].w, x);
-                x = fmaf(q1.x, k[r][1].x, x);
-                x = fmaf(q1.y, k[r][1].y, x);
-                x = fmaf(q1.z, k[r][1].z, x);
-                s[r][h] = fmaf(q1.w, k[r][1].w, x);
+            for (int i = 0; i < 2; i++) {
+                const float4 a = *reinterpret_cast<const float4 *>(kb + at + 128 * i);
+                const float4 b = *reinterpret_cast<const float4 *>(vb + at + 128 * i);
+                k[r][4 * i] = a.x; k[r][4 * i + 1] = a.y; k[r][4 * i + 2] = a.z; k[r][4 * i + 3] = a.w;
+                v[r][4 * i] = b.x; v[r][4 * i + 1] = b.y; v[r][4 * i + 2] = b.z; v[r][4 * i + 3] = b.w;
             }
         }
-        float score = reduce_scatter<kHeads>(s, lane);
-        if (r0 + (lane >> 3) >= hi) score = -INFINITY;
-        float top = fmaxf(score, __shfl_xor_sync(0xffffffffu, score, 8));
-        top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 16));
-        const float m_new = fmaxf(m, top);
-        if (__any_sync(0xffffffffu, m_new > m)) {
-            const float corr = ex2(m - m_new);
-            l *= corr;
-            m = m_new;
-#pragma unroll
-            for (int h = 0; h < kHeads; h++) {
-                const float c = __shfl_sync(0xffffffffu, corr, h);
-#pragma unroll
-                for (int e = 0; e < 8; e++) acc[h][e] *= c;
-            }
-        }
-        const float w = ex2(score - m);
-        l += w;
-        s_w[warp][lane & 7][lane >> 3] = w;
-        __syncwarp();
-#pragma unroll
-        for (int h = 0; h < kHeads; h++) {
-            const float4 wh = *reinterpret_cast<const float4 *>(s_w[warp][h]);
-            const float wr[4] = {wh.x, wh.y, wh.z, wh.w};
-#pragma unroll
-            for (int r = 0; r < kRowsAtOnce; r++) {
-                acc[h][0] = fmaf(wr[r], v[r][0].x, acc[h][0]);
-                acc[h][1] = fmaf(wr[r], v[r][0].y, acc[h][1]);
-                acc[h][2] = fmaf(wr[r], v[r][0].z, acc[h][2]);
-                acc[h][3] = fmaf(wr[r], v[r][0].w, acc[h][3]);
-                acc[h][4] = fmaf(wr[r], v[r][1].x, acc[h][4]);
-                acc[h][5] = fmaf(wr[r], v[r][1].y, acc[h][5]);
-                acc[h][6] = fmaf(wr[r], v[r][1].z, acc[h][6]);
-                acc[h][7] = fmaf(wr[r], v[r][1].w, acc[h][7]);
-            }
-        }
-        __syncwarp();
+        st.add(k, v, s_q + 4 * lane, s_q + 128 + 4 * lane, s_w[warp], r0, hi, lane);
     }
 
     // ---- merge: the warps, the cluster, then the head's clusters (the last to arrive)
-    l += __shfl_xor_sync(0xffffffffu, l, 8);
-    l += __shfl_xor_sync(0xffffffffu, l, 16);
     float2 *const wml = reinterpret_cast<float2 *>(smem + kOffMlF32);
-    if (lane < 8) wml[lane * kWarps + warp] = make_float2(m, l);
+    st.finish(wml, warp, lane);
     float *const mine = reinterpret_cast<float *>(smem) + warp * 8 * kHeadPitch;
 #pragma unroll
     for (int h = 0; h < kHeads; h++) {
-        *reinterpret_cast<float4 *>(mine + h * kHeadPitch + 4 * lane) = make_float4(acc[h][0], acc[h][1], acc[h][2], acc[h][3]);
+        *reinterpret_cast<float4 *>(mine + h * kHeadPitch + 4 * lane) = make_float4(st.acc[h][0], st.acc[h][1], st.acc[h][2], st.acc[h][3]);
         *reinterpret_cast<float4 *>(mine + h * kHeadPitch + 128 + 4 * lane) =
-            make_float4(acc[h][4], acc[h][5], acc[h][6], acc[h][7]);
+            make_float4(st.acc[h][4], st.acc[h][5], st.acc[h][6], st.acc[h][7]);
     }
     __syncthreads();
     const int items = group * 64;

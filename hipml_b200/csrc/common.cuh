@@ -47,11 +47,11 @@ __device__ __forceinline__ void griddep_wait() {
 }
 #endif
 
-// cudaLaunchKernelEx with the programmatic-stream-serialization attribute (and, for
-// cluster_x > 1, the cluster dimension).
+// cudaLaunchKernelEx with the programmatic-stream-serialization attribute (and the cluster
+// dimensions, where they are more than one CTA).
 template <typename... KArgs, typename... Args>
 int launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
-               unsigned cluster_x, Args... args) {
+               dim3 cluster, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -61,11 +61,11 @@ int launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cud
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.numAttrs = 1;
-    if (cluster_x > 1) {
+    if (cluster.x * cluster.y * cluster.z > 1) {
         attr[1].id = cudaLaunchAttributeClusterDimension;
-        attr[1].val.clusterDim.x = cluster_x;
-        attr[1].val.clusterDim.y = 1;
-        attr[1].val.clusterDim.z = 1;
+        attr[1].val.clusterDim.x = cluster.x;
+        attr[1].val.clusterDim.y = cluster.y;
+        attr[1].val.clusterDim.z = cluster.z;
         cfg.numAttrs = 2;
     }
     cfg.attrs = attr;

@@ -593,6 +593,38 @@ int hipml_attn_decode_batch_append(hipml_stream_t stream, int dtype, const int *
                        slots, 1, k_f32, v_f32);
 }
 
+static int check_stage(const void *k_cache, const void *v_cache, int n_kv, int head_dim, int kv_dtype, int stride,
+                       int key_from, int key_to, int key_capacity, const void *workspace, size_t workspace_bytes) {
+    if (head_dim != 256 || n_kv <= 0)
+        return fail(HIPML_ERR_INVALID_ARGUMENT,
+                    "tensor-core chunk attention: only head_dim 256 with a GQA group <= 8");
+    if (kv_dtype < 0 || kv_dtype > 2)
+        return fail(HIPML_ERR_INVALID_ARGUMENT, "unknown KV dtype %d", kv_dtype);
+    if (key_from < 0 || key_to < key_from || key_capacity % 128 != 0 || key_to > key_capacity)
+        return fail(HIPML_ERR_INVALID_ARGUMENT, "stage rows [%d, %d) with capacity %d", key_from,
+                    key_to, key_capacity);
+    if (kv_dtype != 0 && key_to > stride)
+        return fail(HIPML_ERR_INVALID_ARGUMENT, "position %d beyond KV cache %d", key_to, stride);
+    const size_t need = chunk_tc_workspace_bytes(n_kv, key_capacity);
+    if (!workspace || workspace_bytes < need)
+        return fail(HIPML_ERR_WORKSPACE, "chunk attention workspace: %zu bytes given, %zu needed",
+                    workspace_bytes, need);
+    if ((reinterpret_cast<size_t>(workspace) & 255) != 0)
+        return fail(HIPML_ERR_WORKSPACE, "chunk attention workspace must be 256-byte aligned");
+    if (((reinterpret_cast<size_t>(k_cache) | reinterpret_cast<size_t>(v_cache)) & 15) != 0)
+        return fail(HIPML_ERR_INVALID_ARGUMENT, "q, out and the caches must be 16-byte aligned");
+    return 0;
+}
+
+// Whether a one-pass chunk goes straight from the cache on the CUDA cores (attn_chunk_small.cu): the
+// tensor-core path has ~24 us of fixed latency, the small kernel takes ~9 us + 2 us per 1,000 (query, key)
+// pairs of 4 KV heads, so they meet at ~7,000 (37 tokens at 29: 12 us against 24; 100 at 0: 17 against 25;
+// 37 at 200, 8,000 pairs: 28 against 26).
+static bool small_chunk(int n_kv, int pos0, int tokens) {
+    const long long pairs = (long long)tokens * pos0 + (long long)tokens * (tokens + 1) / 2;
+    return pairs * n_kv <= 26000 && tokens <= 65535;
+}
+
 size_t hipml_attn_chunk_workspace_bytes(int n_kv, int head_dim, int pos0, int tokens) {
     if (head_dim != 256 || n_kv <= 0 || pos0 < 0 || tokens <= 0) return 0;
     return chunk_tc_workspace_bytes(n_kv, pos0 + tokens);
@@ -650,6 +682,15 @@ int hipml_attn_chunk(hipml_stream_t stream, const float *q, const void *k_cache,
             return fail(HIPML_ERR_INVALID_ARGUMENT,
                         "tensor-core chunk attention: only head_dim 256 with a GQA group <= 8");
         const int cap = (pos0 + tokens + 127) / 128 * 128;
+        if (mode == 0 && splits < 2 && small_chunk(n_kv, pos0, tokens)) {
+            if (int e = check_stage(k_cache, v_cache, n_kv, head_dim, kv_dtype, stride, 0, pos0 + tokens, cap, workspace,
+                                    workspace_bytes))
+                return e;
+            if (((reinterpret_cast<size_t>(q) | reinterpret_cast<size_t>(out)) & 15) != 0)
+                return fail(HIPML_ERR_INVALID_ARGUMENT, "q, out and the caches must be 16-byte aligned");
+            return launch_chunk_small(as_stream(stream), q, k_cache, v_cache, out, n_heads, n_kv, kv_dtype, stride, pos0,
+                                      tokens);
+        }
         if (int e = hipml_attn_chunk_stage(stream, k_cache, v_cache, n_kv, head_dim, kv_dtype,
                                            stride, 0, pos0 + tokens, cap, workspace,
                                            workspace_bytes))
@@ -668,24 +709,9 @@ int hipml_attn_chunk_stage(hipml_stream_t stream, const void *k_cache, const voi
                            int n_kv, int head_dim, int kv_dtype, int stride, int key_from,
                            int key_to, int key_capacity, void *workspace,
                            size_t workspace_bytes) {
-    if (head_dim != 256 || n_kv <= 0)
-        return fail(HIPML_ERR_INVALID_ARGUMENT,
-                    "tensor-core chunk attention: only head_dim 256 with a GQA group <= 8");
-    if (kv_dtype < 0 || kv_dtype > 2)
-        return fail(HIPML_ERR_INVALID_ARGUMENT, "unknown KV dtype %d", kv_dtype);
-    if (key_from < 0 || key_to < key_from || key_capacity % 128 != 0 || key_to > key_capacity)
-        return fail(HIPML_ERR_INVALID_ARGUMENT, "stage rows [%d, %d) with capacity %d", key_from,
-                    key_to, key_capacity);
-    if (kv_dtype != 0 && key_to > stride)
-        return fail(HIPML_ERR_INVALID_ARGUMENT, "position %d beyond KV cache %d", key_to, stride);
-    const size_t need = chunk_tc_workspace_bytes(n_kv, key_capacity);
-    if (!workspace || workspace_bytes < need)
-        return fail(HIPML_ERR_WORKSPACE, "chunk attention workspace: %zu bytes given, %zu needed",
-                    workspace_bytes, need);
-    if ((reinterpret_cast<size_t>(workspace) & 255) != 0)
-        return fail(HIPML_ERR_WORKSPACE, "chunk attention workspace must be 256-byte aligned");
-    if (((reinterpret_cast<size_t>(k_cache) | reinterpret_cast<size_t>(v_cache)) & 15) != 0)
-        return fail(HIPML_ERR_INVALID_ARGUMENT, "q, out and the caches must be 16-byte aligned");
+    if (int e = check_stage(k_cache, v_cache, n_kv, head_dim, kv_dtype, stride, key_from, key_to, key_capacity,
+                            workspace, workspace_bytes))
+        return e;
     return launch_chunk_stage(as_stream(stream), k_cache, v_cache, n_kv, kv_dtype, stride, key_from,
                               key_to, key_capacity, workspace);
 }

@@ -197,6 +197,10 @@ int launch_chunk_combine(cudaStream_t stream, const float *part_acc, const float
                          float *out, int n_heads, int head_dim, int tokens, int qslots, int splits,
                          const float *gate = nullptr);
 
+// Chunk attention straight from the cache for few (query, key) pairs (attn_chunk_small.cu), head_dim 256.
+int launch_chunk_small(cudaStream_t stream, const float *q, const void *k_cache, const void *v_cache, float *out,
+                       int n_heads, int n_kv, int kv_dtype, int stride, int pos0, int tokens);
+
 // Throughput form of the q8_0 bulk append, head_dim 256 and 16-byte-aligned sources (kv_encode.cu).
 int launch_kv_encode_bulk_rows(cudaStream_t stream, const float *k, const float *v,
                                unsigned char *kc, unsigned char *vc, int n_kv, int stride,

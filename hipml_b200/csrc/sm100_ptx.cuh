@@ -160,14 +160,13 @@ __device__ __forceinline__ void tc_fence_after() {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
 // Arrive on `bar` when every MMA this thread issued so far has completed. In the pair form
-// the arrival goes to the barrier at the same offset in both CTAs.
+// the arrival goes to the barrier at the same offset in both CTAs, whose cluster ranks `both` masks.
 template <int kCtas>
-__device__ __forceinline__ void tc_commit(unsigned bar) {
+__device__ __forceinline__ void tc_commit(unsigned bar, unsigned short both = 3) {
     if constexpr (kCtas == 1) {
         asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
                      : "memory");
     } else {
-        const unsigned short both = 3;
         asm volatile(
             "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 "
             "[%0], %1;"
