@@ -251,7 +251,8 @@ __global__ void __launch_bounds__(256) attn_chunk_stage(StageParams p) {
 
 // kCtas = 1: one CTA per query tile. kCtas = 2: launched as clusters of two along x; the
 // K maps then have 64-key boxes (a CTA loads its half of the keys of a tile).
-template <int kCtas>
+// kFold: the key slices of a tile (grid z) are one cluster, which folds them.
+template <int kCtas, bool kFold>
 __global__ void __launch_bounds__(kTcThreads, 1)
 attn_chunk_tc(const __grid_constant__ CUtensorMap map_k_hi, const __grid_constant__ CUtensorMap map_k_lo,
               const __grid_constant__ CUtensorMap map_vt_hi,
@@ -277,8 +278,9 @@ attn_chunk_tc(const __grid_constant__ CUtensorMap map_k_hi, const __grid_constan
     // The launch order is heaviest first: x = 0 holds the last query tiles, which walk the
     // most keys, so the tail of the grid is made of the short tiles.
     // (a cluster holds one pair, or the pairs of all key slices of a query tile: ranks 2 sp, 2 sp + 1)
-    const unsigned in_cluster = kCtas == 2 ? cluster_rank() : 0, leader = in_cluster & ~1u, rank = in_cluster & 1u;
-    const unsigned short both = (unsigned short)(3u << leader);
+    const unsigned in_cluster = kCtas == 2 ? cluster_rank() : 0;
+    const unsigned leader = kFold ? in_cluster & ~1u : 0, rank = kFold ? in_cluster & 1u : in_cluster;
+    const unsigned short both = kFold ? (unsigned short)(3u << leader) : 3;
     const int unit = (int)(gridDim.x / kCtas) - 1 - (int)(blockIdx.x / kCtas);  // tile or pair
     const int qt = unit * kCtas + (int)rank, kvh = blockIdx.y, sp = blockIdx.z;
     const int t0 = qt * p.qtile;
@@ -298,8 +300,7 @@ attn_chunk_tc(const __grid_constant__ CUtensorMap map_k_hi, const __grid_constan
     // Key tiles the CTA (pair) walks: its rows see cache rows < pos0 + (last live query + 1).
     const int t_end = min(p.tokens, (unit + 1) * kCtas * p.qtile);
     const int n_tiles_all = (p.pos0 + t_end + kKeyTile - 1) / kKeyTile;
-    const bool fold = kCtas == 2 && p.fold > 1;
-    const int nsp = fold ? p.fold : (p.splits < 2 ? 1 : p.splits);
+    const int nsp = kFold ? p.fold : (p.splits < 2 ? 1 : p.splits);
     const int kt_lo = (int)((long long)n_tiles_all * sp / nsp);
     const int kt_hi = (int)((long long)n_tiles_all * (sp + 1) / nsp);
     const int n_tiles = kt_hi - kt_lo;
@@ -584,7 +585,7 @@ attn_chunk_tc(const __grid_constant__ CUtensorMap map_k_hi, const __grid_constan
         const bool live = r < rows_live;
         const int rq = r / p.group, rh = r - rq * p.group;
         const int h = kvh * p.group + rh;
-        const bool norm = p.splits < 2 && !fold;
+        const bool norm = p.splits < 2 && !kFold;
         const size_t slot = ((size_t)sp * p.qslots + (t0 + rq)) * p.n_heads + h;
         float *const dst = (norm ? p.out + ((size_t)(t0 + rq) * p.n_heads + h) * kD : p.part_acc + slot * kD) +
                            128 * half;
@@ -743,12 +744,12 @@ attn_chunk_tc(const __grid_constant__ CUtensorMap map_k_hi, const __grid_constan
                                         __uint_as_float(v[e + 2]) * pre, __uint_as_float(v[e + 3]) * pre);
                 }
             }
-            if (bulk_rows && !fold) fence_async_shared();   // these rows are read by the bulk copies below
+            if (bulk_rows && !kFold) fence_async_shared();   // these rows are read by the bulk copies below
             if (live && half == 0) {
                 const bool flushed = m_glob != -INFINITY;   // part of O is in memory already
-                row_scale[2 * r] = fold ? m_used : (flushed ? exp2f(m_glob - m_used) : -1.0f);
-                row_scale[2 * r + 1] = fold ? l : inv;
-                if (!norm && !fold) {
+                row_scale[2 * r] = kFold ? m_used : (flushed ? exp2f(m_glob - m_used) : -1.0f);
+                row_scale[2 * r + 1] = kFold ? l : inv;
+                if (!norm && !kFold) {
                     p.part_ml[slot * 2] = m_used;
                     p.part_ml[slot * 2 + 1] = l;
                 }
@@ -756,7 +757,7 @@ attn_chunk_tc(const __grid_constant__ CUtensorMap map_k_hi, const __grid_constan
         }
         // (the eight softmax warps; a warp that gave up still arrives, and nothing is written then)
         asm volatile("bar.sync 1, 256;" ::: "memory");
-        if (fold) {
+        if constexpr (kFold) {
             // (the slices meet below)
         } else if (*abort_flag == 0 && bulk_rows) {
             if (lane == 0) {
@@ -806,57 +807,55 @@ attn_chunk_tc(const __grid_constant__ CUtensorMap map_k_hi, const __grid_constan
 
     // Slices of a tile in one cluster: every CTA folds its share of the rows of all slices' staged
     // partials through distributed shared memory and writes the output.
-    if constexpr (kCtas == 2) {
-        if (fold) {
-            cluster_sync_all();
-            if (warp < 8 && *abort_flag == 0) {
-                constexpr int kPitch = kD + 4;
-                const float *const stage = reinterpret_cast<const float *>(smem);
-                const unsigned stage_addr = smem_u32(stage), ml_addr = smem_u32(stage + 128 * kPitch);
-                const int r_lo = rows_live * sp / nsp, r_hi = rows_live * (sp + 1) / nsp;
-                for (int r = r_lo + warp; r < r_hi; r += 8) {
-                    // lane s holds slice s's {maximum, sum}
-                    float2 ml = make_float2(-INFINITY, 0.0f);
-                    if (lane < nsp) ml = ld_cluster_f2(map_to_cta(ml_addr + 8 * r, 2 * lane + rank));
-                    const float big = warp_max(ml.x);
-                    const float wt = ml.x == -INFINITY ? 0.0f : exp2f(ml.x - big);
-                    const float den = warp_sum(ml.y * wt), inv = den > 0.0f ? 1.0f / den : 0.0f;
-                    float4 x[kMaxFold][2];
+    if constexpr (kFold) {
+        cluster_sync_all();
+        if (warp < 8 && *abort_flag == 0) {
+            constexpr int kPitch = kD + 4;
+            const float *const stage = reinterpret_cast<const float *>(smem);
+            const unsigned stage_addr = smem_u32(stage), ml_addr = smem_u32(stage + 128 * kPitch);
+            const int r_lo = rows_live * sp / nsp, r_hi = rows_live * (sp + 1) / nsp;
+            for (int r = r_lo + warp; r < r_hi; r += 8) {
+                // lane s holds slice s's {maximum, sum}
+                float2 ml = make_float2(-INFINITY, 0.0f);
+                if (lane < nsp) ml = ld_cluster_f2(map_to_cta(ml_addr + 8 * r, 2 * lane + rank));
+                const float big = warp_max(ml.x);
+                const float wt = ml.x == -INFINITY ? 0.0f : exp2f(ml.x - big);
+                const float den = warp_sum(ml.y * wt), inv = den > 0.0f ? 1.0f / den : 0.0f;
+                float4 x[kMaxFold][2];
 #pragma unroll
-                    for (int s = 0; s < kMaxFold; s++)
-                        if (s < nsp) {
-                            const unsigned src = map_to_cta(stage_addr + (r * kPitch + 4 * lane) * 4, 2 * s + rank);
-                            x[s][0] = ld_cluster_f4(src);
-                            x[s][1] = ld_cluster_f4(src + 512);
-                        }
-                    float4 y[2] = {make_float4(0.0f, 0.0f, 0.0f, 0.0f), make_float4(0.0f, 0.0f, 0.0f, 0.0f)};
-#pragma unroll
-                    for (int s = 0; s < kMaxFold; s++)
-                        if (s < nsp) {
-                            const float ws = __shfl_sync(0xffffffffu, wt, s);
-#pragma unroll
-                            for (int c = 0; c < 2; c++) {
-                                y[c].x = fmaf(x[s][c].x, ws, y[c].x);
-                                y[c].y = fmaf(x[s][c].y, ws, y[c].y);
-                                y[c].z = fmaf(x[s][c].z, ws, y[c].z);
-                                y[c].w = fmaf(x[s][c].w, ws, y[c].w);
-                            }
-                        }
-                    const int rq = r / p.group;
-                    const size_t row = (size_t)(t0 + rq) * p.n_heads + kvh * p.group + (r - rq * p.group);
-#pragma unroll
-                    for (int c = 0; c < 2; c++) {
-                        const int col = 128 * c + 4 * lane;
-                        float4 w = make_float4(y[c].x * inv, y[c].y * inv, y[c].z * inv, y[c].w * inv);
-                        if (p.gate) {
-                            const float4 g = *reinterpret_cast<const float4 *>(p.gate + row * kD + col);
-                            w.x *= 1.0f / (1.0f + expf(-g.x));
-                            w.y *= 1.0f / (1.0f + expf(-g.y));
-                            w.z *= 1.0f / (1.0f + expf(-g.z));
-                            w.w *= 1.0f / (1.0f + expf(-g.w));
-                        }
-                        *reinterpret_cast<float4 *>(p.out + row * kD + col) = w;
+                for (int s = 0; s < kMaxFold; s++)
+                    if (s < nsp) {
+                        const unsigned src = map_to_cta(stage_addr + (r * kPitch + 4 * lane) * 4, 2 * s + rank);
+                        x[s][0] = ld_cluster_f4(src);
+                        x[s][1] = ld_cluster_f4(src + 512);
                     }
+                float4 y[2] = {make_float4(0.0f, 0.0f, 0.0f, 0.0f), make_float4(0.0f, 0.0f, 0.0f, 0.0f)};
+#pragma unroll
+                for (int s = 0; s < kMaxFold; s++)
+                    if (s < nsp) {
+                        const float ws = __shfl_sync(0xffffffffu, wt, s);
+#pragma unroll
+                        for (int c = 0; c < 2; c++) {
+                            y[c].x = fmaf(x[s][c].x, ws, y[c].x);
+                            y[c].y = fmaf(x[s][c].y, ws, y[c].y);
+                            y[c].z = fmaf(x[s][c].z, ws, y[c].z);
+                            y[c].w = fmaf(x[s][c].w, ws, y[c].w);
+                        }
+                    }
+                const int rq = r / p.group;
+                const size_t row = (size_t)(t0 + rq) * p.n_heads + kvh * p.group + (r - rq * p.group);
+#pragma unroll
+                for (int c = 0; c < 2; c++) {
+                    const int col = 128 * c + 4 * lane;
+                    float4 w = make_float4(y[c].x * inv, y[c].y * inv, y[c].z * inv, y[c].w * inv);
+                    if (p.gate) {
+                        const float4 g = *reinterpret_cast<const float4 *>(p.gate + row * kD + col);
+                        w.x *= 1.0f / (1.0f + expf(-g.x));
+                        w.y *= 1.0f / (1.0f + expf(-g.y));
+                        w.z *= 1.0f / (1.0f + expf(-g.z));
+                        w.w *= 1.0f / (1.0f + expf(-g.w));
+                    }
+                    *reinterpret_cast<float4 *>(p.out + row * kD + col) = w;
                 }
             }
         }
@@ -940,7 +939,7 @@ static int fold_capacity(int slices) {
         attr.val.clusterDim.z = slices;
         cfg.attrs = &attr;
         cfg.numAttrs = 1;
-        if (cudaOccupancyMaxActiveClusters(&n, attn_chunk_tc<2>, &cfg) != cudaSuccess) {
+        if (cudaOccupancyMaxActiveClusters(&n, attn_chunk_tc<2, true>, &cfg) != cudaSuccess) {
             cudaGetLastError();
             n = 0;
         }
@@ -983,13 +982,16 @@ int launch_chunk_tc(cudaStream_t stream, const float *q, float *out, float *part
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !configured[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(attn_chunk_tc<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaError_t e = cudaFuncSetAttribute(attn_chunk_tc<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              kSmemBytes);
         if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(attn_chunk_tc<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            e = cudaFuncSetAttribute(attn_chunk_tc<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      kSmemBytes);
         if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(attn_chunk_tc<2>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+            e = cudaFuncSetAttribute(attn_chunk_tc<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     kSmemBytes);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(attn_chunk_tc<2, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         if (e != cudaSuccess) return (int)e;
         configured[dev] = true;
     }
@@ -1016,7 +1018,7 @@ int launch_chunk_tc(cudaStream_t stream, const float *q, float *out, float *part
     const int nsp = splits < 2 ? 1 : splits;
     const int qtiles = (tokens + p.qtile - 1) / p.qtile;
     if (!pair) {
-        return launch_pdl(attn_chunk_tc<1>, dim3(qtiles, n_kv, nsp), dim3(kTcThreads), (size_t)kSmemBytes,
+        return launch_pdl(attn_chunk_tc<1, false>, dim3(qtiles, n_kv, nsp), dim3(kTcThreads), (size_t)kSmemBytes,
                           stream, 1, mk_hi, mk_lo, mv_hi, mv_lo, p);
     }
     // Clusters of two CTAs along x: consecutive query tiles of one KV head (an odd tile count leaves the
@@ -1024,9 +1026,11 @@ int launch_chunk_tc(cudaStream_t stream, const float *q, float *out, float *part
     const int pairs = (qtiles + 1) / 2;
     const int key_tiles = (pos0 + tokens + kKeyTile - 1) / kKeyTile;
     p.fold = splits < 2 ? fold_slices(pairs * n_kv, key_tiles) : 1;
-    const dim3 grid(pairs * 2, n_kv, p.fold > 1 ? p.fold : nsp);
-    return launch_pdl(attn_chunk_tc<2>, grid, dim3(kTcThreads), (size_t)kSmemBytes, stream,
-                      dim3(2, 1, p.fold > 1 ? p.fold : 1), mk_hi, mk_lo, mv_hi, mv_lo, p);
+    if (p.fold > 1)
+        return launch_pdl(attn_chunk_tc<2, true>, dim3(pairs * 2, n_kv, p.fold), dim3(kTcThreads), (size_t)kSmemBytes,
+                          stream, dim3(2, 1, p.fold), mk_hi, mk_lo, mv_hi, mv_lo, p);
+    return launch_pdl(attn_chunk_tc<2, false>, dim3(pairs * 2, n_kv, nsp), dim3(kTcThreads), (size_t)kSmemBytes, stream,
+                      2, mk_hi, mk_lo, mv_hi, mv_lo, p);
 }
 
 }  // namespace hipml

@@ -44,7 +44,28 @@ struct Cfg {
 
 __device__ int g_arrive_cols[kArriveRegions * kArriveRegionInts];
 
-// grid (n_kv * runs * kC, ceil(columns / kCols)), clusters of kC.
+// Which columns a cluster takes: groups of `each`, from `base` on every `stride` columns, run `run` of them
+// (base >= the column count: nothing). Columns go to clusters of their own while a head has clusters to
+// spare for their runs, and share conversions beyond (4 columns of 300 rows take 2 runs each: 8 clusters of
+// the head's 18; of 8,192 rows 17: one cluster per run takes all four).
+struct Share {
+    int base, each, stride, run;
+};
+template <class LenOf>
+__device__ __forceinline__ Share share_columns(const DecodeParams &p, int cap, int in_head, LenOf len_of) {
+    int runs = 1;
+    for (int c = threadIdx.x & 31; c < p.n_slots; c += 32) runs = max(runs, balance(p, len_of(c), kC, kUnitRows).runs);
+    runs = __reduce_max_sync(0xffffffffu, runs);
+    const int side = cap / runs;   // groups side by side, >= 1
+    Share s;
+    s.each = min(kCols, div_up(p.n_slots, side));
+    s.run = in_head % runs;
+    s.stride = side * s.each;
+    s.base = in_head < side * runs ? in_head / runs * s.each : p.n_slots;
+    return s;
+}
+
+// grid (n_kv * runs * kC), clusters of kC.
 __global__ void __launch_bounds__(kThreads, 1) attn_decode_cols(DecodeParams p, int *status) {
     using C = Cfg;
     extern __shared__ __align__(128) unsigned char smem[];
@@ -63,21 +84,25 @@ __global__ void __launch_bounds__(kThreads, 1) attn_decode_cols(DecodeParams p, 
         mbar_init_fence();
     }
     if (warp == 0) tmem_alloc<1>(smem_u32(&s_tmem), kTmemCols);
-    const int col0 = blockIdx.y * kCols, col_end = min(p.n_slots, col0 + kCols);
+    const int cap = min(p.splits, p.run_cap), cluster = (int)blockIdx.x / kC;
+    const int kvh = cluster / cap, in_head = cluster - kvh * cap;
     const int *const len_at = p.len + p.len_offset;
-    {
-        // Nothing that the grids ahead may write can be relied on yet, but the lengths as they stand are a
-        // good guess: enough to ask L2 for the first rows (the cache rows themselves are read later).
-        const Work w = plan_stream<kC, kUnitRows>(p, col0, rank, min(max(__ldcg(len_at + col0 * p.len_stride), 0), p.stride));
+    auto len_of = [&](int col) { return min(max(__ldcg(len_at + col * p.len_stride), 0), p.stride); };
+    // Nothing that the grids ahead may write can be relied on yet, but the lengths as they stand are a good
+    // guess: enough to ask L2 for the first rows (the cache rows themselves are read later).
+    Share sh = share_columns(p, cap, in_head, len_of);
+    if (sh.base < p.n_slots) {
+        const Work w = plan_run<kC, kUnitRows>(p, sh.base, kvh, sh.run, rank, len_of(sh.base));
         const int first = w.row0 + w.unit * warp;
         if (lane == 0 && first < w.row1) {
-            const size_t at = ((size_t)w.kvh * p.stride + first) * kRowBytes;
+            const size_t at = ((size_t)kvh * p.stride + first) * kRowBytes;
             const unsigned bytes = (unsigned)(min(w.unit, w.row1 - first) * kRowBytes);
             prefetch_l2(p.k + at, bytes);
             prefetch_l2(p.v + at, bytes);
         }
     }
     griddep_wait();
+    sh = share_columns(p, cap, in_head, len_of);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -95,39 +120,24 @@ __global__ void __launch_bounds__(kThreads, 1) attn_decode_cols(DecodeParams p, 
         }
     };
 
-    for (int base = col0; base < col_end;) {
-        // Columns base .. base + n - 1 share a plan: the same units for every warp. (Ascending lengths leave it
-        // only where they cross a multiple of the unit; then the rest is a second round.)
+    for (int base = sh.base, end = min(base + sh.each, p.n_slots); base < p.n_slots;) {
+        // Columns base .. base + n - 1 share a plan: the same units for every warp. (Ascending lengths rarely
+        // leave it; then the rest of the group is another round.)
         Work w[kCols];
-        int n = 0, units = 0;
+        int n = 1;
+        const Balance b0 = balance(p, len_of(base), kC, kUnitRows);
 #pragma unroll
         for (int c = 0; c < kCols; c++) {
-            w[c] = plan_stream<kC, kUnitRows>(p, base + c, rank, base + c < col_end ? __ldcg(len_at + (base + c) * p.len_stride) : 0);
-            const int u = div_up(w[c].len, w[c].unit);
-            if (c == 0) {
-                n = 1;
-                units = u;
-            } else if (n == c && base + c < col_end && u == units && w[c].unit == w[0].unit && w[c].runs == w[0].runs) {
-                n = c + 1;
-            }
+            const int len = base + c < end ? len_of(base + c) : 0;
+            w[c] = plan_run<kC, kUnitRows>(p, base + c, kvh, sh.run, rank, len);
+            const Balance b = balance(p, len, kC, kUnitRows);
+            if (c > 0 && n == c && base + c < end && b.units == b0.units && b.unit == b0.unit && b.runs == b0.runs) n = c + 1;
         }
-        const int kvh = w[0].kvh, unit = w[0].unit;
+        const int unit = w[0].unit;
         int row1 = w[0].row1;
 #pragma unroll
         for (int c = 1; c < kCols; c++)
             if (c < n) row1 = max(row1, w[c].row1);
-        auto neutral = [&](int col, int r) {
-            float *const pa = p.part_acc + (size_t)col * p.acc_slot + (size_t)kvh * group * p.splits * 256;
-            float *const pm = p.part_ml + (size_t)col * p.ml_slot + (size_t)kvh * group * p.splits * 2;
-            for (int i = rank * kThreads + tid; i < group * 256; i += kC * kThreads)
-                pa[((size_t)(i >> 8) * p.splits + r) * 256 + (i & 255)] = 0.0f;
-            if (rank == 0 && tid < group)
-                *reinterpret_cast<float2 *>(pm + ((size_t)tid * p.splits + r) * 2) = make_float2(-INFINITY, 0.0f);
-        };
-        for (int c = 0; c < n; c++) {
-            for (int r = w[0].run + p.run_cap; r < min(p.splits, kNeutralSlots); r += p.run_cap) neutral(base + c, r);
-            if (w[0].run >= w[0].runs) neutral(base + c, w[0].run);
-        }
         if (w[0].run < w[0].runs) {
         const size_t head_byte = (size_t)kvh * p.stride * kRowBytes;   // (the columns share the cache)
         const int first = w[0].row0 + unit * warp;
@@ -206,8 +216,16 @@ __global__ void __launch_bounds__(kThreads, 1) attn_decode_cols(DecodeParams p, 
 #pragma unroll
             for (int c = 0; c < kCols; c++) {
                 if (c >= n) break;
+                const int live = min(unit, w[c].row1 - r0);
+                if (live <= 0) {   // the unit begins past this column's end: it adds nothing
+#pragma unroll
+                    for (int j = 0; j < kT; j++)
+#pragma unroll
+                        for (int e = 0; e < 2; e++) ph[c][j][e] = pl[c][j][e] = __float2half2_rn(0.0f);
+                    continue;
+                }
                 float corr[2];
-                if (softmax<kT>(s[c], min(unit, w[c].row1 - r0), g, run[c], ph[c], pl[c], corr) && i > 0) {
+                if (softmax<kT>(s[c], live, g, run[c], ph[c], pl[c], corr) && i > 0) {
 #pragma unroll 1
                     for (int m = 0; m < 4; m++) {
                         float a[16];
@@ -342,8 +360,12 @@ __global__ void __launch_bounds__(kThreads, 1) attn_decode_cols(DecodeParams p, 
         cluster_wait();
         __syncthreads();
         if (lane == 0) fence_async_shared();   // partials were written over the rings; a next round's copies follow
-        }   // run with rows
+        }   // a live run of these columns
         base += n;
+        if (base >= end) {   // the cluster's next group of columns
+            base = sh.base += sh.stride;
+            end = min(base + sh.each, p.n_slots);
+        }
     }
     if (!landed && status) atomicCAS(status, 0, 21);
     tc_fence_before();
@@ -373,11 +395,10 @@ int setup(int **status) {
 
 }  // namespace
 
-int launch_decode_cols(cudaStream_t stream, const DecodeParams &p, int cols) {
+int launch_decode_cols(cudaStream_t stream, const DecodeParams &p) {
     int *status = nullptr;
     if (int e = setup(&status)) return e;
-    const dim3 grid(p.n_kv * min(p.splits, p.run_cap) * kC, (cols + kCols - 1) / kCols);
-    return launch_pdl(attn_decode_cols, grid, dim3(kThreads), (size_t)Cfg::kSmem, stream, kC, p, status);
+    return launch_pdl(attn_decode_cols, dim3(p.n_kv * min(p.splits, p.run_cap) * kC), dim3(kThreads), (size_t)Cfg::kSmem, stream, kC, p, status);
 }
 
 }  // namespace hipml

@@ -591,7 +591,7 @@ int launch(cudaStream_t stream, const DecodeParams &p, int slots) {
     // several columns over one cache: side by side (not with the tail of an exchange)
     const bool columns = !kQ4 && kC == 2 && kWide && slots > 1 && q.kv_slot_bytes == 0 && q.k_row == nullptr &&
                          q.xch.phases == 0;
-    const int rc = columns ? launch_decode_cols(stream, q, slots)
+    const int rc = columns ? launch_decode_cols(stream, q)
                            : launch_pdl(attn_decode_warps<kQ4, kC, kWide>, grid, dim3(kThreads),
                                         (size_t)Cfg<kQ4, kWide>::kSmem, stream, kC, q, status);
     if (rc != 0 || !second_launch) return rc;

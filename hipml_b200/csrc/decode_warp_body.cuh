@@ -545,42 +545,52 @@ __device__ __forceinline__ int div_up(int a, int b) { return (a + b - 1) / b; }
 
 // The balanced plan of one stream: every warp of every run gets a unit before any gets two, and units
 // are 16 rows as long as one each is enough (half the latency of a short step), then 32 (an eighth
-// fewer instructions per row).
+// fewer instructions per row). Units are counted in eights, so that neighbouring columns of a stream
+// mostly share a plan; the last few can be empty.
 struct Balance {
-    int unit, runs;
+    int unit, units, runs;
 };
 __device__ __forceinline__ Balance balance(const DecodeParams &p, int len, int ctas, int most) {
     const int cap = min(p.splits, p.run_cap), warps = kWarps * ctas;
     Balance b;
     b.unit = div_up(len, 16) <= cap * warps ? 16 : most;
-    b.runs = max(1, min(div_up(div_up(len, b.unit), warps), cap));
+    b.units = div_up(len, b.unit * 8) * 8;
+    b.runs = max(1, min(div_up(b.units, warps), cap));
     return b;
 }
 
-// One stream, or a column of one, of `len` live rows.
+// Run `run` of a head under the balanced plan.
 template <int kC, int kUnitRows>
-__device__ __forceinline__ Work plan_stream(const DecodeParams &p, int slot, int rank, int len) {
+__device__ __forceinline__ Work plan_run(const DecodeParams &p, int slot, int kvh, int run, int rank, int len) {
+    const Balance b = balance(p, len, kC, kUnitRows);
     Work w;
     w.slot = slot;
     w.len = len;
+    w.kvh = kvh;
+    w.run = run;
+    w.runs = b.runs;
+    w.unit = b.unit;
+    w.row0 = w.row1 = 0;
+    if (run < b.runs) {
+        const int c0 = (int)((long long)run * b.units / b.runs), c1 = (int)((long long)(run + 1) * b.units / b.runs);
+        w.row0 = (c0 + (c1 - c0) * rank / kC) * b.unit;   // (past the end for a CTA without rows)
+        w.row1 = min((c0 + (c1 - c0) * (rank + 1) / kC) * b.unit, len);
+    }
+    return w;
+}
+
+// One stream of `len` live rows.
+template <int kC, int kUnitRows>
+__device__ __forceinline__ Work plan_stream(const DecodeParams &p, int slot, int rank, int len) {
     const int cluster = (int)blockIdx.x / kC;
     if (!p.by_stride && p.run_cap > 0) {
-        const int cap = min(p.splits, p.run_cap);
-        const Balance b = balance(p, len, kC, kUnitRows);
-        w.kvh = cluster / cap;
-        w.run = cluster - w.kvh * cap;
-        w.runs = b.runs;
-        w.unit = b.unit;
-        w.row0 = w.row1 = 0;
-        if (w.run < w.runs) {
-            const int units = div_up(len, b.unit);
-            const int c0 = (int)((long long)w.run * units / w.runs), c1 = (int)((long long)(w.run + 1) * units / w.runs);
-            w.row0 = min((c0 + (c1 - c0) * rank / kC) * b.unit, len);
-            w.row1 = min((c0 + (c1 - c0) * (rank + 1) / kC) * b.unit, len);
-        }
-        return w;
+        const int cap = min(p.splits, p.run_cap), kvh = cluster / cap;
+        return plan_run<kC, kUnitRows>(p, slot, kvh, cluster - kvh * cap, rank, len);
     }
     // fixed runs of ceil(span / splits) rows, rounded up to 64
+    Work w;
+    w.slot = slot;
+    w.len = len;
     w.kvh = cluster / p.splits;
     w.run = cluster - w.kvh * p.splits;
     w.runs = p.splits;

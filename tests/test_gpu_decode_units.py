@@ -73,7 +73,7 @@ def test_lengths_that_change_between_launches_are_seen():
 
 # columns whose lengths cross a 16- or 32-row unit, the change of the unit (4,608) or nothing
 @pytest.mark.parametrize("cols", [2, 4, 5, 8])
-@pytest.mark.parametrize("pos0", [0, 13, 29, 200, 4604, 9214])
+@pytest.mark.parametrize("pos0", [0, 13, 29, 125, 200, 1278, 4604, 9214])
 def test_columns_side_by_side_give_each_columns_own_bits(pos0, cols):
     from hipml_b200 import api
     heads, n_kv, hd, scale, stride = 24, 4, 256, 0.0625, pos0 + cols + 2
