@@ -23,22 +23,24 @@ namespace {
 using namespace warp_body;
 
 constexpr int kCols = 4;          // columns side by side
-constexpr int kC = 2;             // CTAs per cluster, as the single-column form
 constexpr int kUnitRows = 32;
 constexpr unsigned kTmemCols = 512;
+constexpr int kMaxCols = 64;      // of a launch
 
 struct Cfg {
     static constexpr int kSlot = kUnitRows * kRowBytes;
-    static constexpr int kRing = 2 * kSlot;                        // per warp: a unit of K and one of V; later a partial
-    static_assert(kRing >= 8 * kHeadPitch * 4, "a warp's partial fits its ring");
+    static constexpr int kRing = 2 * kSlot;                        // per warp: a unit of K and one of V; later two partials
+    static constexpr int kPartial = 8 * kHeadPitch * 4;
+    static_assert(kRing >= 2 * kPartial, "a warp's partials fit its ring");
     static constexpr int kQBytes = 16 * 32 * 16;                   // a column's query fragments, later its partial of the CTA
     static constexpr int kBiasBytes = 8 * 4 * 16;
     static constexpr int kOffQ = kWarps * kRing;
     static constexpr int kOffBias = kOffQ + kCols * kQBytes;
-    static constexpr int kOffMl = kOffBias + kCols * kBiasBytes;   // [8 heads][warps] {reference, sum}
-    static constexpr int kOffCml = kOffMl + kWarps * 8 * 8;        // per column [8 heads]
+    static constexpr int kOffMl = kOffBias + kCols * kBiasBytes;   // two columns' [8 heads][warps] {reference, sum}
+    static constexpr int kOffCml = kOffMl + 2 * kWarps * 8 * 8;    // per column [8 heads]
     static constexpr int kOffBar = kOffCml + kCols * 8 * 8;
-    static constexpr int kSmem = kOffBar + kWarps * 2 * 8;
+    static constexpr int kOffFold = kOffBar + kWarps * 2 * 8 + 8;  // weights of the last fold, after its barrier
+    static constexpr int kSmem = kOffFold + kCols * 5 * kStagedRow * 8;
     static_assert(kSmem + 1024 <= 227 * 1024, "one CTA per SM");
 };
 
@@ -51,10 +53,10 @@ __device__ int g_arrive_cols[kArriveRegions * kArriveRegionInts];
 struct Share {
     int base, each, stride, run;
 };
-template <class LenOf>
-__device__ __forceinline__ Share share_columns(const DecodeParams &p, int cap, int in_head, LenOf len_of) {
+template <int kC>
+__device__ __forceinline__ Share share_columns(const DecodeParams &p, int cap, int in_head, const int *len) {
     int runs = 1;
-    for (int c = threadIdx.x & 31; c < p.n_slots; c += 32) runs = max(runs, balance(p, len_of(c), kC, kUnitRows).runs);
+    for (int c = threadIdx.x & 31; c < p.n_slots; c += 32) runs = max(runs, balance(p, len[c], kC, kUnitRows).runs);
     runs = __reduce_max_sync(0xffffffffu, runs);
     const int side = cap / runs;   // groups side by side, >= 1
     Share s;
@@ -65,12 +67,14 @@ __device__ __forceinline__ Share share_columns(const DecodeParams &p, int cap, i
     return s;
 }
 
-// grid (n_kv * runs * kC), clusters of kC.
+// grid (n_kv * runs * kC), clusters of kC as in the single-column form.
+template <int kC>
 __global__ void __launch_bounds__(kThreads, 1) attn_decode_cols(DecodeParams p, int *status) {
     using C = Cfg;
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ int s_last;
     __shared__ unsigned s_tmem;
+    __shared__ int s_len[kMaxCols];
     griddep_launch();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int g = lane >> 2, t = lane & 3;
@@ -78,38 +82,70 @@ __global__ void __launch_bounds__(kThreads, 1) attn_decode_cols(DecodeParams p, 
     const int rank = (int)cluster_rank();
     unsigned char *const ring = smem + warp * C::kRing;
     const unsigned ring_addr = smem_u32(ring), bar = smem_u32(smem + C::kOffBar) + warp * 16;
+    const unsigned bar_fold = smem_u32(smem + C::kOffFold) - 8;
     if (lane == 0) {
         mbar_init(bar, 1);
         mbar_init(bar + 8, 1);
+        if (warp == 0) mbar_init(bar_fold, 1);
         mbar_init_fence();
     }
     if (warp == 0) tmem_alloc<1>(smem_u32(&s_tmem), kTmemCols);
     const int cap = min(p.splits, p.run_cap), cluster = (int)blockIdx.x / kC;
     const int kvh = cluster / cap, in_head = cluster - kvh * cap;
-    const int *const len_at = p.len + p.len_offset;
-    auto len_of = [&](int col) { return min(max(__ldcg(len_at + col * p.len_stride), 0), p.stride); };
-    // Nothing that the grids ahead may write can be relied on yet, but the lengths as they stand are a good
-    // guess: enough to ask L2 for the first rows (the cache rows themselves are read later).
-    Share sh = share_columns(p, cap, in_head, len_of);
-    if (sh.base < p.n_slots) {
-        const Work w = plan_run<kC, kUnitRows>(p, sh.base, kvh, sh.run, rank, len_of(sh.base));
-        const int first = w.row0 + w.unit * warp;
-        if (lane == 0 && first < w.row1) {
-            const size_t at = ((size_t)kvh * p.stride + first) * kRowBytes;
-            const unsigned bytes = (unsigned)(min(w.unit, w.row1 - first) * kRowBytes);
-            prefetch_l2(p.k + at, bytes);
-            prefetch_l2(p.v + at, bytes);
+    // Nothing that the grids ahead may write can be relied on before they are done, but the lengths as they
+    // stand are a good guess: enough to plan with and to ask L2 for the first rows. They are checked below.
+    auto read_len = [&]() {   // of column tid < n_slots
+        return min(max(__ldcg(p.len + p.len_offset + tid * p.len_stride), 0), p.stride);
+    };
+    if (tid < p.n_slots) s_len[tid] = read_len();
+    __syncthreads();
+    const size_t head_byte = (size_t)kvh * p.stride * kRowBytes;   // (the columns share the cache)
+    Share sh = share_columns<kC>(p, cap, in_head, s_len);
+    int base = sh.base, end = min(base + sh.each, p.n_slots);
+    // Columns base .. base + n - 1 share a plan: the same units for every warp. (Ascending lengths rarely leave
+    // it; then the rest of the group is another round.)
+    int n, len[kCols], first, row1, nw;
+    bool live;
+    Work w;
+    size_t step;
+    const unsigned char *kp, *vp;
+    auto plan = [&]() {
+        live = false;
+        nw = n = 0;
+        if (base >= p.n_slots) return;
+        const Balance b0 = balance(p, s_len[base], kC, kUnitRows);
+        n = 1;
+        int longest = 0;
+#pragma unroll
+        for (int c = 0; c < kCols; c++) {
+            len[c] = base + c < end ? s_len[base + c] : 0;
+            const Balance b = balance(p, len[c], kC, kUnitRows);
+            if (c > 0 && n == c && base + c < end && b.units == b0.units && b.unit == b0.unit && b.runs == b0.runs) n = c + 1;
+            if (n > c) longest = max(longest, len[c]);
         }
+        w = plan_run<kC>(b0, base, kvh, sh.run, rank, longest);
+        live = w.run < w.runs;
+        first = w.row0 + w.unit * warp;
+        row1 = w.row1;
+        nw = live && first < row1 ? div_up(row1 - first, w.unit * kWarps) : 0;
+        step = (size_t)w.unit * kWarps * kRowBytes;
+        kp = p.k + head_byte + (size_t)first * kRowBytes;
+        vp = p.v + head_byte + (size_t)first * kRowBytes;
+    };
+    auto unit_bytes = [&](int i) { return (unsigned)(min(w.unit, row1 - (first + i * w.unit * kWarps)) * kRowBytes); };
+    auto fetch = [&](int i, const unsigned char *src, int slot) {   // unit i: one lane
+        const unsigned bytes = unit_bytes(i);
+        mbar_arrive_expect_tx(bar + 8 * slot, bytes);
+        bulk_load(ring_addr + slot * C::kSlot, src, bytes, bar + 8 * slot);
+    };
+    plan();
+    if (lane == 0 && nw > 0) {
+        prefetch_l2(kp, unit_bytes(0));
+        prefetch_l2(vp, unit_bytes(0));
     }
     griddep_wait();
-    sh = share_columns(p, cap, in_head, len_of);
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    // this warp's accumulators of column c: lanes 32 * (warp % 4), columns 128 c + 64 * (warp / 4)
-    const unsigned tmem = s_tmem + ((unsigned)(warp & 3) << 21) + 64u * (warp >> 2);
-    unsigned phase = 0;
-    bool landed = true;
+    unsigned phase = 0, fold_phase = 0;
+    bool landed = true, checked = false;
     auto wait = [&](int slot) {
         unsigned spin = 0;
         while (!mbar_try_wait(bar + 8 * slot, phase)) {
@@ -120,70 +156,67 @@ __global__ void __launch_bounds__(kThreads, 1) attn_decode_cols(DecodeParams p, 
         }
     };
 
-    for (int base = sh.base, end = min(base + sh.each, p.n_slots); base < p.n_slots;) {
-        // Columns base .. base + n - 1 share a plan: the same units for every warp. (Ascending lengths rarely
-        // leave it; then the rest of the group is another round.)
-        Work w[kCols];
-        int n = 1;
-        const Balance b0 = balance(p, len_of(base), kC, kUnitRows);
+    for (;;) {
+        const int real_len = !checked && tid < p.n_slots ? read_len() : 0;
+        // Query fragments of every column, warp b makes block b's (as in the single-column body).
+        float2 x[kCols][2][2];
 #pragma unroll
         for (int c = 0; c < kCols; c++) {
-            const int len = base + c < end ? len_of(base + c) : 0;
-            w[c] = plan_run<kC, kUnitRows>(p, base + c, kvh, sh.run, rank, len);
-            const Balance b = balance(p, len, kC, kUnitRows);
-            if (c > 0 && n == c && base + c < end && b.units == b0.units && b.unit == b0.unit && b.runs == b0.runs) n = c + 1;
+            const float *const qh = p.q + (size_t)(base + c) * p.q_slot + (size_t)(kvh * group + g) * 256;
+#pragma unroll
+            for (int k = 0; k < 2; k++)
+#pragma unroll
+                for (int i = 0; i < 2; i++) {
+                    x[c][k][i] = make_float2(0.0f, 0.0f);
+                    if (g < group && c < n)
+                        x[c][k][i] = *reinterpret_cast<const float2 *>(qh + k_word_dim(warp, 4 * k + t, 2 * i));
+                }
         }
-        const int unit = w[0].unit;
-        int row1 = w[0].row1;
+        if (lane == 0 && nw > 0) {
+            fetch(0, kp, 0);
+            fetch(0, vp, 1);
+        }
 #pragma unroll
-        for (int c = 1; c < kCols; c++)
-            if (c < n) row1 = max(row1, w[c].row1);
-        if (w[0].run < w[0].runs) {
-        const size_t head_byte = (size_t)kvh * p.stride * kRowBytes;   // (the columns share the cache)
-        const int first = w[0].row0 + unit * warp;
-        const int nw = first < row1 ? div_up(row1 - first, unit * kWarps) : 0;
-        const size_t step = (size_t)unit * kWarps * kRowBytes;
-        const unsigned char *kp = p.k + head_byte + (size_t)first * kRowBytes;
-        const unsigned char *vp = p.v + head_byte + (size_t)first * kRowBytes;
-        auto fetch = [&](int i, const unsigned char *src, int slot) {   // unit i: one lane
-            const unsigned bytes = (unsigned)(min(unit, row1 - (first + i * unit * kWarps)) * kRowBytes);
-            mbar_arrive_expect_tx(bar + 8 * slot, bytes);
-            bulk_load(ring_addr + slot * C::kSlot, src, bytes, bar + 8 * slot);
-        };
-        // Query fragments of every column, warp b makes block b's (as in the single-column body).
-        {
-            float2 x[kCols][2][2];
-#pragma unroll
-            for (int c = 0; c < kCols; c++) {
-                const float *const qh = p.q + (size_t)(base + c) * p.q_slot + (size_t)(kvh * group + g) * 256;
-#pragma unroll
-                for (int k = 0; k < 2; k++)
-#pragma unroll
-                    for (int i = 0; i < 2; i++) {
-                        x[c][k][i] = make_float2(0.0f, 0.0f);
-                        if (g < group && c < n)
-                            x[c][k][i] = *reinterpret_cast<const float2 *>(qh + k_word_dim(warp, 4 * k + t, 2 * i));
-                    }
-            }
-            if (lane == 0 && nw > 0) {
-                fetch(0, kp, 0);
-                fetch(0, vp, 1);
-            }
-#pragma unroll
-            for (int c = 0; c < kCols; c++) {
-                if (c >= n) break;
+        for (int c = 0; c < kCols; c++)
+            if (c < n)
                 store_query<false>(x[c], p.scale_log2, warp, lane, reinterpret_cast<uint4 *>(smem + C::kOffQ + c * C::kQBytes),
                                    reinterpret_cast<float *>(smem + C::kOffBias + c * C::kBiasBytes));
+        tc_fence_before();
+        if (checked) {
+            __syncthreads();
+        } else if (__syncthreads_or(tid < p.n_slots && real_len != s_len[tid])) {
+            // Rare: the lengths changed after they were first looked at. What was fetched lands, unused (its
+            // slots' barriers start over), and the CTA plans again.
+            if (lane == 0 && nw > 0) {
+                for (int i = 0; i < 2; i++) {
+                    for (unsigned spin = 0; !mbar_try_wait(bar + 8 * i, 0) && spin < kSpinLimit; spin++) {}
+                    mbar_inval(bar + 8 * i);
+                    mbar_init(bar + 8 * i, 1);
+                }
+                mbar_init_fence();
             }
+            if (tid < p.n_slots) s_len[tid] = real_len;
+            __syncthreads();
+            sh = share_columns<kC>(p, cap, in_head, s_len);
+            base = sh.base;
+            end = min(base + sh.each, p.n_slots);
+            plan();
+            checked = true;
+            continue;
         }
-        __syncthreads();
+        checked = true;
+        tc_fence_after();
+        if (base >= p.n_slots) break;
+        if (live) {
+        // this warp's accumulators of column c: lanes 32 * (warp % 4), columns 128 c + 64 * (warp / 4)
+        const unsigned tmem = s_tmem + ((unsigned)(warp & 3) << 21) + 64u * (warp >> 2);
 
         Running run[kCols];
 #pragma unroll
         for (int c = 0; c < kCols; c++) start(run[c]);
         auto work = [&](auto tiles, int i, int rows) __attribute__((always_inline)) {
             constexpr int kT = decltype(tiles)::value;
-            const int r0 = first + i * unit * kWarps;
+            const int r0 = first + i * w.unit * kWarps;
             // ---- scores of all columns
             wait(0);
             float s[kCols][kT][4];
@@ -216,8 +249,8 @@ __global__ void __launch_bounds__(kThreads, 1) attn_decode_cols(DecodeParams p, 
 #pragma unroll
             for (int c = 0; c < kCols; c++) {
                 if (c >= n) break;
-                const int live = min(unit, w[c].row1 - r0);
-                if (live <= 0) {   // the unit begins past this column's end: it adds nothing
+                const int rows_c = min(w.unit, min(row1, len[c]) - r0);
+                if (rows_c <= 0) {   // the unit begins past this column's end: it adds nothing
 #pragma unroll
                     for (int j = 0; j < kT; j++)
 #pragma unroll
@@ -225,7 +258,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_decode_cols(DecodeParams p, 
                     continue;
                 }
                 float corr[2];
-                if (softmax<kT>(s[c], live, g, run[c], ph[c], pl[c], corr) && i > 0) {
+                if (softmax<kT>(s[c], rows_c, g, run[c], ph[c], pl[c], corr) && i > 0) {
 #pragma unroll 1
                     for (int m = 0; m < 4; m++) {
                         float a[16];
@@ -290,72 +323,90 @@ __global__ void __launch_bounds__(kThreads, 1) attn_decode_cols(DecodeParams p, 
             phase ^= 1;
         };
         for (int i = 0; i < nw; i++) {
-            const int rows = min(unit, row1 - (first + i * unit * kWarps));
+            const int rows = min(w.unit, row1 - (first + i * w.unit * kWarps));
             if (rows > 16)
                 work(Int<2>{}, i, rows);
             else
                 work(Int<1>{}, i, rows);
         }
 
-        // ---- merge: the warps of the CTA column by column, then the cluster, then the runs
+        // ---- merge: the warps of the CTA, two columns at a time, then the cluster, then the runs
         const int items = group * 64;
-        const bool one_run = w[0].runs == 1 && p.out != nullptr;
+        const bool one_run = w.runs == 1 && p.out != nullptr;
         float2 *const wml = reinterpret_cast<float2 *>(smem + C::kOffMl);
         auto cpart = [&](int c) { return reinterpret_cast<float4 *>(smem + C::kOffQ + c * C::kQBytes); };
         auto cml = [&](int c) { return reinterpret_cast<float2 *>(smem + C::kOffCml) + 8 * c; };
 #pragma unroll
-        for (int c = 0; c < kCols; c++) {
-            if (c >= n) break;
-            sum_rows(run[c]);
-            if (g == 0) {
-                wml[(2 * t) * kWarps + warp] = make_float2(run[c].m[0], run[c].l[0]);
-                wml[(2 * t + 1) * kWarps + warp] = make_float2(run[c].m[1], run[c].l[1]);
-            }
-            float acc[8][2][4];
+        for (int c0 = 0; c0 < kCols; c0 += 2) {
+            if (c0 >= n) break;
 #pragma unroll
-            for (int m = 0; m < 4; m++) {
-                float a[16];
+            for (int c = c0; c < c0 + 2; c++) {
+                if (c >= n) break;
+                sum_rows(run[c]);
+                float2 *const ml = wml + (c - c0) * 8 * kWarps;
+                if (g == 0) {
+                    ml[(2 * t) * kWarps + warp] = make_float2(run[c].m[0], run[c].l[0]);
+                    ml[(2 * t + 1) * kWarps + warp] = make_float2(run[c].m[1], run[c].l[1]);
+                }
+                float a[4][16];
 #pragma unroll
-                for (int e = 0; e < 16; e++) a[e] = 0.0f;
+                for (int m = 0; m < 4; m++)
+#pragma unroll
+                    for (int e = 0; e < 16; e++) a[m][e] = 0.0f;
                 if (nw > 0) {
-                    tmem_ld16(tmem + 128 * c + 16 * m, a);
+#pragma unroll
+                    for (int m = 0; m < 4; m++) tmem_ld16(tmem + 128 * c + 16 * m, a[m]);
                     tmem_wait_ld();
                 }
+                float acc[8][2][4];
 #pragma unroll
-                for (int e = 0; e < 16; e++) acc[2 * m + (e >> 3)][(e >> 2) & 1][e & 3] = a[e];
+                for (int m = 0; m < 4; m++)
+#pragma unroll
+                    for (int e = 0; e < 16; e++) acc[2 * m + (e >> 3)][(e >> 2) & 1][e & 3] = a[m][e];
+                store_warp_partial<false>(reinterpret_cast<float *>(ring + (c - c0) * C::kPartial), acc, group, g, t);
             }
-            store_warp_partial<false>(reinterpret_cast<float *>(ring), acc, group, g, t);
             __syncthreads();
-            fold_warps(smem, C::kRing, wml, items, [&](int item, const Part &r) {
-                cpart(c)[item] = r.a;
-                if ((item & 63) == 0) cml(c)[item >> 6] = make_float2(r.m, r.l);
-            });
-            __syncthreads();
+#pragma unroll
+            for (int c = c0; c < c0 + 2; c++)
+                if (c < n)
+                    fold_warps(smem + (c - c0) * C::kPartial, C::kRing, wml + (c - c0) * 8 * kWarps, items,
+                               [&](int item, const Part &r) {
+                                   cpart(c)[item] = r.a;
+                                   if ((item & 63) == 0) cml(c)[item >> 6] = make_float2(r.m, r.l);
+                               });
+            if (c0 + 2 < n) __syncthreads();
         }
         cluster_sync_all();
-        for (int c = 0; c < n; c++) {
-            const int col = base + c;
-            fold_cluster<kC>(cpart(c), cml(c), items, rank, [&](int item, const Part &r) {
-                if (one_run) emit_item(p, col, kvh, group, item, r);
-                const size_t row = (size_t)(kvh * group + (item >> 6)) * p.splits + w[0].run;
-                reinterpret_cast<float4 *>(p.part_acc + (size_t)col * p.acc_slot + row * 256)[item & 63] = r.a;
-                if ((item & 63) == 0)
-                    *reinterpret_cast<float2 *>(p.part_ml + (size_t)col * p.ml_slot + row * 2) = make_float2(r.m, r.l);
-            });
-        }
+        fold_cluster<kC, kCols>(cpart(0), cml(0), C::kQBytes / 16, n, items, rank, [&](int c, int item, const Part &r) {
+            if (one_run) emit_item(p, base + c, kvh, group, item, r);
+            const size_t row = (size_t)(kvh * group + (item >> 6)) * p.splits + w.run;
+            reinterpret_cast<float4 *>(p.part_acc + (size_t)(base + c) * p.acc_slot + row * 256)[item & 63] = r.a;
+            if ((item & 63) == 0)
+                *reinterpret_cast<float2 *>(p.part_ml + (size_t)(base + c) * p.ml_slot + row * 2) = make_float2(r.m, r.l);
+        });
         cluster_arrive();   // no CTA may leave, or start over, while another still reads its partials
         if (p.out != nullptr && !one_run) {
             int *const ctr = g_arrive_cols + (size_t)p.arrive_region * kArriveRegionInts +
                              (size_t)(base * p.n_kv + kvh) * p.arrive_stride + rank;
             __syncthreads();
             if (tid == 0) {
-                const int last = arrive_acq_rel(ctr) == w[0].runs - 1;
+                const int last = arrive_acq_rel(ctr) == w.runs - 1;
                 if (last) *ctr = 0;
                 s_last = last;
             }
             __syncthreads();
-            if (s_last)
-                for (int c = 0; c < n; c++) fold_runs<kC>(p, base + c, kvh, group, w[0].runs, rank, nullptr);
+            if (s_last) {
+                // as many columns at a time as fit the rings
+                const int slice = (items / kC + 1) * w.runs * 16, fit = max(1, min(n, kWarps * C::kRing / slice));
+                for (int c = 0; c < n; c += fit) {
+                    const int m = min(fit, n - c);
+                    if (fold_runs_staged<kC>(p, base + c, m, kvh, group, w.runs, rank, smem, kWarps * C::kRing, bar_fold,
+                                             fold_phase, reinterpret_cast<float2(*)[kStagedRow]>(smem + C::kOffFold), landed))
+                        fold_phase ^= 1;
+                    else
+                        fold_runs<kC, 1, 8>(p, base + c, m, kvh, group, w.runs, rank, nullptr);
+                }
+            }
         }
         cluster_wait();
         __syncthreads();
@@ -366,6 +417,8 @@ __global__ void __launch_bounds__(kThreads, 1) attn_decode_cols(DecodeParams p, 
             base = sh.base += sh.stride;
             end = min(base + sh.each, p.n_slots);
         }
+        plan();
+        if (base >= p.n_slots) break;
     }
     if (!landed && status) atomicCAS(status, 0, 21);
     tc_fence_before();
@@ -376,29 +429,31 @@ __global__ void __launch_bounds__(kThreads, 1) attn_decode_cols(DecodeParams p, 
     }
 }
 
-int setup(int **status) {
+template <int kC>
+int launch(cudaStream_t stream, const DecodeParams &p) {
     static std::mutex mu;
     static int *status_word[64] = {};   // nullptr: device not set up yet
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) dev = 0;
-    std::lock_guard<std::mutex> lock(mu);
-    if (status_word[dev] == nullptr) {
-        const cudaError_t e = cudaFuncSetAttribute(attn_decode_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem);
-        if (e != cudaSuccess) return (int)e;
-        status_word[dev] = device_status_word();
-        if (status_word[dev] == nullptr) return launch_status();
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        if (status_word[dev] == nullptr) {
+            const cudaError_t e =
+                cudaFuncSetAttribute(attn_decode_cols<kC>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem);
+            if (e != cudaSuccess) return (int)e;
+            status_word[dev] = device_status_word();
+            if (status_word[dev] == nullptr) return launch_status();
+        }
     }
-    *status = status_word[dev];
-    return 0;
+    return launch_pdl(attn_decode_cols<kC>, dim3(p.n_kv * min(p.splits, p.run_cap) * kC), dim3(kThreads),
+                      (size_t)Cfg::kSmem, stream, kC, p, status_word[dev]);
 }
 
 }  // namespace
 
-int launch_decode_cols(cudaStream_t stream, const DecodeParams &p) {
-    int *status = nullptr;
-    if (int e = setup(&status)) return e;
-    return launch_pdl(attn_decode_cols, dim3(p.n_kv * min(p.splits, p.run_cap) * kC), dim3(kThreads), (size_t)Cfg::kSmem, stream, kC, p, status);
+int launch_decode_cols(cudaStream_t stream, const DecodeParams &p, int cluster) {
+    return cluster == 8 ? launch<8>(stream, p) : launch<2>(stream, p);
 }
 
 }  // namespace hipml

@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(kThreads, 2) attn_decode_rows_f32(ColsParams p
     });
     cluster_sync_all();
     const bool one = clusters == 1 && d.out != nullptr;
-    fold_cluster<kF32Cluster>(cpart, cml, items, rank, [&](int item, const Part &r) {
+    fold_cluster<kF32Cluster, 1>(cpart, cml, 0, 1, items, rank, [&](int, int item, const Part &r) {
         if (one) {
             emit_item(d, col, kvh, group, item, r);
             return;
@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(kThreads, 2) attn_decode_rows_f32(ColsParams p
             s_last = last;
         }
         __syncthreads();
-        if (s_last) fold_runs<kF32Cluster>(d, col, kvh, group, clusters, rank, nullptr);
+        if (s_last) fold_runs<kF32Cluster, 1, 8>(d, col, 1, kvh, group, clusters, rank, nullptr);
     }
     cluster_wait();
 }

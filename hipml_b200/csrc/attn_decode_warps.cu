@@ -60,8 +60,8 @@ struct Cfg {
     static constexpr int kOffMl = kOffBias + 8 * 4 * 16;           // [8 heads][warps] {reference, sum}
     static constexpr int kOffCml = kOffMl + kWarps * 8 * 8;        // [8 heads] {reference, sum} of the CTA
     static constexpr int kOffRow = kOffCml + 8 * 8;                // the row to append: K, V
-    static constexpr int kOffBar = kOffRow + 2 * kRow;
-    static constexpr int kSmem = kOffBar + kWarps * kSlots * 8;
+    static constexpr int kOffBar = kOffRow + 2 * kRow;             // a warp's slots each, then the last fold's
+    static constexpr int kSmem = kOffBar + kWarps * kSlots * 8 + 8;
     static_assert((kWide ? 1 : 2) * (kSmem + 512 + 1024) <= 228 * 1024, "CTAs per SM");
 };
 
@@ -136,9 +136,11 @@ __global__ void __launch_bounds__(kThreads, kWide ? 1 : 2) attn_decode_warps(Dec
     const int rank = kC > 1 ? (int)cluster_rank() : 0;
     unsigned char *const ring = smem + warp * C::kRing;
     const unsigned ring_addr = smem_u32(ring), bar = smem_u32(smem + C::kOffBar) + warp * C::kSlots * 8;
+    const unsigned bar_fold = smem_u32(smem + C::kSmem) - 8;
     if (lane == 0) {
 #pragma unroll
         for (int i = 0; i < C::kSlots; i++) mbar_init(bar + 8 * i, 1);
+        if (warp == 0) mbar_init(bar_fold, 1);
         mbar_init_fence();
     }
     uint4 *const qf = reinterpret_cast<uint4 *>(smem + C::kOffQ);
@@ -430,7 +432,7 @@ __global__ void __launch_bounds__(kThreads, kWide ? 1 : 2) attn_decode_warps(Dec
     // ---- merge of the cluster: this CTA folds slice `rank` of the items
     if constexpr (kC > 1) {
         cluster_sync_all();
-        fold_cluster<kC>(cpart, cml, items, rank, run_done);
+        fold_cluster<kC, 1>(cpart, cml, 0, 1, items, rank, [&](int, int item, const Part &r) { run_done(item, r); });
         // no CTA may leave while another still reads its partial
         cluster_arrive();
     }
@@ -446,7 +448,15 @@ __global__ void __launch_bounds__(kThreads, kWide ? 1 : 2) attn_decode_warps(Dec
                 s_plan[0] = last;
             }
             __syncthreads();
-            if (s_plan[0]) fold_runs<kC>(p, w.slot, w.kvh, group, w.runs, rank, nullptr);
+            if (s_plan[0]) {
+                // (in a cluster a CTA has half a head's items or less: ordinary loads, one trip for the runs of a
+                // deep stream, are as fast there)
+                if constexpr (kC > 1)
+                    fold_runs<kC, 1, 18>(p, w.slot, 1, w.kvh, group, w.runs, rank, nullptr);
+                else if (!fold_runs_staged<kC>(p, w.slot, 1, w.kvh, group, w.runs, rank, smem, kWarps * C::kRing, bar_fold, 0,
+                                               reinterpret_cast<float2(*)[kStagedRow]>(smem + C::kOffQ), landed))
+                    fold_runs<kC, 1, 8>(p, w.slot, 1, w.kvh, group, w.runs, rank, nullptr);
+            }
         } else {
             // the exchange wants whole heads in one CTA: the cluster arrives as one
             __threadfence();
@@ -465,7 +475,7 @@ __global__ void __launch_bounds__(kThreads, kWide ? 1 : 2) attn_decode_warps(Dec
                 __syncthreads();
                 if (s_plan[0]) {
                     float *const staged = reinterpret_cast<float *>(smem);
-                    for (int r = 0; r < kC; r++) fold_runs<kC>(p, w.slot, w.kvh, group, w.runs, r, staged);
+                    for (int r = 0; r < kC; r++) fold_runs<kC, 1, 8>(p, w.slot, 1, w.kvh, group, w.runs, r, staged);
                     __syncthreads();
                     FoldAcc f;
                     if (warp < group) {
@@ -509,7 +519,7 @@ __global__ void __launch_bounds__(kThreads) attn_decode_warps_fold(DecodeParams 
         runs = balance(p, len, kC, kUnitRows).runs;
     }
     const bool exchange = p.xch.phases != 0;
-    for (int r = 0; r < kC; r++) fold_runs<kC>(p, slot, kvh, group, runs, r, exchange ? staged : nullptr);
+    for (int r = 0; r < kC; r++) fold_runs<kC, 1, 8>(p, slot, 1, kvh, group, runs, r, exchange ? staged : nullptr);
     if (!exchange) return;
     __syncthreads();
     FoldAcc f;
@@ -589,9 +599,9 @@ int launch(cudaStream_t stream, const DecodeParams &p, int slots) {
         }
     }
     // several columns over one cache: side by side (not with the tail of an exchange)
-    const bool columns = !kQ4 && kC == 2 && kWide && slots > 1 && q.kv_slot_bytes == 0 && q.k_row == nullptr &&
+    const bool columns = !kQ4 && kC > 1 && kWide && slots > 1 && slots <= 64 && q.kv_slot_bytes == 0 && q.k_row == nullptr &&
                          q.xch.phases == 0;
-    const int rc = columns ? launch_decode_cols(stream, q)
+    const int rc = columns ? launch_decode_cols(stream, q, kC)
                            : launch_pdl(attn_decode_warps<kQ4, kC, kWide>, grid, dim3(kThreads),
                                         (size_t)Cfg<kQ4, kWide>::kSmem, stream, kC, q, status);
     if (rc != 0 || !second_launch) return rc;
@@ -608,12 +618,15 @@ int launch_c(cudaStream_t stream, const DecodeParams &p, int slots) {
 
 // Which form. One stream (or columns of one) has ~37 SMs per KV head: clusters of two, wide (8,192
 // rows: 11.5 us a layer, against 14.4 with two small CTAs per SM and 13.1 with clusters of four, of
-// which only 33 fit the device). Several slots: no clusters, a head has too few CTAs to pair them; wide
-// up to 16 (slot, head) pairs (3 slots of 512 .. 8,192 rows: 17.1 us against 19.7), beyond that the
-// twice as fine runs of the small CTAs balance better (16 slots: 43.0 us against 47.7).
+// which only 33 fit the device); clusters of eight up to the 1,023 rows that the engine's policy gives fewer
+// than 128 splits, where one holds a head and nothing is folded through memory (672 rows: KC8_TIME).
+// Several slots: no clusters, a head has too few CTAs to pair them; wide up to 16 (slot, head) pairs (3
+// slots of 512 .. 8,192 rows: 17.1 us against 19.7), beyond that the twice as fine runs of the small CTAs
+// balance better (16 slots: 43.0 us against 47.7).
 int launch_decode_warps(cudaStream_t stream, const DecodeParams &p, int slots) {
     const bool one_stream = !p.by_stride && p.run_cap >= 4 && p.share_slots == 0;
-    if (one_stream) return launch_c<2, true>(stream, p, slots);
+    if (one_stream)
+        return p.splits < 128 && p.run_cap >= 16 ? launch_c<8, true>(stream, p, slots) : launch_c<2, true>(stream, p, slots);
     return p.share_slots > 0 && slots * p.n_kv <= 16 ? launch_c<1, true>(stream, p, slots)
                                                      : launch_c<1, false>(stream, p, slots);
 }

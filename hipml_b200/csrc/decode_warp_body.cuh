@@ -387,13 +387,55 @@ __device__ __forceinline__ void fold_sources(int i0, int i1, Load load, Part (&r
     }
 }
 
-// How the threads of a CTA divide a slice of 1 / kC of a head group's items (at most 512): kShare
-// neighbouring threads per item, each with a contiguous share of the sources, joined by shuffles; or
-// kPer items per thread.
+// The same for sources in memory, independent of the batch: the maximum first (from the {m, l} pairs alone
+// where there is more than one batch), then the sum in source order.
+template <int kPer, int kBatch, class LoadMl, class Load>
+__device__ __forceinline__ void fold_memory(int i0, int i1, LoadMl load_ml, Load load, Part (&r)[kPer]) {
+#pragma unroll
+    for (int j = 0; j < kPer; j++) {
+        r[j].a = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        r[j].m = -INFINITY;
+        r[j].l = 0.0f;
+    }
+    const bool one_batch = i1 - i0 <= kBatch;
+    if (!one_batch) {
+        for (int s0 = i0; s0 < i1; s0 += 16)
+#pragma unroll
+            for (int i = 0; i < 16; i++)
+#pragma unroll
+                for (int j = 0; j < kPer; j++)
+                    if (s0 + i < i1) r[j].m = fmaxf(r[j].m, load_ml(s0 + i, j).x);
+    }
+    for (int s0 = i0; s0 < i1; s0 += kBatch) {
+        float4 x[kPer][kBatch];
+        float2 ml[kPer][kBatch];
+#pragma unroll
+        for (int i = 0; i < kBatch; i++)
+#pragma unroll
+            for (int j = 0; j < kPer; j++) {
+                x[j][i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                ml[j][i] = make_float2(-INFINITY, 0.0f);
+                if (s0 + i < i1) {
+                    x[j][i] = load(s0 + i, j);
+                    ml[j][i] = load_ml(s0 + i, j);
+                }
+            }
+#pragma unroll
+        for (int j = 0; j < kPer; j++) {
+            if (one_batch)
+#pragma unroll
+                for (int i = 0; i < kBatch; i++) r[j].m = fmaxf(r[j].m, ml[j][i].x);
+#pragma unroll
+            for (int i = 0; i < kBatch; i++) add(r[j], x[j][i], ml[j][i]);
+        }
+    }
+}
+
+// In a cluster of kC a CTA has 1 / kC of a head group's items (at most 512) to fold: kShare neighbouring
+// threads take an item, each with a contiguous share of the sources, joined by shuffles.
 template <int kC>
 struct Split {
     static constexpr int kShare = kC > 2 ? kC / 2 : 1;
-    static constexpr int kPer = kC == 1 ? 2 : 1;
 };
 template <int kShare>
 __device__ __forceinline__ void join(Part &r) {
@@ -430,9 +472,9 @@ __device__ __forceinline__ void store_warp_partial(float *dst, const float (&acc
 template <class Done>
 __device__ __forceinline__ void fold_warps(const unsigned char *partials, int pitch, const float2 *ml_at, int items,
                                            Done done) {
-    using S = Split<1>;
-    Part r[S::kPer];
-    fold_sources<S::kPer, kWarps>(
+    constexpr int kPer = 2;   // (at most 512 items)
+    Part r[kPer];
+    fold_sources<kPer, kWarps>(
         0, kWarps,
         [&](int i, int j, float4 &x, float2 &ml) {
             const int item = min((int)threadIdx.x + j * kThreads, items - 1);
@@ -441,28 +483,39 @@ __device__ __forceinline__ void fold_warps(const unsigned char *partials, int pi
         },
         r);
 #pragma unroll
-    for (int j = 0; j < S::kPer; j++)
+    for (int j = 0; j < kPer; j++)
         if ((int)threadIdx.x + j * kThreads < items) done(threadIdx.x + j * kThreads, r[j]);
 }
-// Folds slice `rank` of the items of the kC CTAs of a cluster (cpart: [item], cml: [8 heads], at the same
-// place in each of them).
-template <int kC, class Done>
-__device__ __forceinline__ void fold_cluster(const float4 *cpart, const float2 *cml, int items, int rank, Done done) {
-    using S = Split<kC>;
-    static_assert(S::kPer == 1 && kC % S::kShare == 0, "slices");
-    const int first = items * rank / kC, count = items * (rank + 1) / kC - first;
-    const int at = threadIdx.x / S::kShare, part = threadIdx.x % S::kShare, item = first + min(at, count - 1);
-    const unsigned area = smem_u32(cpart + item), ml_area = smem_u32(cml + (item >> 6));
-    Part r[1];
-    fold_sources<1, kC / S::kShare>(
-        part * (kC / S::kShare), (part + 1) * (kC / S::kShare),
-        [&](int i, int, float4 &x, float2 &ml) {
-            x = ld_cluster_f4(map_to_cta(area, i));
-            ml = ld_cluster_f2(map_to_cta(ml_area, i));
+// Folds slice `rank` of the items of the kC CTAs of a cluster, for each of `cols` <= kPer columns (partials of
+// [item] at cpart, {max, sum} of [8 heads] at cml, a column cpart_pitch / 8 further, at the same place in each
+// CTA); done(column, item, part).
+template <int kC, int kPer, class Done>
+__device__ __forceinline__ void fold_cluster(const float4 *cpart, const float2 *cml, int cpart_pitch, int cols, int items,
+                                             int rank, Done done) {
+    constexpr int kShare = Split<kC>::kShare;
+    static_assert(kC % kShare == 0, "slices");
+    const int first = items * rank / kC, count = items * (rank + 1) / kC - first, total = cols * count;
+    const int at = threadIdx.x / kShare, part = threadIdx.x % kShare;
+    int col[kPer], item[kPer];
+#pragma unroll
+    for (int j = 0; j < kPer; j++) {
+        const int f = min(at + j * (kThreads / kShare), total - 1);
+        col[j] = cols > 1 ? f / count : 0;
+        item[j] = first + f - col[j] * count;
+    }
+    Part r[kPer];
+    fold_sources<kPer, kC / kShare>(
+        part * (kC / kShare), (part + 1) * (kC / kShare),
+        [&](int i, int j, float4 &x, float2 &ml) {
+            x = ld_cluster_f4(map_to_cta(smem_u32(cpart + col[j] * cpart_pitch + item[j]), i));
+            ml = ld_cluster_f2(map_to_cta(smem_u32(cml + col[j] * 8 + (item[j] >> 6)), i));
         },
         r);
-    join<S::kShare>(r[0]);
-    if (at < count && part == 0) done(item, r[0]);
+#pragma unroll
+    for (int j = 0; j < kPer; j++) {
+        join<kShare>(r[j]);
+        if (at + j * (kThreads / kShare) < total && part == 0) done(col[j], item[j], r[j]);
+    }
 }
 
 // One float4 (item = head of the group * 64 + dims / 4) of the output: normalised (and gated), or
@@ -498,38 +551,114 @@ __device__ __forceinline__ void emit_item(const DecodeParams &p, int slot, int k
     }
 }
 
-// Folds the `runs` partials of slice `rank` of a head group from memory and emits it (or, staged !=
-// nullptr, leaves it there: [8 heads][256] sums, then [8 heads]{max, sum}).
-template <int kC>
-__device__ __forceinline__ void fold_runs(const DecodeParams &p, int slot, int kvh, int group, int runs, int rank,
-                                          float *staged) {
-    using S = Split<kC>;
-    const float *pa = p.part_acc + (size_t)slot * p.acc_slot + (size_t)kvh * group * p.splits * 256;
-    const float *pm = p.part_ml + (size_t)slot * p.ml_slot + (size_t)kvh * group * p.splits * 2;
+// Folds the `runs` partials of slice `rank` of a head group (of each of `cols` slots from `slot` on) from
+// memory and emits it (or, staged != nullptr, leaves it there: [8 heads][256] sums, then [8 heads]{max,
+// sum}). kPer items a thread, kBatch runs in one round trip: 18 for the runs of a deep stream (B200: 18 pairs
+// of SMs per KV head; three trips of 8 took 2.9 us at the end of every launch).
+template <int kC, int kPer, int kBatch>
+__device__ __forceinline__ void fold_runs(const DecodeParams &p, int slot, int cols, int kvh, int group, int runs,
+                                          int rank, float *staged) {
+    constexpr int kShare = Split<kC>::kShare;
     const int items = group * 64, first = items * rank / kC, count = items * (rank + 1) / kC - first;
-    const int at0 = threadIdx.x / S::kShare, part = threadIdx.x % S::kShare;
-    Part r[S::kPer];
-    fold_sources<S::kPer, S::kPer == 1 ? 10 : 8>(
-        runs * part / S::kShare, runs * (part + 1) / S::kShare,
-        [&](int i, int j, float4 &x, float2 &ml) {
-            const int item = first + min(at0 + j * kThreads, count - 1);
-            const size_t row = (size_t)(item >> 6) * p.splits + i;
-            x = __ldcg(reinterpret_cast<const float4 *>(pa + row * 256) + (item & 63));
-            ml = __ldcg(reinterpret_cast<const float2 *>(pm + row * 2));
-        },
-        r);
+    const int part = threadIdx.x % kShare, total = cols * count;
+    for (int f0 = threadIdx.x / kShare; f0 - (int)threadIdx.x / kShare < total; f0 += kPer * (kThreads / kShare)) {
+        const float *pa[kPer], *pm[kPer];
+        int item[kPer], col[kPer];
 #pragma unroll
-    for (int j = 0; j < S::kPer; j++) {
-        join<S::kShare>(r[j]);
-        const int item = first + at0 + j * kThreads;
-        if (at0 + j * kThreads >= count || part != 0) continue;
-        if (staged) {
-            reinterpret_cast<float4 *>(staged)[item] = r[j].a;
-            if ((item & 63) == 0) reinterpret_cast<float2 *>(staged + 8 * 256)[item >> 6] = make_float2(r[j].m, r[j].l);
-        } else {
-            emit_item(p, slot, kvh, group, item, r[j]);
+        for (int j = 0; j < kPer; j++) {
+            const int f = min(f0 + j * (kThreads / kShare), total - 1);
+            col[j] = cols > 1 ? f / count : 0;
+            item[j] = first + f - col[j] * count;
+            const int head = kvh * group + (item[j] >> 6);
+            pa[j] = p.part_acc + (size_t)(slot + col[j]) * p.acc_slot + (size_t)head * p.splits * 256 + 4 * (item[j] & 63);
+            pm[j] = p.part_ml + (size_t)(slot + col[j]) * p.ml_slot + (size_t)head * p.splits * 2;
+        }
+        Part r[kPer];
+        fold_memory<kPer, kBatch>(
+            runs * part / kShare, runs * (part + 1) / kShare,
+            [&](int i, int j) { return __ldcg(reinterpret_cast<const float2 *>(pm[j]) + i); },
+            [&](int i, int j) { return __ldcg(reinterpret_cast<const float4 *>(pa[j] + (size_t)i * 256)); }, r);
+#pragma unroll
+        for (int j = 0; j < kPer; j++) {
+            join<kShare>(r[j]);
+            if (f0 + j * (kThreads / kShare) >= total || part != 0) continue;
+            if (staged) {
+                reinterpret_cast<float4 *>(staged)[item[j]] = r[j].a;
+                if ((item[j] & 63) == 0)
+                    reinterpret_cast<float2 *>(staged + 8 * 256)[item[j] >> 6] = make_float2(r[j].m, r[j].l);
+            } else {
+                emit_item(p, slot + col[j], kvh, group, item[j], r[j]);
+            }
         }
     }
+}
+
+// The same fold, bit for bit, with the partials brought to shared memory by bulk copies: ordinary loads
+// keep ~25 KB of a CTA's in flight, and at ~1 us a trip the last CTA of a deep head (17 runs x 3 KB, four
+// times that for four columns) spent 2.3 and 8.4 us in them. `area`: `bytes` of shared memory that no copy
+// is in flight to, `bar`: a barrier in its phase `phase`. False (and nothing done) where they do not fit.
+constexpr int kStagedRow = 32;   // float2s: {weight, sum} of up to 31 runs, the maximum last
+template <int kC>
+__device__ __forceinline__ bool fold_runs_staged(const DecodeParams &p, int slot, int cols, int kvh, int group, int runs,
+                                                 int rank, unsigned char *area, int bytes, unsigned bar, unsigned phase,
+                                                 float2 (*s_ml)[kStagedRow], bool &landed) {
+    const int items = group * 64, first = items * rank / kC, count = items * (rank + 1) / kC - first;
+    if (runs >= kStagedRow || cols * runs * count * 16 > bytes) return false;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int head0 = first >> 6, heads = ((first + count - 1) >> 6) - head0 + 1;
+    auto pa = [&](int c, int head, int run) {
+        return p.part_acc + (size_t)(slot + c) * p.acc_slot + ((size_t)(kvh * group + head) * p.splits + run) * 256;
+    };
+    // generic writes (of this CTA to the area, of all CTAs to the partials) come before the copies' reads
+    asm volatile("fence.proxy.async;" ::: "memory");
+    __syncthreads();
+    if (tid == 0) mbar_arrive_expect_tx(bar, (unsigned)(cols * runs * count * 16));
+    __syncthreads();
+    const int pieces = cols * runs * heads;   // a head's part of the slice of one run
+    for (int i = tid; i < pieces; i += kThreads) {
+        const int h = i % heads, cr = i / heads, run = cr % runs, c = cr / runs;
+        const int lo = max(first, (head0 + h) * 64), hi = min(first + count, (head0 + h + 1) * 64);
+        bulk_load(smem_u32(area) + (unsigned)((cr * count + lo - first) * 16), pa(c, head0 + h, run) + 4 * (lo & 63),
+                  (unsigned)((hi - lo) * 16), bar);
+    }
+    // weights {2^(m - M), l} of every (column, head), a warp each
+    for (int i = warp; i < cols * heads; i += kWarps) {
+        const int h = i % heads, c = i / heads;
+        float2 ml = make_float2(-INFINITY, 0.0f);
+        if (lane < runs)
+            ml = __ldcg(reinterpret_cast<const float2 *>(p.part_ml + (size_t)(slot + c) * p.ml_slot +
+                                                         (size_t)(kvh * group + head0 + h) * p.splits * 2) + lane);
+        const float big = warp_max(ml.x);
+        s_ml[i][lane] = lane == kStagedRow - 1 ? make_float2(big, 0.0f)
+                                               : make_float2(ml.x == -INFINITY ? 0.0f : ex2(ml.x - big), ml.y);
+    }
+    __syncthreads();
+    for (unsigned spin = 0; !mbar_try_wait(bar, phase);)
+        if (++spin > kSpinLimit) {
+            landed = false;
+            break;
+        }
+    for (int f = tid; f < cols * count; f += kThreads) {
+        const int c = cols > 1 ? f / count : 0, at = f - c * count, item = first + at;
+        const float2 *const wl = s_ml[c * heads + (item >> 6) - head0];
+        const float4 *const x = reinterpret_cast<const float4 *>(area) + (size_t)c * runs * count + at;
+        Part r;
+        r.a = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        r.l = 0.0f;
+        r.m = wl[kStagedRow - 1].x;
+#pragma unroll 4
+        for (int i = 0; i < runs; i++) {
+            const float4 v = x[i * count];
+            const float2 w = wl[i];
+            r.a.x = fmaf(v.x, w.x, r.a.x);
+            r.a.y = fmaf(v.y, w.x, r.a.y);
+            r.a.z = fmaf(v.z, w.x, r.a.z);
+            r.a.w = fmaf(v.w, w.x, r.a.w);
+            r.l = fmaf(w.y, w.x, r.l);
+        }
+        emit_item(p, slot + c, kvh, group, item, r);
+    }
+    return true;
 }
 
 // Which rows a CTA works on.
@@ -554,15 +683,15 @@ __device__ __forceinline__ Balance balance(const DecodeParams &p, int len, int c
     const int cap = min(p.splits, p.run_cap), warps = kWarps * ctas;
     Balance b;
     b.unit = div_up(len, 16) <= cap * warps ? 16 : most;
-    b.units = div_up(len, b.unit * 8) * 8;
+    b.units = div_up(len, 16 * 8) * 8;
+    if (b.unit == 32) b.units = div_up(len, 32 * 8) * 8;
     b.runs = max(1, min(div_up(b.units, warps), cap));
     return b;
 }
 
-// Run `run` of a head under the balanced plan.
-template <int kC, int kUnitRows>
-__device__ __forceinline__ Work plan_run(const DecodeParams &p, int slot, int kvh, int run, int rank, int len) {
-    const Balance b = balance(p, len, kC, kUnitRows);
+// Run `run` of a head under plan b; the first units % runs runs get one unit more than the others.
+template <int kC>
+__device__ __forceinline__ Work plan_run(const Balance &b, int slot, int kvh, int run, int rank, int len) {
     Work w;
     w.slot = slot;
     w.len = len;
@@ -572,7 +701,8 @@ __device__ __forceinline__ Work plan_run(const DecodeParams &p, int slot, int kv
     w.unit = b.unit;
     w.row0 = w.row1 = 0;
     if (run < b.runs) {
-        const int c0 = (int)((long long)run * b.units / b.runs), c1 = (int)((long long)(run + 1) * b.units / b.runs);
+        const int each = b.units / b.runs, more = b.units - each * b.runs;
+        const int c0 = run * each + min(run, more), c1 = c0 + each + (run < more ? 1 : 0);
         w.row0 = (c0 + (c1 - c0) * rank / kC) * b.unit;   // (past the end for a CTA without rows)
         w.row1 = min((c0 + (c1 - c0) * (rank + 1) / kC) * b.unit, len);
     }
@@ -585,7 +715,7 @@ __device__ __forceinline__ Work plan_stream(const DecodeParams &p, int slot, int
     const int cluster = (int)blockIdx.x / kC;
     if (!p.by_stride && p.run_cap > 0) {
         const int cap = min(p.splits, p.run_cap), kvh = cluster / cap;
-        return plan_run<kC, kUnitRows>(p, slot, kvh, cluster - kvh * cap, rank, len);
+        return plan_run<kC>(balance(p, len, kC, kUnitRows), slot, kvh, cluster - kvh * cap, rank, len);
     }
     // fixed runs of ceil(span / splits) rows, rounded up to 64
     Work w;

@@ -146,7 +146,7 @@ int launch_decode_tc(cudaStream_t stream, const DecodeParams &p, int slots);
 // The default body of the split pass (attn_decode_warps.cu); launch_decode_tc calls it.
 int launch_decode_warps(cudaStream_t stream, const DecodeParams &p, int slots);
 // The same for several columns of one cache; p as launch_decode_warps set it up for its own launch.
-int launch_decode_cols(cudaStream_t stream, const DecodeParams &p);
+int launch_decode_cols(cudaStream_t stream, const DecodeParams &p, int cluster);
 // Arrival-counter region for a launch on `stream` (-1: none free, use the two-launch form);
 // `counters` = slots * n_kv * arrive_stride must fit a region.
 int decode_arrive_region(cudaStream_t stream, long long counters);
