@@ -949,15 +949,40 @@ static int fold_capacity(int slices) {
     return n;
 }
 
-// Key slices per query tile of a one-pass launch of `pairs` CTA pairs. A launch with fewer pairs than the
-// device has SM pairs leaves the rest idle, and every pair walks its keys alone at ~4.4 us per 128-key tile
-// behind ~13 us of its own (301 tokens at 3,001: 32 pairs, 26 tiles, 127 us). So: as many slices as still
-// start together, at least two key tiles each (the fold costs ~4 us), none past the 64 tiles where a
-// pair would move its sums to memory. (B200: 33 clusters of 2 slices, 15 of 4, 7 of 8.)
-static int fold_slices(int pairs, int key_tiles) {
-    for (int s = kMaxFold; s >= 2; s--)
-        if (key_tiles >= 2 * s && (key_tiles + s - 1) / s <= kFlushTiles && pairs <= fold_capacity(s)) return s;
-    return 1;
+// Query tile and key slices of a one-pass launch. A pair of CTAs walks its keys at ~4.5 us per 128-key tile
+// (the tensor cores' rate; a little faster while other SMs idle) behind ~13 us of its own, of which ~8 go
+// into moving its 2 x 126 query rows in and its output rows out (an SM moves ~30 B/ns). A launch with fewer
+// pairs than the device has SM pairs can therefore be shortened by slices of the keys, which fold in one
+// cluster (~3 us; 301 tokens at 3,001: 32 pairs, 26 tiles, 127 us in one), and by smaller query tiles (300
+// tokens at 0: 36.2 -> 33.4 us; not where the walk is long: 536 at 4,014 179 -> 199 us with tiles of 15
+// instead of 21). This takes the shape that an estimate from those figures says is shortest, among those
+// whose clusters all start together; a slice stays below the 64 tiles where a pair would move its sums to
+// memory. Launches of more pairs than that keep whole tiles and one slice.
+struct ChunkShape {
+    int qtile, fold;
+};
+static ChunkShape chunk_shape(int tokens, int n_kv, int group, int key_tiles) {
+    // (tiles below two thirds of the full one gained nothing more)
+    const int smallest = (2 * (128 / group) + 2) / 3;
+    ChunkShape best = {128 / group, 1};
+    float best_us = 1e30f;
+    for (int fold = 1; fold <= kMaxFold; fold++) {
+        if (fold > 1 && (key_tiles < 2 * fold || (key_tiles + fold - 1) / fold > kFlushTiles)) continue;
+        const int room = fold_capacity(fold) / n_kv;   // clusters per KV head that start together
+        if (room < 1) continue;
+        const int least = (tokens + 2 * room - 1) / (2 * room);
+        for (int qtile = least > smallest ? least : smallest; qtile <= 128 / group; qtile++) {
+            const int pairs = ((tokens + qtile - 1) / qtile + 1) / 2 * n_kv * fold;
+            const float step = 3.1f + 0.022f * (float)pairs;
+            const float us = step * (float)((key_tiles + fold - 1) / fold) + 8.0f * (float)(qtile * group) / 126.0f +
+                             (fold > 1 ? 3.0f : 0.0f);
+            if (us < best_us) {
+                best_us = us;
+                best = {qtile, fold};
+            }
+        }
+    }
+    return best;
 }
 
 // Launches the tensor-core kernel over a workspace staged for `cap` keys per head.
@@ -1016,6 +1041,11 @@ int launch_chunk_tc(cudaStream_t stream, const float *q, float *out, float *part
     p.gate = gate;
     p.fold = 1;
     const int nsp = splits < 2 ? 1 : splits;
+    if (pair && splits < 2) {
+        const ChunkShape s = chunk_shape(tokens, n_kv, p.group, (pos0 + tokens + kKeyTile - 1) / kKeyTile);
+        p.qtile = s.qtile;
+        p.fold = s.fold;
+    }
     const int qtiles = (tokens + p.qtile - 1) / p.qtile;
     if (!pair) {
         return launch_pdl(attn_chunk_tc<1, false>, dim3(qtiles, n_kv, nsp), dim3(kTcThreads), (size_t)kSmemBytes,
@@ -1024,8 +1054,6 @@ int launch_chunk_tc(cudaStream_t stream, const float *q, float *out, float *part
     // Clusters of two CTAs along x: consecutive query tiles of one KV head (an odd tile count leaves the
     // last pair's second CTA without live queries), and along z the key slices that fold in the cluster.
     const int pairs = (qtiles + 1) / 2;
-    const int key_tiles = (pos0 + tokens + kKeyTile - 1) / kKeyTile;
-    p.fold = splits < 2 ? fold_slices(pairs * n_kv, key_tiles) : 1;
     if (p.fold > 1)
         return launch_pdl(attn_chunk_tc<2, true>, dim3(pairs * 2, n_kv, p.fold), dim3(kTcThreads), (size_t)kSmemBytes,
                           stream, dim3(2, 1, p.fold), mk_hi, mk_lo, mv_hi, mv_lo, p);
