@@ -25,7 +25,7 @@ using namespace warp_body;
 constexpr int kCols = 4;          // columns side by side
 constexpr int kUnitRows = 32;
 constexpr unsigned kTmemCols = 512;
-constexpr int kMaxCols = 64;      // of a launch
+constexpr int kMaxCols = 32;      // of a launch
 
 struct Cfg {
     static constexpr int kSlot = kUnitRows * kRowBytes;
@@ -46,28 +46,50 @@ struct Cfg {
 
 __device__ int g_arrive_cols[kArriveRegions * kArriveRegionInts];
 
-// Which columns a cluster takes: groups of `each`, from `base` on every `stride` columns, run `run` of them
-// (base >= the column count: nothing). Columns go to clusters of their own while a head has clusters to
-// spare for their runs, and share conversions beyond (4 columns of 300 rows take 2 runs each: 8 clusters of
-// the head's 18; of 8,192 rows 17: one cluster per run takes all four).
+// Which columns a cluster takes. Neighbouring columns with the same plan (the same units for every warp), at
+// most `each` of them, are a group; a cluster has run `run` of groups `group`, `group` + `hop`, ... Groups go
+// to clusters of their own while a head has clusters to spare for their runs, and columns share conversions
+// beyond (4 columns of 300 rows take 2 runs each: 8 clusters of the head's 18; of 8,192 rows 17: one cluster
+// per run takes all four).
 struct Share {
-    int base, each, stride, run;
+    int each, run, group, hop;
+    unsigned starts;   // bit c: column c's plan is not column c - 1's
 };
 template <int kC>
 __device__ __forceinline__ Share share_columns(const DecodeParams &p, int cap, int in_head, const int *len) {
-    int runs = 1;
-    for (int c = threadIdx.x & 31; c < p.n_slots; c += 32) runs = max(runs, balance(p, len[c], kC, kUnitRows).runs);
-    runs = __reduce_max_sync(0xffffffffu, runs);
+    const int c = threadIdx.x & 31;
+    const bool on = c < p.n_slots;
+    Balance b = {0, 0, 1};
+    if (on) b = balance(p, len[c], kC, kUnitRows);
+    const int units = __shfl_up_sync(0xffffffffu, b.units, 1), unit = __shfl_up_sync(0xffffffffu, b.unit, 1);
+    const int before = __shfl_up_sync(0xffffffffu, b.runs, 1);
+    const int runs = __reduce_max_sync(0xffffffffu, b.runs);
     const int side = cap / runs;   // groups side by side, >= 1
     Share s;
+    s.starts = __ballot_sync(0xffffffffu, on && (c == 0 || units != b.units || unit != b.unit || before != b.runs));
     s.each = min(kCols, div_up(p.n_slots, side));
     s.run = in_head % runs;
-    s.stride = side * s.each;
-    s.base = in_head < side * runs ? in_head / runs * s.each : p.n_slots;
+    s.group = in_head < side * runs ? in_head / runs + (int)blockIdx.y * side : p.n_slots;
+    s.hop = side * gridDim.y;
     return s;
 }
+// Columns [base, end) of group s.group (none past the last); returns how many groups there are.
+__device__ __forceinline__ int find_group(const Share &s, int cols, int &base, int &end) {
+    base = end = cols;
+    int groups = 0;
+    for (int first = 0; first < cols; groups++) {
+        const unsigned later = first < 31 ? s.starts >> (first + 1) : 0;
+        const int last = min(min(first + s.each, cols), later ? first + __ffs(later) : cols);
+        if (groups == s.group) {
+            base = first;
+            end = last;
+        }
+        first = last;
+    }
+    return groups;
+}
 
-// grid (n_kv * runs * kC), clusters of kC as in the single-column form.
+// grid (n_kv * runs * kC, ceil(columns / kCols)), clusters of kC as in the single-column form.
 template <int kC>
 __global__ void __launch_bounds__(kThreads, 1) attn_decode_cols(DecodeParams p, int *status) {
     using C = Cfg;
@@ -101,9 +123,8 @@ __global__ void __launch_bounds__(kThreads, 1) attn_decode_cols(DecodeParams p, 
     __syncthreads();
     const size_t head_byte = (size_t)kvh * p.stride * kRowBytes;   // (the columns share the cache)
     Share sh = share_columns<kC>(p, cap, in_head, s_len);
-    int base = sh.base, end = min(base + sh.each, p.n_slots);
-    // Columns base .. base + n - 1 share a plan: the same units for every warp. (Ascending lengths rarely leave
-    // it; then the rest of the group is another round.)
+    int base, end;
+    int groups = find_group(sh, p.n_slots, base, end);
     int n, len[kCols], first, row1, nw;
     bool live;
     Work w;
@@ -111,17 +132,15 @@ __global__ void __launch_bounds__(kThreads, 1) attn_decode_cols(DecodeParams p, 
     const unsigned char *kp, *vp;
     auto plan = [&]() {
         live = false;
-        nw = n = 0;
-        if (base >= p.n_slots) return;
+        nw = 0;
+        n = end - base;
+        if (n == 0) return;
         const Balance b0 = balance(p, s_len[base], kC, kUnitRows);
-        n = 1;
         int longest = 0;
 #pragma unroll
         for (int c = 0; c < kCols; c++) {
-            len[c] = base + c < end ? s_len[base + c] : 0;
-            const Balance b = balance(p, len[c], kC, kUnitRows);
-            if (c > 0 && n == c && base + c < end && b.units == b0.units && b.unit == b0.unit && b.runs == b0.runs) n = c + 1;
-            if (n > c) longest = max(longest, len[c]);
+            len[c] = c < n ? s_len[base + c] : 0;
+            longest = max(longest, len[c]);
         }
         w = plan_run<kC>(b0, base, kvh, sh.run, rank, longest);
         live = w.run < w.runs;
@@ -198,8 +217,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_decode_cols(DecodeParams p, 
             if (tid < p.n_slots) s_len[tid] = real_len;
             __syncthreads();
             sh = share_columns<kC>(p, cap, in_head, s_len);
-            base = sh.base;
-            end = min(base + sh.each, p.n_slots);
+            groups = find_group(sh, p.n_slots, base, end);
             plan();
             checked = true;
             continue;
@@ -412,13 +430,10 @@ __global__ void __launch_bounds__(kThreads, 1) attn_decode_cols(DecodeParams p, 
         __syncthreads();
         if (lane == 0) fence_async_shared();   // partials were written over the rings; a next round's copies follow
         }   // a live run of these columns
-        base += n;
-        if (base >= end) {   // the cluster's next group of columns
-            base = sh.base += sh.stride;
-            end = min(base + sh.each, p.n_slots);
-        }
+        sh.group += sh.hop;   // the cluster's next group of columns
+        if (sh.group >= groups) break;
+        find_group(sh, p.n_slots, base, end);
         plan();
-        if (base >= p.n_slots) break;
     }
     if (!landed && status) atomicCAS(status, 0, 21);
     tc_fence_before();
@@ -446,8 +461,8 @@ int launch(cudaStream_t stream, const DecodeParams &p) {
             if (status_word[dev] == nullptr) return launch_status();
         }
     }
-    return launch_pdl(attn_decode_cols<kC>, dim3(p.n_kv * min(p.splits, p.run_cap) * kC), dim3(kThreads),
-                      (size_t)Cfg::kSmem, stream, kC, p, status_word[dev]);
+    return launch_pdl(attn_decode_cols<kC>, dim3(p.n_kv * min(p.splits, p.run_cap) * kC, (p.n_slots + kCols - 1) / kCols),
+                      dim3(kThreads), (size_t)Cfg::kSmem, stream, kC, p, status_word[dev]);
 }
 
 }  // namespace
