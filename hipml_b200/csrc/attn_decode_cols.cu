@@ -468,7 +468,7 @@ int launch(cudaStream_t stream, const DecodeParams &p) {
 }  // namespace
 
 int launch_decode_cols(cudaStream_t stream, const DecodeParams &p, int cluster) {
-    return cluster == 8 ? launch<8>(stream, p) : launch<2>(stream, p);
+    return cluster == 8 ? launch<8>(stream, p) : cluster == 4 ? launch<4>(stream, p) : launch<2>(stream, p);
 }
 
 }  // namespace hipml

@@ -10,8 +10,8 @@
 //
 // attn_front_rows_q8: a CTA of 8 warps per token, or several where tokens are few. The rotation angles depend on the
 // position and the channel pair only, so the CTA computes the n_rot/2 (cos, sin) pairs once
-// (f64 sincos over f64 frequencies, as the definition does) and all its heads share them; where the
-// launch carries the positions it does so before the grid dependency resolves. A warp owns a
+// (f64 sincos over f64 frequencies, as the definition does) and all its heads share them, before the
+// grid dependency resolves. A warp owns a
 // whole 256-wide head row: 8 values per lane (two 16-byte loads), the sum of squares by
 // shuffles, the rotation partner (channel +- n_rot/2) in the lane n_rot/16 away. The K row
 // leaves as a q8_0 cache row straight from the normalised, rotated registers and the V row
@@ -259,11 +259,12 @@ __global__ void __launch_bounds__(256) attn_front_rows_q8(const __grid_constant_
             sn[c] = (float)s;
         }
     };
-    if (!p.pos4) {
-        // positions that the launch carries: the angles need not wait for the grids ahead
-        const int p4[4] = {p.pos0 + t, p.pos0 + t, p.pos0 + t, p.pos0 + t};
-        angles(p4);
-    }
+    // The angles need not wait for the grids ahead: positions that the launch carries are known, and those in
+    // memory are most likely what they will be (a step's layers share them); they are checked below.
+    int p4[4] = {p.pos0 + t, p.pos0 + t, p.pos0 + t, p.pos0 + t};
+    if (p.pos4)
+        for (int i = 0; i < 4; i++) p4[i] = __ldcg(p.pos4 + i);
+    angles(p4);
     griddep_wait();   // positions and rows may come from a grid that is still running
     const int rows = p.n_heads + 2 * p.n_kv, hop = 8 * gridDim.y;
     float x[8], g[8];   // the row at hand (and the gate half of a query row)
@@ -281,11 +282,17 @@ __global__ void __launch_bounds__(256) attn_front_rows_q8(const __grid_constant_
     int r = blockIdx.y * 8 + warp;
     load_row(r);
     const int cache_row = p.step ? p.step[0] : p.pos0 + t;
-    if (p.pos4) {
-        const int p4[4] = {p.pos4[0], p.pos4[1], p.pos4[2], p.pos4[3]};
+    bool moved = false;
+    if (p.pos4)
+        for (int i = 0; i < 4; i++) {
+            const int x = __ldcg(p.pos4 + i);
+            moved = moved || x != p4[i];
+            p4[i] = x;
+        }
+    if (__syncthreads_or(moved)) {
         angles(p4);
+        __syncthreads();
     }
-    __syncthreads();
     for (; r < rows; r += hop) {
         if (r < p.n_heads) {
             store8(p.gate + ((size_t)t * p.n_heads + r) * 256 + 8 * lane, g);

@@ -229,3 +229,25 @@ def test_gated_chunk_attention_equals_chunk_then_gate(splits):
     got = gated.cpu().numpy().ravel()
     assert np.all(np.isfinite(got))
     assert O.max_abs(want, got) <= 5e-7
+
+
+def test_positions_that_change_between_launches_are_seen():
+    """The one-token kernel makes its angles from the position ids as they stand before the grids ahead are
+    done; ids written right before it must win."""
+    from hipml_b200 import api
+    n_heads, n_kv, hd = 24, 4, 256
+    qg, k, v, qn, kn = (_dev(x) for x in _front_inputs(21, n_heads, n_kv, hd, 1))
+    ids = [_ints([p, p + 1, p + 2, p]) for p in (0, 90_000, 17, 31_000)]
+    step, moving = _ints([0, 1]), _ints([0, 0, 0, 0])
+
+    def front(pos):
+        q, gate, k_out = (torch.empty(1, n * hd, device="cuda") for n in (n_heads, n_heads, n_kv))
+        api.attn_front_append_q8(qg, k, v, q, gate, qn, kn, None, None, n_heads, n_kv, hd, 64, THETA, EPS, tokens=1,
+                                 sections=SECTIONS, pos=pos, step=step, k_out=k_out)
+        return q, k_out
+
+    want = [front(p) for p in ids]
+    for p, (wq, wk) in zip(ids, want):
+        moving.copy_(p)
+        q, k_out = front(moving)
+        assert torch.equal(q, wq) and torch.equal(k_out, wk)
