@@ -621,16 +621,16 @@ int launch_c(cudaStream_t stream, const DecodeParams &p, int slots) {
 // which only 33 fit the device); clusters of eight up to the 1,023 rows that the engine's policy gives fewer
 // than 128 splits, where one holds a head and nothing is folded through memory (672 rows: 8.7 us with
 // pairs, 8.2), of four up to 519 (300 rows: 8.0 us with eight, 7.4).
-// Several slots: no clusters, a head has too few CTAs to pair them; wide up to 16 (slot, head) pairs (3
-// slots of 512 .. 8,192 rows: 17.1 us against 19.7), beyond that the twice as fine runs of the small CTAs
-// balance better (16 slots: 43.0 us against 47.7).
+// Several slots: no clusters, a head has too few CTAs to pair them; wide up to 28 (slot, head) pairs (4 KV
+// heads, 5 slots of 512 .. 3,000 rows: 14.9 us a layer against 16.5), beyond that the twice as fine runs of
+// the small CTAs balance better (8 slots of 512 .. 8,192: 24.6 us against 25.4, 10 slots 32.8 against 34.2).
 int launch_decode_warps(cudaStream_t stream, const DecodeParams &p, int slots) {
     const bool one_stream = !p.by_stride && p.run_cap >= 4 && p.share_slots == 0;
     if (one_stream)
         return p.splits >= 128 || p.run_cap < 16 ? launch_c<2, true>(stream, p, slots)
                : p.splits > 64                  ? launch_c<8, true>(stream, p, slots)
                                                 : launch_c<4, true>(stream, p, slots);
-    return p.share_slots > 0 && slots * p.n_kv <= 16 ? launch_c<1, true>(stream, p, slots)
+    return p.share_slots > 0 && slots * p.n_kv <= 28 ? launch_c<1, true>(stream, p, slots)
                                                      : launch_c<1, false>(stream, p, slots);
 }
 
