@@ -29,8 +29,8 @@
 // tiles with CTA barriers and softmax through shared memory took 2,370, 57 us a layer); short ones
 // the chain of dependent latencies (8,192 rows: 11.5 us, before 16).
 //
-// Merge: the eight warps' partials through shared memory, then the CTAs of a cluster through
-// distributed shared memory (every CTA folds a slice of the outputs), then, where a head has more
+// Merge: the eight warps' partials through shared memory, then the CTAs of a cluster, each of which
+// folds a slice of the outputs and is sent the others' share of it, then, where a head has more
 // than one cluster, through memory: the last cluster to arrive at the slice's counter folds it.
 // Every sum runs in a fixed order, so the result does not depend on who arrives last.
 #include <atomic>
@@ -55,13 +55,14 @@ struct Cfg {
     static constexpr int kSlots = kQ4 ? 5 : 3;                     // odd (see release)
     static constexpr int kRing = kSlots * kSlot;                   // per warp; later the warp's partial (8 heads)
     static_assert(kRing >= 8 * kHeadPitch * 4, "a warp's partial fits its ring");
-    static constexpr int kOffQ = kWarps * kRing;                   // query fragments [16 steps][32 lanes], later the CTA's partial
+    static constexpr int kOffQ = kWarps * kRing;                   // query fragments [16 steps][32 lanes]
     static constexpr int kOffBias = kOffQ + 16 * 32 * 16;          // [8 blocks][4] {head 2t, 2t + 1, 2t, 2t + 1}
     static constexpr int kOffMl = kOffBias + 8 * 4 * 16;           // [8 heads][warps] {reference, sum}
-    static constexpr int kOffCml = kOffMl + kWarps * 8 * 8;        // [8 heads] {reference, sum} of the CTA
-    static constexpr int kOffRow = kOffCml + 8 * 8;                // the row to append: K, V
+    static constexpr int kOffRow = kOffMl + kWarps * 8 * 8;        // the row to append: K, V
     static constexpr int kOffBar = kOffRow + 2 * kRow;             // a warp's slots each, then the last fold's
-    static constexpr int kSmem = kOffBar + kWarps * kSlots * 8 + 8;
+    static constexpr int kOffInMl = kOffBar + kWarps * kSlots * 8 + 16;   // (two more: the last fold's, the inbox's)
+    static constexpr int kOffIn = (kOffInMl + 8 * 8 * 8 + 15) / 16 * 16;  // partials of the cluster's CTAs (wide)
+    static constexpr int kSmem = kWide ? kOffIn + 8 * 256 * 4 : kOffInMl;
     static_assert((kWide ? 1 : 2) * (kSmem + 512 + 1024) <= 228 * 1024, "CTAs per SM");
 };
 
@@ -136,13 +137,20 @@ __global__ void __launch_bounds__(kThreads, kWide ? 1 : 2) attn_decode_warps(Dec
     const int rank = kC > 1 ? (int)cluster_rank() : 0;
     unsigned char *const ring = smem + warp * C::kRing;
     const unsigned ring_addr = smem_u32(ring), bar = smem_u32(smem + C::kOffBar) + warp * C::kSlots * 8;
-    const unsigned bar_fold = smem_u32(smem + C::kSmem) - 8;
+    const unsigned bar_fold = smem_u32(smem + C::kOffInMl) - 16, bar_in = bar_fold + 8;
+    const int items = group * 64;
+    static_assert(kC == 1 || kWide, "clusters are wide");
     if (lane == 0) {
 #pragma unroll
         for (int i = 0; i < C::kSlots; i++) mbar_init(bar + 8 * i, 1);
-        if (warp == 0) mbar_init(bar_fold, 1);
+        if (warp == 0) {
+            mbar_init(bar_fold, 1);
+            if (kC > 1) mbar_init(bar_in, 1);
+        }
         mbar_init_fence();
+        if (kC > 1 && warp == 0) mbar_arrive_expect_tx(bar_in, inbox_bytes<kC>(items, rank));
     }
+    if constexpr (kC > 1) cluster_arrive();   // (waited for before anything is sent to another CTA)
     uint4 *const qf = reinterpret_cast<uint4 *>(smem + C::kOffQ);
     const float4 *const bias = reinterpret_cast<const float4 *>(smem + C::kOffBias);
     bool landed = true;
@@ -205,6 +213,7 @@ __global__ void __launch_bounds__(kThreads, kWide ? 1 : 2) attn_decode_warps(Dec
             }
     }
     griddep_wait();
+    if constexpr (kC > 1) cluster_wait();
     for (;;) {
         // (the small loads first: behind the rows they would wait for all of them)
         const int real_len = reads_len ? __ldcg(len_at) : 0;
@@ -410,7 +419,6 @@ __global__ void __launch_bounds__(kThreads, kWide ? 1 : 2) attn_decode_warps(Dec
     }
     store_warp_partial<kQ4>(reinterpret_cast<float *>(ring), acc, group, g, t);
     __syncthreads();
-    const int items = group * 64;
     const bool one_run = w.runs == 1 && p.out != nullptr && p.xch.phases == 0;
     // the run's partial of one item, and the output where there is no other run
     auto run_done = [&](int item, const Part &r) {
@@ -419,22 +427,23 @@ __global__ void __launch_bounds__(kThreads, kWide ? 1 : 2) attn_decode_warps(Dec
         reinterpret_cast<float4 *>(part_acc + row * 256)[item & 63] = r.a;
         if ((item & 63) == 0) *reinterpret_cast<float2 *>(part_ml + row * 2) = make_float2(r.m, r.l);
     };
-    float4 *const cpart = reinterpret_cast<float4 *>(smem + C::kOffQ);     // [8 heads][64] (the query is dead)
-    float2 *const cml = reinterpret_cast<float2 *>(smem + C::kOffCml);     // [8 heads]
+    float4 *const inbox = reinterpret_cast<float4 *>(smem + C::kOffIn);
+    float2 *const inbox_ml = reinterpret_cast<float2 *>(smem + C::kOffInMl);
     fold_warps(smem, C::kRing, wml, items, [&](int item, const Part &r) {
-        if (kC > 1) {
-            cpart[item] = r.a;
-            if ((item & 63) == 0) cml[item >> 6] = make_float2(r.m, r.l);
-        } else {
+        if constexpr (kC > 1)
+            send_item<kC>(inbox, inbox_ml, bar_in, items, rank, item, r);
+        else
             run_done(item, r);
-        }
     });
     // ---- merge of the cluster: this CTA folds slice `rank` of the items
     if constexpr (kC > 1) {
-        cluster_sync_all();
-        fold_cluster<kC, 1>(cpart, cml, 0, 1, items, rank, [&](int, int item, const Part &r) { run_done(item, r); });
-        // no CTA may leave while another still reads its partial
-        cluster_arrive();
+        __syncthreads();
+        for (unsigned spin = 0; !mbar_try_wait_cluster(bar_in, 0);)
+            if (++spin > kSpinLimit) {
+                landed = false;
+                break;
+            }
+        fold_inbox<kC>(inbox, inbox_ml, items, rank, run_done);
     }
     // ---- merge of the runs: the last to arrive at the slice's counter folds it
     if (p.out != nullptr && !one_run) {
@@ -461,8 +470,7 @@ __global__ void __launch_bounds__(kThreads, kWide ? 1 : 2) attn_decode_warps(Dec
             // the exchange wants whole heads in one CTA: the cluster arrives as one
             __threadfence();
             if constexpr (kC > 1) {
-                cluster_wait();
-                cluster_arrive();
+                cluster_sync_all();
             } else {
                 __syncthreads();
             }
@@ -491,7 +499,6 @@ __global__ void __launch_bounds__(kThreads, kWide ? 1 : 2) attn_decode_warps(Dec
             }
         }
     }
-    if constexpr (kC > 1) cluster_wait();
     if (!landed && status) atomicCAS(status, 0, 21);
 }
 

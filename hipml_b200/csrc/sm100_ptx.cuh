@@ -56,6 +56,18 @@ __device__ __forceinline__ bool mbar_try_wait(unsigned bar, unsigned parity) {
         : "memory");
     return ok != 0;
 }
+// For what other CTAs of the cluster wrote.
+__device__ __forceinline__ bool mbar_try_wait_cluster(unsigned bar, unsigned parity) {
+    unsigned ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
 
 
 // ---- thread-block cluster (CTA pair) helpers
@@ -89,6 +101,18 @@ __device__ __forceinline__ void mbar_inval(unsigned bar) {
 // Asks L2 for `bytes` (a multiple of 16, 16-byte aligned); touches nothing of this CTA.
 __device__ __forceinline__ void prefetch_l2(const void *src, unsigned bytes) {
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
+}
+// Stores to another CTA's shared memory whose bytes are counted on a barrier of that CTA (both shared::cluster
+// addresses): the receiver waits on its own barrier and reads locally.
+__device__ __forceinline__ void st_async_f4(unsigned addr, const float4 &v, unsigned bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(addr),
+                 "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void st_async_f2(unsigned addr, const float2 &v, unsigned bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];" ::"r"(addr), "f"(v.x),
+                 "f"(v.y), "r"(bar)
+                 : "memory");
 }
 // loads from a shared::cluster address
 __device__ __forceinline__ float4 ld_cluster_f4(unsigned addr) {
