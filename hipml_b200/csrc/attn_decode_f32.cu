@@ -15,6 +15,8 @@
 // a time with all loads in flight; the four rows' dot products are summed over the lanes by one
 // reduce-scatter (25 shuffles for 24 sums, where a butterfly each took 120). Other head sizes:
 // attn_decode_cols_f32, one warp per (query head, run, column).
+#include <atomic>
+
 #include "decode_rows_f32.cuh"
 
 namespace hipml {
@@ -36,16 +38,17 @@ namespace {
 using namespace warp_body;
 
 constexpr int kOffMlF32 = kWarps * 8 * kHeadPitch * 4;             // after the warps' partials: [8 heads][warp]
-constexpr int kOffPartF32 = kOffMlF32 + kWarps * 8 * 8;            // the CTA's partial [8 heads][256]
-constexpr int kOffCmlF32 = kOffPartF32 + 8 * 256 * 4;              // [8 heads]
-constexpr int kSmemF32 = kOffCmlF32 + 8 * 8;
+constexpr int kOffInF32 = kOffMlF32 + kWarps * 8 * 8;              // partials of the cluster's CTAs
+constexpr int kOffInMlF32 = kOffInF32 + 8 * 256 * 4;
+constexpr int kOffBarF32 = kOffInMlF32 + 8 * 8 * 8;
+constexpr int kSmemF32 = kOffBarF32 + 8;
 
 __device__ int g_arrive_f32[kArriveRegions * kArriveRegionInts];
 
-// kC: CTAs (runs) per cluster, folded through distributed shared memory. grid (n_kv * clusters * kC,
+// kC: CTAs (runs) per cluster, each sent its slice of the others' partials to fold. grid (n_kv * clusters * kC,
 // columns). d: out, scratch and counters (as the quantised body's).
 template <int kHeads, int kC>
-__global__ void __launch_bounds__(kThreads, 2) attn_decode_rows_f32(ColsParams p, DecodeParams d, int clusters) {
+__global__ void __launch_bounds__(kThreads, 2) attn_decode_rows_f32(ColsParams p, DecodeParams d, int clusters, int *status) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ __align__(16) float s_q[8 * 256];
     __shared__ __align__(16) float s_w[kWarps][8][kRowsAtOnce];
@@ -55,6 +58,14 @@ __global__ void __launch_bounds__(kThreads, 2) attn_decode_rows_f32(ColsParams p
     const int rank = (int)cluster_rank(), cluster = (int)blockIdx.x / kC;
     const int kvh = cluster / clusters, in_head = cluster - kvh * clusters, col = blockIdx.y;
     const int group = p.n_heads / p.n_kv, width = p.n_kv * 256, seq = p.pos0 + col + 1;
+    const int items = group * 64;
+    const unsigned bar_in = smem_u32(smem + kOffBarF32);
+    if (tid == 0) {
+        mbar_init(bar_in, 1);
+        mbar_init_fence();
+        mbar_arrive_expect_tx(bar_in, inbox_bytes<kC>(items, rank));
+    }
+    cluster_arrive();   // (waited for before anything is sent to another CTA)
     // this warp's share of the run, fixed in cache positions, cut at the column's last row
     const int run = in_head * kC + rank;
     const int run0 = run * p.per, run_rows = run < p.splits ? p.per : 0;
@@ -64,6 +75,7 @@ __global__ void __launch_bounds__(kThreads, 2) attn_decode_rows_f32(ColsParams p
     for (int i = lane; i < 2 * (hi - lo); i += 32)
         prefetch_l2(((i & 1) ? vb : kb) + (size_t)(lo + (i >> 1)) * width, 1024);
     griddep_wait();
+    cluster_wait();
     for (int i = tid; i < 8 * 64; i += kThreads) {
         float4 x = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         if (i < group * 64)
@@ -106,16 +118,14 @@ __global__ void __launch_bounds__(kThreads, 2) attn_decode_rows_f32(ColsParams p
             make_float4(st.acc[h][4], st.acc[h][5], st.acc[h][6], st.acc[h][7]);
     }
     __syncthreads();
-    const int items = group * 64;
-    float4 *const cpart = reinterpret_cast<float4 *>(smem + kOffPartF32);
-    float2 *const cml = reinterpret_cast<float2 *>(smem + kOffCmlF32);
+    float4 *const inbox = reinterpret_cast<float4 *>(smem + kOffInF32);
+    float2 *const inbox_ml = reinterpret_cast<float2 *>(smem + kOffInMlF32);
     fold_warps(smem, 8 * kHeadPitch * 4, wml, items, [&](int item, const Part &r) {
-        cpart[item] = r.a;
-        if ((item & 63) == 0) cml[item >> 6] = make_float2(r.m, r.l);
+        send_item<kC>(inbox, inbox_ml, bar_in, items, rank, item, r);
     });
-    cluster_sync_all();
+    if (!await_inbox(bar_in, 0) && status) atomicCAS(status, 0, 21);
     const bool one = clusters == 1 && d.out != nullptr;
-    fold_cluster<kC, 1>(cpart, cml, 0, 1, items, rank, [&](int, int item, const Part &r) {
+    fold_inbox<kC>(inbox, inbox_ml, items, rank, [&](int item, const Part &r) {
         if (one) {
             emit_item(d, col, kvh, group, item, r);
             return;
@@ -125,7 +135,6 @@ __global__ void __launch_bounds__(kThreads, 2) attn_decode_rows_f32(ColsParams p
         if ((item & 63) == 0)
             *reinterpret_cast<float2 *>(d.part_ml + (size_t)col * d.ml_slot + row * 2) = make_float2(r.m, r.l);
     });
-    cluster_arrive();   // no CTA may leave while another still reads its partial
     if (d.out != nullptr && !one) {
         int *const ctr = g_arrive_f32 + (size_t)d.arrive_region * kArriveRegionInts +
                          (size_t)(col * p.n_kv + kvh) * kC + rank;
@@ -138,7 +147,6 @@ __global__ void __launch_bounds__(kThreads, 2) attn_decode_rows_f32(ColsParams p
         __syncthreads();
         if (s_last) fold_runs<kC, 1, 8>(d, col, 1, kvh, group, clusters, rank, nullptr);
     }
-    cluster_wait();
 }
 
 // One warp per (query head, run, column), any head size.
@@ -223,17 +231,21 @@ namespace {
 
 template <int kHeads, int kC>
 int launch_rows_f32_heads(cudaStream_t stream, const ColsParams &p, const DecodeParams &d, int clusters) {
-    static bool configured[64] = {};
+    static std::atomic<int *> status_word[64] = {};   // nullptr: device not set up yet
     int dev = 0;
     cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64 || !configured[dev]) {
+    if (dev < 0 || dev >= 64) dev = 0;
+    int *status = status_word[dev].load(std::memory_order_acquire);
+    if (status == nullptr) {
         const cudaError_t e =
             cudaFuncSetAttribute(attn_decode_rows_f32<kHeads, kC>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemF32);
         if (e != cudaSuccess) return (int)e;
-        if (dev >= 0 && dev < 64) configured[dev] = true;
+        status = device_status_word();
+        if (status == nullptr) return launch_status();
+        status_word[dev].store(status, std::memory_order_release);
     }
     return launch_pdl(attn_decode_rows_f32<kHeads, kC>, dim3(p.n_kv * clusters * kC, p.rows), dim3(kThreads),
-                      (size_t)kSmemF32, stream, kC, p, d, clusters);
+                      (size_t)kSmemF32, stream, kC, p, d, clusters, status);
 }
 
 int launch_rows_f32(cudaStream_t stream, const ColsParams &p, float *out, long long acc_slot, long long ml_slot,

@@ -437,12 +437,7 @@ __global__ void __launch_bounds__(kThreads, kWide ? 1 : 2) attn_decode_warps(Dec
     });
     // ---- merge of the cluster: this CTA folds slice `rank` of the items
     if constexpr (kC > 1) {
-        __syncthreads();
-        for (unsigned spin = 0; !mbar_try_wait_cluster(bar_in, 0);)
-            if (++spin > kSpinLimit) {
-                landed = false;
-                break;
-            }
+        landed &= await_inbox(bar_in, 0);
         fold_inbox<kC>(inbox, inbox_ml, items, rank, run_done);
     }
     // ---- merge of the runs: the last to arrive at the slice's counter folds it

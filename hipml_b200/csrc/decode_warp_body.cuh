@@ -486,9 +486,9 @@ __device__ __forceinline__ void fold_warps(const unsigned char *partials, int pi
     for (int j = 0; j < kPer; j++)
         if ((int)threadIdx.x + j * kThreads < items) done(threadIdx.x + j * kThreads, r[j]);
 }
-// Folds slice `rank` of the items of the kC CTAs of a cluster, for each of `cols` <= kPer columns (partials of
-// [item] at cpart, {max, sum} of [8 heads] at cml, a column cpart_pitch / 8 further, at the same place in each
-// CTA); done(column, item, part).
+// Merge of a cluster, several columns: folds slice `rank` of the items of the kC CTAs of a cluster, for each of
+// `cols` <= kPer columns (partials of [item] at cpart, {max, sum} of [8 heads] at cml, a column cpart_pitch / 8
+// further, at the same place in each CTA); done(column, item, part).
 template <int kC, int kPer, class Done>
 __device__ __forceinline__ void fold_cluster(const float4 *cpart, const float2 *cml, int cpart_pitch, int cols, int items,
                                              int rank, Done done) {
@@ -518,10 +518,11 @@ __device__ __forceinline__ void fold_cluster(const float4 *cpart, const float2 *
     }
 }
 
-// The same exchange pushed instead of pulled: every CTA sends each item of its partial to the CTA that folds it
-// as soon as it has it, and that one waits on its own barrier and reads locally; none has to stay for another's
-// reads either. (A barrier of the cluster, remote loads and another barrier were 0.9 us of the 8.3 us that a
-// layer of 672 rows takes, 0.7 of 14.9 with the rest of its layer's chain at 8,192.)
+// Merge of a cluster, one column: every CTA sends each item of its partial to the CTA that folds it (slice r of
+// the items: CTA r) as soon as it has it, and that one waits on its own barrier and reads locally; none has to
+// stay for another's reads. (A barrier of the cluster, remote loads and another barrier were 0.9 us of the 8.3 us
+// that a layer of 672 rows takes, 0.7 of 14.9 with its front end at 8,192 rows, 0.6 of 12.6 over the f32 cache at
+// 2,048; four columns of 8,192 rows took 34.1 us a layer sent this way and 33.3 read.)
 // inbox: [kC sources][items / kC] float4, inbox_ml: [kC][8 heads]; kC divides 64. The receiver's barrier expects
 // inbox_bytes.
 template <int kC>
@@ -561,6 +562,13 @@ __device__ __forceinline__ void fold_inbox(const float4 *inbox, const float2 *in
         r);
     join<kShare>(r[0]);
     if (at < count && part == 0) done(item, r[0]);
+}
+// This CTA's partials of the cluster are all there (its own behind the CTA barrier).
+__device__ __forceinline__ bool await_inbox(unsigned bar, unsigned phase) {
+    __syncthreads();
+    for (unsigned spin = 0; !mbar_try_wait_cluster(bar, phase);)
+        if (++spin > kSpinLimit) return false;
+    return true;
 }
 
 // One float4 (item = head of the group * 64 + dims / 4) of the output: normalised (and gated), or

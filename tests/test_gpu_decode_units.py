@@ -42,6 +42,30 @@ def test_step_with_append_at_the_edges_of_a_unit(seq, dtype):
     assert ok and ma <= 2e-5 and rl <= 2e-5, (ma, rl)
 
 
+# clusters of four, eight and two; slices of the outputs that lie within, begin or cross a head
+@pytest.mark.parametrize("seq", [40, 700, 1500])
+@pytest.mark.parametrize("group", [1, 3, 5, 7, 8])
+def test_partials_sent_within_a_cluster_for_any_group(group, seq):
+    from hipml_b200 import api
+    n_kv, hd, scale = 4, 256, 0.0625
+    heads = n_kv * group
+    gen = torch.Generator(device="cuda").manual_seed(seq + group)
+    k, v = (torch.randn(seq, n_kv * hd, device="cuda", generator=gen) for _ in range(2))
+    q = torch.randn(heads * hd, device="cuda", generator=gen)
+    kc, vc = (torch.zeros(n_kv * seq * 272, dtype=torch.uint8, device="cuda") for _ in range(2))
+    api.kv_encode_bulk(k, v, kc, vc, n_kv, hd, seq, 0, 0, seq)
+    splits = api.decode_splits(seq)
+    acc, ml = torch.empty(heads * splits * hd, device="cuda"), torch.empty(heads * splits * 2, device="cuda")
+    out = torch.full((heads * hd,), float("nan"), device="cuda")
+    step = torch.tensor([seq - 1, seq] + [0] * 6, dtype=torch.int32, device="cuda")
+    api.attn_decode_kv(step, q, kc, vc, acc, ml, out, heads, n_kv, hd, seq, scale, splits)
+    assert api.check_device_status() == 0
+    want = O.attn_decode_kv(q.cpu().numpy(), kc.cpu().numpy().reshape(n_kv, seq, 272), vc.cpu().numpy().reshape(n_kv, seq, 272),
+                            0, heads, n_kv, hd, seq, scale, stride=seq)
+    ok, ma, rl = cases.attention_within_bar(want, out.cpu().numpy())
+    assert ok and ma <= 2e-5 and rl <= 2e-5, (ma, rl)
+
+
 def test_lengths_that_change_between_launches_are_seen():
     """The kernel plans from the length as it stands before the grids ahead are done; a length written by
     the kernel right before it must win."""
