@@ -27,7 +27,7 @@
 // What bounds it: long caches the HBM stream and the issue rate together (100,000 rows: 42.6 us a
 // layer = 5.1 TB/s, 33 us of it in the loop; 1,555 warp instructions per 32 rows of K and V, where 64-row
 // tiles with CTA barriers and softmax through shared memory took 2,370, 57 us a layer); short ones
-// the chain of dependent latencies (8,192 rows: 11.5 us, before 16).
+// the chain of dependent latencies (8,192 rows: 10.7 us, before 16).
 //
 // Merge: the eight warps' partials through shared memory, then the CTAs of a cluster, each of which
 // folds a slice of the outputs and is sent the others' share of it, then, where a head has more
@@ -618,11 +618,11 @@ int launch_c(cudaStream_t stream, const DecodeParams &p, int slots) {
 
 }  // namespace
 
-// Which form. One stream (or columns of one) has ~37 SMs per KV head: clusters of two, wide (8,192
-// rows: 11.5 us a layer, against 14.4 with two small CTAs per SM and 13.1 with clusters of four, of
-// which only 33 fit the device); clusters of eight up to the 1,023 rows that the engine's policy gives fewer
-// than 128 splits, where one holds a head and nothing is folded through memory (672 rows: 8.7 us with
-// pairs, 8.2), of four up to 519 (300 rows: 8.0 us with eight, 7.4).
+// Which form. One stream (or columns of one) has ~37 SMs per KV head: clusters of two, wide (8,192 rows: 11.5 us
+// a layer while partials were still read, against 14.4 with two small CTAs per SM and 13.1 with clusters of four,
+// of which only 33 fit the device; 1,100 rows: 8.2 us, of four 8.4, of eight 9.4); clusters of eight up to the 1,023
+// rows that the engine's policy gives fewer than 128 splits, where one holds a head and nothing is folded through
+// memory (672 rows: 8.2 us with pairs, 7.3; 1,000: 8.3, 7.6), of four up to 519 (300 rows: 7.1 us with eight, 6.8).
 // Several slots: no clusters, a head has too few CTAs to pair them; wide up to 28 (slot, head) pairs (4 KV
 // heads, 5 slots of 512 .. 3,000 rows: 14.9 us a layer against 16.5), beyond that the twice as fine runs of
 // the small CTAs balance better (8 slots of 512 .. 8,192: 24.6 us against 25.4, 10 slots 32.8 against 34.2).
