@@ -399,7 +399,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_decode_cols(DecodeParams p, 
             if (one_run) emit_item(p, base + c, kvh, group, item, r);
             const size_t row = (size_t)(kvh * group + (item >> 6)) * p.splits + w.run;
             reinterpret_cast<float4 *>(p.part_acc + (size_t)(base + c) * p.acc_slot + row * 256)[item & 63] = r.a;
-            if ((item & 63) == 0)
+            if (writes_pair<kC>(items, rank, item))
                 *reinterpret_cast<float2 *>(p.part_ml + (size_t)(base + c) * p.ml_slot + row * 2) = make_float2(r.m, r.l);
         });
         cluster_arrive();   // no CTA may leave, or start over, while another still reads its partials

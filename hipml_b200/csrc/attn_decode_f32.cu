@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(kThreads, 2) attn_decode_rows_f32(ColsParams p
         }
         const size_t row = (size_t)(kvh * group + (item >> 6)) * d.splits + in_head;
         reinterpret_cast<float4 *>(d.part_acc + (size_t)col * d.acc_slot + row * 256)[item & 63] = r.a;
-        if ((item & 63) == 0)
+        if (writes_pair<kC>(items, rank, item))
             *reinterpret_cast<float2 *>(d.part_ml + (size_t)col * d.ml_slot + row * 2) = make_float2(r.m, r.l);
     });
     if (d.out != nullptr && !one) {

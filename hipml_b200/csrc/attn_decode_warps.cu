@@ -425,7 +425,7 @@ __global__ void __launch_bounds__(kThreads, kWide ? 1 : 2) attn_decode_warps(Dec
         if (one_run) emit_item(p, w.slot, w.kvh, group, item, r);
         const size_t row = (size_t)(item >> 6) * p.splits + w.run;
         reinterpret_cast<float4 *>(part_acc + row * 256)[item & 63] = r.a;
-        if ((item & 63) == 0) *reinterpret_cast<float2 *>(part_ml + row * 2) = make_float2(r.m, r.l);
+        if (writes_pair<kC>(items, rank, item)) *reinterpret_cast<float2 *>(part_ml + row * 2) = make_float2(r.m, r.l);
     };
     float4 *const inbox = reinterpret_cast<float4 *>(smem + C::kOffIn);
     float2 *const inbox_ml = reinterpret_cast<float2 *>(smem + C::kOffInMl);

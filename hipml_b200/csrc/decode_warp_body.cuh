@@ -330,6 +330,15 @@ __device__ __forceinline__ int value_dim(int blk, int g, int half) {
     return base + 4 * j + 2 + 2 * half;
 }
 
+// Whether the CTA that folds slice `rank` of the items writes the {maximum, sum} of this item's head to memory: with
+// the first item of the head, and with the first of the slice where that lies inside a head. The counter of the runs is
+// one per slice, so whoever folds the slice there may only read what CTAs of the same rank wrote; the CTAs that share a
+// head write the same bits.
+template <int kC>
+__device__ __forceinline__ bool writes_pair(int items, int rank, int item) {
+    return (item & 63) == 0 || item == items * rank / kC;
+}
+
 // ---- folds. A partial of a head is (acc, m, l) with weights relative to 2^m; folding partials is
 // associative up to rounding, and always runs in one order with explicit operations.
 struct Part {

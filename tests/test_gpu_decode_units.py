@@ -110,7 +110,10 @@ def test_columns_side_by_side_give_each_columns_own_bits(pos0, cols):
     acc, ml = (torch.empty(cols * heads * splits * n, device="cuda") for n in (hd, 2))
     out = torch.full((cols, heads * hd), float("nan"), device="cuda")
     pos = torch.tensor([[pos0 + c, pos0 + c + 1] for c in range(cols)], dtype=torch.int32, device="cuda")
-    for _ in range(2):   # the second launch finds the first one's counters
+    for _ in range(2):   # the second launch finds the first one's counters, and scratch that was never written
+        acc.fill_(float("nan"))
+        ml.fill_(float("nan"))
+        out.fill_(float("nan"))
         api.attn_decode_cols(pos, q, kc, vc, acc, ml, out, heads, n_kv, hd, stride, scale, splits, cols,
                              heads * splits * hd, heads * splits * 2, heads * hd)
     for c in range(cols):
@@ -119,6 +122,101 @@ def test_columns_side_by_side_give_each_columns_own_bits(pos0, cols):
         api.attn_decode_kv(step, q[c], kc, vc, acc, ml, one, heads, n_kv, hd, stride, scale, splits)
         assert torch.equal(one, out[c]), f"column {c}"
     assert api.check_device_status() == 0
+
+
+def _attend(q, k, v, n_kv, hd, scale):
+    """softmax(q k^T) v of one query row per head, 64 bits: q [heads * hd], k and v [rows, n_kv * hd]."""
+    heads = q.numel() // hd
+    q = q.double().view(n_kv, heads // n_kv, hd)
+    k, v = (x.double().view(-1, n_kv, hd).transpose(0, 1) for x in (k, v))
+    return (torch.softmax(q @ k.transpose(1, 2) * scale, dim=-1) @ v).reshape(-1)
+
+
+def _close(got, want):
+    """The bar of the decode tests: largest difference and relative 2-norm."""
+    d = got.double() - want
+    return bool(torch.isfinite(got).all()) and d.abs().max() <= 2e-5 and d.norm() <= 2e-5 * want.norm()
+
+
+LAUNCHES = 24   # with scratch that would poison an output that read any of it too early, and a query each
+
+
+# few splits keep their clusters of four or eight when the stream is longer than one cluster holds; at 128 pairs
+@pytest.mark.parametrize("splits,seq", [(8, 600), (32, 2000), (64, 519), (64, 2500), (100, 2000), (128, 3000)])
+@pytest.mark.parametrize("group", [1, 5, 6, 7, 8])
+def test_no_launch_reads_partials_that_are_not_written_yet(group, splits, seq):
+    """A head's runs meet in memory, slice by slice of its outputs: slices begin inside a head here."""
+    from hipml_b200 import api
+    n_kv, hd, scale = 4, 256, 0.0625
+    heads = n_kv * group
+    gen = torch.Generator(device="cuda").manual_seed(seq + group)
+    k, v = (torch.randn(seq, n_kv * hd, device="cuda", generator=gen) for _ in range(2))
+    kc, vc = (torch.zeros(n_kv * seq * 272, dtype=torch.uint8, device="cuda") for _ in range(2))
+    api.kv_encode_bulk(k, v, kc, vc, n_kv, hd, seq, 0, 0, seq)
+    kq, vq = (torch.from_numpy(cases.unpack_head_major(O.dequantize_q8(c.cpu().numpy().reshape(n_kv, seq, 272)), n_kv,
+                                                       seq, hd)).cuda() for c in (kc, vc))
+    acc, ml = (torch.empty(heads * splits * n, device="cuda") for n in (hd, 2))
+    q = torch.randn(LAUNCHES, heads * hd, device="cuda", generator=gen)
+    out = torch.full((LAUNCHES, heads * hd), float("nan"), device="cuda")
+    step = torch.tensor([seq - 1, seq] + [0] * 6, dtype=torch.int32, device="cuda")
+    for i in range(LAUNCHES):
+        acc.fill_(float("nan"))
+        ml.fill_(float("nan"))
+        api.attn_decode_kv(step, q[i], kc, vc, acc, ml, out[i], heads, n_kv, hd, seq, scale, splits)
+    assert api.check_device_status() == 0
+    for i in range(LAUNCHES):
+        assert _close(out[i], _attend(q[i], kq, vq, n_kv, hd, scale)), f"launch {i}"
+
+
+@pytest.mark.parametrize("splits,pos0", [(32, 2000), (64, 2500), (100, 2000), (128, 3000)])
+@pytest.mark.parametrize("group", [5, 6, 7])
+def test_no_launch_of_columns_reads_partials_that_are_not_written_yet(group, splits, pos0):
+    from hipml_b200 import api
+    n_kv, hd, scale, cols = 4, 256, 0.0625, 4
+    heads, seq = n_kv * group, pos0 + cols
+    gen = torch.Generator(device="cuda").manual_seed(pos0 + group)
+    k, v = (torch.randn(seq, n_kv * hd, device="cuda", generator=gen) for _ in range(2))
+    kc, vc = (torch.zeros(n_kv * seq * 272, dtype=torch.uint8, device="cuda") for _ in range(2))
+    api.kv_encode_bulk(k, v, kc, vc, n_kv, hd, seq, 0, 0, seq)
+    kq, vq = (torch.from_numpy(cases.unpack_head_major(O.dequantize_q8(c.cpu().numpy().reshape(n_kv, seq, 272)), n_kv,
+                                                       seq, hd)).cuda() for c in (kc, vc))
+    acc, ml = (torch.empty(cols * heads * splits * n, device="cuda") for n in (hd, 2))
+    q = torch.randn(LAUNCHES, cols, heads * hd, device="cuda", generator=gen)
+    out = torch.full((LAUNCHES, cols, heads * hd), float("nan"), device="cuda")
+    pos = torch.tensor([[pos0 + c, pos0 + c + 1] for c in range(cols)], dtype=torch.int32, device="cuda")
+    for i in range(LAUNCHES):
+        acc.fill_(float("nan"))
+        ml.fill_(float("nan"))
+        api.attn_decode_cols(pos, q[i], kc, vc, acc, ml, out[i], heads, n_kv, hd, seq, scale, splits, cols,
+                             heads * splits * hd, heads * splits * 2, heads * hd)
+    assert api.check_device_status() == 0
+    for i in range(LAUNCHES):
+        for c in range(cols):
+            n = pos0 + c + 1
+            assert _close(out[i, c], _attend(q[i, c], kq[:n], vq[:n], n_kv, hd, scale)), f"launch {i}, column {c}"
+
+
+@pytest.mark.parametrize("group", [1, 3, 5, 6, 7, 8])
+@pytest.mark.parametrize("n_ctx,pos0,rows", [(300, 298, 1), (600, 590, 2), (2100, 2047, 1), (2100, 2092, 8)])
+def test_no_launch_over_the_f32_cache_reads_partials_that_are_not_written_yet(group, n_ctx, pos0, rows):
+    from hipml_b200 import api
+    n_kv, hd = 4, 256
+    heads, seq = n_kv * group, pos0 + rows
+    gen = torch.Generator(device="cuda").manual_seed(n_ctx + group)
+    k, v = (torch.randn(n_ctx, n_kv * hd, device="cuda", generator=gen) for _ in range(2))
+    splits = api.cols_splits(n_ctx)
+    acc, ml = (torch.empty(rows * heads * splits * n, device="cuda") for n in (hd, 2))
+    q = torch.randn(LAUNCHES, rows, heads * hd, device="cuda", generator=gen)
+    out = torch.full((LAUNCHES, rows, heads * hd), float("nan"), device="cuda")
+    for i in range(LAUNCHES):
+        acc.fill_(float("nan"))
+        ml.fill_(float("nan"))
+        api.attn_decode_cols_f32(q[i], k, v, acc, ml, out[i], heads, n_kv, hd, n_ctx, pos0, rows)
+    assert api.check_device_status() == 0
+    for i in range(LAUNCHES):
+        for c in range(rows):
+            n = pos0 + c + 1
+            assert _close(out[i, c], _attend(q[i, c], k[:n], v[:n], n_kv, hd, 0.0625)), f"launch {i}, column {c}"
 
 
 @pytest.mark.parametrize("heads,n_kv", [(24, 4), (8, 1), (2, 2)])
@@ -137,7 +235,10 @@ def test_f32_cache_decode_at_the_edges_of_runs(heads, n_kv, n_ctx, pos0, rows):
     splits = api.cols_splits(n_ctx)
     acc, ml = (torch.full((rows * heads * splits * n,), float("nan"), device="cuda") for n in (hd, 2))
     out = torch.full((rows, heads * hd), float("nan"), device="cuda")
-    for _ in range(2):
+    for _ in range(2):   # (the second finds the first one's counters, and scratch that was never written)
+        acc.fill_(float("nan"))
+        ml.fill_(float("nan"))
+        out.fill_(float("nan"))
         api.attn_decode_cols_f32(q, k, v, acc, ml, out, heads, n_kv, hd, n_ctx, pos0, rows)
     kn, vn, qn = k.cpu().numpy(), v.cpu().numpy(), q.cpu().numpy()
     for c in range(rows):
