@@ -424,8 +424,21 @@ __global__ void __launch_bounds__(kThreads, kWide ? 1 : 2) attn_decode_warps(Dec
     auto run_done = [&](int item, const Part &r) {
         if (one_run) emit_item(p, w.slot, w.kvh, group, item, r);
         const size_t row = (size_t)(item >> 6) * p.splits + w.run;
-        reinterpret_cast<float4 *>(part_acc + row * 256)[item & 63] = r.a;
-        if (writes_pair<kC>(items, rank, item)) *reinterpret_cast<float2 *>(part_ml + row * 2) = make_float2(r.m, r.l);
+        float *const acc_at = part_acc + row * 256 + 4 * (item & 63), *const ml_at = part_ml + row * 2;
+        const bool with_ml = writes_pair<kC>(items, rank, item);
+        if (p.out != nullptr) {
+            *reinterpret_cast<float4 *>(acc_at) = r.a;
+            if (with_ml) *reinterpret_cast<float2 *>(ml_at) = make_float2(r.m, r.l);
+        } else {   // partials that are folded by a launch of their own: scratch on any 4-byte boundary
+            acc_at[0] = r.a.x;
+            acc_at[1] = r.a.y;
+            acc_at[2] = r.a.z;
+            acc_at[3] = r.a.w;
+            if (with_ml) {
+                ml_at[0] = r.m;
+                ml_at[1] = r.l;
+            }
+        }
     };
     float4 *const inbox = reinterpret_cast<float4 *>(smem + C::kOffIn);
     float2 *const inbox_ml = reinterpret_cast<float2 *>(smem + C::kOffInMl);

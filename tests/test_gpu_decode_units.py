@@ -219,6 +219,48 @@ def test_no_launch_over_the_f32_cache_reads_partials_that_are_not_written_yet(gr
             assert _close(out[i, c], _attend(q[i, c], k[:n], v[:n], n_kv, hd, 0.0625)), f"launch {i}, column {c}"
 
 
+# floats by which part_acc, part_ml and their slots are off the alignment that the fold inside the kernel wants
+@pytest.mark.parametrize("acc_off,ml_off,acc_odd,ml_odd", [(0, 1, 0, 0), (0, 0, 0, 1), (0, 1, 0, 1), (1, 0, 3, 0), (3, 1, 1, 1)])
+@pytest.mark.parametrize("entry", ["rows q8_0", "rows q4_0", "batch append q8_0", "one slot", "columns"])
+def test_scratch_of_several_slots_may_lie_on_any_float(entry, acc_off, ml_off, acc_odd, ml_odd):
+    from hipml_b200 import api
+    heads, n_kv, hd, scale = 24, 4, 256, 0.0625
+    dtype = 1 if "q4" in entry else 0
+    row, deq = ((272, O.dequantize_q8), (144, O.dequantize_q4))[dtype]
+    lens = [700] if entry == "one slot" else [300, 301, 302] if entry == "columns" else [1, 700, 333]
+    slots, stride = len(lens), 704
+    caches = 1 if entry == "columns" else slots
+    gen = torch.Generator(device="cuda").manual_seed(acc_off + 8 * ml_off + 64 * acc_odd)
+    k, v = (torch.randn(caches, max(lens), n_kv * hd, device="cuda", generator=gen) for _ in range(2))
+    kc, vc = (torch.zeros(caches, n_kv * stride * row, dtype=torch.uint8, device="cuda") for _ in range(2))
+    for s in range(caches):
+        api.kv_encode_bulk(k[s], v[s], kc[s], vc[s], n_kv, hd, stride, 0, 0, max(lens), dtype)
+    kq, vq = (torch.from_numpy(np.stack([cases.unpack_head_major(deq(c[s].cpu().numpy().reshape(n_kv, stride, row)), n_kv,
+                                                                 stride, hd) for s in range(caches)])).cuda() for c in (kc, vc))
+    splits = 6
+    acc_slot, ml_slot = heads * splits * hd + acc_odd, heads * splits * 2 + ml_odd
+    acc = torch.full((slots * acc_slot + 4,), float("nan"), device="cuda")[acc_off:]
+    ml = torch.full((slots * ml_slot + 4,), float("nan"), device="cuda")[ml_off:]
+    q = torch.randn(slots, heads * hd, device="cuda", generator=gen)
+    out = torch.full((slots, heads * hd), float("nan"), device="cuda")
+    pos = torch.tensor([[n - 1, n] for n in lens], dtype=torch.int32, device="cuda")
+    tail = (splits, n_kv * stride * row, acc_slot, ml_slot, heads * hd, slots)
+    if entry == "columns":
+        api.attn_decode_cols(pos, q, kc, vc, acc, ml, out, heads, n_kv, hd, stride, scale, splits, slots, acc_slot, ml_slot,
+                             heads * hd)
+    elif entry == "one slot":
+        api.attn_decode_batch(pos, q, kc, vc, acc, ml, out, heads, n_kv, hd, stride, scale, *tail, lens[0])
+    elif entry == "batch append q8_0":
+        new = [torch.stack([x[s, n - 1] for s, n in enumerate(lens)]).contiguous() for x in (k, v)]
+        api.attn_decode_batch_append(pos, new[0], new[1], q, kc, vc, acc, ml, out, heads, n_kv, hd, stride, scale, *tail)
+    else:
+        api.attn_decode_rows(pos, q, kc, vc, acc, ml, out, heads, n_kv, hd, stride, scale, *tail, dtype=dtype)
+    assert api.check_device_status() == 0
+    for s, n in enumerate(lens):
+        c = 0 if entry == "columns" else s
+        assert _close(out[s], _attend(q[s], kq[c, :n], vq[c, :n], n_kv, hd, scale)), f"slot {s}"
+
+
 @pytest.mark.parametrize("heads,n_kv", [(24, 4), (8, 1), (2, 2)])
 @pytest.mark.parametrize("n_ctx,pos0,rows", [(1, 0, 1), (33, 31, 2), (260, 250, 3), (2100, 2090, 8), (8200, 8199, 1),
                                              (8200, 3, 2)])
