@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_decode_cols(DecodeParams p, 
     // Nothing that the grids ahead may write can be relied on before they are done, but the lengths as they
     // stand are a good guess: enough to plan with and to ask L2 for the first rows. They are checked below.
     auto read_len = [&]() {   // of column tid < n_slots
-        return min(max(__ldcg(p.len + p.len_offset + tid * p.len_stride), 0), p.stride);
+        return live_len(p, __ldcg(p.len + p.len_offset + tid * p.len_stride));
     };
     if (tid < p.n_slots) s_len[tid] = read_len();
     __syncthreads();

@@ -165,14 +165,14 @@ __global__ void __launch_bounds__(kThreads, kWide ? 1 : 2) attn_decode_warps(Dec
     const int first_slot = shared_plan ? tid : (int)blockIdx.y;
     const bool reads_len = !shared_plan || tid < p.n_slots;
     const int *len_at = p.len + p.len_offset + first_slot * p.len_stride;
-    auto clamp_len = [&](int n) { return min(max(n, 0), p.stride); };
+    auto read_len = [&]() { return live_len(p, __ldcg(len_at)); };
     Work w;
     if (shared_plan) {
-        if (reads_len) s_len[tid] = clamp_len(__ldcg(len_at));
+        if (reads_len) s_len[tid] = read_len();
         __syncthreads();
         w = plan_slots<C::kUnitRows>(p, s_len, s_plan);
     } else {
-        w = plan_stream<kC, C::kUnitRows>(p, first_slot, rank, clamp_len(__ldcg(len_at)));
+        w = plan_stream<kC, C::kUnitRows>(p, first_slot, rank, read_len());
     }
     // This warp's units are rows row0 + unit * (warp + 8 i), i < nw. Only the last one can be short or
     // hold the row to append (the last live row).
@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(kThreads, kWide ? 1 : 2) attn_decode_warps(Dec
     if constexpr (kC > 1) cluster_wait();
     for (;;) {
         // (the small loads first: behind the rows they would wait for all of them)
-        const int real_len = reads_len ? __ldcg(len_at) : 0;
+        const int real_len = reads_len ? read_len() : 0;
         float2 x[2][2];
         const float *const qh = p.q + (size_t)max(w.slot, 0) * p.q_slot + (size_t)(w.kvh * group + g) * 256;
 #pragma unroll
@@ -515,17 +515,19 @@ __global__ void __launch_bounds__(kThreads, kWide ? 1 : 2) attn_decode_warps(Dec
 template <int kC, int kUnitRows>
 __global__ void __launch_bounds__(kThreads) attn_decode_warps_fold(DecodeParams p, int *status) {
     __shared__ int s_quota;
+    __shared__ int s_len[64];
     __shared__ __align__(16) float staged[8 * 256 + 16];
     griddep_launch();
     griddep_wait();
     const int kvh = blockIdx.x, slot = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int group = p.n_heads / p.n_kv;
-    const int len = p.len[slot * p.len_stride + p.len_offset];
+    const int len = live_len(p, p.len[slot * p.len_stride + p.len_offset]);
     int runs = p.splits;
     if (p.share_slots > 0) {
+        if (tid < p.n_slots) s_len[tid] = live_len(p, p.len[tid * p.len_stride + p.len_offset]);
+        __syncthreads();
         if (warp == 0) {
-            const int q = shared_quota_warp(p.len, p.len_stride, p.len_offset, p.n_slots, p.splits, p.share_slots,
-                                            p.n_kv);
+            const int q = shared_quota_warp(s_len, 1, 0, p.n_slots, p.splits, p.share_slots, p.n_kv);
             if (lane == 0) s_quota = q;
         }
         __syncthreads();

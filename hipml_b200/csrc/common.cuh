@@ -33,8 +33,9 @@ inline int launch_status() { return static_cast<int>(cudaGetLastError()); }
 // start of the next costs as much as the small kernels themselves. Every kernel of this
 // library therefore (1) lets the next launch of the stream be scheduled as soon as all of
 // its own CTAs have started (griddep_launch at its top), and (2) waits for the previous
-// grid to have completed and flushed before it touches memory (griddep_wait; anything
-// before it is index arithmetic or loads of inputs that no kernel of the chain writes).
+// grid to have completed and flushed before it relies on memory (griddep_wait; before it there is
+// index arithmetic, and guesses: values read early to plan with, live lengths and position ids,
+// which are read again after it and compared, and requests to L2, which deliver nothing).
 // Because every kernel waits before it writes, completion is transitive along the chain.
 // Both instructions are no-ops in a launch without the attribute (a launch by name through
 // hipml_module_launch_kernel, a kernel that follows a foreign kernel).

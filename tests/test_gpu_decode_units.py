@@ -1,5 +1,7 @@
 """Decode at the edges of the default body's work units: a warp takes 16 rows, or 32 once a step has
 more 16-row units than warps; 8 warps per CTA, two CTAs per run. CPU definition: ops.rs:449-518."""
+import re
+
 import numpy as np
 import pytest
 import torch
@@ -93,6 +95,64 @@ def test_lengths_that_change_between_launches_are_seen():
     assert api.check_device_status() == 0
     for a, b in zip(outs, want):
         assert torch.equal(a, b)
+
+
+def _device_status():
+    from hipml_b200 import _lib, api
+    try:
+        return api.check_device_status()
+    except _lib.HipmlError as e:
+        return int(re.search(r"code (\d+)", e.text).group(1))
+
+
+@pytest.mark.parametrize("fold_mode", [0, 1], ids=["fold_inside", "fold_launch"])
+@pytest.mark.parametrize("entry", ["step", "step append", "columns", "slots", "slots append"])
+def test_a_length_past_the_cache_counts_as_the_cache_s(entry, fold_mode):
+    """No form reads or writes past the `stride` rows of a head; an append past them is reported (status 22)."""
+    from hipml_b200 import api
+    heads, n_kv, hd, scale, stride, beyond = 24, 4, 256, 0.0625, 300, 40
+    gen = torch.Generator(device="cuda").manual_seed(8)
+    # (rows follow the last head, so that a kernel that went on would be seen and not fault)
+    room = n_kv * stride * 272 + 4096 * 272
+    kc, vc = (torch.full((2, room), 0x7E, dtype=torch.uint8, device="cuda") for _ in range(2))
+    k, v = (torch.randn(stride, n_kv * hd, device="cuda", generator=gen) for _ in range(2))
+    for s in range(2):
+        api.kv_encode_bulk(k, v, kc[s], vc[s], n_kv, hd, stride, 0, 0, stride)
+    want_k, want_v = kc.clone(), vc.clone()
+    live = n_kv * stride * 272
+    kq, vq = (torch.from_numpy(cases.unpack_head_major(O.dequantize_q8(c[0, :live].cpu().numpy().reshape(n_kv, stride, 272)),
+                                                       n_kv, stride, hd)).cuda() for c in (kc, vc))
+    q = torch.randn(2, heads * hd, device="cuda", generator=gen)
+    new = torch.randn(2, n_kv * hd, device="cuda", generator=gen)
+    splits = 8
+    acc, ml = (torch.empty(2 * heads * splits * n, device="cuda") for n in (hd, 2))
+    out = torch.full((2, heads * hd), float("nan"), device="cuda")
+    lens = [stride + beyond, 7] if entry.startswith("slots") else [stride + beyond, stride + 1]
+    pos = torch.tensor([[n - 1, n] for n in lens], dtype=torch.int32, device="cuda")
+    args = (heads, n_kv, hd, stride, scale, splits)
+    slots = (heads * splits * hd, heads * splits * 2, heads * hd, 2)
+    api.set_decode_fold_mode(fold_mode)
+    try:
+        if entry == "step":
+            api.attn_decode_kv(pos[0], q[0], kc[0], vc[0], acc, ml, out[0], *args)
+        elif entry == "step append":
+            api.attn_decode_kv_append(pos[0], new[0], new[0], q[0], kc[0], vc[0], acc, ml, out[0], *args)
+        elif entry == "columns":
+            api.attn_decode_cols(pos, q, kc, vc, acc, ml, out, *args, 2, *slots[:3])
+        elif entry == "slots":
+            api.attn_decode_rows(pos, q, kc, vc, acc, ml, out, *args, room, *slots)
+        else:
+            new_rows = torch.stack([new[0], k[6]])   # (slot 1 appends what it holds already)
+            new_v = torch.stack([new[1], v[6]])
+            api.attn_decode_batch_append(pos, new_rows, new_v, q, kc, vc, acc, ml, out, *args, room, *slots)
+    finally:
+        api.set_decode_fold_mode(0)
+    assert _device_status() == (22 if "append" in entry else 0)
+    assert torch.equal(kc, want_k) and torch.equal(vc, want_v)
+    for s, n in enumerate(lens):
+        if s == 0 or not entry.startswith("step"):
+            n = min(n, stride)
+            assert _close(out[s], _attend(q[s], kq[:n], vq[:n], n_kv, hd, scale)), f"row {s}"
 
 
 # columns whose lengths cross a 16- or 32-row unit, the change of the unit (4,608) or nothing
