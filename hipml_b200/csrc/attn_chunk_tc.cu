@@ -809,7 +809,11 @@ attn_chunk_tc(const __grid_constant__ CUtensorMap map_k_hi, const __grid_constan
     // partials through distributed shared memory and writes the output.
     if constexpr (kFold) {
         cluster_sync_all();
-        if (warp < 8 && *abort_flag == 0) {
+        // A slice that gave up left no partial: then no CTA of the cluster writes output. (The flags are as they
+        // stood before the barrier, the same for all; one read per warp, on its way beside the first row's.)
+        const unsigned flag_addr = smem_u32(const_cast<int *>(abort_flag));
+        const int gave_up = lane < 2 * nsp ? ld_cluster_s32(map_to_cta(flag_addr, lane)) : 0;
+        if (warp < 8 && !__any_sync(0xffffffffu, gave_up != 0)) {
             constexpr int kPitch = kD + 4;
             const float *const stage = reinterpret_cast<const float *>(smem);
             const unsigned stage_addr = smem_u32(stage), ml_addr = smem_u32(stage + 128 * kPitch);

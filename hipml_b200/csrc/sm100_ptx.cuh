@@ -123,6 +123,11 @@ __device__ __forceinline__ float4 ld_cluster_f4(unsigned addr) {
                  : "memory");
     return v;
 }
+__device__ __forceinline__ int ld_cluster_s32(unsigned addr) {
+    int v;
+    asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+    return v;
+}
 __device__ __forceinline__ float2 ld_cluster_f2(unsigned addr) {
     float2 v;
     asm volatile("ld.shared::cluster.v2.f32 {%0,%1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr) : "memory");
