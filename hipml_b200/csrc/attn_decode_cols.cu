@@ -292,11 +292,30 @@ __global__ void __launch_bounds__(kThreads, 1) attn_decode_cols(DecodeParams p, 
             // ---- values
             wait(1);
             unsigned char *const vt = ring + C::kSlot;
-            if (rows < 16 * kT) {
-                // stale rows have weight 0, but their scales must not be NaN or infinite
-                for (int j = lane; j < (16 * kT - rows) * (kRowBytes / 16); j += 32)
-                    reinterpret_cast<uint4 *>(vt + rows * kRowBytes)[j] = make_uint4(0, 0, 0, 0);
+            // rows past the end have weight 0, but their scales must not be NaN or infinite
+            auto clear_rows = [&](int from, int to) {
+                for (int j = lane; j < (to - from) * (kRowBytes / 16); j += 32)
+                    reinterpret_cast<uint4 *>(vt + from * kRowBytes)[j] = make_uint4(0, 0, 0, 0);
                 __syncwarp();
+            };
+            if (rows < 16 * kT) clear_rows(rows, 16 * kT);
+            // Where a column ends inside the unit, the rows past its end are other columns': they stay. If one of them
+            // has such a scale, the columns take turns, the longest first, and each clears what it does not see.
+            unsigned on = (1u << n) - 1, left = 0;   // columns of the pass, columns of later passes
+            int upto = rows, shortest = rows;
+            auto rows_of = [&](int c) { return max(0, min(w.unit, min(row1, len[c]) - r0)); };
+#pragma unroll
+            for (int c = 0; c < kCols; c++)
+                if (c < n) shortest = min(shortest, rows_of(c));
+            bool apart = false;
+            if (shortest < rows) {
+                bool bad = false;
+                for (int j = lane; j < (rows - shortest) * 8; j += 32) {
+                    const unsigned char *const scale = vt + (shortest + (j >> 3)) * kRowBytes + (j & 7) * kQ8BlockBytes;
+                    bad = bad || (*reinterpret_cast<const unsigned short *>(scale) & 0x7c00u) == 0x7c00u;
+                }
+                apart = __any_sync(0xffffffffu, bad);
+                if (apart) left = on;
             }
             const unsigned *const vrow = reinterpret_cast<const unsigned *>(vt) + 2 * t * Row<false>::kPitch;
             auto value = [&](auto m) __attribute__((always_inline)) {
@@ -306,7 +325,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_decode_cols(DecodeParams p, 
                 for (int j = 0; j < kT; j++) load_v<M, false>(vrow + j * 16 * Row<false>::kPitch, g, f[j]);
 #pragma unroll
                 for (int c = 0; c < kCols; c++) {
-                    if (c >= n) break;
+                    if (!(on >> c & 1)) continue;
                     float a[16];
 #pragma unroll
                     for (int e = 0; e < 16; e++) a[e] = 0.0f;
@@ -330,14 +349,34 @@ __global__ void __launch_bounds__(kThreads, 1) attn_decode_cols(DecodeParams p, 
                     tmem_st16(tmem + 128 * c + 16 * M, a);
                 }
             };
-            value(Int<0>{});
-            value(Int<1>{});
-            value(Int<2>{});
-            value(Int<3>{});
+            for (;;) {
+                if (apart) {
+                    __syncwarp();
+                    int c_at = 0, most = -1;
+#pragma unroll
+                    for (int c = 0; c < kCols; c++)
+                        if ((left >> c & 1) && rows_of(c) > most) {
+                            most = rows_of(c);
+                            c_at = c;
+                        }
+                    clear_rows(most, upto);
+                    upto = most;
+                    on = 1u << c_at;
+                    left &= ~on;
+                }
+                value(Int<0>{});
+                value(Int<1>{});
+                value(Int<2>{});
+                value(Int<3>{});
+                if (left == 0) break;
+            }
             tmem_wait_st();
             __syncwarp();
             vp += step;
-            if (lane == 0 && i + 1 < nw) fetch(i + 1, vp, 1);
+            if (lane == 0 && i + 1 < nw) {
+                if (apart) fence_async_shared();   // generic writes to the slot come before the copy's
+                fetch(i + 1, vp, 1);
+            }
             phase ^= 1;
         };
         for (int i = 0; i < nw; i++) {

@@ -184,6 +184,36 @@ def test_columns_side_by_side_give_each_columns_own_bits(pos0, cols):
     assert api.check_device_status() == 0
 
 
+# the last columns' rows in the first one's last unit, or in one of their own
+@pytest.mark.parametrize("cols", [2, 4, 7])
+@pytest.mark.parametrize("pos0", [0, 13, 29, 200, 1278, 4604, 9214])
+@pytest.mark.parametrize("which", ["k", "v"])
+def test_a_column_does_not_see_the_next_one_s_infinite_scale(pos0, cols, which):
+    """A row whose values overflow f16 has infinite scales: what an earlier column does not see has no weight there,
+    whatever it holds."""
+    from hipml_b200 import api
+    heads, n_kv, hd, scale, stride = 24, 4, 256, 0.0625, pos0 + cols + 2
+    gen = torch.Generator(device="cuda").manual_seed(pos0 + cols)
+    kc, vc = (torch.zeros(n_kv * stride * 272, dtype=torch.uint8, device="cuda") for _ in range(2))
+    k, v = (torch.randn(pos0 + cols, n_kv * hd, device="cuda", generator=gen) for _ in range(2))
+    (k if which == "k" else v)[pos0 + 1:] = 1e9   # f16 scale: infinity
+    api.kv_encode_bulk(k, v, kc, vc, n_kv, hd, stride, 0, 0, pos0 + cols)
+    q = torch.randn(cols, heads * hd, device="cuda", generator=gen)
+    splits = api.decode_splits(pos0 + cols)
+    acc, ml = (torch.empty(cols * heads * splits * n, device="cuda") for n in (hd, 2))
+    out = torch.empty(cols, heads * hd, device="cuda")
+    pos = torch.tensor([[pos0 + c, pos0 + c + 1] for c in range(cols)], dtype=torch.int32, device="cuda")
+    api.attn_decode_cols(pos, q, kc, vc, acc, ml, out, heads, n_kv, hd, stride, scale, splits, cols,
+                         heads * splits * hd, heads * splits * 2, heads * hd)
+    assert torch.isfinite(out[0]).all()
+    for c in range(cols):
+        one = torch.empty(heads * hd, device="cuda")
+        step = torch.tensor([pos0 + c, pos0 + c + 1] + [0] * 6, dtype=torch.int32, device="cuda")
+        api.attn_decode_kv(step, q[c], kc, vc, acc, ml, one, heads, n_kv, hd, stride, scale, splits)
+        assert torch.equal(one.nan_to_num(7.0), out[c].nan_to_num(7.0)), f"column {c}"
+    assert api.check_device_status() == 0
+
+
 def _attend(q, k, v, n_kv, hd, scale):
     """softmax(q k^T) v of one query row per head, 64 bits: q [heads * hd], k and v [rows, n_kv * hd]."""
     heads = q.numel() // hd
