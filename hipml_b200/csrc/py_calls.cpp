@@ -76,6 +76,12 @@ struct From<float> {
     }
 };
 
+// Nothing is converted once an argument has failed: Python must not be called with an exception set.
+template <class T>
+T take(PyObject *o, bool &ok) {
+    return ok ? From<T>::py(o, ok) : T();
+}
+
 bool current_stream(hipml_stream_t &stream) {
     PyObject *dev = PyObject_CallNoArgs(g_get_device);
     if (!dev) return false;
@@ -101,7 +107,7 @@ struct Call<int (*)(hipml_stream_t, A...), fn> {
     static PyObject *go(PyObject *const *args, std::index_sequence<I...>) {
         bool ok = true;
         hipml_stream_t stream = nullptr;
-        std::tuple<A...> v{From<A>::py(args[I], ok)...};
+        std::tuple<A...> v{take<A>(args[I], ok)...};   // (braces: in order)
         if (!ok || !current_stream(stream)) return nullptr;
         int rc;
         Py_BEGIN_ALLOW_THREADS;   // (a launch waits when the device's queue is full)
