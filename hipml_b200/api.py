@@ -324,9 +324,8 @@ def attn_front_append_q8(qg, k, v, q, gate, q_norm, k_norm, k_cache, v_cache, n_
                          pos=None, step=None, k_out=None):
     """Split + norm + rope + q8_0 append of `tokens` rows in one launch."""
     rc = _c.attn_front_append_q8(qg, k, v, q, gate, k_out, q_norm, k_norm, k_cache, v_cache,
-                                 n_heads, n_kv, head_dim, n_rot, sections is not None, *(sections
-                                 or (0, 0, 0, 0)), pos, step, pos0, tokens, stride, theta_base,
-                                 eps)
+                                 n_heads, n_kv, head_dim, n_rot, sections, pos, step, pos0, tokens,
+                                 stride, theta_base, eps)
     if rc:
         _lib.check("attn_front_append_q8", rc)
 

@@ -76,6 +76,36 @@ struct From<float> {
     }
 };
 
+// A host array of up to four ints (the rest are 0), or None: any sequence of what int() takes.
+struct Sections {
+    bool given;
+    int s[4];
+};
+template <>
+struct From<Sections> {
+    static Sections py(PyObject *o, bool &ok) {
+        Sections r = {o != Py_None, {0, 0, 0, 0}};
+        PyObject *items = r.given ? PySequence_Tuple(o) : nullptr;
+        if (!items) {
+            ok = ok && !r.given;
+            return r;
+        }
+        const Py_ssize_t n = PyTuple_GET_SIZE(items);
+        if (n > 4) {
+            PyErr_Format(PyExc_IndexError, "%zd sections given, 4 at most", n);
+            ok = false;
+        }
+        for (Py_ssize_t i = 0; i < n && ok; i++) {
+            PyObject *v = PyNumber_Long(PyTuple_GET_ITEM(items, i));
+            ok = v != nullptr;
+            if (ok) r.s[i] = From<int>::py(v, ok);
+            Py_XDECREF(v);
+        }
+        Py_DECREF(items);
+        return r;
+    }
+};
+
 // Nothing is converted once an argument has failed: Python must not be called with an exception set.
 template <class T>
 T take(PyObject *o, bool &ok) {
@@ -121,15 +151,13 @@ struct Call<int (*)(hipml_stream_t, A...), fn> {
     }
 };
 
-// hipml_attn_front_append_q8: as above, but argument 14 (`sections`) is a host array: None or a
-// sequence of four ints.
+// hipml_attn_front_append_q8: as above, but argument 14 (`sections`) is a host array.
 int front_append(hipml_stream_t stream, const float *qg, const float *k, const float *v, float *q, float *gate,
                  float *k_out, const float *q_norm, const float *k_norm, void *k_cache, void *v_cache, int n_heads,
-                 int n_kv, int head_dim, int n_rot, int has_sections, int s0, int s1, int s2, int s3, const int *pos,
-                 const int *step, int pos0, int tokens, int stride, float theta_base, float eps) {
-    const int sections[4] = {s0, s1, s2, s3};
+                 int n_kv, int head_dim, int n_rot, Sections sections, const int *pos, const int *step,
+                 int pos0, int tokens, int stride, float theta_base, float eps) {
     return hipml_attn_front_append_q8(stream, qg, k, v, q, gate, k_out, q_norm, k_norm, k_cache, v_cache, n_heads,
-                                      n_kv, head_dim, n_rot, has_sections ? sections : nullptr, pos, step, pos0,
+                                      n_kv, head_dim, n_rot, sections.given ? sections.s : nullptr, pos, step, pos0,
                                       tokens, stride, theta_base, eps);
 }
 
