@@ -246,7 +246,10 @@ __device__ __forceinline__ void norm_rope_lane8(float (&x)[8], const float *w, i
 }
 
 // grid (tokens, row groups), block 256: CTA (t, y) takes head rows y * 8 + warp, + 8 * groups, ... of token t.
-__global__ void __launch_bounds__(256) attn_front_rows_q8(const __grid_constant__ FrontRowsParams p) {
+// kPerSm: CTAs per SM. Four (60 registers) is the quicker form of a few rounds (one token with its decode step: 0.14 us
+// a layer). Many tokens are bound by how many warps wait at once, each with one row's loads in flight: six.
+template <int kPerSm>
+__global__ void __launch_bounds__(256, kPerSm) attn_front_rows_q8(const __grid_constant__ FrontRowsParams p) {
     __shared__ float cs[kMaxHeadDim / 2], sn[kMaxHeadDim / 2];
     __shared__ __align__(16) unsigned char img[8][kMaxRowBytes];
     griddep_launch();
@@ -392,12 +395,15 @@ int launch_front_rows_q8(cudaStream_t stream, const float *qg, const float *k, c
     p.rope.theta_base = theta_base;
     p.eps = eps;
     rope_freqs(theta_base, n_rot, p.freq);
-    // A head row per warp while that leaves SMs free (one token of 24 + 8 rows took 9.0 us in one CTA, 4 in
-    // four); two CTAs per token beyond, where the angles' cost shows (2,048 tokens: 41.3 us with two, 45.1
-    // with four; 700 tokens: 17.1 us with two, 19.8 with one).
+    // A head row per warp while that leaves SMs free (one token of 24 + 8 rows: 6.1 us in one CTA, 3.1 in four);
+    // two CTAs per token beyond, where the angles' cost shows (2,048 tokens: 37.9 us with two, 40.4 with one, 40.0 with
+    // four; 700 tokens: 14.4, 16.4, 14.9). Six CTAs per SM from where four would need more than two rounds (2,048
+    // tokens: 44.9 us with four, 42.4 with five, 37.9 with six, 42.7 with eight, which spill; 700: 16.5, 14.8, 14.4, 17.4;
+    // 301 tokens with staging and attention after them: 109.8 us with six, 108.3 with four).
     const int all = (n_heads + 2 * n_kv + 7) / 8;
     const int groups = tokens <= 2 * 148 ? all : (all < 2 ? all : 2);
-    return launch_pdl(attn_front_rows_q8, dim3(tokens, groups), dim3(256), 0, stream, 1, p);
+    return launch_pdl(tokens > 4 * 148 ? attn_front_rows_q8<6> : attn_front_rows_q8<4>, dim3(tokens, groups), dim3(256), 0,
+                      stream, 1, p);
 }
 
 }  // namespace hipml

@@ -155,6 +155,27 @@ def test_fused_front_with_q8_append_chunk():
     _check_fused(tokens=50, pos0=131, stride=300, decode=False)
 
 
+@pytest.mark.parametrize("tokens", [296, 297, 592, 593, 700])
+def test_fused_front_gives_a_token_the_same_bits_at_every_size(tokens):
+    """The launch's form changes with the number of tokens (at 296 and 592): a token's rows do not."""
+    from hipml_b200 import api
+    n_heads, n_kv, hd, stride, pos0 = 24, 4, 256, tokens + 9, 5
+    gen = torch.Generator(device="cuda").manual_seed(tokens)
+    qg, k, v = (torch.randn(tokens, n * hd, device="cuda", generator=gen) for n in (2 * n_heads, n_kv, n_kv))
+    qn, kn = (1 + 0.1 * torch.randn(hd, device="cuda", generator=gen) for _ in range(2))
+    got = []
+    for piece in (tokens, 50):
+        q, gate = (torch.full((tokens, n_heads * hd), float("nan"), device="cuda") for _ in range(2))
+        kc, vc = (torch.full((n_kv * stride * 272,), CANARY, dtype=torch.uint8, device="cuda") for _ in range(2))
+        for t in range(0, tokens, piece):
+            n = min(piece, tokens - t)
+            api.attn_front_append_q8(qg[t:t + n], k[t:t + n], v[t:t + n], q[t:t + n], gate[t:t + n], qn, kn, kc, vc,
+                                     n_heads, n_kv, hd, 64, THETA, EPS, pos0=pos0 + t, tokens=n, stride=stride)
+        got.append((q, gate, kc, vc))
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
+
+
 def test_fused_front_with_q8_append_one_decode_token():
     _check_fused(tokens=1, pos0=37, stride=64, decode=True)
 
