@@ -401,8 +401,9 @@ int launch_front_rows_q8(cudaStream_t stream, const float *qg, const float *k, c
     // tokens: 44.9 us with four, 42.4 with five, 37.9 with six, 42.7 with eight, which spill; 700: 16.5, 14.8, 14.4, 17.4;
     // 301 tokens with staging and attention after them: 109.8 us with six, 108.3 with four).
     const int all = (n_heads + 2 * n_kv + 7) / 8;
-    const int groups = tokens <= 2 * 148 ? all : (all < 2 ? all : 2);
-    return launch_pdl(tokens > 4 * 148 ? attn_front_rows_q8<6> : attn_front_rows_q8<4>, dim3(tokens, groups), dim3(256), 0,
+    const int sms = device_sms();
+    const int groups = tokens <= 2 * sms ? all : (all < 2 ? all : 2);
+    return launch_pdl(tokens > 4 * sms ? attn_front_rows_q8<6> : attn_front_rows_q8<4>, dim3(tokens, groups), dim3(256), 0,
                       stream, 1, p);
 }
 

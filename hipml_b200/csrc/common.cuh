@@ -101,6 +101,9 @@ const void *lookup_front_kernel(const char *name);
 // Device status word set by kernels whose bounded waits ran out.
 int *device_status_word();
 
+// SMs of the current device (148 where it cannot be asked).
+int device_sms();
+
 // ---- device helpers -------------------------------------------------------
 
 // Byte offset of row (kvh, pos) of a head-major q8 cache with `stride` rows per head.

@@ -3,6 +3,7 @@
 // runtime. Same conventions: int status, 0 = success, opaque handles, memcpy kinds 1/2/3.
 // Also the error-message plumbing shared by the launchers and the built-in kernel table
 // behind hipml_module_get_function.
+#include <atomic>
 #include <cstring>
 
 #include "common.cuh"
@@ -44,6 +45,19 @@ int *device_status_word() {
     if (cudaGetSymbolAddress(reinterpret_cast<void **>(&p), g_device_status) != cudaSuccess)
         return nullptr;
     return p;
+}
+
+int device_sms() {
+    static std::atomic<int> cached[64];
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64) dev = 0;
+    int sms = cached[dev].load();
+    if (sms == 0) {
+        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
+        cached[dev].store(sms);
+    }
+    return sms;
 }
 
 }  // namespace hipml

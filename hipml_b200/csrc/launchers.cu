@@ -27,24 +27,11 @@ int check_encode(int dtype, int n_kv, int head_dim, int stride) {
 
 // Live runs per KV head of the single-stream split pass: one round of the device's CTA slots
 // (two CTAs per SM), so that every CTA streams one long run instead of several short ones.
-// Cached per device; hipml_set_decode_cta_slots overrides it for every device.
+// hipml_set_decode_cta_slots overrides it for every device.
 std::atomic<int> g_cta_slots_override{0};
 int decode_cta_slots() {
     const int forced = g_cta_slots_override.load();
-    if (forced > 0) return forced;
-    static std::atomic<int> cached[64];
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64) dev = 0;
-    int slots = cached[dev].load();
-    if (slots == 0) {
-        int sms = 0;
-        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
-            sms = 148;
-        slots = 2 * sms;
-        cached[dev].store(slots);
-    }
-    return slots;
+    return forced > 0 ? forced : 2 * device_sms();
 }
 int decode_run_cap(int n_kv) {
     const int cap = decode_cta_slots() / (n_kv > 0 ? n_kv : 1);
