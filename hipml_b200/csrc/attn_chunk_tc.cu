@@ -957,26 +957,33 @@ static int fold_capacity(int slices) {
 // (the tensor cores' rate; a little faster while other SMs idle) behind ~13 us of its own, of which ~8 go
 // into moving its 2 x 126 query rows in and its output rows out (an SM moves ~30 B/ns). A launch with fewer
 // pairs than the device has SM pairs can therefore be shortened by slices of the keys, which fold in one
-// cluster (~3 us; 301 tokens at 3,001: 32 pairs, 26 tiles, 127 us in one), and by smaller query tiles (300
-// tokens at 0: 36.2 -> 33.4 us; not where the walk is long: 536 at 4,014 179 -> 199 us with tiles of 15
-// instead of 21). This takes the shape that an estimate from those figures says is shortest, among those
-// whose clusters all start together; a slice stays below the 64 tiles where a pair would move its sums to
-// memory. Launches of more pairs than that keep whole tiles and one slice.
+// cluster (~3 us; 301 tokens at 3,001: 32 pairs, 26 tiles, 127 us in one), and by smaller query tiles. Those
+// shorten what a pair does before and after its walk, but more pairs slow each other down: two thirds of the
+// size gain ~1 us up to 48 pairs (240 tokens at 0: 23.0 us against 23.9; 300: 27.2, 28.3) and lose it beyond
+// (400 tokens at 0, 60 pairs: 35.0 against 32.6; 500, 72 pairs: 38.8, 34.2), so they are for launches that leave
+// a third of the places free; slices also take the size that fills the pairs a whole tile needs (64 tokens at
+// 2,000 in five slices: 39.2 us with tiles of 16, 40.5 of 21; one slice gains nothing from it). This takes the
+// shape that an estimate from those figures says is shortest, among those whose clusters all start together;
+// a slice stays below the 64 tiles where a pair would move its sums to memory. Launches of more pairs than
+// that keep whole tiles and one slice.
 struct ChunkShape {
     int qtile, fold;
 };
 static ChunkShape chunk_shape(int tokens, int n_kv, int group, int key_tiles) {
     // (tiles below two thirds of the full one gained nothing more)
-    const int smallest = (2 * (128 / group) + 2) / 3;
-    ChunkShape best = {128 / group, 1};
+    const int full = 128 / group, smallest = (2 * full + 2) / 3;
+    const int few = fold_capacity(1) * 2 / 3;
+    auto pairs_of = [&](int qtile) { return ((tokens + qtile - 1) / qtile + 1) / 2 * n_kv; };
+    ChunkShape best = {full, 1};
     float best_us = 1e30f;
     for (int fold = 1; fold <= kMaxFold; fold++) {
         if (fold > 1 && (key_tiles < 2 * fold || (key_tiles + fold - 1) / fold > kFlushTiles)) continue;
         const int room = fold_capacity(fold) / n_kv;   // clusters per KV head that start together
         if (room < 1) continue;
         const int least = (tokens + 2 * room - 1) / (2 * room);
-        for (int qtile = least > smallest ? least : smallest; qtile <= 128 / group; qtile++) {
-            const int pairs = ((tokens + qtile - 1) / qtile + 1) / 2 * n_kv * fold;
+        for (int qtile = least > smallest ? least : smallest; qtile <= full; qtile++) {
+            const int pairs = pairs_of(qtile) * fold;
+            if (qtile < full && pairs > few && (fold == 1 || pairs > pairs_of(full) * fold)) continue;
             const float step = 3.1f + 0.022f * (float)pairs;
             const float us = step * (float)((key_tiles + fold - 1) / fold) + 8.0f * (float)(qtile * group) / 126.0f +
                              (fold > 1 ? 3.0f : 0.0f);
