@@ -607,12 +607,13 @@ static int check_stage(const void *k_cache, const void *v_cache, int n_kv, int h
 // tensor-core path has ~17 us of fixed latency and takes 21 - 28 us up to 1,024 keys. The small kernel is bound by
 // the walk of the last token's CTA, 4 us + 5.6 us per 100 keys (6.9 with groups of more than six), and from about a
 // wave of CTAs on by their number (tokens * n_kv: 2 us per 1,000 (query, key) pairs of 4 KV heads). 1 to 37 tokens
-// with 256 keys to see: 18.3 - 19.5 us against 21.2 - 23.2; with 384: 25.3 - 27.2 against 25.5 - 27.2; with 1,000, where
-// pairs alone would let one token in, 59 against 24. Groups of eight, 192 keys: 18.1 against 20.4, 256: 23 against 20.
+// with 256 keys to see: 18.3 - 19.5 us against 21.2 - 23.2; with 384: 25.3 - 27.2 against 25.5 - 27.2; with 448, two key
+// slices there: 28.8 - 30.7 against 22.4 - 27.5; with 1,000, where pairs alone would let one token in, 59 against 24.
+// Groups of eight, 192 keys: 18.1 against 20.4, 256: 23 against 20.
 // 100 tokens at 0: 17 against 25; 64 at 128 (10,300 pairs): 22.4 against 23.5; 100 at 92: 31 against 23.
 static bool small_chunk(int n_heads, int n_kv, int pos0, int tokens) {
     const long long pairs = (long long)tokens * pos0 + (long long)tokens * (tokens + 1) / 2;
-    return pos0 + tokens <= (n_heads > 6 * n_kv ? 208 : 256) && pairs * n_kv <= 26000;
+    return pos0 + tokens <= (n_heads > 6 * n_kv ? 208 : 384) && pairs * n_kv <= 26000;
 }
 
 size_t hipml_attn_chunk_workspace_bytes(int n_kv, int head_dim, int pos0, int tokens) {

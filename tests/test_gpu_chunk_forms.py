@@ -16,7 +16,7 @@ def _sampled(tokens):
 
 
 # (tokens, pos0): small form at its edges; 8, 7, .. 2 slices; odd tile counts; slices without keys; none
-SIZES = [(1, 0), (3, 4), (1, 255), (1, 256), (20, 236), (20, 237), (5, 127), (37, 29), (90, 45), (91, 46), (37, 700), (21, 1900), (43, 1111), (64, 2500),
+SIZES = [(1, 0), (3, 4), (1, 383), (1, 384), (9, 375), (9, 376), (5, 127), (37, 29), (90, 45), (91, 46), (37, 700), (21, 1900), (43, 1111), (64, 2500),
          (130, 1500), (170, 1024), (301, 3001), (230, 90), (337, 120)]
 
 
