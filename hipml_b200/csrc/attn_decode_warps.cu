@@ -511,15 +511,19 @@ __global__ void __launch_bounds__(kThreads, kWide ? 1 : 2) attn_decode_warps(Dec
 }
 
 
-// The fold of the runs as a launch of its own (grid (n_kv, slots)): the same arithmetic, bit for bit.
-template <int kC, int kUnitRows>
+// The fold of the runs as a launch of its own: the same arithmetic, bit for bit. Grid (n_kv * slices, slots), a CTA a
+// slice of the outputs; with the exchange, which wants whole heads in one CTA, (n_kv, slots). kBatch: runs whose
+// loads are issued together.
+template <int kC, int kUnitRows, int kBatch>
 __global__ void __launch_bounds__(kThreads) attn_decode_warps_fold(DecodeParams p, int *status) {
     __shared__ int s_quota;
     __shared__ int s_len[64];
     __shared__ __align__(16) float staged[8 * 256 + 16];
     griddep_launch();
     griddep_wait();
-    const int kvh = blockIdx.x, slot = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const bool exchange = p.xch.phases != 0;
+    const int slices = gridDim.x / p.n_kv, kvh = blockIdx.x / slices, slice = blockIdx.x - kvh * slices;
+    const int slot = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int group = p.n_heads / p.n_kv;
     const int len = live_len(p, p.len[slot * p.len_stride + p.len_offset]);
     int runs = p.splits;
@@ -535,9 +539,11 @@ __global__ void __launch_bounds__(kThreads) attn_decode_warps_fold(DecodeParams 
     } else if (!p.by_stride && p.run_cap > 0) {
         runs = balance(p, len, kC, kUnitRows).runs;
     }
-    const bool exchange = p.xch.phases != 0;
-    for (int r = 0; r < kC; r++) fold_runs<kC, 1, 8>(p, slot, 1, kvh, group, runs, r, exchange ? staged : nullptr);
-    if (!exchange) return;
+    if (!exchange) {
+        fold_runs<kC, 1, kBatch>(p, slot, 1, kvh, group, runs, slice, nullptr, slices);
+        return;
+    }
+    for (int r = 0; r < kC; r++) fold_runs<kC, 1, 8>(p, slot, 1, kvh, group, runs, r, staged);
     __syncthreads();
     FoldAcc f;
     if (warp < group) {
@@ -623,7 +629,14 @@ int launch(cudaStream_t stream, const DecodeParams &p, int slots) {
                                         (size_t)Cfg<kQ4, kWide>::kSmem, stream, kC, q, status);
     if (rc != 0 || !second_launch) return rc;
     q.out = p.out;
-    return launch_pdl(attn_decode_warps_fold<kC, Cfg<kQ4, kWide>::kUnitRows>, dim3(q.n_kv, slots), dim3(kThreads), 0, stream, 1, q, status);
+    // Slices while their CTAs are few (672 rows 16.4 us with the split pass in one, 10.0 in eight; 16 slots of up to 3,000
+    // rows 24.3 in one, 26.4 in four); many loads at once where there can be many runs (one slot of 256: 39.8 us by
+    // eights, 25.4; 64 slots of few: 16.4, 18.7).
+    constexpr int kUnitRows = Cfg<kQ4, kWide>::kUnitRows;
+    int slices = q.xch.phases ? 1 : (kC > 4 ? kC : 4);
+    while (slices > 1 && slots * q.n_kv * slices > (kC > 1 ? 2 * device_sms() : 64)) slices /= 2;
+    return launch_pdl(q.splits > 16 ? attn_decode_warps_fold<kC, kUnitRows, 18> : attn_decode_warps_fold<kC, kUnitRows, 8>,
+                      dim3(q.n_kv * slices, slots), dim3(kThreads), 0, stream, 1, q, status);
 }
 
 template <int kC, bool kWide>

@@ -613,15 +613,15 @@ __device__ __forceinline__ void emit_item(const DecodeParams &p, int slot, int k
     }
 }
 
-// Folds the `runs` partials of slice `rank` of a head group (of each of `cols` slots from `slot` on) from
+// Folds the `runs` partials of slice `rank` of `slices` of a head group (of each of `cols` slots from `slot` on) from
 // memory and emits it (or, staged != nullptr, leaves it there: [8 heads][256] sums, then [8 heads]{max,
 // sum}). kPer items a thread, kBatch runs in one round trip: 18 for the runs of a deep stream (B200: 18 pairs
 // of SMs per KV head; three trips of 8 took 2.9 us at the end of every launch).
 template <int kC, int kPer, int kBatch>
 __device__ __forceinline__ void fold_runs(const DecodeParams &p, int slot, int cols, int kvh, int group, int runs,
-                                          int rank, float *staged) {
+                                          int rank, float *staged, int slices = kC) {
     constexpr int kShare = Split<kC>::kShare;
-    const int items = group * 64, first = items * rank / kC, count = items * (rank + 1) / kC - first;
+    const int items = group * 64, first = items * rank / slices, count = items * (rank + 1) / slices - first;
     const int part = threadIdx.x % kShare, total = cols * count;
     for (int f0 = threadIdx.x / kShare; f0 - (int)threadIdx.x / kShare < total; f0 += kPer * (kThreads / kShare)) {
         const float *pa[kPer], *pm[kPer];
