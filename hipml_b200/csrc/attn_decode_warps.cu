@@ -648,18 +648,20 @@ int launch_c(cudaStream_t stream, const DecodeParams &p, int slots) {
 
 // Which form. One stream (or columns of one) has ~37 SMs per KV head: clusters of two, wide (8,192 rows: 11.5 us
 // a layer while partials were still read, against 14.4 with two small CTAs per SM and 13.1 with clusters of four,
-// of which only 33 fit the device; 1,100 rows: 8.2 us, of four 8.4, of eight 9.4); clusters of eight up to the 1,023
-// rows that the engine's policy gives fewer than 128 splits, where one holds a head and nothing is folded through
-// memory (672 rows: 8.2 us with pairs, 7.3; 1,000: 8.3, 7.6), of four up to 519 (300 rows: 7.1 us with eight, 6.8).
+// of which only 33 fit the device); clusters of eight up to the 1,023 rows that the engine's policy gives fewer than
+// 128 splits, where one holds a head and nothing is folded through memory (700 rows, launches in a row: 7.4 us, of four
+// 8.4, of two 8.0), while the device holds those of two launches (15: with eight KV heads the next launch waits for
+// this one, 10.5 us against 8.7 with pairs); of four up to 519 (300 rows: 6.4 us, of eight 7.0, of two 8.0; below ~200
+// rows pairs would be 0.5 us quicker still, but how long a stream is the host does not know from so few splits).
 // Several slots: no clusters, a head has too few CTAs to pair them; wide up to 28 (slot, head) pairs (4 KV
 // heads, 5 slots of 512 .. 3,000 rows: 14.9 us a layer against 16.5), beyond that the twice as fine runs of
 // the small CTAs balance better (8 slots of 512 .. 8,192: 24.6 us against 25.4, 10 slots 32.8 against 34.2).
 int launch_decode_warps(cudaStream_t stream, const DecodeParams &p, int slots) {
     const bool one_stream = !p.by_stride && p.run_cap >= 4 && p.share_slots == 0;
     if (one_stream)
-        return p.splits >= 128 || p.run_cap < 16 ? launch_c<2, true>(stream, p, slots)
-               : p.splits > 64                  ? launch_c<8, true>(stream, p, slots)
-                                                : launch_c<4, true>(stream, p, slots);
+        return p.splits >= 128 || p.run_cap < 16 || (p.splits > 64 && p.n_kv > 6) ? launch_c<2, true>(stream, p, slots)
+               : p.splits > 64                                                    ? launch_c<8, true>(stream, p, slots)
+                                                                                  : launch_c<4, true>(stream, p, slots);
     return p.share_slots > 0 && slots * p.n_kv <= 28 ? launch_c<1, true>(stream, p, slots)
                                                      : launch_c<1, false>(stream, p, slots);
 }

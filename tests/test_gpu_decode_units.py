@@ -68,6 +68,28 @@ def test_partials_sent_within_a_cluster_for_any_group(group, seq):
     assert ok and ma <= 2e-5 and rl <= 2e-5, (ma, rl)
 
 
+# more KV heads than the device holds clusters of eight for two launches, and a tensor-parallel rank's one
+@pytest.mark.parametrize("n_kv,group", [(8, 4), (7, 3), (6, 4), (1, 6)])
+@pytest.mark.parametrize("seq", [300, 600, 1000, 1300])
+def test_step_with_other_numbers_of_heads(seq, n_kv, group):
+    from hipml_b200 import api
+    heads, hd, scale = n_kv * group, 256, 0.0625
+    gen = torch.Generator(device="cuda").manual_seed(seq + n_kv)
+    k, v = (torch.randn(seq, n_kv * hd, device="cuda", generator=gen) for _ in range(2))
+    q = torch.randn(heads * hd, device="cuda", generator=gen)
+    kc, vc = (torch.zeros(n_kv * seq * 272, dtype=torch.uint8, device="cuda") for _ in range(2))
+    api.kv_encode_bulk(k, v, kc, vc, n_kv, hd, seq, 0, 0, seq)
+    kq, vq = (torch.from_numpy(cases.unpack_head_major(O.dequantize_q8(c.cpu().numpy().reshape(n_kv, seq, 272)), n_kv,
+                                                       seq, hd)).cuda() for c in (kc, vc))
+    splits = api.decode_splits(seq)
+    acc, ml = (torch.full((heads * splits * n,), float("nan"), device="cuda") for n in (hd, 2))
+    out = torch.full((heads * hd,), float("nan"), device="cuda")
+    step = torch.tensor([seq - 1, seq] + [0] * 6, dtype=torch.int32, device="cuda")
+    api.attn_decode_kv(step, q, kc, vc, acc, ml, out, heads, n_kv, hd, seq, scale, splits)
+    assert api.check_device_status() == 0
+    assert _close(out, _attend(q, kq, vq, n_kv, hd, scale))
+
+
 def test_lengths_that_change_between_launches_are_seen():
     """The kernel plans from the length as it stands before the grids ahead are done; a length written by
     the kernel right before it must win."""
