@@ -24,8 +24,8 @@
 //     8 x 8 tiles, as an exact f16 high + low pair after multiplication with the block's scale; the
 //     codes are the A operand (16 dims x 16 keys), converted exactly (0x6400 | (code + 128) is
 //     1152 + code). 64 accumulators per lane hold all 256 dims x 8 heads.
-// What bounds it: long caches the HBM stream and the issue rate together (100,000 rows: 42.6 us a
-// layer = 5.1 TB/s, 33 us of it in the loop; 1,555 warp instructions per 32 rows of K and V, where 64-row
+// What bounds it: long caches the HBM stream and the issue rate together (100,000 rows: 43 - 45 us a
+// layer in a captured chain = 4.85 - 5.04 TB/s, 33 us of it in the loop; 1,555 warp instructions per 32 rows of K and V, where 64-row
 // tiles with CTA barriers and softmax through shared memory took 2,370, 57 us a layer); short ones
 // the chain of dependent latencies (8,192 rows: 10.7 us, before 16).
 //

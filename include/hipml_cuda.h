@@ -172,10 +172,10 @@ int hipml_kv_append_chunk_f32(hipml_stream_t stream, float *k_cache, float *v_ca
  * attn_decode_kv_reduce, launch_kv.rs:232-279) with split s over positions [s*per, (s+1)*per),
  * per = ceil(seq/splits). The scalar kernel (selector 6, or any head_dim other than 256) keeps
  * exactly that and fills every slot. The tensor-core kernel is ONE launch and deals the rows
- * out for this device instead: at most R = min(splits, the device's pairs of SMs / n_kv) runs per
- * KV head, only as many as the live rows can occupy, partial of run r in slot r; of the other slots
- * those below R and the first 32 receive neutral partials (max -inf, sum 0), the rest are not
- * written. The last CTA to finish a part of a KV head's outputs folds the runs into `out`. A
+ * out for this device instead: at most R = min(splits, the device's clusters / n_kv) runs per KV
+ * head (a cluster of two SMs, or of four or eight where splits < 128), only as many as the live rows
+ * can occupy, partial of run r in slot r; of the other slots those below R and the first 32 receive
+ * neutral partials (max -inf, sum 0), the rest are not written. The last CTA to finish a part of a KV head's outputs folds the runs into `out`. A
  * caller must therefore not point the by-name attn_decode_kv_reduce kernel at these partials.
  * The tensor-core kernel needs out, part_acc (16 bytes) and part_ml (8 bytes) aligned. Two
  * calls that may overlap on the device must not share scratch (as in the reference); the
@@ -209,8 +209,8 @@ int hipml_kv_append_cols_f32(hipml_stream_t stream, float *k_cache, float *v_cac
  * (position, length) pair (pos[2c], pos[2c+1]), scratch slices (c*acc_slot, c*ml_slot floats)
  * and output row (out + c*q_slot). Every column is partitioned over its own live length with
  * the given split count, so its result is bit-identical to its one-column hipml_attn_decode_kv
- * launch (the caller groups columns of equal split count, as the reference does). selector 0
- * or 4. */
+ * launch (the caller groups columns of equal split count, as the reference does). Columns that share
+ * a launch write the partials of their live runs only, no neutral ones. selector 0 or 4. */
 int hipml_attn_decode_cols(hipml_stream_t stream, int selector, const int *pos, const float *q,
                            const void *k, const void *v, float *part_acc, float *part_ml,
                            float *out, int n_heads, int n_kv, int head_dim, int stride, float scale,
@@ -411,11 +411,15 @@ size_t hipml_attn_chunk_workspace_bytes(int n_kv, int head_dim, int pos0, int to
  * [splits][qslots][n_heads][2] with qslots = tokens rounded up to 32, and a combine pass
  * writes out (attn_chunk_split.hip:343-376).
  * mode: 0 = tensor-core kernel with error-compensated half-precision operands (meets the f32
- * tolerance), 1 = tensor-core kernel, single half-precision pass (the reference kernel's own
- * precision), 2 = scalar f32 kernel (any head_dim multiple of 32 up to 256; no workspace),
- * 3 = as 0 but one CTA per query tile instead of CTA pairs (A/B form of the same arithmetic).
- * workspace: device memory of at least hipml_attn_chunk_workspace_bytes(...) for modes 0/1/3,
- * 256-byte aligned. The tensor-core modes want q, out, the caches and part_acc 16-byte aligned
+ * tolerance); one-pass calls with few (query, key) pairs instead take a CUDA-core kernel that
+ * reads the cache as it lies, in f32, and leaves the workspace alone (do not count on a staged
+ * image after this call; hipml_attn_chunk_stage makes one). 1 = tensor-core kernel, single
+ * half-precision pass (the reference kernel's own precision), 2 = scalar f32 kernel (any head_dim
+ * multiple of 32 up to 256; no workspace), 3 = as 0 but always one CTA per query tile on the tensor
+ * cores (A/B form; modes 0 and 1 run CTA pairs and, where a launch has few query tiles, smaller
+ * tiles and up to eight key slices per tile folded inside the kernel).
+ * workspace: device memory of at least hipml_attn_chunk_workspace_bytes(...) for modes 0/1/3 at
+ * every size, 256-byte aligned. The tensor-core modes want q, out, the caches and part_acc 16-byte aligned
  * and part_ml 8-byte aligned (rows leave the kernel as whole 1 KB bulk copies). */
 int hipml_attn_chunk(hipml_stream_t stream, const float *q, const void *k_cache,
                      const void *v_cache, float *out, int n_heads, int n_kv, int head_dim,
