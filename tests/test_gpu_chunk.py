@@ -51,6 +51,20 @@ def _run_chunk(c: cases.ChunkCase, kv_dtype, mode, splits=1, poison_scratch=True
     return out.cpu().numpy()
 
 
+def _run_staged(c: cases.ChunkCase, splits=1):
+    """The q8_0 case through the staged entry, which takes the tensor-core kernel at every size (mode 0)."""
+    from hipml_b200 import api
+    nhd = c.heads * c.hd
+    seq = c.pos0 + c.tok
+    cap = (seq + 127) // 128 * 128
+    ws = torch.full((api.attn_chunk_workspace_bytes(c.n_kv, c.hd, 0, cap),), 0xFF, dtype=torch.uint8, device="cuda")
+    api.attn_chunk_stage(_dev(c.kb), _dev(c.vb), c.n_kv, c.hd, 1, c.stride, 0, seq, cap, ws)
+    out = torch.full((c.tok, nhd), float("nan"), device="cuda")
+    api.attn_chunk_staged(_dev(c.q), out, c.heads, c.n_kv, c.hd, c.pos0, c.tok, cap, ws)
+    assert api.check_device_status() == 0
+    return out.cpu().numpy()
+
+
 def _assert_bar(expected, got, mode, label=""):
     assert np.all(np.isfinite(got)), f"{label}: non-finite output"
     ok, ma, rl = cases.attention_within_bar(expected, got)
@@ -88,16 +102,29 @@ def test_q8_cache_with_stride_beyond_live_length(mode):
 def test_tile_edges_tensor_core(tok, pos0):
     """Query counts around the 21-query tile and key counts around the 128-key tile."""
     c = cases.chunk_case_q8(tok=tok, pos0=pos0, seed=0xED6E + tok + pos0)
-    _assert_bar(cases.chunk_expected(c, threads=4), _run_chunk(c, 1, 0), 0, f"{tok}@{pos0}")
+    expected = cases.chunk_expected(c, threads=4)
+    _assert_bar(expected, _run_chunk(c, 1, 0), 0, f"{tok}@{pos0}")
+    # (few pairs go straight from the cache there: the tensor-core kernel through the staged entry)
+    _assert_bar(expected, _run_staged(c), 0, f"{tok}@{pos0} staged")
 
 
 def test_other_gqa_groups_and_head_dims():
-    # group 8 and group 4 on the tensor-core kernel; head_dim 64 on the scalar kernel
+    # group 8 and group 4 straight from the cache and on the tensor-core kernel; head_dim 64 on the scalar kernel
     for heads, n_kv in ((16, 2), (8, 2)):
         c = cases.chunk_case_q8(heads=heads, n_kv=n_kv, tok=40, pos0=70, seed=0x6A + heads)
-        _assert_bar(cases.chunk_expected(c), _run_chunk(c, 1, 0), 0, f"group {heads // n_kv}")
+        expected = cases.chunk_expected(c)
+        _assert_bar(expected, _run_chunk(c, 1, 0), 0, f"group {heads // n_kv}")
+        _assert_bar(expected, _run_staged(c), 0, f"group {heads // n_kv} staged")
     c = cases.chunk_case_f32(heads=8, n_kv=2, hd=64, tok=19, pos0=11)
     _assert_bar(cases.chunk_expected(c), _run_chunk(c, 0, 2), 2, "hd64 scalar")
+
+
+# query tile and key slices follow the group: one slice, two, four, eight
+@pytest.mark.parametrize("heads,n_kv", [(4, 4), (16, 4), (32, 4), (8, 1)])
+@pytest.mark.parametrize("tok,pos0", [(60, 30), (50, 600), (70, 1100), (33, 2300)])
+def test_tensor_core_kernel_for_other_groups(tok, pos0, heads, n_kv):
+    c = cases.chunk_case_q8(heads=heads, n_kv=n_kv, tok=tok, pos0=pos0, seed=0x6B + heads + tok)
+    _assert_bar(cases.chunk_expected(c, threads=4), _run_staged(c), 0, f"{heads}/{n_kv} {tok}@{pos0}")
 
 
 def test_config1_prefill_672_tokens_f32_cache():
