@@ -379,7 +379,8 @@ int hipml_attn_decode_kv_static(hipml_stream_t stream, const int *step, int sele
  * `splits` runs per head and slot. The reference cuts every slot's cache into `splits` runs of
  * ceil(stride/splits) rows fixed in cache positions; at head_dim 256 with up to 64 slots this
  * library instead reads the live lengths on the device and deals the batch's 64-key tiles out
- * to one round of CTAs, each slot getting runs in proportion to its live length (still safe to
+ * to one round of CTAs, each slot getting runs in proportion to its live length, and one slot is
+ * taken as hipml_attn_decode_kv takes a stream (still safe to
  * replay from a captured graph: nothing of the plan is baked into the launch). */
 int hipml_attn_decode_rows(hipml_stream_t stream, int dtype, const int *pos, const float *q,
                            const void *k_cache, const void *v_cache, float *part_acc,
