@@ -50,7 +50,8 @@ __device__ int g_arrive_cols[kArriveRegions * kArriveRegionInts];
 // most `each` of them, are a group; a cluster has run `run` of groups `group`, `group` + `hop`, ... Groups go
 // to clusters of their own while a head has clusters to spare for their runs, and columns share conversions
 // beyond (4 columns of 300 rows take 2 runs each: 8 clusters of the head's 18; of 8,192 rows 17: one cluster
-// per run takes all four).
+// per run takes all four). `cap`: the clusters of a head; what its groups do not need ends at once, so there is one
+// round of them and they take the groups in turn.
 struct Share {
     int each, run, group, hop;
     unsigned starts;   // bit c: column c's plan is not column c - 1's
@@ -69,8 +70,8 @@ __device__ __forceinline__ Share share_columns(const DecodeParams &p, int cap, i
     s.starts = __ballot_sync(0xffffffffu, on && (c == 0 || units != b.units || unit != b.unit || before != b.runs));
     s.each = min(kCols, div_up(p.n_slots, side));
     s.run = in_head % runs;
-    s.group = in_head < side * runs ? in_head / runs + (int)blockIdx.y * side : p.n_slots;
-    s.hop = side * gridDim.y;
+    s.group = in_head < side * runs ? in_head / runs : p.n_slots;
+    s.hop = side;
     return s;
 }
 // Columns [base, end) of group s.group (none past the last); returns how many groups there are.
@@ -89,7 +90,7 @@ __device__ __forceinline__ int find_group(const Share &s, int cols, int &base, i
     return groups;
 }
 
-// grid (n_kv * runs * kC, ceil(columns / kCols)), clusters of kC as in the single-column form.
+// grid (n_kv * run_cap * kC), clusters of kC as in the single-column form.
 template <int kC>
 __global__ void __launch_bounds__(kThreads, 1) attn_decode_cols(DecodeParams p, int *status) {
     using C = Cfg;
@@ -112,7 +113,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_decode_cols(DecodeParams p, 
         mbar_init_fence();
     }
     if (warp == 0) tmem_alloc<1>(smem_u32(&s_tmem), kTmemCols);
-    const int cap = min(p.splits, p.run_cap), cluster = (int)blockIdx.x / kC;
+    const int cap = p.run_cap, cluster = (int)blockIdx.x / kC;
     const int kvh = cluster / cap, in_head = cluster - kvh * cap;
     // Nothing that the grids ahead may write can be relied on before they are done, but the lengths as they
     // stand are a good guess: enough to plan with and to ask L2 for the first rows. They are checked below.
@@ -457,7 +458,10 @@ __global__ void __launch_bounds__(kThreads, 1) attn_decode_cols(DecodeParams p, 
                 const int slice = (items / kC + 1) * w.runs * 16, fit = max(1, min(n, kWarps * C::kRing / slice));
                 for (int c = 0; c < n; c += fit) {
                     const int m = min(fit, n - c);
-                    if (fold_runs_staged<kC>(p, base + c, m, kvh, group, w.runs, rank, smem, kWarps * C::kRing, bar_fold,
+                    // (the staged fold takes the runs in one order; clusters of four and eight join shares of them, as
+                    // the single-column body does)
+                    if (Split<kC>::kShare == 1 &&
+                        fold_runs_staged<kC>(p, base + c, m, kvh, group, w.runs, rank, smem, kWarps * C::kRing, bar_fold,
                                              fold_phase, reinterpret_cast<float2(*)[kStagedRow]>(smem + C::kOffFold), landed))
                         fold_phase ^= 1;
                     else
@@ -484,7 +488,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_decode_cols(DecodeParams p, 
 }
 
 template <int kC>
-int launch(cudaStream_t stream, const DecodeParams &p) {
+int launch(cudaStream_t stream, DecodeParams p) {
     static std::mutex mu;
     static int *status_word[64] = {};   // nullptr: device not set up yet
     int dev = 0;
@@ -500,8 +504,19 @@ int launch(cudaStream_t stream, const DecodeParams &p) {
             if (status_word[dev] == nullptr) return launch_status();
         }
     }
-    return launch_pdl(attn_decode_cols<kC>, dim3(p.n_kv * min(p.splits, p.run_cap) * kC, (p.n_slots + kCols - 1) / kCols),
-                      dim3(kThreads), (size_t)Cfg::kSmem, stream, kC, p, status_word[dev]);
+    // (up to kMaxCols in a launch: 40 columns of 100 rows took 115 us as grids of the single-column body)
+    for (int left = p.n_slots; left > 0; left -= kMaxCols) {
+        p.n_slots = min(left, kMaxCols);
+        if (int e = launch_pdl(attn_decode_cols<kC>, dim3(p.n_kv * p.run_cap * kC), dim3(kThreads), (size_t)Cfg::kSmem, stream,
+                               kC, p, status_word[dev]))
+            return e;
+        p.len += kMaxCols * p.len_stride;
+        p.q += kMaxCols * p.q_slot;
+        p.part_acc += kMaxCols * p.acc_slot;
+        p.part_ml += kMaxCols * p.ml_slot;
+        if (p.out) p.out += kMaxCols * p.out_slot;
+    }
+    return 0;
 }
 
 }  // namespace

@@ -622,7 +622,7 @@ int launch(cudaStream_t stream, const DecodeParams &p, int slots) {
         }
     }
     // several columns over one cache: side by side (not with the tail of an exchange)
-    const bool columns = !kQ4 && kC > 1 && kWide && slots > 1 && slots <= 32 && q.kv_slot_bytes == 0 && q.k_row == nullptr &&
+    const bool columns = !kQ4 && kC > 1 && kWide && slots > 1 && q.kv_slot_bytes == 0 && q.k_row == nullptr &&
                          q.xch.phases == 0;
     const int rc = columns ? launch_decode_cols(stream, q, kC)
                            : launch_pdl(attn_decode_warps<kQ4, kC, kWide>, grid, dim3(kThreads),

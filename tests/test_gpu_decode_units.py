@@ -68,6 +68,37 @@ def test_partials_sent_within_a_cluster_for_any_group(group, seq):
     assert ok and ma <= 2e-5 and rl <= 2e-5, (ma, rl)
 
 
+@pytest.mark.parametrize("append", [False, True], ids=["rows", "rows and append"])
+@pytest.mark.parametrize("dtype", [0, 1], ids=["q8_0", "q4_0"])
+@pytest.mark.parametrize("seq,stride", [(1, 40), (700, 704), (700, 9000), (8999, 9000)])
+def test_one_slot_is_a_stream(seq, stride, dtype, append):
+    from hipml_b200 import api
+    heads, n_kv, hd, scale, row = 24, 4, 256, 0.0625, (272, 144)[dtype]
+    gen = torch.Generator(device="cuda").manual_seed(seq + dtype)
+    k, v = (torch.randn(seq, n_kv * hd, device="cuda", generator=gen) for _ in range(2))
+    q = torch.randn(heads * hd, device="cuda", generator=gen)
+    kc, vc = (torch.full((n_kv * stride * row,), 0x7E, dtype=torch.uint8, device="cuda") for _ in range(2))
+    api.kv_encode_bulk(k, v, kc, vc, n_kv, hd, stride, 0, 0, seq, dtype)
+    want_k, want_v = kc.clone(), vc.clone()
+    deq = (O.dequantize_q8, O.dequantize_q4)[dtype]
+    kq, vq = (torch.from_numpy(cases.unpack_head_major(deq(np.ascontiguousarray(
+        c.cpu().numpy().reshape(n_kv, stride, row)[:, :seq])), n_kv, seq, hd)).cuda() for c in (kc, vc))
+    splits = api.batch_splits(stride, 1)
+    acc, ml = (torch.full((heads * splits * n,), float("nan"), device="cuda") for n in (hd, 2))
+    out = torch.full((heads * hd,), float("nan"), device="cuda")
+    pos = torch.tensor([[seq - 1, seq]], dtype=torch.int32, device="cuda")
+    tail = (heads, n_kv, hd, stride, scale, splits, n_kv * stride * row, heads * splits * hd, heads * splits * 2, heads * hd, 1)
+    if append:
+        for c in (kc, vc):   # the row to append arrives with the step
+            c.view(n_kv, stride, row)[:, seq - 1] = 0x7E
+        api.attn_decode_batch_append(pos, k[seq - 1:], v[seq - 1:], q, kc, vc, acc, ml, out, *tail, dtype=dtype)
+    else:
+        api.attn_decode_rows(pos, q, kc, vc, acc, ml, out, *tail, dtype=dtype)
+    assert api.check_device_status() == 0
+    assert torch.equal(kc, want_k) and torch.equal(vc, want_v)
+    assert _close(out, _attend(q, kq, vq, n_kv, hd, scale))
+
+
 # more KV heads than the device holds clusters of eight for two launches, and a tensor-parallel rank's one
 @pytest.mark.parametrize("n_kv,group", [(8, 4), (7, 3), (6, 4), (1, 6)])
 @pytest.mark.parametrize("seq", [300, 600, 1000, 1300])
@@ -198,6 +229,38 @@ def test_columns_side_by_side_give_each_columns_own_bits(pos0, cols):
         out.fill_(float("nan"))
         api.attn_decode_cols(pos, q, kc, vc, acc, ml, out, heads, n_kv, hd, stride, scale, splits, cols,
                              heads * splits * hd, heads * splits * 2, heads * hd)
+    for c in range(cols):
+        one = torch.empty(heads * hd, device="cuda")
+        step = torch.tensor([pos0 + c, pos0 + c + 1] + [0] * 6, dtype=torch.int32, device="cuda")
+        api.attn_decode_kv(step, q[c], kc, vc, acc, ml, one, heads, n_kv, hd, stride, scale, splits)
+        assert torch.equal(one, out[c]), f"column {c}"
+    assert api.check_device_status() == 0
+
+
+# groups of columns in turn and side by side, columns of two launches, few splits over a long stream
+@pytest.mark.parametrize("fold_mode", [0, 1], ids=["fold_inside", "fold_launch"])
+@pytest.mark.parametrize("pos0,cols,splits", [(0, 3, 1), (10, 33, 5), (100, 16, 13), (700, 40, 90), (1278, 40, 128),
+                                              (3000, 3, 64), (5000, 9, 24), (5000, 12, 128)])
+def test_columns_of_every_form_give_each_columns_own_bits(pos0, cols, splits, fold_mode):
+    from hipml_b200 import api
+    heads, n_kv, hd, scale, stride = 24, 4, 256, 0.0625, pos0 + cols + 2
+    gen = torch.Generator(device="cuda").manual_seed(pos0 + cols)
+    kc, vc = (torch.full((n_kv * stride * 272,), 0x7E, dtype=torch.uint8, device="cuda") for _ in range(2))
+    k, v = (torch.randn(pos0 + cols, n_kv * hd, device="cuda", generator=gen) for _ in range(2))
+    api.kv_encode_bulk(k, v, kc, vc, n_kv, hd, stride, 0, 0, pos0 + cols)
+    q = torch.randn(cols, heads * hd, device="cuda", generator=gen)
+    acc, ml = (torch.empty(cols * heads * splits * n, device="cuda") for n in (hd, 2))
+    out = torch.empty(cols, heads * hd, device="cuda")
+    pos = torch.tensor([[pos0 + c, pos0 + c + 1] for c in range(cols)], dtype=torch.int32, device="cuda")
+    api.set_decode_fold_mode(fold_mode)
+    try:
+        for _ in range(2):
+            for x in (acc, ml, out):
+                x.fill_(float("nan"))
+            api.attn_decode_cols(pos, q, kc, vc, acc, ml, out, heads, n_kv, hd, stride, scale, splits, cols,
+                                 heads * splits * hd, heads * splits * 2, heads * hd)
+    finally:
+        api.set_decode_fold_mode(0)
     for c in range(cols):
         one = torch.empty(heads * hd, device="cuda")
         step = torch.tensor([pos0 + c, pos0 + c + 1] + [0] * 6, dtype=torch.int32, device="cuda")
