@@ -249,6 +249,82 @@ __global__ void __launch_bounds__(256) attn_chunk_stage(StageParams p) {
 
 // ------------------------------------------------------------------ main kernel
 
+// w times the layer's output gate, sigmoid(g).
+__device__ __forceinline__ void apply_gate(float4 &w, const float4 &g) {
+    w.x *= 1.0f / (1.0f + expf(-g.x));
+    w.y *= 1.0f / (1.0f + expf(-g.y));
+    w.z *= 1.0f / (1.0f + expf(-g.z));
+    w.w *= 1.0f / (1.0f + expf(-g.w));
+}
+
+// Rows [r_lo, r_hi) of a query tile, whose `nsp` <= kS key slices lie staged in the CTAs of the cluster (slice s in
+// CTA 2 s + rank: rows of kPitch floats at stage_addr, their {maximum, sum} at ml_addr): folded and written by eight
+// warps, a warp kMaxFold / kS rows at a time with all their loads in flight. (One at a time a row costs three trips,
+// to the other CTAs' pairs, to their rows and to the gate's row in memory: 16 us for the 63 rows of a CTA in two
+// slices, 301 tokens at 3,001, now 3.)
+template <int kS>
+__device__ __forceinline__ void fold_slices(const ChunkTcParams &p, unsigned stage_addr, unsigned ml_addr, int nsp, int rank,
+                                            int r_lo, int r_hi, int t0, int kvh, int warp, int lane) {
+    constexpr int kPitch = kD + 4, kR = kMaxFold / kS;
+    for (int r0 = r_lo + warp * kR; r0 < r_hi; r0 += 8 * kR) {
+        // lane kS * j + s holds slice s's pair of row r0 + j
+        const int mine = r0 + lane / kS;
+        float2 ml = make_float2(-INFINITY, 0.0f);
+        if (lane < kMaxFold && lane % kS < nsp && mine < r_hi)
+            ml = ld_cluster_f2(map_to_cta(ml_addr + 8 * mine, 2 * (lane % kS) + rank));
+        size_t row[kR];
+        float4 x[kR][kS][2], g[kR][2];
+#pragma unroll
+        for (int j = 0; j < kR; j++) {
+            const int r = min(r0 + j, r_hi - 1), rq = r / p.group;
+            row[j] = ((size_t)(t0 + rq) * p.n_heads + kvh * p.group + (r - rq * p.group)) * kD + 4 * lane;
+            if (p.gate) {
+                g[j][0] = *reinterpret_cast<const float4 *>(p.gate + row[j]);
+                g[j][1] = *reinterpret_cast<const float4 *>(p.gate + row[j] + 128);
+            }
+#pragma unroll
+            for (int s = 0; s < kS; s++)
+                if (s < nsp) {
+                    const unsigned src = map_to_cta(stage_addr + (r * kPitch + 4 * lane) * 4, 2 * s + rank);
+                    x[j][s][0] = ld_cluster_f4(src);
+                    x[j][s][1] = ld_cluster_f4(src + 512);
+                }
+        }
+        float big = ml.x;
+#pragma unroll
+        for (int o = kS / 2; o > 0; o /= 2) big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, o));
+        const float wt = ml.x == -INFINITY ? 0.0f : exp2f(ml.x - big);
+        float den = ml.y * wt;
+#pragma unroll
+        for (int o = kS / 2; o > 0; o /= 2) den += __shfl_xor_sync(0xffffffffu, den, o);
+        const float inv_of = den > 0.0f ? 1.0f / den : 0.0f;
+#pragma unroll
+        for (int j = 0; j < kR; j++) {
+            float4 y[2] = {make_float4(0.0f, 0.0f, 0.0f, 0.0f), make_float4(0.0f, 0.0f, 0.0f, 0.0f)};
+#pragma unroll
+            for (int s = 0; s < kS; s++)
+                if (s < nsp) {
+                    const float ws = __shfl_sync(0xffffffffu, wt, kS * j + s);
+#pragma unroll
+                    for (int c = 0; c < 2; c++) {
+                        y[c].x = fmaf(x[j][s][c].x, ws, y[c].x);
+                        y[c].y = fmaf(x[j][s][c].y, ws, y[c].y);
+                        y[c].z = fmaf(x[j][s][c].z, ws, y[c].z);
+                        y[c].w = fmaf(x[j][s][c].w, ws, y[c].w);
+                    }
+                }
+            const float inv = __shfl_sync(0xffffffffu, inv_of, kS * j);
+            if (r0 + j >= r_hi) continue;
+#pragma unroll
+            for (int c = 0; c < 2; c++) {
+                float4 w = make_float4(y[c].x * inv, y[c].y * inv, y[c].z * inv, y[c].w * inv);
+                if (p.gate) apply_gate(w, g[j][c]);
+                *reinterpret_cast<float4 *>(p.out + row[j] + 128 * c) = w;
+            }
+        }
+    }
+}
+
 // kCtas = 1: one CTA per query tile. kCtas = 2: launched as clusters of two along x; the
 // K maps then have 64-key boxes (a CTA loads its half of the keys of a tile).
 // kFold: the key slices of a tile (grid z) are one cluster, which folds them.
@@ -770,36 +846,47 @@ attn_chunk_tc(const __grid_constant__ CUtensorMap map_k_hi, const __grid_constan
                 bulk_store_commit_wait_read();
             }
         } else if (*abort_flag == 0) {
-            for (int rr = warp; rr < rows_live; rr += 8) {
-                const int q2 = rr / p.group, h2 = kvh * p.group + (rr - q2 * p.group);
-                const size_t row = norm ? ((size_t)(t0 + q2) * p.n_heads + h2)
-                                        : (((size_t)sp * p.qslots + (t0 + q2)) * p.n_heads + h2);
-                float *const drow = (norm ? p.out : p.part_acc) + row * kD;
-                const float *const grow = (norm && p.gate) ? p.gate + row * kD : nullptr;
-                const float cg = row_scale[2 * rr], inv = row_scale[2 * rr + 1];
+            // (four rows at a time: what they take from memory is on its way together)
+            constexpr int kR = 4;
+            for (int r0 = warp * kR; r0 < rows_live; r0 += 8 * kR) {
+                float *drow[kR];
+                float4 old[kR][2], g[kR][2];
+                float cg[kR];
 #pragma unroll
-                for (int c = 0; c < 2; c++) {
-                    const int col = 128 * c + 4 * lane;
-                    float4 w = *reinterpret_cast<const float4 *>(stage + rr * kPitch + col);
-                    if (cg >= 0.0f) {
-                        const float4 g = *reinterpret_cast<const float4 *>(drow + col);
-                        w.x = fmaf(g.x, cg, w.x);
-                        w.y = fmaf(g.y, cg, w.y);
-                        w.z = fmaf(g.z, cg, w.z);
-                        w.w = fmaf(g.w, cg, w.w);
+                for (int k = 0; k < kR; k++) {
+                    const int rr = min(r0 + k, rows_live - 1), q2 = rr / p.group, h2 = kvh * p.group + (rr - q2 * p.group);
+                    const size_t row = norm ? ((size_t)(t0 + q2) * p.n_heads + h2)
+                                            : (((size_t)sp * p.qslots + (t0 + q2)) * p.n_heads + h2);
+                    drow[k] = (norm ? p.out : p.part_acc) + row * kD + 4 * lane;
+                    cg[k] = row_scale[2 * rr];
+#pragma unroll
+                    for (int c = 0; c < 2; c++) {
+                        if (cg[k] >= 0.0f) old[k][c] = *reinterpret_cast<const float4 *>(drow[k] + 128 * c);
+                        if (norm && p.gate)
+                            g[k][c] = *reinterpret_cast<const float4 *>(p.gate + row * kD + 4 * lane + 128 * c);
                     }
-                    w.x *= inv;
-                    w.y *= inv;
-                    w.z *= inv;
-                    w.w *= inv;
-                    if (grow) {   // the layer's output gate, applied where the row is produced
-                        const float4 g = *reinterpret_cast<const float4 *>(grow + col);
-                        w.x *= 1.0f / (1.0f + expf(-g.x));
-                        w.y *= 1.0f / (1.0f + expf(-g.y));
-                        w.z *= 1.0f / (1.0f + expf(-g.z));
-                        w.w *= 1.0f / (1.0f + expf(-g.w));
+                }
+#pragma unroll
+                for (int k = 0; k < kR; k++) {
+                    const int rr = r0 + k;
+                    if (rr >= rows_live) break;
+                    const float inv = row_scale[2 * rr + 1];
+#pragma unroll
+                    for (int c = 0; c < 2; c++) {
+                        float4 w = *reinterpret_cast<const float4 *>(stage + rr * kPitch + 128 * c + 4 * lane);
+                        if (cg[k] >= 0.0f) {
+                            w.x = fmaf(old[k][c].x, cg[k], w.x);
+                            w.y = fmaf(old[k][c].y, cg[k], w.y);
+                            w.z = fmaf(old[k][c].z, cg[k], w.z);
+                            w.w = fmaf(old[k][c].w, cg[k], w.w);
+                        }
+                        w.x *= inv;
+                        w.y *= inv;
+                        w.z *= inv;
+                        w.w *= inv;
+                        if (norm && p.gate) apply_gate(w, g[k][c]);   // the layer's output gate, where the row is produced
+                        *reinterpret_cast<float4 *>(drow[k] + 128 * c) = w;
                     }
-                    *reinterpret_cast<float4 *>(drow + col) = w;
                 }
             }
         }
@@ -815,53 +902,14 @@ attn_chunk_tc(const __grid_constant__ CUtensorMap map_k_hi, const __grid_constan
         const int gave_up = lane < 2 * nsp ? ld_cluster_s32(map_to_cta(flag_addr, lane)) : 0;
         if (warp < 8 && !__any_sync(0xffffffffu, gave_up != 0)) {
             constexpr int kPitch = kD + 4;
-            const float *const stage = reinterpret_cast<const float *>(smem);
-            const unsigned stage_addr = smem_u32(stage), ml_addr = smem_u32(stage + 128 * kPitch);
+            const unsigned stage_addr = smem_u32(smem), ml_addr = stage_addr + 128 * kPitch * 4;
             const int r_lo = rows_live * sp / nsp, r_hi = rows_live * (sp + 1) / nsp;
-            for (int r = r_lo + warp; r < r_hi; r += 8) {
-                // lane s holds slice s's {maximum, sum}
-                float2 ml = make_float2(-INFINITY, 0.0f);
-                if (lane < nsp) ml = ld_cluster_f2(map_to_cta(ml_addr + 8 * r, 2 * lane + rank));
-                const float big = warp_max(ml.x);
-                const float wt = ml.x == -INFINITY ? 0.0f : exp2f(ml.x - big);
-                const float den = warp_sum(ml.y * wt), inv = den > 0.0f ? 1.0f / den : 0.0f;
-                float4 x[kMaxFold][2];
-#pragma unroll
-                for (int s = 0; s < kMaxFold; s++)
-                    if (s < nsp) {
-                        const unsigned src = map_to_cta(stage_addr + (r * kPitch + 4 * lane) * 4, 2 * s + rank);
-                        x[s][0] = ld_cluster_f4(src);
-                        x[s][1] = ld_cluster_f4(src + 512);
-                    }
-                float4 y[2] = {make_float4(0.0f, 0.0f, 0.0f, 0.0f), make_float4(0.0f, 0.0f, 0.0f, 0.0f)};
-#pragma unroll
-                for (int s = 0; s < kMaxFold; s++)
-                    if (s < nsp) {
-                        const float ws = __shfl_sync(0xffffffffu, wt, s);
-#pragma unroll
-                        for (int c = 0; c < 2; c++) {
-                            y[c].x = fmaf(x[s][c].x, ws, y[c].x);
-                            y[c].y = fmaf(x[s][c].y, ws, y[c].y);
-                            y[c].z = fmaf(x[s][c].z, ws, y[c].z);
-                            y[c].w = fmaf(x[s][c].w, ws, y[c].w);
-                        }
-                    }
-                const int rq = r / p.group;
-                const size_t row = (size_t)(t0 + rq) * p.n_heads + kvh * p.group + (r - rq * p.group);
-#pragma unroll
-                for (int c = 0; c < 2; c++) {
-                    const int col = 128 * c + 4 * lane;
-                    float4 w = make_float4(y[c].x * inv, y[c].y * inv, y[c].z * inv, y[c].w * inv);
-                    if (p.gate) {
-                        const float4 g = *reinterpret_cast<const float4 *>(p.gate + row * kD + col);
-                        w.x *= 1.0f / (1.0f + expf(-g.x));
-                        w.y *= 1.0f / (1.0f + expf(-g.y));
-                        w.z *= 1.0f / (1.0f + expf(-g.z));
-                        w.w *= 1.0f / (1.0f + expf(-g.w));
-                    }
-                    *reinterpret_cast<float4 *>(p.out + row * kD + col) = w;
-                }
-            }
+            if (nsp == 2)
+                fold_slices<2>(p, stage_addr, ml_addr, nsp, rank, r_lo, r_hi, t0, kvh, warp, lane);
+            else if (nsp <= 4)
+                fold_slices<4>(p, stage_addr, ml_addr, nsp, rank, r_lo, r_hi, t0, kvh, warp, lane);
+            else
+                fold_slices<8>(p, stage_addr, ml_addr, nsp, rank, r_lo, r_hi, t0, kvh, warp, lane);
         }
     }
 
