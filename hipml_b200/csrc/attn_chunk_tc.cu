@@ -403,9 +403,86 @@ attn_chunk_tc(const __grid_constant__ CUtensorMap map_k_hi, const __grid_constan
         tmem_alloc<kCtas>(smem_u32(tmem_slot), 512);  // in the pair form: warp 0 of both CTAs
     }
 
+    // Ahead of the grid dependency nothing is read, but L2 can be asked for what is wanted first: the query
+    // tile and the gate rows (a query's heads of the group are one run), and the tensor maps.
+    if (tid < nq) {
+        const size_t at = ((size_t)(t0 + tid) * p.n_heads + kvh * p.group) * kD;
+        prefetch_l2(p.q + at, (unsigned)(p.group * kD * 4));
+        if (p.gate) prefetch_l2(p.gate + at, (unsigned)(p.group * kD * 4));
+    }
+    if (warp == 8 && lane == 0) {
+        prefetch_map(&map_k_hi);
+        prefetch_map(&map_k_lo);
+        prefetch_map(&map_vt_hi);
+        prefetch_map(&map_vt_lo);
+    }
+    if constexpr (kCtas == 2) cluster_arrive();
+    constexpr int kHalf = kStageBytes / 2;   // low plane of a ring slot
+    // TMA producer (warp 8, lane 0): ring slots issued, and whether every wait came through.
+    unsigned n = 0;
+    bool ok = true;
+    // Takes the next ring slot once the MMAs that read it have completed and arms its
+    // full barrier; in a pair only the leader arms, with both CTAs' bytes (the peer's
+    // copies complete on the leader's barrier).
+    auto acquire = [&](unsigned &dst, unsigned &full) {
+        const unsigned stage = n % kStages, phase = (n / kStages) & 1;
+        ok = ok && mbar_wait(bar_empty + 8 * stage, phase ^ 1, abort_flag, peer_abort, p.status, 1);
+        if (!ok) return;
+        dst = smem_u32(ring + stage * kStageBytes);
+        full = lead_full + 8 * stage;
+        if (rank == 0)
+            mbar_arrive_expect_tx(bar_full + 8 * stage,
+                                  kCtas * (p.single_pass ? kStageBytes / 2 : kStageBytes));
+        n++;
+    };
+    auto load_k = [&](int kt) {
+        unsigned dst = 0, full = 0;
+        if constexpr (kCtas == 1) {
+            // slot = 128 keys x 64 dims (hi, lo)
+            for (int c = 0; c < 4 && ok; c++) {
+                acquire(dst, full);
+                if (!ok) return;
+                const int y = kvh * p.lpad + kt * kKeyTile;
+                tma_load_2d<1>(dst, &map_k_hi, c * 64, y, full);
+                if (!p.single_pass) tma_load_2d<1>(dst + kHalf, &map_k_lo, c * 64, y, full);
+            }
+        } else {
+            // slot = this CTA's 64 keys x two 64-dim chunks (hi c, hi c+1, lo c, lo c+1)
+            for (int cp = 0; cp < 2 && ok; cp++) {
+                acquire(dst, full);
+                if (!ok) return;
+                const int y = kvh * p.lpad + kt * kKeyTile + 64 * (int)rank;
+                for (int cc = 0; cc < 2; cc++) {
+                    const int x = (2 * cp + cc) * 64;
+                    tma_load_2d<2>(dst + cc * (kHalf / 2), &map_k_hi, x, y, full);
+                    if (!p.single_pass)
+                        tma_load_2d<2>(dst + kHalf + cc * (kHalf / 2), &map_k_lo, x, y, full);
+                }
+            }
+        }
+    };
+    auto load_v = [&](int kt) {
+        unsigned dst = 0, full = 0;
+        // slot = 128 dims x 64 keys (hi, lo); a pair CTA loads only its half of the dims
+        for (int kc = 0; kc < 2 && ok; kc++)
+            for (int dh = 0; dh < (kCtas == 1 ? 2 : 1) && ok; dh++) {
+                acquire(dst, full);
+                if (!ok) return;
+                const int x = kt * kKeyTile + kc * 64;
+                const int y = kvh * kD + (kCtas == 1 ? dh : (int)rank) * 128;
+                tma_load_2d<kCtas>(dst, &map_vt_hi, x, y, full);
+                if (!p.single_pass) tma_load_2d<kCtas>(dst + kHalf, &map_vt_lo, x, y, full);
+            }
+    };
     // The query rows may come from a grid that is still running (a dependent launch can start
     // while the grid before its predecessor has not finished): nothing is read before this.
     griddep_wait();
+    if constexpr (kCtas == 2) {
+        // The first key tile is on its way while the query tile is converted (the barriers of both CTAs are there).
+        cluster_wait();
+        if (warp == 8 && lane == 0 && n_tiles > 0) load_k(kt_lo);
+        __syncwarp();
+    }
     // Q tile: f32 -> scaled hi/lo f16 in the swizzled K-major image. Row r = query r/group,
     // head r%group; rows past the live queries are zero. An item is 8 dims of a row; a thread's
     // items are taken in batches whose loads are all issued before the first is converted (one
@@ -452,8 +529,7 @@ attn_chunk_tc(const __grid_constant__ CUtensorMap map_k_hi, const __grid_constan
     // Make the generic-proxy writes of Q visible to the tensor-core (async) proxy.
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     tc_fence_before();
-    // Barriers initialised, Q written, TMEM allocated: in every CTA of the pair before any
-    // of them signals the other or the leader's MMAs read the peer's shared memory.
+    // Q written, TMEM allocated: in every CTA of the pair before the leader's MMAs read the peer's shared memory.
     if constexpr (kCtas == 2) cluster_sync_all(); else __syncthreads();
     tc_fence_after();
     const unsigned tmem = *tmem_slot;
@@ -462,69 +538,11 @@ attn_chunk_tc(const __grid_constant__ CUtensorMap map_k_hi, const __grid_constan
     const int terms = p.single_pass ? 1 : 3;
     constexpr unsigned kIdescS = idesc_f16(128 * kCtas, 128);         // S = Q K^T
     constexpr unsigned kIdescO = idesc_f16(128 * kCtas, 128 * kCtas); // O += P V (per MMA)
-    constexpr int kHalf = kStageBytes / 2;   // low plane of a ring slot
 
     if (warp == 8) {
         // ---------------------------------------------------------------- TMA producer
         if (lane == 0 && n_tiles > 0) {
-            unsigned n = 0;  // chunks issued
-            bool ok = true;
-            // (the staged image, the scratch and the output rows belong to the previous grids:
-            // every thread waited for them before the query tile was read)
-            // Takes the next ring slot once the MMAs that read it have completed and arms its
-            // full barrier; in a pair only the leader arms, with both CTAs' bytes (the peer's
-            // copies complete on the leader's barrier).
-            auto acquire = [&](unsigned &dst, unsigned &full) {
-                const unsigned stage = n % kStages, phase = (n / kStages) & 1;
-                ok = ok && mbar_wait(bar_empty + 8 * stage, phase ^ 1, abort_flag, peer_abort, p.status, 1);
-                if (!ok) return;
-                dst = smem_u32(ring + stage * kStageBytes);
-                full = lead_full + 8 * stage;
-                if (rank == 0)
-                    mbar_arrive_expect_tx(bar_full + 8 * stage,
-                                          kCtas * (p.single_pass ? kStageBytes / 2 : kStageBytes));
-                n++;
-            };
-            auto load_k = [&](int kt) {
-                unsigned dst = 0, full = 0;
-                if constexpr (kCtas == 1) {
-                    // slot = 128 keys x 64 dims (hi, lo)
-                    for (int c = 0; c < 4 && ok; c++) {
-                        acquire(dst, full);
-                        if (!ok) return;
-                        const int y = kvh * p.lpad + kt * kKeyTile;
-                        tma_load_2d<1>(dst, &map_k_hi, c * 64, y, full);
-                        if (!p.single_pass) tma_load_2d<1>(dst + kHalf, &map_k_lo, c * 64, y, full);
-                    }
-                } else {
-                    // slot = this CTA's 64 keys x two 64-dim chunks (hi c, hi c+1, lo c, lo c+1)
-                    for (int cp = 0; cp < 2 && ok; cp++) {
-                        acquire(dst, full);
-                        if (!ok) return;
-                        const int y = kvh * p.lpad + kt * kKeyTile + 64 * (int)rank;
-                        for (int cc = 0; cc < 2; cc++) {
-                            const int x = (2 * cp + cc) * 64;
-                            tma_load_2d<2>(dst + cc * (kHalf / 2), &map_k_hi, x, y, full);
-                            if (!p.single_pass)
-                                tma_load_2d<2>(dst + kHalf + cc * (kHalf / 2), &map_k_lo, x, y, full);
-                        }
-                    }
-                }
-            };
-            auto load_v = [&](int kt) {
-                unsigned dst = 0, full = 0;
-                // slot = 128 dims x 64 keys (hi, lo); a pair CTA loads only its half of the dims
-                for (int kc = 0; kc < 2 && ok; kc++)
-                    for (int dh = 0; dh < (kCtas == 1 ? 2 : 1) && ok; dh++) {
-                        acquire(dst, full);
-                        if (!ok) return;
-                        const int x = kt * kKeyTile + kc * 64;
-                        const int y = kvh * kD + (kCtas == 1 ? dh : (int)rank) * 128;
-                        tma_load_2d<kCtas>(dst, &map_vt_hi, x, y, full);
-                        if (!p.single_pass) tma_load_2d<kCtas>(dst + kHalf, &map_vt_lo, x, y, full);
-                    }
-            };
-            load_k(kt_lo);
+            if constexpr (kCtas == 1) load_k(kt_lo);
             for (int kt = kt_lo; kt < kt_hi && ok; kt++) {
                 if (kt + 1 < kt_hi) load_k(kt + 1);
                 load_v(kt);

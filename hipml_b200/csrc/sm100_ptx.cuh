@@ -159,6 +159,11 @@ __device__ __forceinline__ void tma_load_2d(unsigned dst, const CUtensorMap *map
     }
 }
 
+// Asks for a tensor map (a kernel parameter) ahead of its first use.
+__device__ __forceinline__ void prefetch_map(const CUtensorMap *map) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
+}
+
 template <int kCtas>
 __device__ __forceinline__ void tmem_alloc(unsigned smem_dst, unsigned cols) {
     if constexpr (kCtas == 1) {
