@@ -212,15 +212,14 @@ __global__ void __launch_bounds__(kThreads, kWide ? 1 : 2) attn_decode_warps(Dec
                 prefetch_l2(vp + (size_t)i * step, bytes);
             }
         // and for the small inputs, whose trip to memory is on the path of every launch that finds them cold: the query
-        // rows of the group, the row to append, the gate
-        if (warp == 0 && w.slot >= 0) {
-            ask_l2(p.q + (size_t)w.slot * p.q_slot + (size_t)w.kvh * group * 256, 1024LL * group);
-            if (p.k_row != nullptr && w.row1 == w.len) {
-                const size_t at = (size_t)w.slot * p.row_slot + (size_t)w.kvh * 256;
-                ask_l2(p.k_row + at, 1024);
-                ask_l2(p.v_row + at, 1024);
-            }
-            if (p.gate != nullptr && w.run == 0)
+        // rows of the group, the row to append, the gate (a warp each)
+        if (w.slot >= 0) {
+            const size_t row = (size_t)w.slot * p.row_slot + (size_t)w.kvh * 256;
+            const bool appends = p.k_row != nullptr && w.row1 == w.len;
+            if (warp == 1) ask_l2(p.q + (size_t)w.slot * p.q_slot + (size_t)w.kvh * group * 256, 1024LL * group);
+            if (warp == 2 && appends) ask_l2(p.k_row + row, 1024);
+            if (warp == 3 && appends) ask_l2(p.v_row + row, 1024);
+            if (warp == 4 && p.gate != nullptr && w.run == 0)
                 ask_l2(p.gate + (size_t)w.slot * p.out_slot + (size_t)w.kvh * group * p.out_head_stride, 1024LL * group);
         }
     }
@@ -271,29 +270,32 @@ __global__ void __launch_bounds__(kThreads, kWide ? 1 : 2) attn_decode_warps(Dec
     // kNeutralSlots of the others that the caller has. The runs without rows write them, which have nothing else to do
     // (written by the live ones ahead of their first unit they were 1.2 of the 7.4 us of a layer of 672 rows, whose one
     // run has 31 empty slots beside it); the live ones only where there are no others.
-    auto neutral = [&](int run) {
-        const int at = rank * kThreads + tid;
-        if (p.out != nullptr) {
-            for (int i = at; i < items; i += kC * kThreads)
-                reinterpret_cast<float4 *>(part_acc + ((size_t)(i >> 6) * p.splits + run) * 256)[i & 63] =
-                    make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        } else {   // (scratch on any 4-byte boundary)
-            for (int i = at; i < group * 256; i += kC * kThreads)
-                part_acc[((size_t)(i >> 8) * p.splits + run) * 256 + (i & 255)] = 0.0f;
+    // (a wide CTA alone shares the device with other slots, and has no such runs)
+    if constexpr (kC > 1 || !kWide) {
+        auto neutral = [&](int run) {
+            const int at = rank * kThreads + tid;
+            if (p.out != nullptr) {
+                for (int i = at; i < items; i += kC * kThreads)
+                    reinterpret_cast<float4 *>(part_acc + ((size_t)(i >> 6) * p.splits + run) * 256)[i & 63] =
+                        make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            } else {   // (scratch on any 4-byte boundary)
+                for (int i = at; i < group * 256; i += kC * kThreads)
+                    part_acc[((size_t)(i >> 8) * p.splits + run) * 256 + (i & 255)] = 0.0f;
+            }
+            if (rank == 0 && tid < group) {
+                float *const ml = part_ml + ((size_t)tid * p.splits + run) * 2;
+                ml[0] = -INFINITY;
+                ml[1] = 0.0f;
+            }
+        };
+        if (p.share_slots == 0 && !p.by_stride && p.run_cap > 0) {
+            const int launched = min(p.splits, p.run_cap), idle = launched - w.runs;
+            const int from = idle > 0 ? w.run : launched + w.run, hop = idle > 0 ? idle : launched;
+            if (idle <= 0 || w.run >= w.runs)
+                for (int r = from; r < max(launched, min(p.splits, kNeutralSlots)); r += hop) neutral(r);
         }
-        if (rank == 0 && tid < group) {
-            float *const ml = part_ml + ((size_t)tid * p.splits + run) * 2;
-            ml[0] = -INFINITY;
-            ml[1] = 0.0f;
-        }
-    };
-    if (!p.by_stride && p.run_cap > 0 && p.share_slots == 0) {
-        const int launched = min(p.splits, p.run_cap), idle = launched - w.runs;
-        const int from = idle > 0 ? w.run : launched + w.run, hop = idle > 0 ? idle : launched;
-        if (idle <= 0 || w.run >= w.runs)
-            for (int r = from; r < max(launched, min(p.splits, kNeutralSlots)); r += hop) neutral(r);
+        if (w.run >= w.runs) return;
     }
-    if (w.run >= w.runs) return;
 
     // Fused append: the warp whose last unit holds the new row quantises it (with the encoder's own
     // arithmetic) while its first unit is on the way, stores it to the cache and keeps its bytes for the
