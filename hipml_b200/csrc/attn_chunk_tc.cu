@@ -216,9 +216,19 @@ __device__ __forceinline__ void stage_store8(__half *hi, __half *lo, size_t at, 
 __global__ void __launch_bounds__(256) attn_chunk_stage(StageParams p) {
     __shared__ float vs[64][129];
     griddep_launch();
-    griddep_wait();
     const int kvh = blockIdx.y, key0 = (p.tile0 + blockIdx.x) * 64;
     const int tid = threadIdx.x;
+    if (blockIdx.z < 2 && tid < 64 && key0 + tid < p.n_keys) {   // (the second half of V asks for the same rows)
+        const unsigned char *const cache = (const unsigned char *)(blockIdx.z == 0 ? p.k : p.v);
+        const int key = key0 + tid;
+        if (p.kv_dtype == 0)
+            ask_l2(cache + ((size_t)key * p.n_kv + kvh) * (kD * 4), kD * 4);
+        else if (p.kv_dtype == 1)
+            ask_l2(cache + q8_row_offset(kvh, p.stride, key, kD), 8 * kQ8BlockBytes);
+        else
+            ask_l2(cache + q4_row_offset(kvh, p.stride, key, kD), 8 * kQ4BlockBytes);
+    }
+    griddep_wait();
     if (blockIdx.z == 0) {
         // K: row-major copy. Thread -> dims [8*(tid%32), +8) of keys tid/32 + 8*i.
 #pragma unroll 4
@@ -266,18 +276,18 @@ __device__ __forceinline__ void apply_gate(float4 &w, const float4 &g) {
 
 // Rows [r_lo, r_hi) of a query tile, whose `nsp` <= kS key slices lie staged in the CTAs of the cluster (slice s in
 // CTA 2 s + rank: rows of kPitch floats at stage_addr, their {maximum, sum} at ml_addr): folded and written by eight
-// warps, a warp kMaxFold / kS rows at a time with all their loads in flight. (One at a time a row costs three trips,
+// warps, a warp two to four rows at a time with all their loads in flight. (One at a time a row costs three trips,
 // to the other CTAs' pairs, to their rows and to the gate's row in memory: 16 us for the 63 rows of a CTA in two
 // slices, 301 tokens at 3,001, now 3.)
 template <int kS>
 __device__ __forceinline__ void fold_slices(const ChunkTcParams &p, unsigned stage_addr, unsigned ml_addr, int nsp, int rank,
                                             int r_lo, int r_hi, int t0, int kvh, int warp, int lane) {
-    constexpr int kPitch = kD + 4, kR = kMaxFold / kS;
+    constexpr int kPitch = kD + 4, kR = kS == 8 ? 2 : kMaxFold / kS;
     for (int r0 = r_lo + warp * kR; r0 < r_hi; r0 += 8 * kR) {
         // lane kS * j + s holds slice s's pair of row r0 + j
         const int mine = r0 + lane / kS;
         float2 ml = make_float2(-INFINITY, 0.0f);
-        if (lane < kMaxFold && lane % kS < nsp && mine < r_hi)
+        if (lane < kS * kR && lane % kS < nsp && mine < r_hi)
             ml = ld_cluster_f2(map_to_cta(ml_addr + 8 * mine, 2 * (lane % kS) + rank));
         size_t row[kR];
         float4 x[kR][kS][2], g[kR][2];

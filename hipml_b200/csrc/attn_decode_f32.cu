@@ -74,6 +74,7 @@ __global__ void __launch_bounds__(kThreads, 2) attn_decode_rows_f32(ColsParams p
     // (asks L2 only; the rows are read once the grids ahead are done)
     for (int i = lane; i < 2 * (hi - lo); i += 32)
         prefetch_l2(((i & 1) ? vb : kb) + (size_t)(lo + (i >> 1)) * width, 1024);
+    if (tid == 0) ask_l2(p.q + ((size_t)col * p.n_heads + kvh * group) * 256, 1024LL * group);
     griddep_wait();
     cluster_wait();
     for (int i = tid; i < 8 * 64; i += kThreads) {
@@ -210,11 +211,14 @@ extern "C" __global__ void kv_append_cols_f32(float *__restrict__ k_cache,
                                               const float *__restrict__ v, int pos0, int rows,
                                               int width) {
     griddep_launch();
-    griddep_wait();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= 2LL * width * rows) return;
     const int c = (int)(i / (2 * width));
     const int j = (int)(i - (long long)c * 2 * width);
+    if ((threadIdx.x & 31) == 0)   // a warp's 32 floats, as far as they are of the same row
+        ask_l2(j < width ? k + (size_t)c * width + j : v + (size_t)c * width + j - width,
+               4LL * min(32, j < width ? width - j : 2 * width - j));
+    griddep_wait();
     const size_t base = (size_t)(pos0 + c) * width;
     if (j < width)
         k_cache[base + j] = k[(size_t)c * width + j];

@@ -267,9 +267,18 @@ __global__ void __launch_bounds__(256, kPerSm) attn_front_rows_q8(const __grid_c
     int p4[4] = {p.pos0 + t, p.pos0 + t, p.pos0 + t, p.pos0 + t};
     if (p.pos4)
         for (int i = 0; i < 4; i++) p4[i] = __ldcg(p.pos4 + i);
+    const int rows = p.n_heads + 2 * p.n_kv, hop = 8 * gridDim.y;
+    if (lane == 0) {   // the warp's first row, and the weights
+        const int r = blockIdx.y * 8 + warp;
+        if (r < p.n_heads)
+            ask_l2(p.qg + ((size_t)t * p.n_heads + r) * 512, 2048);
+        else if (r < rows)
+            ask_l2(r < p.n_heads + p.n_kv ? p.k + ((size_t)t * p.n_kv + r - p.n_heads) * 256
+                                          : p.v + ((size_t)t * p.n_kv + r - p.n_heads - p.n_kv) * 256, 1024);
+        if (t == 0 && warp < 2) ask_l2(warp ? p.k_norm : p.q_norm, 1024);
+    }
     angles(p4);
     griddep_wait();   // positions and rows may come from a grid that is still running
-    const int rows = p.n_heads + 2 * p.n_kv, hop = 8 * gridDim.y;
     float x[8], g[8];   // the row at hand (and the gate half of a query row)
     auto load_row = [&](int r) {
         if (r < p.n_heads) {

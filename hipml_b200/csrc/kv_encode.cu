@@ -114,13 +114,14 @@ __global__ void __launch_bounds__(256) kv_encode_bulk_q8_w(const float *__restri
                                                            int src0) {
     __shared__ __align__(16) unsigned char img[8][2][kMaxRowBytes];
     griddep_launch();
-    griddep_wait();   // the f32 rows may come from a grid that is still running
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const long long idx = (long long)blockIdx.x * 8 + warp;
     if (idx >= (long long)n_kv * rows) return;
     const int r = (int)(idx / n_kv);
     const int h = (int)(idx - (long long)r * n_kv);
     const size_t src = ((size_t)(src0 + r) * n_kv + h) * 256 + (size_t)lane * 8;
+    if (lane < 2) ask_l2((lane ? v : k) + (src - (size_t)lane * 8), 1024);
+    griddep_wait();   // the f32 rows may come from a grid that is still running
     const float4 ka = __ldg(reinterpret_cast<const float4 *>(k + src));
     const float4 kb = __ldg(reinterpret_cast<const float4 *>(k + src) + 1);
     const float4 va = __ldg(reinterpret_cast<const float4 *>(v + src));
@@ -220,13 +221,14 @@ __global__ void __launch_bounds__(256) kv_encode_bulk_q4_w(const float *__restri
                                                            int src0) {
     __shared__ __align__(16) unsigned char img[8][2][8 * kQ4BlockBytes];
     griddep_launch();
-    griddep_wait();   // the f32 rows may come from a grid that is still running
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const long long idx = (long long)blockIdx.x * 8 + warp;
     if (idx >= (long long)n_kv * rows) return;
     const int r = (int)(idx / n_kv);
     const int h = (int)(idx - (long long)r * n_kv);
     const size_t src = ((size_t)(src0 + r) * n_kv + h) * 256 + (size_t)lane * 8;
+    if (lane < 2) ask_l2((lane ? v : k) + (src - (size_t)lane * 8), 1024);
+    griddep_wait();   // the f32 rows may come from a grid that is still running
     const float4 ka = __ldg(reinterpret_cast<const float4 *>(k + src));
     const float4 kb = __ldg(reinterpret_cast<const float4 *>(k + src) + 1);
     const float4 va = __ldg(reinterpret_cast<const float4 *>(v + src));
@@ -272,8 +274,12 @@ extern "C" __global__ void kv_append_chunk_f32(float *__restrict__ k_cache,
                                                const float *__restrict__ v, int pos0, int width,
                                                int tokens) {
     griddep_launch();
-    griddep_wait();
     const size_t n = (size_t)tokens * (size_t)width;
+    if (threadIdx.x < 2) {   // the block's first pieces, four floats a thread
+        const size_t at = (size_t)blockIdx.x * blockDim.x * 4;
+        if (at < n) ask_l2((threadIdx.x ? v : k) + at, (long long)min(n - at, (size_t)blockDim.x * 4) * 4);
+    }
+    griddep_wait();
     const size_t base = (size_t)pos0 * (size_t)width;
     const size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     const size_t nthreads = (size_t)gridDim.x * blockDim.x;
