@@ -2,13 +2,19 @@
 // the body of attn_decode_warps.cu with the columns side by side. CPU definition per column:
 // crates/hipml-core/src/ops.rs:449-518; launcher replaced: launch_kv::launch_cols_ptrs.
 //
-// The columns see the same rows but for the last few, so a warp loads and converts a unit's codes once
-// and runs every column's MMAs on them: of the ~635 warp instructions that 16 rows cost a column, ~430
-// are the codes' and only ~205 the column's own. What does not fit is the accumulators (64 a lane and
-// column): they live in tensor memory, 128 of its columns per decode column, and come to the registers
-// 16 at a time for the pair of blocks at hand (tcgen05.ld / st, 2 x 64 words a lane per unit).
-// One launch per layer takes up to four columns in the time of about two; 4 columns of 8,192 rows took
-// 36 us a layer as four grids of the single-column body.
+// The columns see the same rows but for the last few, so a warp loads and converts a unit's codes once and runs the
+// MMAs of all of them on it. The heads of a group of columns are packed into tiles of eight, the MMA's eight result
+// columns, up to four tiles: four columns of six heads take three (a column each took four: 512 of the tensor pipe's
+// eight-cycle MMAs a unit, 8.6 us of scores, softmax and values for 8,192 rows), and five share a launch's CTAs. What
+// does not fit the registers is the accumulators (64 a lane and tile): they live in tensor memory, 128 of its columns
+// per tile, and come to the registers 16 at a time for the pair of blocks at hand (tcgen05.ld / st), so that the loops
+// over these pairs can be loops: unrolled four times, as the single-column body with its accumulators in registers has
+// them, their code came from beyond the SM's instruction cache in every launch (4 columns of 8,192 rows, with their
+// append: 27.9 us a layer, rolled 24.6; of 32,768: 53.0 and 50.9).
+//
+// The cluster's and the runs' partials meet column after column, each run beginning with another column: so the CTAs
+// that arrive last, and fold the runs of a column, are different ones. (One CTA with all four columns of 17 runs, 209 KB,
+// took 8.4 us at the end of every launch.)
 //
 // Each column's arithmetic is that of its own launch, operation for operation -- the plan, the order of
 // every sum, the movements of the references -- so its result is the same bits.
@@ -22,32 +28,34 @@ namespace {
 
 using namespace warp_body;
 
-constexpr int kCols = 4;          // columns side by side
+constexpr int kTiles = 4;         // of eight heads, of the columns side by side
+constexpr int kCols = 8;          // most columns side by side (of four heads or fewer)
 constexpr int kUnitRows = 32;
 constexpr unsigned kTmemCols = 512;
 constexpr int kMaxCols = 32;      // of a launch
+constexpr int kArriveBar = 1;     // named barriers of the columns' arrivals
 
 struct Cfg {
     static constexpr int kSlot = kUnitRows * kRowBytes;
     static constexpr int kRing = 2 * kSlot;                        // per warp: a unit of K and one of V; later two partials
     static constexpr int kPartial = 8 * kHeadPitch * 4;
     static_assert(kRing >= 2 * kPartial, "a warp's partials fit its ring");
-    static constexpr int kQBytes = 16 * 32 * 16;                   // a column's query fragments, later its partial of the CTA
+    static constexpr int kQBytes = 16 * 32 * 16;                   // a tile's query fragments, later its partial of the CTA
+    static_assert(kQBytes == 8 * 1024, "eight heads of a partial");
     static constexpr int kBiasBytes = 8 * 4 * 16;
     static constexpr int kOffQ = kWarps * kRing;
-    static constexpr int kOffBias = kOffQ + kCols * kQBytes;
-    static constexpr int kOffMl = kOffBias + kCols * kBiasBytes;   // two columns' [8 heads][warps] {reference, sum}
-    static constexpr int kOffCml = kOffMl + 2 * kWarps * 8 * 8;    // per column [8 heads]
-    static constexpr int kOffBar = kOffCml + kCols * 8 * 8;
-    static constexpr int kOffFold = kOffBar + kWarps * 2 * 8 + 8;  // weights of the last fold, after its barrier
-    static constexpr int kSmem = kOffFold + kCols * 5 * kStagedRow * 8;
+    static constexpr int kOffBias = kOffQ + kTiles * kQBytes;
+    static constexpr int kOffMl = kOffBias + kTiles * kBiasBytes;  // [heads][warps] {reference, sum}
+    static constexpr int kOffCml = kOffMl + kTiles * kWarps * 8 * 8;   // the CTA's, per head
+    static constexpr int kOffBar = kOffCml + kTiles * 8 * 8;
+    static constexpr int kSmem = kOffBar + kWarps * 2 * 8;
     static_assert(kSmem + 1024 <= 227 * 1024, "one CTA per SM");
 };
 
 __device__ int g_arrive_cols[kArriveRegions * kArriveRegionInts];
 
 // Which columns a cluster takes. Neighbouring columns with the same plan (the same units for every warp), at
-// most `each` of them, are a group; a cluster has run `run` of groups `group`, `group` + `hop`, ... Groups go
+// most `each` of them (as many as fit the tiles, in groups of one size), are a group; a cluster has run `run` of groups `group`, `group` + `hop`, ... Groups go
 // to clusters of their own while a head has clusters to spare for their runs, and columns share conversions
 // beyond (4 columns of 300 rows take 2 runs each: 8 clusters of the head's 18; of 8,192 rows 17: one cluster
 // per run takes all four). `cap`: the clusters of a head; what its groups do not need ends at once, so there is one
@@ -57,7 +65,7 @@ struct Share {
     unsigned starts;   // bit c: column c's plan is not column c - 1's
 };
 template <int kC>
-__device__ __forceinline__ Share share_columns(const DecodeParams &p, int cap, int in_head, const int *len) {
+__device__ __forceinline__ Share share_columns(const DecodeParams &p, int cap, int in_head, int group, const int *len) {
     const int c = threadIdx.x & 31;
     const bool on = c < p.n_slots;
     Balance b = {0, 0, 1};
@@ -68,7 +76,8 @@ __device__ __forceinline__ Share share_columns(const DecodeParams &p, int cap, i
     const int side = cap / runs;   // groups side by side, >= 1
     Share s;
     s.starts = __ballot_sync(0xffffffffu, on && (c == 0 || units != b.units || unit != b.unit || before != b.runs));
-    s.each = min(kCols, div_up(p.n_slots, side));
+    const int most = min(kCols, 8 * kTiles / group);
+    s.each = div_up(p.n_slots, max(side, div_up(p.n_slots, most)));
     s.run = in_head % runs;
     s.group = in_head < side * runs ? in_head / runs : p.n_slots;
     s.hop = side;
@@ -95,7 +104,7 @@ template <int kC>
 __global__ void __launch_bounds__(kThreads, 1) attn_decode_cols(DecodeParams p, int *status) {
     using C = Cfg;
     extern __shared__ __align__(128) unsigned char smem[];
-    __shared__ int s_last;
+    __shared__ int s_last[kCols];
     __shared__ unsigned s_tmem;
     __shared__ int s_len[kMaxCols];
     griddep_launch();
@@ -105,11 +114,9 @@ __global__ void __launch_bounds__(kThreads, 1) attn_decode_cols(DecodeParams p, 
     const int rank = (int)cluster_rank();
     unsigned char *const ring = smem + warp * C::kRing;
     const unsigned ring_addr = smem_u32(ring), bar = smem_u32(smem + C::kOffBar) + warp * 16;
-    const unsigned bar_fold = smem_u32(smem + C::kOffFold) - 8;
     if (lane == 0) {
         mbar_init(bar, 1);
         mbar_init(bar + 8, 1);
-        if (warp == 0) mbar_init(bar_fold, 1);
         mbar_init_fence();
     }
     if (warp == 0) tmem_alloc<1>(smem_u32(&s_tmem), kTmemCols);
@@ -123,10 +130,10 @@ __global__ void __launch_bounds__(kThreads, 1) attn_decode_cols(DecodeParams p, 
     if (tid < p.n_slots) s_len[tid] = read_len();
     __syncthreads();
     const size_t head_byte = (size_t)kvh * p.stride * kRowBytes;   // (the columns share the cache)
-    Share sh = share_columns<kC>(p, cap, in_head, s_len);
+    Share sh = share_columns<kC>(p, cap, in_head, group, s_len);
     int base, end;
     int groups = find_group(sh, p.n_slots, base, end);
-    int n, len[kCols], first, row1, nw;
+    int n, first, row1, nw;
     bool live;
     Work w;
     size_t step;
@@ -138,11 +145,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_decode_cols(DecodeParams p, 
         if (n == 0) return;
         const Balance b0 = balance(p, s_len[base], kC, kUnitRows);
         int longest = 0;
-#pragma unroll
-        for (int c = 0; c < kCols; c++) {
-            len[c] = c < n ? s_len[base + c] : 0;
-            longest = max(longest, len[c]);
-        }
+        for (int c = 0; c < n; c++) longest = max(longest, s_len[base + c]);
         w = plan_run<kC>(b0, base, kvh, sh.run, rank, longest);
         live = w.run < w.runs;
         first = w.row0 + w.unit * warp;
@@ -163,8 +166,10 @@ __global__ void __launch_bounds__(kThreads, 1) attn_decode_cols(DecodeParams p, 
         prefetch_l2(kp, unit_bytes(0));
         prefetch_l2(vp, unit_bytes(0));
     }
+    if (lane == 0 && warp < n)
+        ask_l2(p.q + (size_t)(base + warp) * p.q_slot + (size_t)kvh * group * 256, 1024LL * group);
     griddep_wait();
-    unsigned phase = 0, fold_phase = 0;
+    unsigned phase = 0;
     bool landed = true, checked = false;
     auto wait = [&](int slot) {
         unsigned spin = 0;
@@ -178,29 +183,31 @@ __global__ void __launch_bounds__(kThreads, 1) attn_decode_cols(DecodeParams p, 
 
     for (;;) {
         const int real_len = !checked && tid < p.n_slots ? read_len() : 0;
-        // Query fragments of every column, warp b makes block b's (as in the single-column body).
-        float2 x[kCols][2][2];
+        // Head f of the group's columns is head f % group of column f / group. Query fragments of every tile, warp b
+        // makes block b's (as in the single-column body).
+        const int heads = n * group, tiles = div_up(heads, 8);
+        float2 x[kTiles][2][2];
 #pragma unroll
-        for (int c = 0; c < kCols; c++) {
-            const float *const qh = p.q + (size_t)(base + c) * p.q_slot + (size_t)(kvh * group + g) * 256;
+        for (int a = 0; a < kTiles; a++) {
+            const int f = 8 * a + g, c = f / group;
+            const float *const qh = p.q + (size_t)(base + c) * p.q_slot + (size_t)(kvh * group + f - c * group) * 256;
 #pragma unroll
             for (int k = 0; k < 2; k++)
 #pragma unroll
                 for (int i = 0; i < 2; i++) {
-                    x[c][k][i] = make_float2(0.0f, 0.0f);
-                    if (g < group && c < n)
-                        x[c][k][i] = *reinterpret_cast<const float2 *>(qh + k_word_dim(warp, 4 * k + t, 2 * i));
+                    x[a][k][i] = make_float2(0.0f, 0.0f);
+                    if (f < heads) x[a][k][i] = *reinterpret_cast<const float2 *>(qh + k_word_dim(warp, 4 * k + t, 2 * i));
                 }
         }
         if (lane == 0 && nw > 0) {
             fetch(0, kp, 0);
             fetch(0, vp, 1);
         }
+        auto query_of = [&](int a) { return reinterpret_cast<uint4 *>(smem + C::kOffQ + a * C::kQBytes); };
+        auto bias_of = [&](int a) { return reinterpret_cast<float *>(smem + C::kOffBias + a * C::kBiasBytes); };
 #pragma unroll
-        for (int c = 0; c < kCols; c++)
-            if (c < n)
-                store_query<false>(x[c], p.scale_log2, warp, lane, reinterpret_cast<uint4 *>(smem + C::kOffQ + c * C::kQBytes),
-                                   reinterpret_cast<float *>(smem + C::kOffBias + c * C::kBiasBytes));
+        for (int a = 0; a < kTiles; a++)
+            if (a < tiles) store_query<false>(x[a], p.scale_log2, warp, lane, query_of(a), bias_of(a));
         tc_fence_before();
         if (checked) {
             __syncthreads();
@@ -217,7 +224,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_decode_cols(DecodeParams p, 
             }
             if (tid < p.n_slots) s_len[tid] = real_len;
             __syncthreads();
-            sh = share_columns<kC>(p, cap, in_head, s_len);
+            sh = share_columns<kC>(p, cap, in_head, group, s_len);
             groups = find_group(sh, p.n_slots, base, end);
             plan();
             checked = true;
@@ -227,65 +234,89 @@ __global__ void __launch_bounds__(kThreads, 1) attn_decode_cols(DecodeParams p, 
         tc_fence_after();
         if (base >= p.n_slots) break;
         if (live) {
-        // this warp's accumulators of column c: lanes 32 * (warp % 4), columns 128 c + 64 * (warp / 4)
+        // this warp's accumulators of tile a: lanes 32 * (warp % 4), columns 128 a + 64 * (warp / 4)
         const unsigned tmem = s_tmem + ((unsigned)(warp & 3) << 21) + 64u * (warp >> 2);
+        // live rows of heads 2t, 2t + 1 of every tile (heads past the last: the longest's)
+        int len[kTiles][2];
+#pragma unroll
+        for (int a = 0; a < kTiles; a++)
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int f = 8 * a + 2 * t + h;
+                len[a][h] = f < heads ? s_len[base + f / group] : row1;
+            }
 
-        Running run[kCols];
+        Running run[kTiles];
 #pragma unroll
-        for (int c = 0; c < kCols; c++) start(run[c]);
-        auto work = [&](auto tiles, int i, int rows) __attribute__((always_inline)) {
-            constexpr int kT = decltype(tiles)::value;
+        for (int a = 0; a < kTiles; a++) start(run[a]);
+        auto work = [&](auto row_tiles, int i, int rows) __attribute__((always_inline)) {
+            constexpr int kT = decltype(row_tiles)::value;
             const int r0 = first + i * w.unit * kWarps;
-            // ---- scores of all columns
+            // ---- scores of all tiles
             wait(0);
-            float s[kCols][kT][4];
+            float s[kTiles][kT][4];
 #pragma unroll
-            for (int c = 0; c < kCols; c++)
+            for (int a = 0; a < kTiles; a++)
 #pragma unroll
                 for (int j = 0; j < kT; j++)
 #pragma unroll
-                    for (int e = 0; e < 4; e++) s[c][j][e] = 0.0f;
+                    for (int e = 0; e < 4; e++) s[a][j][e] = 0.0f;
             const unsigned *const krow = reinterpret_cast<const unsigned *>(ring) + g * Row<false>::kPitch;
-            auto score = [&](auto m) __attribute__((always_inline)) {
-                constexpr int M = decltype(m)::value;
+#pragma unroll 1
+            for (int M = 0; M < 4; M++) {   // pairs of blocks
                 KFrag<kT> f;
-                load_k<M, false, kT>(krow, t, f);
+                load_k<0, false, kT>(krow + M * Row<false>::kPair, t, f);
 #pragma unroll
-                for (int c = 0; c < kCols; c++)
-                    if (c < n)
-                        add_scores<M, kT>(f, reinterpret_cast<const uint4 *>(smem + C::kOffQ + c * C::kQBytes) + lane,
-                                          reinterpret_cast<const float4 *>(smem + C::kOffBias + c * C::kBiasBytes) + t, s[c]);
-            };
-            score(Int<0>{});
-            score(Int<1>{});
-            score(Int<2>{});
-            score(Int<3>{});
+                for (int a = 0; a < kTiles; a++)
+                    if (a < tiles)
+                        add_scores<0, kT>(f, query_of(a) + lane + 4 * 32 * M,
+                                          reinterpret_cast<const float4 *>(bias_of(a)) + t + 8 * M, s[a]);
+            }
             __syncwarp();
             kp += step;
             if (lane == 0 && i + 1 < nw) fetch(i + 1, kp, 0);
-            // ---- softmax
-            __half2 ph[kCols][kT][2], pl[kCols][kT][2];
+            // ---- softmax (where the unit begins past a column's end, that column gets nothing from it)
+            __half2 ph[kTiles][kT][2], pl[kTiles][kT][2];
+            auto sight = [&](int a, int h) { return min(w.unit, min(row1, len[a][h]) - r0); };
+            // Heads (a bit each) whose references move: all of a column as soon as one of them is exceeded, no others, as
+            // in the column's own launch.
+            unsigned moving = 0;
 #pragma unroll
-            for (int c = 0; c < kCols; c++) {
-                if (c >= n) break;
-                const int rows_c = min(w.unit, min(row1, len[c]) - r0);
-                if (rows_c <= 0) {   // the unit begins past this column's end: it adds nothing
+            for (int a = 0; a < kTiles; a++) {
+                if (a >= tiles) break;
+                const int rows_of[2] = {sight(a, 0), sight(a, 1)};
+                float nm[2], x[kT][4];
+                bool over[2];
+                exponents<kT, true>(s[a], rows_of, g, run[a], nm, x, over);
+                // (lane t of each group of four has heads 2t, 2t + 1)
+                if (over[0]) moving |= 1u << (8 * a + 2 * t);
+                if (over[1]) moving |= 2u << (8 * a + 2 * t);
+            }
+            if (__any_sync(0xffffffffu, moving != 0)) {
+                moving = __reduce_or_sync(0xffffffffu, moving);
+                const unsigned one = (1u << group) - 1;
+                for (int c = 0; c < n; c++)
+                    if (moving >> (c * group) & one) moving |= one << (c * group);
+            }
 #pragma unroll
-                    for (int j = 0; j < kT; j++)
-#pragma unroll
-                        for (int e = 0; e < 2; e++) ph[c][j][e] = pl[c][j][e] = __float2half2_rn(0.0f);
-                    continue;
-                }
+            for (int a = 0; a < kTiles; a++) {
+                if (a >= tiles) break;
+                const int rows_of[2] = {sight(a, 0), sight(a, 1)};
+                const unsigned mine = moving >> (8 * a);
+                auto decide = [&](const bool (&)[2], bool (&move)[2]) {
+                    move[0] = mine >> (2 * t) & 1;
+                    move[1] = mine >> (2 * t + 1) & 1;
+                    return (mine & 0xff) != 0;
+                };
                 float corr[2];
-                if (softmax<kT>(s[c], rows_c, g, run[c], ph[c], pl[c], corr) && i > 0) {
+                if (softmax<kT, true>(s[a], rows_of, g, run[a], ph[a], pl[a], corr, decide) && i > 0) {
 #pragma unroll 1
-                    for (int m = 0; m < 4; m++) {
-                        float a[16];
-                        tmem_ld16(tmem + 128 * c + 16 * m, a);
-                        tmem_wait_ld();
+                    for (int b = 0; b < 4; b++) {
+                        float v[16];
+                        tmem_ld16(tmem + 128 * a + 16 * b, v);
 #pragma unroll
-                        for (int e = 0; e < 16; e++) a[e] *= corr[e & 1];
-                        tmem_st16(tmem + 128 * c + 16 * m, a);
+                        for (int e = 0; e < 16; e++) v[e] *= corr[e & 1];
+                        tmem_st16(tmem + 128 * a + 16 * b, v);
                     }
                     tmem_wait_st();
                 }
@@ -302,12 +333,9 @@ __global__ void __launch_bounds__(kThreads, 1) attn_decode_cols(DecodeParams p, 
             if (rows < 16 * kT) clear_rows(rows, 16 * kT);
             // Where a column ends inside the unit, the rows past its end are other columns': they stay. If one of them
             // has such a scale, the columns take turns, the longest first, and each clears what it does not see.
-            unsigned on = (1u << n) - 1, left = 0;   // columns of the pass, columns of later passes
-            int upto = rows, shortest = rows;
-            auto rows_of = [&](int c) { return max(0, min(w.unit, min(row1, len[c]) - r0)); };
-#pragma unroll
-            for (int c = 0; c < kCols; c++)
-                if (c < n) shortest = min(shortest, rows_of(c));
+            auto rows_of = [&](int c) { return max(0, min(w.unit, min(row1, s_len[base + c]) - r0)); };
+            int shortest = rows;
+            for (int c = 0; c < n; c++) shortest = min(shortest, rows_of(c));
             bool apart = false;
             if (shortest < rows) {
                 bool bad = false;
@@ -316,60 +344,60 @@ __global__ void __launch_bounds__(kThreads, 1) attn_decode_cols(DecodeParams p, 
                     bad = bad || (*reinterpret_cast<const unsigned short *>(scale) & 0x7c00u) == 0x7c00u;
                 }
                 apart = __any_sync(0xffffffffu, bad);
-                if (apart) left = on;
             }
             const unsigned *const vrow = reinterpret_cast<const unsigned *>(vt) + 2 * t * Row<false>::kPitch;
-            auto value = [&](auto m) __attribute__((always_inline)) {
-                constexpr int M = decltype(m)::value;
+            // the values of the unit for all heads, or for those of column `only` (begun: there is something to add to)
+            auto value = [&](int M, auto masked, int only, bool begun) __attribute__((always_inline)) {
+                constexpr bool kMasked = decltype(masked)::value != 0;
                 VFrag f[kT];
 #pragma unroll
-                for (int j = 0; j < kT; j++) load_v<M, false>(vrow + j * 16 * Row<false>::kPitch, g, f[j]);
+                for (int j = 0; j < kT; j++)
+                    load_v<0, false>(vrow + M * Row<false>::kPair + j * 16 * Row<false>::kPitch, g, f[j]);
 #pragma unroll
-                for (int c = 0; c < kCols; c++) {
-                    if (!(on >> c & 1)) continue;
-                    float a[16];
+                for (int a = 0; a < kTiles; a++) {
+                    if (a >= tiles) break;
+                    float v[16];
 #pragma unroll
-                    for (int e = 0; e < 16; e++) a[e] = 0.0f;
-                    if (i > 0) {
-                        tmem_ld16(tmem + 128 * c + 16 * M, a);
-                        tmem_wait_ld();
-                    }
-                    float ae[2][4], ao[2][4];
+                    for (int e = 0; e < 16; e++) v[e] = 0.0f;
+                    if (begun) tmem_ld16(tmem + 128 * a + 16 * M, v);
+                    float ve[2][4], vo[2][4];
 #pragma unroll
                     for (int e = 0; e < 8; e++) {
-                        ae[e >> 2][e & 3] = a[e];
-                        ao[e >> 2][e & 3] = a[8 + e];
+                        ve[e >> 2][e & 3] = v[e];
+                        vo[e >> 2][e & 3] = v[8 + e];
                     }
+                    const bool keep = !kMasked || (8 * a + g) / group == only;
 #pragma unroll
-                    for (int j = 0; j < kT; j++) add_values(f[j], ph[c][j], pl[c][j], ae, ao);
+                    for (int j = 0; j < kT; j++) add_values<kMasked>(f[j], ph[a][j], pl[a][j], ve, vo, keep);
 #pragma unroll
                     for (int e = 0; e < 8; e++) {
-                        a[e] = ae[e >> 2][e & 3];
-                        a[8 + e] = ao[e >> 2][e & 3];
+                        v[e] = ve[e >> 2][e & 3];
+                        v[8 + e] = vo[e >> 2][e & 3];
                     }
-                    tmem_st16(tmem + 128 * c + 16 * M, a);
+                    tmem_st16(tmem + 128 * a + 16 * M, v);
                 }
             };
-            for (;;) {
-                if (apart) {
-                    __syncwarp();
+            if (!apart) {
+#pragma unroll 1
+                for (int M = 0; M < 4; M++) value(M, Int<0>{}, 0, i > 0);
+            } else {
+                int upto = rows;
+                unsigned left = (1u << n) - 1;
+                for (bool begun = i > 0; left != 0; begun = true) {
                     int c_at = 0, most = -1;
-#pragma unroll
-                    for (int c = 0; c < kCols; c++)
+                    for (int c = 0; c < n; c++)
                         if ((left >> c & 1) && rows_of(c) > most) {
                             most = rows_of(c);
                             c_at = c;
                         }
+                    __syncwarp();
                     clear_rows(most, upto);
                     upto = most;
-                    on = 1u << c_at;
-                    left &= ~on;
+                    left &= ~(1u << c_at);
+                    tmem_wait_st();   // what the turn before stored is loaded again
+#pragma unroll 1
+                    for (int M = 0; M < 4; M++) value(M, Int<1>{}, c_at, begun);
                 }
-                value(Int<0>{});
-                value(Int<1>{});
-                value(Int<2>{});
-                value(Int<3>{});
-                if (left == 0) break;
             }
             tmem_wait_st();
             __syncwarp();
@@ -388,86 +416,88 @@ __global__ void __launch_bounds__(kThreads, 1) attn_decode_cols(DecodeParams p, 
                 work(Int<1>{}, i, rows);
         }
 
-        // ---- merge: the warps of the CTA, two columns at a time, then the cluster, then the runs
-        const int items = group * 64;
+        // ---- merge: the warps of the CTA, two tiles at a time, then the cluster, then the runs
+        const int items = group * 64;   // of a column
         const bool one_run = w.runs == 1 && p.out != nullptr;
-        float2 *const wml = reinterpret_cast<float2 *>(smem + C::kOffMl);
-        auto cpart = [&](int c) { return reinterpret_cast<float4 *>(smem + C::kOffQ + c * C::kQBytes); };
-        auto cml = [&](int c) { return reinterpret_cast<float2 *>(smem + C::kOffCml) + 8 * c; };
+        float2 *const wml = reinterpret_cast<float2 *>(smem + C::kOffMl);    // [heads][warps]
+        float4 *const cpart = reinterpret_cast<float4 *>(smem + C::kOffQ);   // [heads][64]: over the query fragments
+        float2 *const cml = reinterpret_cast<float2 *>(smem + C::kOffCml);   // [heads]
 #pragma unroll
-        for (int c0 = 0; c0 < kCols; c0 += 2) {
-            if (c0 >= n) break;
+        for (int a = 0; a < kTiles; a++) {
+            if (a >= tiles) break;
+            sum_rows(run[a]);
+            if (g == 0) {
+                wml[(8 * a + 2 * t) * kWarps + warp] = make_float2(run[a].m[0], run[a].l[0]);
+                wml[(8 * a + 2 * t + 1) * kWarps + warp] = make_float2(run[a].m[1], run[a].l[1]);
+            }
+        }
+#pragma unroll 1
+        for (int a0 = 0; a0 < tiles; a0 += 2) {
+            const int a1 = min(a0 + 2, tiles);
+#pragma unroll 1
+            for (int a = a0; a < a1; a++) {
+                float v[64];
 #pragma unroll
-            for (int c = c0; c < c0 + 2; c++) {
-                if (c >= n) break;
-                sum_rows(run[c]);
-                float2 *const ml = wml + (c - c0) * 8 * kWarps;
-                if (g == 0) {
-                    ml[(2 * t) * kWarps + warp] = make_float2(run[c].m[0], run[c].l[0]);
-                    ml[(2 * t + 1) * kWarps + warp] = make_float2(run[c].m[1], run[c].l[1]);
-                }
-                float a[4][16];
-#pragma unroll
-                for (int m = 0; m < 4; m++)
-#pragma unroll
-                    for (int e = 0; e < 16; e++) a[m][e] = 0.0f;
-                if (nw > 0) {
-#pragma unroll
-                    for (int m = 0; m < 4; m++) tmem_ld16(tmem + 128 * c + 16 * m, a[m]);
-                    tmem_wait_ld();
-                }
+                for (int e = 0; e < 64; e++) v[e] = 0.0f;
+                if (nw > 0) tmem_ld64(tmem + 128 * a, v);
                 float acc[8][2][4];
 #pragma unroll
-                for (int m = 0; m < 4; m++)
-#pragma unroll
-                    for (int e = 0; e < 16; e++) acc[2 * m + (e >> 3)][(e >> 2) & 1][e & 3] = a[m][e];
-                store_warp_partial<false>(reinterpret_cast<float *>(ring + (c - c0) * C::kPartial), acc, group, g, t);
+                for (int e = 0; e < 64; e++) acc[e >> 3][(e >> 2) & 1][e & 3] = v[e];
+                store_warp_partial<false>(reinterpret_cast<float *>(ring + (a - a0) * C::kPartial), acc,
+                                          min(8, heads - 8 * a), g, t);
             }
             __syncthreads();
-#pragma unroll
-            for (int c = c0; c < c0 + 2; c++)
-                if (c < n)
-                    fold_warps(smem + (c - c0) * C::kPartial, C::kRing, wml + (c - c0) * 8 * kWarps, items,
-                               [&](int item, const Part &r) {
-                                   cpart(c)[item] = r.a;
-                                   if ((item & 63) == 0) cml(c)[item >> 6] = make_float2(r.m, r.l);
-                               });
-            if (c0 + 2 < n) __syncthreads();
+#pragma unroll 1
+            for (int a = a0; a < a1; a++)
+                fold_warps(smem + (a - a0) * C::kPartial, C::kRing, wml + 8 * a * kWarps, min(8, heads - 8 * a) * 64, tid,
+                           [&](int item, const Part &r) {
+                               cpart[a * 512 + item] = r.a;
+                               if ((item & 63) == 0) cml[a * 8 + (item >> 6)] = make_float2(r.m, r.l);
+                           });
+            if (a1 < tiles) __syncthreads();
         }
         cluster_sync_all();
-        fold_cluster<kC, kCols>(cpart(0), cml(0), C::kQBytes / 16, n, items, rank, [&](int c, int item, const Part &r) {
-            if (one_run) emit_item(p, base + c, kvh, group, item, r);
-            const size_t row = (size_t)(kvh * group + (item >> 6)) * p.splits + w.run;
-            reinterpret_cast<float4 *>(p.part_acc + (size_t)(base + c) * p.acc_slot + row * 256)[item & 63] = r.a;
-            if (writes_pair<kC>(items, rank, item))
-                *reinterpret_cast<float2 *>(p.part_ml + (size_t)(base + c) * p.ml_slot + row * 2) = make_float2(r.m, r.l);
-        });
-        cluster_arrive();   // no CTA may leave, or start over, while another still reads its partials
-        if (p.out != nullptr && !one_run) {
-            int *const ctr = g_arrive_cols + (size_t)p.arrive_region * kArriveRegionInts +
-                             (size_t)(base * p.n_kv + kvh) * p.arrive_stride + rank;
-            __syncthreads();
-            if (tid == 0) {
-                const int last = arrive_acq_rel(ctr) == w.runs - 1;
-                if (last) *ctr = 0;
-                s_last = last;
-            }
-            __syncthreads();
-            if (s_last) {
-                // as many columns at a time as fit the rings
-                const int slice = (items / kC + 1) * w.runs * 16, fit = max(1, min(n, kWarps * C::kRing / slice));
-                for (int c = 0; c < n; c += fit) {
-                    const int m = min(fit, n - c);
-                    // (the staged fold takes the runs in one order; clusters of four and eight join shares of them, as
-                    // the single-column body does)
-                    if (Split<kC>::kShare == 1 &&
-                        fold_runs_staged<kC>(p, base + c, m, kvh, group, w.runs, rank, smem, kWarps * C::kRing, bar_fold,
-                                             fold_phase, reinterpret_cast<float2(*)[kStagedRow]>(smem + C::kOffFold), landed))
-                        fold_phase ^= 1;
-                    else
-                        fold_runs<kC, 1, 8>(p, base + c, m, kvh, group, w.runs, rank, nullptr);
+        // Column after column, beginning with another one in every run. Warps 0 .. group - 1 fold the cluster's partials
+        // of a column; another one (the s-th itself where there is none) announces the run.
+        auto column = [&](int s) { return (s + w.run) % n; };
+        const bool meet = p.out != nullptr && !one_run;
+        for (int s = 0; s < n; s++) {
+            const int c = column(s), announcer = group < 8 ? group + s % (8 - group) : s;
+            if (warp < group)
+                fold_cluster<kC>(cpart + c * items, cml + c * group, items, rank, [&](int item, const Part &r) {
+                    if (one_run) emit_item(p, base + c, kvh, group, item, r);
+                    const size_t row = (size_t)(kvh * group + (item >> 6)) * p.splits + w.run;
+                    reinterpret_cast<float4 *>(p.part_acc + (size_t)(base + c) * p.acc_slot + row * 256)[item & 63] = r.a;
+                    if (writes_pair<kC>(items, rank, item))
+                        *reinterpret_cast<float2 *>(p.part_ml + (size_t)(base + c) * p.ml_slot + row * 2) =
+                            make_float2(r.m, r.l);
+                });
+            if (!meet) continue;
+            const int threads = 32 * (group < 8 ? group + 1 : 8);
+            if (warp == announcer) {
+                named_sync(kArriveBar + s, threads);
+                if (lane == 0) {
+                    int *const ctr = g_arrive_cols + (size_t)p.arrive_region * kArriveRegionInts +
+                                     (size_t)((base + c) * p.n_kv + kvh) * p.arrive_stride + rank;
+                    const int last = arrive_acq_rel(ctr) == w.runs - 1;
+                    if (last) *ctr = 0;
+                    s_last[s] = last;
                 }
+                __syncwarp();
+            } else if (warp < group) {
+                named_arrive(kArriveBar + s, threads);
             }
+        }
+        cluster_arrive();   // no CTA may leave, or start over, while another still reads its partials
+        if (meet) {
+            __syncthreads();
+            for (int s = 0; s < n; s++)
+                if (s_last[s]) {
+                    if constexpr (kC == 2)
+                        fold_runs<kC, 1, 18>(p, base + column(s), 1, kvh, group, w.runs, rank, nullptr);
+                    else
+                        fold_runs<kC, 1, 8>(p, base + column(s), 1, kvh, group, w.runs, rank, nullptr);
+                }
         }
         cluster_wait();
         __syncthreads();

@@ -392,7 +392,8 @@ __global__ void __launch_bounds__(kThreads, kWide ? 1 : 2) attn_decode_warps(Dec
         release(!plain, i + (C::kSlots - 1) / 2, vp + (size_t)((C::kSlots - 1) / 2) * step);
         __half2 ph[kT][2], pl[kT][2];
         float corr[2];
-        if (softmax<kT>(s, rows, g, run, ph, pl, corr)) {
+        const int rows_of[2] = {rows, rows};
+        if (softmax<kT>(s, rows_of, g, run, ph, pl, corr)) {
 #pragma unroll
             for (int b = 0; b < 8; b++)
 #pragma unroll
@@ -469,7 +470,7 @@ __global__ void __launch_bounds__(kThreads, kWide ? 1 : 2) attn_decode_warps(Dec
     };
     float4 *const inbox = reinterpret_cast<float4 *>(smem + C::kOffIn);
     float2 *const inbox_ml = reinterpret_cast<float2 *>(smem + C::kOffInMl);
-    fold_warps(smem, C::kRing, wml, items, [&](int item, const Part &r) {
+    fold_warps(smem, C::kRing, wml, items, tid, [&](int item, const Part &r) {
         if constexpr (kC > 1)
             send_item<kC>(inbox, inbox_ml, bar_in, items, rank, item, r);
         else

@@ -185,28 +185,53 @@ __device__ __forceinline__ void sum_rows(Running &r) {   // over the lanes of a 
         r.l[h] += __shfl_xor_sync(0xffffffffu, r.l[h], 16);
     }
 }
-// The weights 2^(score - reference + 10) of kT tiles, as f16 high and low pairs in the B operand's
-// layout: ph[j][0] = rows 2t, 2t + 1 of tile j for head g, ph[j][1] = rows 2t + 8, 2t + 9. Rows from `rows` on
-// get weight 0. True when the references moved: what was accumulated must be multiplied by corr.
-template <int kT>
-__device__ __forceinline__ bool softmax(float (&s)[kT][4], int rows, int g, Running &r, __half2 (&ph)[kT][2],
-                                        __half2 (&pl)[kT][2], float (&corr)[2]) {
-    if (rows < 16 * kT) {   // rows past the end hold stale bytes
+// The exponents score - reference + 10 of kT tiles. Rows from rows[h] on are out of head 2t + h's sight; with kApart the
+// heads differ in that, and one may see none (rows[h] <= 0). over[h]: one of the lane's scores is above the head's
+// reference (not kApart: over[0], of either head).
+template <int kT, bool kApart>
+__device__ __forceinline__ void exponents(float (&s)[kT][4], const int (&rows)[2], int g, const Running &r, float (&nm)[2],
+                                          float (&x)[kT][4], bool (&over)[2]) {
+    nm[0] = r.nm[0];
+    nm[1] = r.nm[1];
+    if ((kApart ? min(rows[0], rows[1]) : rows[0]) < 16 * kT) {   // rows past the end hold stale bytes
 #pragma unroll
-        for (int j = 0; j < kT; j++) {
-            if (16 * j + g >= rows) s[j][0] = s[j][1] = -INFINITY;
-            if (16 * j + g + 8 >= rows) s[j][2] = s[j][3] = -INFINITY;
+        for (int h = 0; h < 2; h++) {
+            if (kApart && rows[h] <= 0) nm[h] = 0.0f;   // (-infinity from here on, not NaN)
+#pragma unroll
+            for (int j = 0; j < kT; j++) {
+                if (16 * j + g >= rows[kApart ? h : 0]) s[j][h] = -INFINITY;
+                if (16 * j + g + 8 >= rows[kApart ? h : 0]) s[j][h + 2] = -INFINITY;
+            }
         }
     }
-    float x[kT][4], xm = -INFINITY;
+    float xm[2] = {-INFINITY, -INFINITY};
 #pragma unroll
     for (int j = 0; j < kT; j++)
 #pragma unroll
         for (int c = 0; c < 4; c++) {
-            x[j][c] = fmaf(s[j][c], kCodeUnit, r.nm[c & 1]);
-            xm = fmaxf(xm, x[j][c]);
+            x[j][c] = fmaf(s[j][c], kCodeUnit, nm[c & 1]);
+            float &m = xm[kApart ? c & 1 : 0];
+            m = fmaxf(m, x[j][c]);
         }
-    const bool moved = __any_sync(0xffffffffu, xm > kPScaleLog2);
+    over[0] = xm[0] > kPScaleLog2;
+    over[1] = xm[1] > kPScaleLog2;
+}
+// Moving the references of one column's heads: all of them as soon as one is exceeded.
+struct MoveAll {
+    __device__ __forceinline__ bool operator()(const bool (&over)[2], bool (&move)[2]) const {
+        return move[0] = move[1] = __any_sync(0xffffffffu, over[0] || over[1]);
+    }
+};
+// The weights 2^(score - reference + 10) of kT tiles, as f16 high and low pairs in the B operand's
+// layout: ph[j][0] = rows 2t, 2t + 1 of tile j for head g, ph[j][1] = rows 2t + 8, 2t + 9; weight 0 out of sight, and a
+// head that sees no row keeps its state. True when references moved: what was accumulated must be multiplied by corr.
+template <int kT, bool kApart = false, class Move = MoveAll>
+__device__ __forceinline__ bool softmax(float (&s)[kT][4], const int (&rows)[2], int g, Running &r, __half2 (&ph)[kT][2],
+                                        __half2 (&pl)[kT][2], float (&corr)[2], Move decide = {}) {
+    float nm[2], x[kT][4];
+    bool over[2], move[2];
+    exponents<kT, kApart>(s, rows, g, r, nm, x, over);
+    const bool moved = decide(over, move);
     if (moved) {
 #pragma unroll
         for (int h = 0; h < 2; h++) {
@@ -219,15 +244,18 @@ __device__ __forceinline__ bool softmax(float (&s)[kT][4], int rows, int g, Runn
             // (rounded up to 1/16, so that the shift by 10 is exact)
             const float top = ceilf(mx * (kCodeUnit * 16.0f)) * 0.0625f;
             const float mn = top > r.m[h] ? top + kMargin : r.m[h];
-            corr[h] = ex2(r.m[h] - mn);
-            r.m[h] = mn;
-            r.nm[h] = kPScaleLog2 - mn;
-            r.l[h] *= corr[h];
+            corr[h] = 1.0f;
+            if (!kApart || (move[h] && rows[h] > 0)) {
+                corr[h] = ex2(r.m[h] - mn);
+                r.m[h] = mn;
+                r.nm[h] = nm[h] = kPScaleLog2 - mn;
+                r.l[h] *= corr[h];
+            }
         }
 #pragma unroll
         for (int j = 0; j < kT; j++)
 #pragma unroll
-            for (int c = 0; c < 4; c++) x[j][c] = fmaf(s[j][c], kCodeUnit, r.nm[c & 1]);
+            for (int c = 0; c < 4; c++) x[j][c] = fmaf(s[j][c], kCodeUnit, nm[c & 1]);
     }
 #pragma unroll
     for (int j = 0; j < kT; j++) {
@@ -305,9 +333,11 @@ __device__ __forceinline__ void load_v(const unsigned *row, int g, VFrag &f) {
 }
 // acc[block][i][c] += weights * values: code bytes {0, 1} (i = 0) and {2, 3} of the lane's word of the even /
 // odd block, c = {byte 0, 1} x {head 2t, 2t + 1} (value_dim).
+// kMasked: heads g of lanes without `keep` get nothing, whatever the rows' scales are.
+template <bool kMasked = false>
 __device__ __forceinline__ void add_values(const VFrag &f, const __half2 (&ph)[2], const __half2 (&pl)[2],
-                                           float (&acc_e)[2][4], float (&acc_o)[2][4]) {
-    auto bits = [](const __half2 &h) { return *reinterpret_cast<const unsigned *>(&h); };
+                                           float (&acc_e)[2][4], float (&acc_o)[2][4], bool keep = true) {
+    auto bits = [&](const __half2 &h) { return !kMasked || keep ? *reinterpret_cast<const unsigned *>(&h) : 0u; };
     auto block = [&](const __half2 d01, const __half2 d23, const unsigned (&a)[2][4], float (&acc)[2][4]) {
         const __half2 h01 = __hmul2(ph[0], d01), h23 = __hmul2(ph[1], d23);
         const __half2 l01 = __hfma2(pl[0], d01, __hfma2(ph[0], d01, __hneg2(h01)));
@@ -477,54 +507,45 @@ __device__ __forceinline__ void store_warp_partial(float *dst, const float (&acc
                         make_float2(acc[b][i][h], acc[b][i][2 + h]);
         }
 }
-// Folds the partials of a CTA's warps (`pitch` bytes apart; ml: [8 heads][warp]); done(item, part).
+// Folds the partials of eight warps (`pitch` bytes apart; ml: [8 heads][warp]) by 256 threads, of which this is number
+// `tid`; done(item, part).
 template <class Done>
 __device__ __forceinline__ void fold_warps(const unsigned char *partials, int pitch, const float2 *ml_at, int items,
-                                           Done done) {
+                                           int tid, Done done) {
     constexpr int kPer = 2;   // (at most 512 items)
     Part r[kPer];
     fold_sources<kPer, kWarps>(
         0, kWarps,
         [&](int i, int j, float4 &x, float2 &ml) {
-            const int item = min((int)threadIdx.x + j * kThreads, items - 1);
+            const int item = min(tid + j * kThreads, items - 1);
             x = *reinterpret_cast<const float4 *>(partials + i * pitch + ((item >> 6) * kHeadPitch + 4 * (item & 63)) * 4);
             ml = ml_at[(item >> 6) * kWarps + i];
         },
         r);
 #pragma unroll
     for (int j = 0; j < kPer; j++)
-        if ((int)threadIdx.x + j * kThreads < items) done(threadIdx.x + j * kThreads, r[j]);
+        if (tid + j * kThreads < items) done(tid + j * kThreads, r[j]);
 }
-// Merge of a cluster, several columns: folds slice `rank` of the items of the kC CTAs of a cluster, for each of
-// `cols` <= kPer columns (partials of [item] at cpart, {max, sum} of [8 heads] at cml, a column cpart_pitch / 8
-// further, at the same place in each CTA); done(column, item, part).
-template <int kC, int kPer, class Done>
-__device__ __forceinline__ void fold_cluster(const float4 *cpart, const float2 *cml, int cpart_pitch, int cols, int items,
-                                             int rank, Done done) {
+// Merge of a cluster by reading: folds slice `rank` of the items of the kC CTAs of a cluster (partials of [item] at
+// cpart, {max, sum} of [8 heads] at cml, at the same place in each CTA), for threads 0 .. kThreads - 1 or more;
+// done(item, part).
+template <int kC, class Done>
+__device__ __forceinline__ void fold_cluster(const float4 *cpart, const float2 *cml, int items, int rank, Done done) {
     constexpr int kShare = Split<kC>::kShare;
-    static_assert(kC % kShare == 0, "slices");
-    const int first = items * rank / kC, count = items * (rank + 1) / kC - first, total = cols * count;
-    const int at = threadIdx.x / kShare, part = threadIdx.x % kShare;
-    int col[kPer], item[kPer];
-#pragma unroll
-    for (int j = 0; j < kPer; j++) {
-        const int f = min(at + j * (kThreads / kShare), total - 1);
-        col[j] = cols > 1 ? f / count : 0;
-        item[j] = first + f - col[j] * count;
-    }
-    Part r[kPer];
-    fold_sources<kPer, kC / kShare>(
+    static_assert(kC % kShare == 0 && 512 / kC * kShare <= kThreads, "slices");
+    const int first = items * rank / kC, count = items * (rank + 1) / kC - first;
+    const int at = threadIdx.x / kShare, part = threadIdx.x % kShare, item = first + min(at, count - 1);
+    if ((int)(threadIdx.x & ~31u) / kShare >= count) return;   // (whole warps: the others join by shuffles)
+    Part r[1];
+    fold_sources<1, kC / kShare>(
         part * (kC / kShare), (part + 1) * (kC / kShare),
-        [&](int i, int j, float4 &x, float2 &ml) {
-            x = ld_cluster_f4(map_to_cta(smem_u32(cpart + col[j] * cpart_pitch + item[j]), i));
-            ml = ld_cluster_f2(map_to_cta(smem_u32(cml + col[j] * 8 + (item[j] >> 6)), i));
+        [&](int i, int, float4 &x, float2 &ml) {
+            x = ld_cluster_f4(map_to_cta(smem_u32(cpart + item), i));
+            ml = ld_cluster_f2(map_to_cta(smem_u32(cml + (item >> 6)), i));
         },
         r);
-#pragma unroll
-    for (int j = 0; j < kPer; j++) {
-        join<kShare>(r[j]);
-        if (at + j * (kThreads / kShare) < total && part == 0) done(col[j], item[j], r[j]);
-    }
+    join<kShare>(r[0]);
+    if (at < count && part == 0) done(item, r[0]);
 }
 
 // Merge of a cluster, one column: every CTA sends each item of its partial to the CTA that folds it (slice r of

@@ -287,10 +287,11 @@ __device__ __forceinline__ void tmem_ld64(unsigned taddr, float (&r)[64]) {
         : "r"(taddr)
         : "memory");
 }
-// 16 columns of a lane, without the wait
+// 16 columns of a lane
 __device__ __forceinline__ void tmem_ld16(unsigned taddr, float (&r)[16]) {
     asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
         : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]), "=f"(r[4]), "=f"(r[5]), "=f"(r[6]), "=f"(r[7]),
           "=f"(r[8]), "=f"(r[9]), "=f"(r[10]), "=f"(r[11]), "=f"(r[12]), "=f"(r[13]), "=f"(r[14]), "=f"(r[15])
         : "r"(taddr)
@@ -302,9 +303,6 @@ __device__ __forceinline__ void tmem_st16(unsigned taddr, const float (&r)[16]) 
         ::"r"(taddr), "f"(r[0]), "f"(r[1]), "f"(r[2]), "f"(r[3]), "f"(r[4]), "f"(r[5]), "f"(r[6]), "f"(r[7]),
           "f"(r[8]), "f"(r[9]), "f"(r[10]), "f"(r[11]), "f"(r[12]), "f"(r[13]), "f"(r[14]), "f"(r[15])
         : "memory");
-}
-__device__ __forceinline__ void tmem_wait_ld() {
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void tmem_wait_st() {
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
@@ -369,6 +367,13 @@ __device__ __forceinline__ void bulk_store(void *dst, unsigned src, unsigned byt
 __device__ __forceinline__ void bulk_store_commit_wait_read() {
     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
     asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+}
+// Named barrier `id` for `threads` of the CTA: wait for all of them, or only announce.
+__device__ __forceinline__ void named_sync(int id, int threads) {
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void named_arrive(int id, int threads) {
+    asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 // Generic-proxy shared-memory writes -> visible to the async proxy (bulk copies, tensor cores).
 __device__ __forceinline__ void fence_async_shared() {
