@@ -279,38 +279,32 @@ __device__ __forceinline__ bool softmax(float (&s)[kT][4], const int (&rows)[2],
 
 // ---- values. A warp's V operands of blocks 2M, 2M + 1 for one tile of 16 rows (`row`: its row 2t).
 struct VFrag {
-    unsigned e[2][4], o[2][4];         // A fragments: code bytes {0, 1} and {2, 3} of the lane's word of each row
+    unsigned e[2][4], o[2][4];         // A fragments of the even / odd block: two code bytes of the lane's of each row (see value_dim)
     __half2 de01, de23, do01, do23;    // scales of rows 2t, 2t + 1 / 2t + 8, 2t + 9
 };
-template <int M, bool kQ4>
-__device__ __forceinline__ void load_v(const unsigned *row, int g, VFrag &f) {
-    using R = Row<kQ4>;
+__device__ __forceinline__ __half2 as_half2(unsigned x) { return *reinterpret_cast<const __half2 *>(&x); }
+__device__ __forceinline__ unsigned as_bits(const __half2 &x) { return *reinterpret_cast<const unsigned *>(&x); }
+// q8_0: code bytes {0, 1} and {2, 3} of word g of each row.
+template <int M>
+__device__ __forceinline__ void load_v_q8(const unsigned *row, int g, VFrag &f) {
+    using R = Row<false>;
     constexpr int kRowOf[4] = {0, 1, 8, 9};
-    const int j = kQ4 ? (g & 3) : g;
     unsigned w0[4], wh[4], we[4], wo[4];
 #pragma unroll
     for (int e = 0; e < 4; e++) {
         const unsigned *w = row + kRowOf[e] * R::kPitch + M * R::kPair;
         w0[e] = w[0];
         wh[e] = w[R::kHalf];
-        we[e] = w[1 + j];
-        wo[e] = w[R::kHalf + 1 + j];
+        we[e] = w[1 + g];
+        wo[e] = w[R::kHalf + 1 + g];
     }
-    auto half2_of = [](unsigned x) { return *reinterpret_cast<const __half2 *>(&x); };
     auto convert = [&](unsigned (&x)[4], unsigned (&a)[2][4]) {
 #pragma unroll
-        for (int e = 0; e < 4; e++) {
-            if constexpr (kQ4)
-                x[e] = (x[e] >> ((g >> 2) * 4)) & 0x0f0f0f0fu;
-            else
-                x[e] ^= 0x80808080u;
-        }
-        // 0x64xx = 1024 + xx, minus 1152 (nibbles: 1032): exact. (The weights are all positive, an offset
+        for (int e = 0; e < 4; e++) x[e] ^= 0x80808080u;
+        // 0x64xx = 1024 + xx, minus 1152: exact. (The weights are all positive, an offset
         // left to the accumulators would cost several bits: 4e-5 relative on a flat 256-key run.)
         auto conv = [&](unsigned y, unsigned sel) {
-            const __half2 r = __hsub2(half2_of(__byte_perm(y, 0x64646464u, sel)),
-                                      __half2half2(__ushort_as_half(kQ4 ? 0x6408 : 0x6480)));
-            return *reinterpret_cast<const unsigned *>(&r);
+            return as_bits(__hsub2(as_half2(__byte_perm(y, 0x64646464u, sel)), as_half2(0x64806480u)));
         };
 #pragma unroll
         for (int i = 0; i < 2; i++) {
@@ -323,16 +317,61 @@ __device__ __forceinline__ void load_v(const unsigned *row, int g, VFrag &f) {
         }
     };
 #pragma unroll
-    for (int e = 0; e < 4; e++) we[e] = j == R::kWords - 1 ? stitch(w0[e], wh[e]) : we[e];
-    f.de01 = half2_of(__byte_perm(w0[0], w0[1], 0x5410));
-    f.de23 = half2_of(__byte_perm(w0[2], w0[3], 0x5410));
-    f.do01 = half2_of(__byte_perm(wh[0], wh[1], 0x7632));
-    f.do23 = half2_of(__byte_perm(wh[2], wh[3], 0x7632));
+    for (int e = 0; e < 4; e++) we[e] = g == R::kWords - 1 ? stitch(w0[e], wh[e]) : we[e];
+    f.de01 = as_half2(__byte_perm(w0[0], w0[1], 0x5410));
+    f.de23 = as_half2(__byte_perm(w0[2], w0[3], 0x5410));
+    f.do01 = as_half2(__byte_perm(wh[0], wh[1], 0x7632));
+    f.do23 = as_half2(__byte_perm(wh[2], wh[3], 0x7632));
     convert(we, f.e);
     convert(wo, f.o);
 }
-// acc[block][i][c] += weights * values: code bytes {0, 1} (i = 0) and {2, 3} of the lane's word of the even /
-// odd block, c = {byte 0, 1} x {head 2t, 2t + 1} (value_dim).
+// q4_0: the low (i = 0) and the high nibbles of code bytes 2g and 2g + 1 of each row. Both nibbles of a byte serve the
+// same lane, and its two bytes are a half word, so that a pair of rows is one word and a nibble of it one mask: ten
+// instructions for eight values and none to stitch a word across the scale, where a word a row with one nibble of each
+// byte took 14 and four more (32,768 rows: 20.2 -> 19.0 us a layer).
+template <int M>
+__device__ __forceinline__ void load_v_q4(const unsigned *row, int g, VFrag &f) {
+    using R = Row<true>;
+    constexpr int kRowOf[4] = {0, 1, 8, 9};
+    unsigned se[4], so[4], ce[4], co[4];
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+        const unsigned short *w = reinterpret_cast<const unsigned short *>(row + kRowOf[e] * R::kPitch + M * R::kPair);
+        se[e] = w[0];
+        ce[e] = w[1 + g];
+        so[e] = w[R::kPair];
+        co[e] = w[R::kPair + 1 + g];
+    }
+    auto both = [](unsigned lo, unsigned hi) { return __byte_perm(lo, hi, 0x5410); };
+    auto convert = [&](const unsigned (&x)[4], unsigned (&a)[2][4]) {
+#pragma unroll
+        for (int p = 0; p < 2; p++) {   // rows 2t, 2t + 1 / 2t + 8, 2t + 9
+            const unsigned y = both(x[2 * p], x[2 * p + 1]);
+#pragma unroll
+            for (int byte = 0; byte < 2; byte++) {
+                const unsigned z = y >> (8 * byte);
+                // 1024 + n, minus 1032; (1024 + 16 n) / 16 - 72: both exact
+                a[0][2 * p + byte] = as_bits(__hsub2(as_half2((z & 0x000f000fu) | 0x64006400u), as_half2(0x64086408u)));
+                a[1][2 * p + byte] = as_bits(__hfma2(as_half2((z & 0x00f000f0u) | 0x64006400u), as_half2(0x2c002c00u),
+                                                     as_half2(0xd480d480u)));
+            }
+        }
+    };
+    f.de01 = as_half2(both(se[0], se[1]));
+    f.de23 = as_half2(both(se[2], se[3]));
+    f.do01 = as_half2(both(so[0], so[1]));
+    f.do23 = as_half2(both(so[2], so[3]));
+    convert(ce, f.e);
+    convert(co, f.o);
+}
+template <int M, bool kQ4>
+__device__ __forceinline__ void load_v(const unsigned *row, int g, VFrag &f) {
+    if constexpr (kQ4)
+        load_v_q4<M>(row, g, f);
+    else
+        load_v_q8<M>(row, g, f);
+}
+// acc[block][i][c] += weights * values, c = {dim, dim + 1} x {head 2t, 2t + 1} from value_dim(block, g, i) on.
 // kMasked: heads g of lanes without `keep` get nothing, whatever the rows' scales are.
 template <bool kMasked = false>
 __device__ __forceinline__ void add_values(const VFrag &f, const __half2 (&ph)[2], const __half2 (&pl)[2],
@@ -351,13 +390,15 @@ __device__ __forceinline__ void add_values(const VFrag &f, const __half2 (&ph)[2
     block(f.de01, f.de23, f.e, acc_e);
     block(f.do01, f.do23, f.o, acc_o);
 }
-// First dim (within the block) of code bytes {0, 1} (half 0) and {2, 3} (half 1) of lane group g's word.
+// First of the two dims (within the block) that lane group g has in half 0 and in half 1 of its operands: q8_0 code bytes
+// {0, 1} and {2, 3} of its word (of an even block, whose words begin with byte 2, the last is stitched); q4_0 the low and
+// the high nibbles of its two bytes.
 template <bool kQ4>
 __device__ __forceinline__ int value_dim(int blk, int g, int half) {
-    const int j = kQ4 ? (g & 3) : g, base = kQ4 ? 16 * (g >> 2) : 0, words = Row<kQ4>::kWords;
-    if (blk & 1) return base + 4 * j + 2 * half;
-    if (j == words - 1) return base + (half ? 4 * words - 2 : 0);
-    return base + 4 * j + 2 + 2 * half;
+    if (kQ4) return 2 * g + 16 * half;
+    if (blk & 1) return 4 * g + 2 * half;
+    if (g == Row<false>::kWords - 1) return half ? 30 : 0;
+    return 4 * g + 2 + 2 * half;
 }
 
 // Whether the CTA that folds slice `rank` of the items writes the {maximum, sum} of this item's head to memory: with
