@@ -494,12 +494,12 @@ __global__ void __launch_bounds__(kThreads, kWide ? 1 : 2) attn_decode_warps(Dec
             }
             __syncthreads();
             if (s_plan[0]) {
-                // (in a cluster a CTA has half a head's items or less: ordinary loads, one trip for the runs of a
-                // deep stream, are as fast there)
+                // (in a cluster a CTA has half a head group's items or less: ordinary loads, one trip for the runs of a
+                // deep stream, are as fast for 17 runs, 137 us against 141 for 16 layers of 3,000 rows)
                 if constexpr (kC > 1)
                     fold_runs<kC, 1, 18>(p, w.slot, 1, w.kvh, group, w.runs, rank, nullptr);
-                else if (!fold_runs_staged<kC>(p, w.slot, 1, w.kvh, group, w.runs, rank, smem, kWarps * C::kRing, bar_fold, 0,
-                                               reinterpret_cast<float2(*)[kStagedRow]>(smem + C::kOffQ), landed))
+                else if (!fold_runs_staged(p, w.slot, w.kvh, group, w.runs, smem, kWarps * C::kRing, bar_fold,
+                                           reinterpret_cast<float2(*)[kStagedRow]>(smem + C::kOffQ), landed))
                     fold_runs<kC, 1, 8>(p, w.slot, 1, w.kvh, group, w.runs, rank, nullptr);
             }
         } else {

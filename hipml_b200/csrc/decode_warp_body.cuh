@@ -717,62 +717,54 @@ __device__ __forceinline__ void fold_runs(const DecodeParams &p, int slot, int c
     }
 }
 
-// The same fold, bit for bit, with the partials brought to shared memory by bulk copies: ordinary loads
-// keep ~25 KB of a CTA's in flight, and at ~1 us a trip the last CTA of a deep head (17 runs x 3 KB, four
-// times that for four columns) spent 2.3 and 8.4 us in them. `area`: `bytes` of shared memory that no copy
-// is in flight to, `bar`: a barrier in its phase `phase`. False (and nothing done) where they do not fit.
+// The same fold of all a head group's items, bit for bit, with the partials brought to shared memory by bulk copies: a
+// head's runs are one piece of memory, so six heads of 16 runs (98 KB) are six copies. (Ordinary loads keep ~25 KB of a
+// CTA's in flight, at ~1 us a trip. Copied run by run, 1 KB each at ~60 ns a copy, they took the last CTA of the head 5
+// of the 26 us of a layer of 8 slots of 512 .. 8,192 rows; 16 layers 393 -> 380 us, of 3 slots of up to 3,139 rows 197 ->
+// 184.) `area`: `bytes` of shared memory that no copy is in flight to, `bar`: a fresh barrier. False (and nothing done)
+// where they do not fit.
 constexpr int kStagedRow = 32;   // float2s: {weight, sum} of up to 31 runs, the maximum last
-template <int kC>
-__device__ __forceinline__ bool fold_runs_staged(const DecodeParams &p, int slot, int cols, int kvh, int group, int runs,
-                                                 int rank, unsigned char *area, int bytes, unsigned bar, unsigned phase,
-                                                 float2 (*s_ml)[kStagedRow], bool &landed) {
-    const int items = group * 64, first = items * rank / kC, count = items * (rank + 1) / kC - first;
-    if (runs >= kStagedRow || cols * runs * count * 16 > bytes) return false;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int head0 = first >> 6, heads = ((first + count - 1) >> 6) - head0 + 1;
-    auto pa = [&](int c, int head, int run) {
-        return p.part_acc + (size_t)(slot + c) * p.acc_slot + ((size_t)(kvh * group + head) * p.splits + run) * 256;
-    };
-    // generic writes (of this CTA to the area, of all CTAs to the partials) come before the copies' reads
+__device__ __forceinline__ bool fold_runs_staged(const DecodeParams &p, int slot, int kvh, int group, int runs,
+                                                 unsigned char *area, int bytes, unsigned bar, float2 (*s_ml)[kStagedRow],
+                                                 bool &landed) {
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, row = runs * 1024;
+    if (runs >= kStagedRow || group * row > bytes) return false;
+    // generic writes (of this CTA to the area, of all CTAs to the partials) come before the copies
     asm volatile("fence.proxy.async;" ::: "memory");
     __syncthreads();
-    if (tid == 0) mbar_arrive_expect_tx(bar, (unsigned)(cols * runs * count * 16));
-    __syncthreads();
-    const int pieces = cols * runs * heads;   // a head's part of the slice of one run
-    for (int i = tid; i < pieces; i += kThreads) {
-        const int h = i % heads, cr = i / heads, run = cr % runs, c = cr / runs;
-        const int lo = max(first, (head0 + h) * 64), hi = min(first + count, (head0 + h + 1) * 64);
-        bulk_load(smem_u32(area) + (unsigned)((cr * count + lo - first) * 16), pa(c, head0 + h, run) + 4 * (lo & 63),
-                  (unsigned)((hi - lo) * 16), bar);
+    if (tid == 0) {
+        mbar_arrive_expect_tx(bar, (unsigned)(group * row));
+        for (int h = 0; h < group; h++)
+            bulk_load(smem_u32(area) + (unsigned)(h * row),
+                      p.part_acc + (size_t)slot * p.acc_slot + (size_t)(kvh * group + h) * p.splits * 256, (unsigned)row, bar);
     }
-    // weights {2^(m - M), l} of every (column, head), a warp each
-    for (int i = warp; i < cols * heads; i += kWarps) {
-        const int h = i % heads, c = i / heads;
+    // weights {2^(m - M), l} of every head, a warp each
+    for (int h = warp; h < group; h += kWarps) {
         float2 ml = make_float2(-INFINITY, 0.0f);
         if (lane < runs)
-            ml = __ldcg(reinterpret_cast<const float2 *>(p.part_ml + (size_t)(slot + c) * p.ml_slot +
-                                                         (size_t)(kvh * group + head0 + h) * p.splits * 2) + lane);
+            ml = __ldcg(reinterpret_cast<const float2 *>(p.part_ml + (size_t)slot * p.ml_slot +
+                                                         (size_t)(kvh * group + h) * p.splits * 2) + lane);
         const float big = warp_max(ml.x);
-        s_ml[i][lane] = lane == kStagedRow - 1 ? make_float2(big, 0.0f)
+        s_ml[h][lane] = lane == kStagedRow - 1 ? make_float2(big, 0.0f)
                                                : make_float2(ml.x == -INFINITY ? 0.0f : ex2(ml.x - big), ml.y);
     }
     __syncthreads();
-    for (unsigned spin = 0; !mbar_try_wait(bar, phase);)
+    for (unsigned spin = 0; !mbar_try_wait(bar, 0);)
         if (++spin > kSpinLimit) {
             landed = false;
             break;
         }
-    for (int f = tid; f < cols * count; f += kThreads) {
-        const int c = cols > 1 ? f / count : 0, at = f - c * count, item = first + at;
-        const float2 *const wl = s_ml[c * heads + (item >> 6) - head0];
-        const float4 *const x = reinterpret_cast<const float4 *>(area) + (size_t)c * runs * count + at;
+    for (int item = tid; item < group * 64; item += kThreads) {
+        const int h = item >> 6;
+        const float2 *const wl = s_ml[h];
+        const float4 *const x = reinterpret_cast<const float4 *>(area + h * row) + (item & 63);
         Part r;
         r.a = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         r.l = 0.0f;
         r.m = wl[kStagedRow - 1].x;
 #pragma unroll 4
         for (int i = 0; i < runs; i++) {
-            const float4 v = x[i * count];
+            const float4 v = x[i * 64];
             const float2 w = wl[i];
             r.a.x = fmaf(v.x, w.x, r.a.x);
             r.a.y = fmaf(v.y, w.x, r.a.y);
@@ -780,7 +772,7 @@ __device__ __forceinline__ bool fold_runs_staged(const DecodeParams &p, int slot
             r.a.w = fmaf(v.w, w.x, r.a.w);
             r.l = fmaf(w.y, w.x, r.l);
         }
-        emit_item(p, slot + c, kvh, group, item, r);
+        emit_item(p, slot, kvh, group, item, r);
     }
     return true;
 }
