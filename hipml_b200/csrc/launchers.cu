@@ -181,6 +181,8 @@ static int decode_kv(hipml_stream_t stream, const int *step, int selector, const
     p.kv_slot_bytes = p.acc_slot = p.ml_slot = p.q_slot = 0;
     if (tensor_core && ((reinterpret_cast<size_t>(p.k) | reinterpret_cast<size_t>(p.v)) & 15) != 0)
         return fail(HIPML_ERR_INVALID_ARGUMENT, "the KV cache must be 16-byte aligned");
+    // (a shard's scratch on an 8-byte boundary only: the split pass stores 16 bytes at a time)
+    if (shard && !xch && (reinterpret_cast<size_t>(part_acc) & 15) != 0) tensor_core = false;
     if (tensor_core && (reinterpret_cast<size_t>(q) & 7) != 0)
         return fail(HIPML_ERR_INVALID_ARGUMENT, "the query row must be 8-byte aligned");
     if (k_row) {

@@ -253,6 +253,25 @@ def test_sequence_split_shards_fold_to_the_whole_cache(shards, seq):
     assert O.max_abs(mirror.ravel(), out.cpu().numpy()) < 1e-6
 
 
+def test_a_shard_takes_scratch_on_an_8_byte_boundary():
+    """The unnormalised rows are 8-byte aligned, and so may the scratch be: what stores 16 bytes at a time is not used."""
+    from hipml_b200 import api
+    heads, n_kv, hd, seq, scale = 24, 4, 256, 300, 0.0625
+    rng = O.Rng(0x5A4E)
+    q = rng.normals(heads * hd)
+    kb = O.quantize_q8(rng.normals(n_kv * seq * hd)).reshape(n_kv, seq, 272)
+    vb = O.quantize_q8(rng.normals(n_kv * seq * hd)).reshape(n_kv, seq, 272)
+    splits = api.decode_splits(seq)
+    acc = torch.full((heads * splits * hd + 2,), float("nan"), device="cuda")[2:]
+    ml = torch.full((heads * splits * 2,), float("nan"), device="cuda")
+    gathered = torch.full((1, heads, hd + 2), float("nan"), device="cuda")
+    api.attn_decode_kv_shard(_step(seq - 1, seq), _dev(q), _dev(kb), _dev(vb), acc, ml, gathered[0], heads, n_kv, hd, seq,
+                             scale, splits)
+    out = torch.full((heads * hd,), float("nan"), device="cuda")
+    api.attn_decode_combine(gathered, out, heads, hd, 1)
+    _assert_close(O.attn_decode_kv_q8(q, kb, vb, heads, n_kv, hd, seq, scale), out.cpu().numpy())
+
+
 @pytest.mark.parametrize("by_head", [0, 4], ids=["replicated", "by_head"])
 @pytest.mark.parametrize("shards,seq", [(2, 700), (4, 3000), (8, 5)])
 def test_peer_memory_exchange_on_one_gpu_in_two_phases(shards, seq, by_head):
