@@ -278,7 +278,7 @@ __device__ __forceinline__ void apply_gate(float4 &w, const float4 &g) {
 // CTA 2 s + rank: rows of kPitch floats at stage_addr, their {maximum, sum} at ml_addr): folded and written by eight
 // warps, a warp two to four rows at a time with all their loads in flight. (One at a time a row costs three trips,
 // to the other CTAs' pairs, to their rows and to the gate's row in memory: 16 us for the 63 rows of a CTA in two
-// slices, 301 tokens at 3,001, now 3.)
+// slices, 301 tokens at 3,001, now ~5.)
 template <int kS>
 __device__ __forceinline__ void fold_slices(const ChunkTcParams &p, unsigned stage_addr, unsigned ml_addr, int nsp, int rank,
                                             int r_lo, int r_hi, int t0, int kvh, int warp, int lane) {

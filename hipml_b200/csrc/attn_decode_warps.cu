@@ -27,7 +27,7 @@
 // What bounds it: long caches the HBM stream and the issue rate together (100,000 rows: 43 - 45 us a
 // layer in a captured chain = 4.85 - 5.04 TB/s, 33 us of it in the loop; 1,555 warp instructions per 32 rows of K and V, where 64-row
 // tiles with CTA barriers and softmax through shared memory took 2,370, 57 us a layer); short ones
-// the chain of dependent latencies (8,192 rows: 10.7 us, before 16).
+// the chain of dependent latencies (8,192 rows: 10.0 us, before 16).
 //
 // Merge: the eight warps' partials through shared memory, then the CTAs of a cluster, each of which
 // folds a slice of the outputs and is sent the others' share of it, then, where a head has more

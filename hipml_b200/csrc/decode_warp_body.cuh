@@ -328,7 +328,7 @@ __device__ __forceinline__ void load_v_q8(const unsigned *row, int g, VFrag &f) 
 // q4_0: the low (i = 0) and the high nibbles of code bytes 2g and 2g + 1 of each row. Both nibbles of a byte serve the
 // same lane, and its two bytes are a half word, so that a pair of rows is one word and a nibble of it one mask: ten
 // instructions for eight values and none to stitch a word across the scale, where a word a row with one nibble of each
-// byte took 14 and four more (32,768 rows: 20.2 -> 19.0 us a layer).
+// byte took 14 and four more (30,000 rows: 19.2 -> 18.8 us a layer; two slots of up to 6,667: 13.9 -> 13.3).
 template <int M>
 __device__ __forceinline__ void load_v_q4(const unsigned *row, int g, VFrag &f) {
     using R = Row<true>;

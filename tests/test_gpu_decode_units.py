@@ -269,6 +269,34 @@ def test_columns_of_every_form_give_each_columns_own_bits(pos0, cols, splits, fo
     assert api.check_device_status() == 0
 
 
+# heads packed into one to four tiles of eight, full and not, columns across a tile's end; five and more columns a group
+@pytest.mark.parametrize("group,n_kv,cols", [(1, 4, 8), (2, 4, 7), (3, 2, 8), (4, 4, 8), (5, 2, 6), (6, 4, 5), (7, 2, 4), (8, 4, 5)])
+@pytest.mark.parametrize("pos0,bad", [(300, False), (4601, True), (9300, False)], ids=["short", "infinite_scales", "two_units"])
+def test_columns_packed_into_tiles_give_each_columns_own_bits(group, n_kv, cols, pos0, bad):
+    from hipml_b200 import api
+    heads, hd, scale, stride = group * n_kv, 256, 0.0625, pos0 + cols + 2
+    gen = torch.Generator(device="cuda").manual_seed(pos0 + 10 * group + cols)
+    kc, vc = (torch.zeros(n_kv * stride * 272, dtype=torch.uint8, device="cuda") for _ in range(2))
+    k, v = (torch.randn(pos0 + cols, n_kv * hd, device="cuda", generator=gen) for _ in range(2))
+    if bad:
+        v[pos0 + cols - 2:] = 1e9   # rows that only the last two columns see have an infinite scale
+    api.kv_encode_bulk(k, v, kc, vc, n_kv, hd, stride, 0, 0, pos0 + cols)
+    q = torch.randn(cols, heads * hd, device="cuda", generator=gen)
+    splits = api.decode_splits(pos0 + cols)
+    acc, ml = (torch.empty(cols * heads * splits * n, device="cuda") for n in (hd, 2))
+    out = torch.full((cols, heads * hd), float("nan"), device="cuda")
+    pos = torch.tensor([[pos0 + c, pos0 + c + 1] for c in range(cols)], dtype=torch.int32, device="cuda")
+    api.attn_decode_cols(pos, q, kc, vc, acc, ml, out, heads, n_kv, hd, stride, scale, splits, cols,
+                         heads * splits * hd, heads * splits * 2, heads * hd)
+    assert torch.isfinite(out[:cols - 2] if bad else out).all()
+    for c in range(cols):
+        one = torch.empty(heads * hd, device="cuda")
+        step = torch.tensor([pos0 + c, pos0 + c + 1] + [0] * 6, dtype=torch.int32, device="cuda")
+        api.attn_decode_kv(step, q[c], kc, vc, acc, ml, one, heads, n_kv, hd, stride, scale, splits)
+        assert torch.equal(one.nan_to_num(7.0), out[c].nan_to_num(7.0)), f"column {c}"
+    assert api.check_device_status() == 0
+
+
 # the last columns' rows in the first one's last unit, or in one of their own
 @pytest.mark.parametrize("cols", [2, 4, 7])
 @pytest.mark.parametrize("pos0", [0, 13, 29, 200, 1278, 4604, 9214])
