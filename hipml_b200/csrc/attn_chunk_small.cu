@@ -75,15 +75,6 @@ __global__ void __launch_bounds__(kThreads, 2) attn_chunk_small(SmallParams p) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int kvh = blockIdx.x, token = p.tokens - 1 - (int)blockIdx.y, group = p.n_heads / p.n_kv;
     const int seq = p.pos0 + token + 1;
-    if (tid == 0) ask_l2(p.q + ((size_t)token * p.n_heads + kvh * group) * 256, 1024LL * group);
-    if (blockIdx.y == 0) {   // the rows of earlier chunks, a few for each thread
-        for (int r = tid; r < p.pos0; r += kThreads) {
-            constexpr int kRow = kType == 0 ? 1024 : kType == 1 ? kRowBytes : kQ4RowBytes;
-            const size_t at = kType == 0 ? ((size_t)r * p.n_kv + kvh) * 1024 : ((size_t)kvh * p.stride + r) * kRow;
-            ask_l2((const unsigned char *)p.k + at, kRow);
-            ask_l2((const unsigned char *)p.v + at, kRow);
-        }
-    }
     griddep_wait();
     for (int i = tid; i < 8 * 64; i += kThreads) {
         float4 x = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
