@@ -442,8 +442,8 @@ __global__ void __launch_bounds__(kThreads, kWide ? 1 : 2) attn_decode_warps(Dec
     sum_rows(run);
     float2 *const wml = reinterpret_cast<float2 *>(smem + C::kOffMl);      // [8 heads][warp]
     if (g == 0) {
-        wml[(2 * t) * kWarps + warp] = make_float2(run.m[0], run.l[0]);
-        wml[(2 * t + 1) * kWarps + warp] = make_float2(run.m[1], run.l[1]);
+        wml[(2 * t) * kWarps + warp] = make_float2(-run.nm[0], run.l[0]);
+        wml[(2 * t + 1) * kWarps + warp] = make_float2(-run.nm[1], run.l[1]);
     }
     store_warp_partial<kQ4>(reinterpret_cast<float *>(ring), acc, group, g, t);
     __syncthreads();

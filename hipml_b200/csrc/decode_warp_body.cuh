@@ -410,8 +410,9 @@ __device__ __forceinline__ bool writes_pair(int items, int rank, int item) {
     return (item & 63) == 0 || item == items * rank / kC;
 }
 
-// ---- folds. A partial of a head is (acc, m, l) with weights relative to 2^m; folding partials is
-// associative up to rounding, and always runs in one order with explicit operations.
+// ---- folds. A partial of a head is (acc, m, l) with weights relative to 2^m (the weights that the warps add up are
+// 2^(score - reference + 10): m is the reference less 10, so that partials of other kernels mean the same); folding
+// partials is associative up to rounding, and always runs in one order with explicit operations.
 struct Part {
     float4 a;
     float m, l;
@@ -643,7 +644,7 @@ __device__ __forceinline__ bool await_inbox(unsigned bar, unsigned phase) {
 }
 
 // One float4 (item = head of the group * 64 + dims / 4) of the output: normalised (and gated), or
-// the raw triple of a shard, whose reference maximum leaves the weights' scale of 2^10 out.
+// the raw triple of a shard, in weights without the scale of 2^10.
 __device__ __forceinline__ void emit_item(const DecodeParams &p, int slot, int kvh, int group, int item,
                                           const Part &r) {
     const int h = kvh * group + (item >> 6), j = item & 63;

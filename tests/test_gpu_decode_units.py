@@ -1,5 +1,6 @@
 """Decode at the edges of the default body's work units: a warp takes 16 rows, or 32 once a step has
 more 16-row units than warps; 8 warps per CTA, two CTAs per run. CPU definition: ops.rs:449-518."""
+import math
 import re
 
 import numpy as np
@@ -267,6 +268,73 @@ def test_columns_of_every_form_give_each_columns_own_bits(pos0, cols, splits, fo
         api.attn_decode_kv(step, q[c], kc, vc, acc, ml, one, heads, n_kv, hd, stride, scale, splits)
         assert torch.equal(one, out[c]), f"column {c}"
     assert api.check_device_status() == 0
+
+
+def _quantised_cache(gen, rows, stride, n_kv, dtype, room=0):
+    """K and V bytes of `rows` random rows per head (NaN scales past them), and the rows as f64 [rows][n_kv * 256]."""
+    from hipml_b200 import api
+    row = (272, 144)[dtype]
+    kc, vc = (torch.full((n_kv * stride * row + room,), 0x7E, dtype=torch.uint8, device="cuda") for _ in range(2))
+    if rows:
+        k, v = (torch.randn(rows, n_kv * 256, device="cuda", generator=gen) for _ in range(2))
+        api.kv_encode_bulk(k, v, kc, vc, n_kv, 256, stride, 0, 0, rows, dtype)
+    deq = (O.dequantize_q8, O.dequantize_q4)[dtype]
+    return kc, vc, [torch.from_numpy(cases.unpack_head_major(
+        deq(np.ascontiguousarray(c[:n_kv * stride * row].cpu().numpy().reshape(n_kv, stride, row)[:, :rows])), n_kv, rows,
+        256)).double().cuda() for c in (kc, vc)]
+
+
+def _triple(q, k, v, n_kv, scale):
+    """log2 of the sum of 2^score per head, and the attention output [heads][256], in f64."""
+    group = q.numel() // 256 // n_kv
+    s = torch.einsum("hgd,nhd->hgn", q.double().view(n_kv, group, 256), k.view(-1, n_kv, 256)) * scale
+    out = torch.einsum("hgn,nhd->hgd", s.softmax(-1), v.view(-1, n_kv, 256))
+    return s.logsumexp(-1).flatten() / math.log(2.0), out.reshape(n_kv * group, 256)
+
+
+# every body of the head_dim-256 kernel: one run, several, a head in one cluster
+@pytest.mark.parametrize("selector", [0, 1, 6, 7, 8])
+@pytest.mark.parametrize("seq", [1, 40, 700, 5000])
+def test_a_shard_s_triple_is_its_sum_of_weights(seq, selector):
+    """acc * 2^max and sum * 2^max are the sums over the rows, whichever body made them: a caller folds them with others."""
+    from hipml_b200 import api
+    heads, n_kv, hd, scale = 24, 4, 256, 0.0625
+    gen = torch.Generator(device="cuda").manual_seed(seq)
+    kc, vc, (k, v) = _quantised_cache(gen, seq, seq + 3, n_kv, int(selector == 1))
+    q = torch.randn(heads * hd, device="cuda", generator=gen)
+    splits = api.decode_splits(seq)
+    acc, ml = (torch.full((heads * splits * n,), float("nan"), device="cuda") for n in (hd, 2))
+    got = torch.full((heads, hd + 2), float("nan"), device="cuda")
+    step = torch.tensor([seq - 1, seq] + [0] * 6, dtype=torch.int32, device="cuda")
+    api.attn_decode_kv_shard(step, q, kc, vc, acc, ml, got, heads, n_kv, hd, seq + 3, scale, splits, selector=selector)
+    assert api.check_device_status() == 0
+    total, out = _triple(q, k, v, n_kv, scale)
+    got = got.double()
+    # (a sum is good to 1e-5, the bar of decode: 1.5e-5 of its logarithm; f32 holds a maximum of up to 32 to 4e-6)
+    assert (got[:, hd] + got[:, hd + 1].log2() - total).abs().max() <= 2e-5
+    assert _close(got[:, :hd] / got[:, hd + 1:], out)
+
+
+def test_shards_of_different_bodies_fold_to_the_whole_cache():
+    from hipml_b200 import api
+    heads, n_kv, hd, scale = 24, 4, 256, 0.0625
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    q = torch.randn(heads * hd, device="cuda", generator=gen)
+    parts = [(0, 0, 700), (6, 0, 300), (8, 0, 900), (1, 1, 500), (7, 0, 20)]
+    gathered = torch.full((len(parts), heads, hd + 2), float("nan"), device="cuda")
+    keys, values = [], []
+    for i, (selector, dtype, n) in enumerate(parts):
+        kc, vc, (k, v) = _quantised_cache(gen, n, n, n_kv, dtype)
+        keys.append(k)
+        values.append(v)
+        splits = api.decode_splits(n)
+        acc, ml = (torch.full((heads * splits * m,), float("nan"), device="cuda") for m in (hd, 2))
+        step = torch.tensor([n - 1, n] + [0] * 6, dtype=torch.int32, device="cuda")
+        api.attn_decode_kv_shard(step, q, kc, vc, acc, ml, gathered[i], heads, n_kv, hd, n, scale, splits, selector=selector)
+    out = torch.full((heads, hd), float("nan"), device="cuda")
+    api.attn_decode_combine(gathered, out, heads, hd, len(parts))
+    assert api.check_device_status() == 0
+    assert _close(out, _triple(q, torch.cat(keys), torch.cat(values), n_kv, scale)[1])
 
 
 # heads packed into one to four tiles of eight, full and not, columns across a tile's end; five and more columns a group
