@@ -181,8 +181,6 @@ static int decode_kv(hipml_stream_t stream, const int *step, int selector, const
     p.kv_slot_bytes = p.acc_slot = p.ml_slot = p.q_slot = 0;
     if (tensor_core && ((reinterpret_cast<size_t>(p.k) | reinterpret_cast<size_t>(p.v)) & 15) != 0)
         return fail(HIPML_ERR_INVALID_ARGUMENT, "the KV cache must be 16-byte aligned");
-    // (a shard's scratch on an 8-byte boundary only: the split pass stores 16 bytes at a time)
-    if (shard && !xch && (reinterpret_cast<size_t>(part_acc) & 15) != 0) tensor_core = false;
     if (tensor_core && (reinterpret_cast<size_t>(q) & 7) != 0)
         return fail(HIPML_ERR_INVALID_ARGUMENT, "the query row must be 8-byte aligned");
     if (k_row) {
@@ -193,6 +191,10 @@ static int decode_kv(hipml_stream_t stream, const int *step, int selector, const
         p.vw = const_cast<unsigned char *>(p.v);
         p.row_slot = 0;
     }
+    // A shard's scratch may lie on any 8 bytes, as its rows do; the split pass that folds its own partials stores 16 at a
+    // time, the one whose partials are folded by a launch of their own stores floats (8,192 rows: 10.0 and 16.8 us; by the
+    // scalar body 86).
+    bool fold_launch = !tensor_core;
     if (tensor_core) {
         // one launch: the split pass folds its own partials (and runs the exchange)
         const size_t align = reinterpret_cast<size_t>(out) | reinterpret_cast<size_t>(gate) |
@@ -201,6 +203,10 @@ static int decode_kv(hipml_stream_t stream, const int *step, int selector, const
             return fail(HIPML_ERR_INVALID_ARGUMENT, "out, gate and part_acc must be 16-byte aligned");
         if ((reinterpret_cast<size_t>(part_ml) & 7) != 0)
             return fail(HIPML_ERR_INVALID_ARGUMENT, "part_ml must be 8-byte aligned");
+        fold_launch = (reinterpret_cast<size_t>(part_acc) & 15) != 0;
+        if (fold_launch) p.run_cap = 0;   // (every slot is written: that fold reads all `splits`)
+    }
+    if (!fold_launch) {
         p.out = out;
         p.out_slot = 0;
         p.out_head_stride = (shard && !xch) ? head_dim + 2 : head_dim;
@@ -236,7 +242,7 @@ static int decode_kv(hipml_stream_t stream, const int *step, int selector, const
     if (xch)
         return fail(HIPML_ERR_INVALID_ARGUMENT,
                     "exchange: only the head_dim 256 kernel (selectors 0, 1, 4) publishes to peers");
-    if (int e = launch_decode_split(as_stream(stream), p, 1, false)) return e;
+    if (int e = launch_decode_split(as_stream(stream), p, 1, tensor_core)) return e;
     if (!shard)
         return launch_decode_reduce(as_stream(stream), part_acc, part_ml, out, n_heads, head_dim,
                                     splits, 1, 0, 0, 0, gate);

@@ -304,7 +304,8 @@ int hipml_attn_front_append_q8(hipml_stream_t stream, const float *qg, const flo
  * output it writes the folded triple of its shard: shard_out f32 [n_heads][head_dim + 2] =
  * (unnormalised acc[head_dim], max in log2 units, sum). The shards' rows are exchanged with any
  * all-gather (NCCL) into gathered f32 [shards][n_heads][head_dim + 2], and
- * hipml_attn_decode_combine folds them into out f32 [n_heads][head_dim]. */
+ * hipml_attn_decode_combine folds them into out f32 [n_heads][head_dim]. shard_out and the scratch
+ * may lie on any 8 bytes; with part_acc on 16 the local fold is part of the same launch. */
 int hipml_attn_decode_kv_shard(hipml_stream_t stream, const int *step, int selector,
                                const float *q, const void *k, const void *v, float *part_acc,
                                float *part_ml, float *shard_out, int n_heads, int n_kv,
