@@ -22,7 +22,7 @@ namespace {
 
 __device__ __forceinline__ void split_range(const DecodeParams &p, int slot, int split, int &lo,
                                             int &hi) {
-    const int len = p.len[slot * p.len_stride + p.len_offset];
+    const int len = live_len(p, p.len[slot * p.len_stride + p.len_offset]);
     const int span = p.by_stride ? p.stride : len;
     const int per = (span + p.splits - 1) / p.splits;
     lo = min(split * per, len);

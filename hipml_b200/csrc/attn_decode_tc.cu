@@ -80,7 +80,7 @@ __device__ __forceinline__ int live_runs(const DecodeParams &p, int slot, int qu
 }
 __device__ __forceinline__ void split_range(const DecodeParams &p, int slot, int split, int quota,
                                             int &lo, int &hi) {
-    const int len = p.len[slot * p.len_stride + p.len_offset];
+    const int len = live_len(p, p.len[slot * p.len_stride + p.len_offset]);
     const RunPlan plan = plan_runs(p.len, p.len_stride, p.len_offset, slot, p.splits,
                                    p.by_stride ? 0 : p.run_cap, p.share_slots, quota);
     if (plan.runs >= 0) {
@@ -88,7 +88,8 @@ __device__ __forceinline__ void split_range(const DecodeParams &p, int slot, int
             lo = hi = len;
             return;
         }
-        lo = (int)((long long)split * plan.tiles / plan.runs) * kTile;
+        // (the tiles are counted before the length is bounded by the cache: runs past it are empty)
+        lo = min((int)((long long)split * plan.tiles / plan.runs) * kTile, len);
         hi = min((int)((long long)(split + 1) * plan.tiles / plan.runs) * kTile, len);
         return;
     }
@@ -395,7 +396,7 @@ attn_decode_kv_i8(const __grid_constant__ CUtensorMap vmap, int v3d, DecodeParam
     if (p.k_row != nullptr) {
         append_pos = p.len[slot * p.len_stride + p.len_offset - 1];
         if (split == 0 && kvh == 0 && tid == 0 &&
-            append_pos != p.len[slot * p.len_stride + p.len_offset] - 1 && status)
+            append_pos != live_len(p, p.len[slot * p.len_stride + p.len_offset]) - 1 && status)
             atomicCAS(status, 0, 22);
     }
     const unsigned bar_k = smem_u32(smem + kOffBar), bar_v = bar_k + 16, bar_mma = bar_k + 40;

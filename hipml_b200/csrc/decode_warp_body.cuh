@@ -789,9 +789,6 @@ struct Work {
 
 __device__ __forceinline__ int div_up(int a, int b) { return (a + b - 1) / b; }
 
-// A live length as the plans take it: none reaches past the rows that the cache has for a head.
-__device__ __forceinline__ int live_len(const DecodeParams &p, int n) { return min(max(n, 0), p.stride); }
-
 // The balanced plan of one stream: every warp of every run gets a unit before any gets two, and units
 // are 16 rows as long as one each is enough (half the latency of a short step), then 32 (an eighth
 // fewer instructions per row). Units are counted in eights, so that neighbouring columns of a stream

@@ -60,6 +60,10 @@ struct DecodeParams {
         int by_head = 0;
     } xch;
 };
+#ifdef __CUDACC__
+// A live length as the bodies take it: none reaches past the rows that the cache has for a head.
+__device__ __forceinline__ int live_len(const DecodeParams &p, int n) { return min(max(n, 0), p.stride); }
+#endif
 // Live runs of one slot in the tensor-core split pass, in 64-key tiles: `runs` runs deal the
 // slot's `tiles` tiles out to within one tile (run i covers tiles [i*tiles/runs,
 // (i+1)*tiles/runs)). Single stream: min(splits, tiles, run_cap). Several slots sharing the

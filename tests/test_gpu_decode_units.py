@@ -209,6 +209,49 @@ def test_a_length_past_the_cache_counts_as_the_cache_s(entry, fold_mode):
             assert _close(out[s], _attend(q[s], kq[:n], vq[:n], n_kv, hd, scale)), f"row {s}"
 
 
+@pytest.mark.parametrize("entry,selector,hd", [("step", 6, 256), ("step", 6, 64), ("step", 0, 64), ("step", 1, 64),
+                                               ("step", 8, 256), ("append", 8, 256), ("slots", 0, 64), ("slots", 1, 64),
+                                               ("shared slots", 8, 256)])
+def test_a_length_past_the_cache_counts_as_the_cache_s_in_every_body(entry, selector, hd):
+    """The scalar body (any head size) and the tcgen05 one: as the default one in the test above."""
+    from hipml_b200 import api
+    heads, n_kv, scale, stride, beyond, slots = 12, 2, 0.0625, 300, 200, 2
+    dtype = int(selector == 1)
+    row = (34, 18)[dtype] * hd // 32
+    gen = torch.Generator(device="cuda").manual_seed(hd)
+    room = n_kv * stride * row + 1024 * 272   # (rows follow the last head: a kernel that went on would be seen and not fault)
+    kc, vc = (torch.full((slots, room), 0x7E, dtype=torch.uint8, device="cuda") for _ in range(2))
+    k, v = (torch.randn(stride, n_kv * hd, device="cuda", generator=gen) for _ in range(2))
+    for s in range(slots):
+        api.kv_encode_bulk(k, v, kc[s], vc[s], n_kv, hd, stride, 0, 0, stride, dtype)
+    before = kc.clone(), vc.clone()
+    live, deq = n_kv * stride * row, (O.dequantize_q8, O.dequantize_q4)[dtype]
+    kq, vq = (torch.from_numpy(cases.unpack_head_major(deq(c[0, :live].cpu().numpy().reshape(n_kv, stride, row)), n_kv, stride,
+                                                       hd)).cuda() for c in (kc, vc))
+    q = torch.randn(slots, heads * hd, device="cuda", generator=gen)
+    new = torch.randn(n_kv * hd, device="cuda", generator=gen)
+    splits = 8
+    acc, ml = (torch.full((slots * heads * splits * n,), float("nan"), device="cuda") for n in (hd, 2))
+    out = torch.full((slots, heads * hd), float("nan"), device="cuda")
+    pos = torch.tensor([[stride + beyond - 1, stride + beyond], [6, 7]], dtype=torch.int32, device="cuda")
+    args = (heads, n_kv, hd, stride, scale, splits)
+    try:
+        if entry == "step":
+            api.attn_decode_kv(pos[0], q[0], kc[0], vc[0], acc, ml, out[0], *args, selector=selector)
+        elif entry == "append":
+            api.attn_decode_kv_append(pos[0], new, new, q[0], kc[0], vc[0], acc, ml, out[0], *args, selector=selector)
+        else:
+            api.set_decode_body(2 if selector == 8 else 1)
+            api.attn_decode_rows(pos, q, kc, vc, acc, ml, out, *args, room, heads * splits * hd, heads * splits * 2,
+                                 heads * hd, slots, dtype=dtype)
+    finally:
+        api.set_decode_body(1)
+    assert _device_status() == (22 if entry == "append" else 0)
+    assert torch.equal(kc, before[0]) and torch.equal(vc, before[1])
+    for s, n in enumerate([stride, 7] if "slots" in entry else [stride]):
+        assert _close(out[s], _attend(q[s], kq[:n], vq[:n], n_kv, hd, scale)), f"row {s}"
+
+
 # columns whose lengths cross a 16- or 32-row unit, the change of the unit (4,608) or nothing
 @pytest.mark.parametrize("cols", [2, 4, 5, 8])
 @pytest.mark.parametrize("pos0", [0, 13, 29, 125, 200, 1278, 4604, 9214])
@@ -342,8 +385,6 @@ def test_shards_of_different_bodies_fold_to_the_whole_cache():
 @pytest.mark.parametrize("seq,stride", [(0, 5), (1, 1), (300, 300), (4700, 4710), (340, 300)])
 def test_a_shard_with_scratch_on_8_bytes_keeps_its_body(seq, stride, selector):
     from hipml_b200 import _lib, api
-    if selector == 8 and seq > stride:
-        pytest.skip("the tcgen05 body takes the length as it is given")
     heads, n_kv, hd, scale = 24, 4, 256, 0.0625
     gen = torch.Generator(device="cuda").manual_seed(seq)
     live = min(seq, stride)
