@@ -314,7 +314,7 @@ __device__ __forceinline__ void fold_slices(const ChunkTcParams &p, unsigned sta
         float den = ml.y * wt;
 #pragma unroll
         for (int o = kS / 2; o > 0; o /= 2) den += __shfl_xor_sync(0xffffffffu, den, o);
-        const float inv_of = den > 0.0f ? 1.0f / den : 0.0f;
+        const float inv_of = 1.0f / den;   // (0 only for a row without a finite score: 0 * infinity, not a number)
 #pragma unroll
         for (int j = 0; j < kR; j++) {
             float4 y[2] = {make_float4(0.0f, 0.0f, 0.0f, 0.0f), make_float4(0.0f, 0.0f, 0.0f, 0.0f)};
@@ -843,7 +843,8 @@ attn_chunk_tc(const __grid_constant__ CUtensorMap map_k_hi, const __grid_constan
         if (ok) {
             griddep_wait();   // (already satisfied unless the CTA had no key tiles to wait for)
             tc_fence_after();
-            const float inv = norm ? (l > 0.0f ? 1.0f / l : 0.0f) : 1.0f;
+            // (every row sees a key; where none of its scores is finite, O and l are 0 and the row is not a number)
+            const float inv = norm ? 1.0f / l : 1.0f;
 #pragma unroll 1
             for (int j = 0; j < 4; j++) {
                 if (n_tiles > 0) {

@@ -60,3 +60,30 @@ def test_chunk_form_follows_the_size(tokens, pos0, dtype):
     assert api.check_device_status() == 0
     ma = O.max_abs(got * torch.sigmoid(gate).cpu().numpy(), gated.cpu().numpy())
     assert ma <= 2e-5, ma
+
+
+# one slice written by bulk copies; read back through the gate; 2, 4 and 8 slices folded in a cluster
+@pytest.mark.parametrize("tokens,pos0", [(2048, 0), (301, 3001), (130, 1500), (37, 700)])
+def test_a_row_without_a_finite_score_is_not_a_number(tokens, pos0):
+    """Keys past the largest f16 overflow in the single-pass form. A row that sees one finite score has its value; one
+    whose scores are all -infinity has no softmax, and says so."""
+    from hipml_b200 import api
+    heads, n_kv, hd = 24, 4, 256
+    seq, cap = pos0 + tokens, (pos0 + tokens + 127) // 128 * 128
+    gen = torch.Generator(device="cuda").manual_seed(seq)
+    k = torch.full((seq, n_kv * hd), 1e5, device="cuda")
+    k[0, 2 * hd:] = 0.0   # (KV heads 2 and 3: the first key is finite)
+    v = torch.randn(seq, n_kv * hd, device="cuda", generator=gen)
+    q = -1.0 - torch.rand(tokens, heads * hd, device="cuda", generator=gen)
+    gate = torch.randn(tokens, heads * hd, device="cuda", generator=gen)
+    ws = torch.full((api.attn_chunk_workspace_bytes(n_kv, hd, 0, cap),), 0x7E, dtype=torch.uint8, device="cuda")
+    api.attn_chunk_stage(k, v, n_kv, hd, 0, seq, 0, seq, cap, ws)
+    out, gated = (torch.full((tokens, heads * hd), 3.0, device="cuda") for _ in range(2))
+    api.attn_chunk_staged(q, out, heads, n_kv, hd, pos0, tokens, cap, ws, mode=1)
+    api.attn_chunk_staged_gated(q, gated, gate, heads, n_kv, hd, pos0, tokens, cap, ws, mode=1)
+    assert api.check_device_status() == 0
+    want = v[0].view(n_kv, 1, hd)[2:].expand(2, heads // n_kv, hd).reshape(-1)   # (f16 values: half a unit in 2^-11)
+    half = heads * hd // 2
+    for got, scale in ((out, torch.ones_like(gate)), (gated, torch.sigmoid(gate))):
+        assert torch.isnan(got[:, :half]).all()
+        assert ((got[:, half:] - want * scale[:, half:]).abs() <= 5e-4 * want.abs() + 1e-6).all()
