@@ -87,3 +87,34 @@ def test_a_row_without_a_finite_score_is_not_a_number(tokens, pos0):
     for got, scale in ((out, torch.ones_like(gate)), (gated, torch.sigmoid(gate))):
         assert torch.isnan(got[:, :half]).all()
         assert ((got[:, half:] - want * scale[:, half:]).abs() <= 5e-4 * want.abs() + 1e-6).all()
+
+
+# rows_live is 126 and 6 (21 queries of six heads, one left over) or 128 and 96: rows in fours, and a remainder
+@pytest.mark.parametrize("heads,n_kv,tokens", [(24, 4, 1996), (32, 4, 2044)], ids=["group6", "group8"])
+def test_gated_rows_that_were_also_moved_to_memory(heads, n_kv, tokens):
+    """More than 64 key tiles in one slice: part of a row is in memory when it is read out, and the gate with it."""
+    from hipml_b200 import api
+    hd, pos0 = 256, 9000
+    seq, cap = pos0 + tokens, (pos0 + tokens + 127) // 128 * 128
+    gen = torch.Generator(device="cuda").manual_seed(tokens)
+    kc, vc = (torch.zeros(n_kv * seq * 272, dtype=torch.uint8, device="cuda") for _ in range(2))
+    k, v = (torch.randn(seq, n_kv * hd, device="cuda", generator=gen) for _ in range(2))
+    api.kv_encode_bulk(k, v, kc, vc, n_kv, hd, seq, 0, 0, seq)
+    q, gate = (torch.randn(tokens, heads * hd, device="cuda", generator=gen) for _ in range(2))
+    ws = torch.full((api.attn_chunk_workspace_bytes(n_kv, hd, 0, cap),), 0x7E, dtype=torch.uint8, device="cuda")
+    api.attn_chunk_stage(kc, vc, n_kv, hd, 1, seq, 0, seq, cap, ws)
+    plain, gated = (torch.full((tokens, heads * hd), float("nan"), device="cuda") for _ in range(2))
+    api.attn_chunk_staged(q, plain, heads, n_kv, hd, pos0, tokens, cap, ws)
+    api.attn_chunk_staged_gated(q, gated, 2.0 * gate, heads, n_kv, hd, pos0, tokens, cap, ws)
+    assert api.check_device_status() == 0
+    assert torch.isfinite(plain).all()
+    want = plain.double() * torch.sigmoid(2.0 * gate.double())
+    # (the attention's bits are the ungated call's; expf, a sum, a division and a product: four roundings and expf's two)
+    assert ((gated.double() - want).abs() <= 4e-7 * want.abs() + 1e-30).all()
+    for t in (0, 20, 21, tokens - 2, tokens - 1):   # and against the definition
+        n = pos0 + t + 1
+        kq, vq = (cases.unpack_head_major(O.dequantize_q8(np.ascontiguousarray(
+            c.cpu().numpy().reshape(n_kv, seq, 272)[:, :n])), n_kv, n, hd) for c in (kc, vc))
+        ok, ma, rl = cases.attention_within_bar(
+            O.attn_causal_f32(q[t].cpu().numpy(), kq, vq, heads, n_kv, hd, n, 0.0625), plain[t].cpu().numpy())
+        assert ok and rl <= 5e-5, (t, ma, rl)

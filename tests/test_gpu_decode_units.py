@@ -151,6 +151,51 @@ def test_lengths_that_change_between_launches_are_seen():
         assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("cols", [2, 5, 8])
+def test_column_lengths_that_change_between_launches_are_seen(cols):
+    """The columns are grouped and planned from the lengths as they stand before the grids ahead are done; lengths written
+    by the kernel right before must win: other units, runs, groups and tiles of heads."""
+    from hipml_b200 import api
+    heads, n_kv, hd, scale, stride = 24, 4, 256, 0.0625, 6000
+    gen = torch.Generator(device="cuda").manual_seed(6)
+    kc, vc = (torch.zeros(n_kv * stride * 272, dtype=torch.uint8, device="cuda") for _ in range(2))
+    k, v = (torch.randn(stride, n_kv * hd, device="cuda", generator=gen) for _ in range(2))
+    api.kv_encode_bulk(k, v, kc, vc, n_kv, hd, stride, 0, 0, stride)
+    q = torch.randn(cols, heads * hd, device="cuda", generator=gen)
+    splits = api.decode_splits(stride)
+    acc, ml = (torch.empty(cols * heads * splits * n, device="cuda") for n in (hd, 2))
+    args = (heads, n_kv, hd, stride, scale, splits, cols, heads * splits * hd, heads * splits * 2, heads * hd)
+    # neighbours of one plan; across the change of the unit (4,608); every column its own plan; empty ones among them
+    sets = [[1 + c for c in range(cols)], [5000 + c for c in range(cols)], [700 + c for c in range(cols)],
+            [4607 + c for c in range(cols)], [100 + 733 * c for c in range(cols)], [(c % 2) * 5990 + c for c in range(cols)],
+            [300 + c // 2 for c in range(cols)]]
+    tables = [torch.tensor([[n - 1, n] for n in s], dtype=torch.int32, device="cuda") for s in sets]
+
+    def attend(pos):
+        out = torch.full((cols, heads * hd), float("nan"), device="cuda")
+        api.attn_decode_cols(pos, q, kc, vc, acc, ml, out, *args)
+        return out
+
+    want = []
+    for t in tables:
+        attend(t)
+        want.append(attend(t))
+        torch.cuda.synchronize()
+    moving, outs = tables[-1].clone(), []
+    for t in tables:
+        moving.copy_(t)
+        outs.append(attend(moving))
+    assert api.check_device_status() == 0
+    for s, a, b in zip(sets, outs, want):
+        assert torch.isfinite(a).all() and torch.equal(a, b), s
+    kq, vq = (torch.from_numpy(cases.unpack_head_major(O.dequantize_q8(c.cpu().numpy().reshape(n_kv, stride, 272)), n_kv,
+                                                       stride, hd)).cuda() for c in (kc, vc))
+    for s, a in zip(sets, outs):
+        for c, n in enumerate(s):
+            if n:
+                assert _close(a[c], _attend(q[c], kq[:n], vq[:n], n_kv, hd, scale)), (s, c)
+
+
 def _device_status():
     from hipml_b200 import _lib, api
     try:
