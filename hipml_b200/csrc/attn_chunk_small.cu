@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(kThreads, 2) attn_chunk_small(SmallParams p) {
             make_float4(st.acc[h][4], st.acc[h][5], st.acc[h][6], st.acc[h][7]);
     }
     __syncthreads();
-    fold_warps(smem, 8 * kHeadPitch * 4, s_ml, group * 64, tid, [&](int item, const Part &r) {
+    fold_warps(smem, 8 * kHeadPitch * 4, s_ml, group * 64, [&](int item, const Part &r) {
         float4 y;
         y.x = __fdiv_rn(r.a.x, r.l);
         y.y = __fdiv_rn(r.a.y, r.l);

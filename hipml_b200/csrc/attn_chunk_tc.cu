@@ -149,13 +149,6 @@ __device__ __forceinline__ void split_half2(float a, float b, unsigned &hi, unsi
     lo = *reinterpret_cast<const unsigned *>(&l);
 }
 
-// 2^x; results below the smallest normal number are 0.
-__device__ __forceinline__ float ex2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
 // Dequantised (or copied) values of 8 consecutive dims of one cache row; zeros past n_keys.
 __device__ __forceinline__ void stage_fetch(const StageParams &p, const void *cache, int kvh,
                                             int key, int d0, float (&x)[8]) {

@@ -55,9 +55,9 @@ struct Cfg {
 __device__ int g_arrive_cols[kArriveRegions * kArriveRegionInts];
 
 // Which columns a cluster takes. Neighbouring columns with the same plan (the same units for every warp), at
-// most `each` of them (as many as fit the tiles, in groups of one size), are a group; a cluster has run `run` of groups `group`, `group` + `hop`, ... Groups go
-// to clusters of their own while a head has clusters to spare for their runs, and columns share conversions
-// beyond (4 columns of 300 rows take 2 runs each: 8 clusters of the head's 18; of 8,192 rows 17: one cluster
+// most `each` of them (as many as fit the tiles, in groups of one size), are a group; a cluster has run `run` of
+// groups `group`, `group` + `hop`, ... Groups go to clusters of their own while a head has clusters to spare for their
+// runs, and columns share conversions beyond (4 columns of 300 rows take 2 runs each: 8 clusters of the head's 18; of 8,192 rows 17: one cluster
 // per run takes all four). `cap`: the clusters of a head; what its groups do not need ends at once, so there is one
 // round of them and they take the groups in turn.
 struct Share {
@@ -449,7 +449,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_decode_cols(DecodeParams p, 
             __syncthreads();
 #pragma unroll 1
             for (int a = a0; a < a1; a++)
-                fold_warps(smem + (a - a0) * C::kPartial, C::kRing, wml + 8 * a * kWarps, min(8, heads - 8 * a) * 64, tid,
+                fold_warps(smem + (a - a0) * C::kPartial, C::kRing, wml + 8 * a * kWarps, min(8, heads - 8 * a) * 64,
                            [&](int item, const Part &r) {
                                cpart[a * 512 + item] = r.a;
                                if ((item & 63) == 0) cml[a * 8 + (item >> 6)] = make_float2(r.m, r.l);
@@ -494,9 +494,9 @@ __global__ void __launch_bounds__(kThreads, 1) attn_decode_cols(DecodeParams p, 
             for (int s = 0; s < n; s++)
                 if (s_last[s]) {
                     if constexpr (kC == 2)
-                        fold_runs<kC, 1, 18>(p, base + column(s), 1, kvh, group, w.runs, rank, nullptr);
+                        fold_runs<kC, 18>(p, base + column(s), kvh, group, w.runs, rank, nullptr);
                     else
-                        fold_runs<kC, 1, 8>(p, base + column(s), 1, kvh, group, w.runs, rank, nullptr);
+                        fold_runs<kC, 8>(p, base + column(s), kvh, group, w.runs, rank, nullptr);
                 }
         }
         cluster_wait();

@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(kThreads, 2) attn_decode_rows_f32(ColsParams p
     __syncthreads();
     float4 *const inbox = reinterpret_cast<float4 *>(smem + kOffInF32);
     float2 *const inbox_ml = reinterpret_cast<float2 *>(smem + kOffInMlF32);
-    fold_warps(smem, 8 * kHeadPitch * 4, wml, items, tid, [&](int item, const Part &r) {
+    fold_warps(smem, 8 * kHeadPitch * 4, wml, items, [&](int item, const Part &r) {
         send_item<kC>(inbox, inbox_ml, bar_in, items, rank, item, r);
     });
     if (!await_inbox(bar_in, 0) && status) atomicCAS(status, 0, 21);
@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(kThreads, 2) attn_decode_rows_f32(ColsParams p
             s_last = last;
         }
         __syncthreads();
-        if (s_last) fold_runs<kC, 1, 8>(d, col, 1, kvh, group, clusters, rank, nullptr);
+        if (s_last) fold_runs<kC, 8>(d, col, kvh, group, clusters, rank, nullptr);
     }
 }
 

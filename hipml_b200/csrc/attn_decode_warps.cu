@@ -470,7 +470,7 @@ __global__ void __launch_bounds__(kThreads, kWide ? 1 : 2) attn_decode_warps(Dec
     };
     float4 *const inbox = reinterpret_cast<float4 *>(smem + C::kOffIn);
     float2 *const inbox_ml = reinterpret_cast<float2 *>(smem + C::kOffInMl);
-    fold_warps(smem, C::kRing, wml, items, tid, [&](int item, const Part &r) {
+    fold_warps(smem, C::kRing, wml, items, [&](int item, const Part &r) {
         if constexpr (kC > 1)
             send_item<kC>(inbox, inbox_ml, bar_in, items, rank, item, r);
         else
@@ -497,10 +497,10 @@ __global__ void __launch_bounds__(kThreads, kWide ? 1 : 2) attn_decode_warps(Dec
                 // (in a cluster a CTA has half a head group's items or less: ordinary loads, one trip for the runs of a
                 // deep stream, are as fast for 17 runs, 137 us against 141 for 16 layers of 3,000 rows)
                 if constexpr (kC > 1)
-                    fold_runs<kC, 1, 18>(p, w.slot, 1, w.kvh, group, w.runs, rank, nullptr);
+                    fold_runs<kC, 18>(p, w.slot, w.kvh, group, w.runs, rank, nullptr);
                 else if (!fold_runs_staged(p, w.slot, w.kvh, group, w.runs, smem, kWarps * C::kRing, bar_fold,
                                            reinterpret_cast<float2(*)[kStagedRow]>(smem + C::kOffQ), landed))
-                    fold_runs<kC, 1, 8>(p, w.slot, 1, w.kvh, group, w.runs, rank, nullptr);
+                    fold_runs<kC, 8>(p, w.slot, w.kvh, group, w.runs, rank, nullptr);
             }
         } else {
             // the exchange wants whole heads in one CTA: the cluster arrives as one
@@ -519,7 +519,7 @@ __global__ void __launch_bounds__(kThreads, kWide ? 1 : 2) attn_decode_warps(Dec
                 __syncthreads();
                 if (s_plan[0]) {
                     float *const staged = reinterpret_cast<float *>(smem);
-                    for (int r = 0; r < kC; r++) fold_runs<kC, 1, 8>(p, w.slot, 1, w.kvh, group, w.runs, r, staged);
+                    for (int r = 0; r < kC; r++) fold_runs<kC, 8>(p, w.slot, w.kvh, group, w.runs, r, staged);
                     __syncthreads();
                     FoldAcc f;
                     if (warp < group) {
@@ -568,10 +568,10 @@ __global__ void __launch_bounds__(kThreads) attn_decode_warps_fold(DecodeParams 
         runs = balance(p, len, kC, kUnitRows).runs;
     }
     if (!exchange) {
-        fold_runs<kC, 1, kBatch>(p, slot, 1, kvh, group, runs, slice, nullptr, slices);
+        fold_runs<kC, kBatch>(p, slot, kvh, group, runs, slice, nullptr, slices);
         return;
     }
-    for (int r = 0; r < kC; r++) fold_runs<kC, 1, 8>(p, slot, 1, kvh, group, runs, r, staged);
+    for (int r = 0; r < kC; r++) fold_runs<kC, 8>(p, slot, kvh, group, runs, r, staged);
     __syncthreads();
     FoldAcc f;
     if (warp < group) {

@@ -46,14 +46,23 @@ __device__ __forceinline__ void griddep_launch() {
 __device__ __forceinline__ void griddep_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
-// Asks L2 for `bytes` from `src` on, as far as they are whole pieces of 16 from a 16-byte boundary; touches nothing.
+// Asks L2 for `bytes` (a multiple of 16, 16-byte aligned); touches nothing of this CTA.
+__device__ __forceinline__ void prefetch_l2(const void *src, unsigned bytes) {
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
+}
+// The same for any `bytes` from any `src` on, as far as they are whole pieces of 16 from a 16-byte boundary.
 // Inputs that no kernel has just written come from memory, and a launch whose rows are on their way while it waits
 // for the grids ahead has that trip behind it.
 __device__ __forceinline__ void ask_l2(const void *src, long long bytes) {
     const size_t from = (reinterpret_cast<size_t>(src) + 15) & ~(size_t)15;
     const size_t to = (reinterpret_cast<size_t>(src) + (size_t)(bytes > 0 ? bytes : 0)) & ~(size_t)15;
-    if (to > from)
-        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(from), "r"((unsigned)(to - from)) : "memory");
+    if (to > from) prefetch_l2(reinterpret_cast<const void *>(from), (unsigned)(to - from));
+}
+// 2^x; results below the smallest normal number are 0.
+__device__ __forceinline__ float ex2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
 }
 #endif
 

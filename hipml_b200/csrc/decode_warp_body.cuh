@@ -28,11 +28,6 @@ constexpr float kMargin = 1.5f;
 constexpr int kNeutralSlots = 32;   // partial slots that are written whether or not a run of rows has them
 constexpr int kPrefetch = 2;   // units of K and of V a warp asks L2 for ahead of the grid dependency
 
-__device__ __forceinline__ float ex2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
 // Transpose of an 8 x 8 tile of f16 held one 32-bit pair per lane (row = lane / 4).
 __device__ __forceinline__ unsigned transpose8(unsigned x) {
     unsigned y;
@@ -468,47 +463,37 @@ __device__ __forceinline__ void fold_sources(int i0, int i1, Load load, Part (&r
     }
 }
 
-// The same for sources in memory, independent of the batch: the maximum first (from the {m, l} pairs alone
-// where there is more than one batch), then the sum in source order.
-template <int kPer, int kBatch, class LoadMl, class Load>
-__device__ __forceinline__ void fold_memory(int i0, int i1, LoadMl load_ml, Load load, Part (&r)[kPer]) {
-#pragma unroll
-    for (int j = 0; j < kPer; j++) {
-        r[j].a = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        r[j].m = -INFINITY;
-        r[j].l = 0.0f;
-    }
+// The same for the sources of one item in memory, independent of the batch: the maximum first (from the {m, l} pairs
+// alone where there is more than one batch), then the sum in source order.
+template <int kBatch, class LoadMl, class Load>
+__device__ __forceinline__ void fold_memory(int i0, int i1, LoadMl load_ml, Load load, Part &r) {
+    r.a = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    r.m = -INFINITY;
+    r.l = 0.0f;
     const bool one_batch = i1 - i0 <= kBatch;
     if (!one_batch) {
         for (int s0 = i0; s0 < i1; s0 += 16)
 #pragma unroll
             for (int i = 0; i < 16; i++)
-#pragma unroll
-                for (int j = 0; j < kPer; j++)
-                    if (s0 + i < i1) r[j].m = fmaxf(r[j].m, load_ml(s0 + i, j).x);
+                if (s0 + i < i1) r.m = fmaxf(r.m, load_ml(s0 + i).x);
     }
     for (int s0 = i0; s0 < i1; s0 += kBatch) {
-        float4 x[kPer][kBatch];
-        float2 ml[kPer][kBatch];
+        float4 x[kBatch];
+        float2 ml[kBatch];
 #pragma unroll
-        for (int i = 0; i < kBatch; i++)
-#pragma unroll
-            for (int j = 0; j < kPer; j++) {
-                x[j][i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                ml[j][i] = make_float2(-INFINITY, 0.0f);
-                if (s0 + i < i1) {
-                    x[j][i] = load(s0 + i, j);
-                    ml[j][i] = load_ml(s0 + i, j);
-                }
+        for (int i = 0; i < kBatch; i++) {
+            x[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            ml[i] = make_float2(-INFINITY, 0.0f);
+            if (s0 + i < i1) {
+                x[i] = load(s0 + i);
+                ml[i] = load_ml(s0 + i);
             }
-#pragma unroll
-        for (int j = 0; j < kPer; j++) {
-            if (one_batch)
-#pragma unroll
-                for (int i = 0; i < kBatch; i++) r[j].m = fmaxf(r[j].m, ml[j][i].x);
-#pragma unroll
-            for (int i = 0; i < kBatch; i++) add(r[j], x[j][i], ml[j][i]);
         }
+        if (one_batch)
+#pragma unroll
+            for (int i = 0; i < kBatch; i++) r.m = fmaxf(r.m, ml[i].x);
+#pragma unroll
+        for (int i = 0; i < kBatch; i++) add(r, x[i], ml[i]);
     }
 }
 
@@ -549,12 +534,12 @@ __device__ __forceinline__ void store_warp_partial(float *dst, const float (&acc
                         make_float2(acc[b][i][h], acc[b][i][2 + h]);
         }
 }
-// Folds the partials of eight warps (`pitch` bytes apart; ml: [8 heads][warp]) by 256 threads, of which this is number
-// `tid`; done(item, part).
+// Folds the partials of a CTA's warps (`pitch` bytes apart; ml: [8 heads][warp]); done(item, part).
 template <class Done>
 __device__ __forceinline__ void fold_warps(const unsigned char *partials, int pitch, const float2 *ml_at, int items,
-                                           int tid, Done done) {
+                                           Done done) {
     constexpr int kPer = 2;   // (at most 512 items)
+    const int tid = threadIdx.x;
     Part r[kPer];
     fold_sources<kPer, kWarps>(
         0, kWarps,
@@ -676,44 +661,31 @@ __device__ __forceinline__ void emit_item(const DecodeParams &p, int slot, int k
     }
 }
 
-// Folds the `runs` partials of slice `rank` of `slices` of a head group (of each of `cols` slots from `slot` on) from
-// memory and emits it (or, staged != nullptr, leaves it there: [8 heads][256] sums, then [8 heads]{max,
-// sum}). kPer items a thread, kBatch runs in one round trip: 18 for the runs of a deep stream (B200: 18 pairs
-// of SMs per KV head; three trips of 8 took 2.9 us at the end of every launch).
-template <int kC, int kPer, int kBatch>
-__device__ __forceinline__ void fold_runs(const DecodeParams &p, int slot, int cols, int kvh, int group, int runs,
-                                          int rank, float *staged, int slices = kC) {
+// Folds the `runs` partials of slice `rank` of `slices` of a slot's head group from memory and emits it (or, staged !=
+// nullptr, leaves it there: [8 heads][256] sums, then [8 heads]{max, sum}). kBatch runs in one round trip: 18 for the
+// runs of a deep stream (B200: 18 pairs of SMs per KV head; three trips of 8 took 2.9 us at the end of every launch).
+template <int kC, int kBatch>
+__device__ __forceinline__ void fold_runs(const DecodeParams &p, int slot, int kvh, int group, int runs, int rank,
+                                          float *staged, int slices = kC) {
     constexpr int kShare = Split<kC>::kShare;
     const int items = group * 64, first = items * rank / slices, count = items * (rank + 1) / slices - first;
-    const int part = threadIdx.x % kShare, total = cols * count;
-    for (int f0 = threadIdx.x / kShare; f0 - (int)threadIdx.x / kShare < total; f0 += kPer * (kThreads / kShare)) {
-        const float *pa[kPer], *pm[kPer];
-        int item[kPer], col[kPer];
-#pragma unroll
-        for (int j = 0; j < kPer; j++) {
-            const int f = min(f0 + j * (kThreads / kShare), total - 1);
-            col[j] = cols > 1 ? f / count : 0;
-            item[j] = first + f - col[j] * count;
-            const int head = kvh * group + (item[j] >> 6);
-            pa[j] = p.part_acc + (size_t)(slot + col[j]) * p.acc_slot + (size_t)head * p.splits * 256 + 4 * (item[j] & 63);
-            pm[j] = p.part_ml + (size_t)(slot + col[j]) * p.ml_slot + (size_t)head * p.splits * 2;
-        }
-        Part r[kPer];
-        fold_memory<kPer, kBatch>(
+    const int part = threadIdx.x % kShare, at = threadIdx.x / kShare;
+    for (int f0 = at; f0 - at < count; f0 += kThreads / kShare) {   // (whole rounds: the shares join by shuffles)
+        const int item = first + min(f0, count - 1), head = kvh * group + (item >> 6);
+        const float *const pa = p.part_acc + (size_t)slot * p.acc_slot + (size_t)head * p.splits * 256 + 4 * (item & 63);
+        const float *const pm = p.part_ml + (size_t)slot * p.ml_slot + (size_t)head * p.splits * 2;
+        Part r;
+        fold_memory<kBatch>(
             runs * part / kShare, runs * (part + 1) / kShare,
-            [&](int i, int j) { return __ldcg(reinterpret_cast<const float2 *>(pm[j]) + i); },
-            [&](int i, int j) { return __ldcg(reinterpret_cast<const float4 *>(pa[j] + (size_t)i * 256)); }, r);
-#pragma unroll
-        for (int j = 0; j < kPer; j++) {
-            join<kShare>(r[j]);
-            if (f0 + j * (kThreads / kShare) >= total || part != 0) continue;
-            if (staged) {
-                reinterpret_cast<float4 *>(staged)[item[j]] = r[j].a;
-                if ((item[j] & 63) == 0)
-                    reinterpret_cast<float2 *>(staged + 8 * 256)[item[j] >> 6] = make_float2(r[j].m, r[j].l);
-            } else {
-                emit_item(p, slot + col[j], kvh, group, item[j], r[j]);
-            }
+            [&](int i) { return __ldcg(reinterpret_cast<const float2 *>(pm) + i); },
+            [&](int i) { return __ldcg(reinterpret_cast<const float4 *>(pa + (size_t)i * 256)); }, r);
+        join<kShare>(r);
+        if (f0 >= count || part != 0) continue;
+        if (staged) {
+            reinterpret_cast<float4 *>(staged)[item] = r.a;
+            if ((item & 63) == 0) reinterpret_cast<float2 *>(staged + 8 * 256)[item >> 6] = make_float2(r.m, r.l);
+        } else {
+            emit_item(p, slot, kvh, group, item, r);
         }
     }
 }

@@ -98,10 +98,6 @@ __device__ __forceinline__ void cluster_wait() {
 __device__ __forceinline__ void mbar_inval(unsigned bar) {
     asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
 }
-// Asks L2 for `bytes` (a multiple of 16, 16-byte aligned); touches nothing of this CTA.
-__device__ __forceinline__ void prefetch_l2(const void *src, unsigned bytes) {
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
-}
 // Stores to another CTA's shared memory whose bytes are counted on a barrier of that CTA (both shared::cluster
 // addresses): the receiver waits on its own barrier and reads locally.
 __device__ __forceinline__ void st_async_f4(unsigned addr, const float4 &v, unsigned bar) {
