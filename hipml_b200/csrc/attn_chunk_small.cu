@@ -2,14 +2,14 @@
 //
 // CPU definition: crates/hipml-core/src/attention.rs:56-102 per query row with seq = pos0 + t + 1.
 //
-// The tensor-core path (attn_chunk_tc.cu) is two launches with ~13 us of fixed cost per CTA pair, however
+// The tensor-core path (attn_chunk_tc.cu) is two launches with ~10 us of fixed cost per CTA pair, however
 // short the chunk; a follow-up of a few dozen tokens to a short conversation is all latency there (37
-// tokens at position 29: 5 us of staging and 13 us of attention). Here a CTA of eight warps takes one
+// tokens at position 29: 19 us of staging and attention, here 8). Here a CTA of eight warps takes one
 // query token and KV head; a warp takes four keys at a time for all heads of the group, reads and
 // dequantises each row once, and sums the 24 dot products over the lanes by one reduce-scatter. Plain f32
-// products and sums. Bound by latency, 5.6 us per 100 keys, up to about a wave of CTAs, by the CUDA cores'
+// products and sums. Bound by latency, 5.4 us per 100 keys, up to about a wave of CTAs, by the CUDA cores'
 // FMA rate beyond; where either passes the tensor cores' time the dispatch goes back to them (small_chunk).
-// 37 tokens at 29 with their append: 26.2 -> 13.4 us.
+// 37 tokens at 29 with their append: 26.2 -> 12.4 us.
 #include "decode_rows_f32.cuh"
 #include "decode_warp_body.cuh"
 

@@ -1037,19 +1037,21 @@ static int fold_capacity(int slices) {
     return n;
 }
 
-// Query tile and key slices of a one-pass launch. A pair of CTAs walks its keys at ~4.5 us per 128-key tile
-// (the tensor cores' rate; a little faster while other SMs idle) behind ~13 us of its own, of which ~8 go
-// into moving its 2 x 126 query rows in and its output rows out (an SM moves ~30 B/ns). A launch with fewer
-// pairs than the device has SM pairs can therefore be shortened by slices of the keys, which fold in one
-// cluster (~3 us; 301 tokens at 3,001: 32 pairs, 26 tiles, 127 us in one), and by smaller query tiles. Those
-// shorten what a pair does before and after its walk, but more pairs slow each other down: two thirds of the
-// size gain ~1 us up to 48 pairs (240 tokens at 0: 23.0 us against 23.9; 300: 27.2, 28.3) and lose it beyond
-// (400 tokens at 0, 60 pairs: 35.0 against 32.6; 500, 72 pairs: 38.8, 34.2), so they are for launches that leave
-// a third of the places free; slices also take the size that fills the pairs a whole tile needs (64 tokens at
-// 2,000 in five slices: 39.2 us with tiles of 16, 40.5 of 21; one slice gains nothing from it). This takes the
-// shape that an estimate from those figures says is shortest, among those whose clusters all start together;
-// a slice stays below the 64 tiles where a pair would move its sums to memory. Launches of more pairs than
-// that keep whole tiles and one slice.
+// Query tile and key slices of a one-pass launch (times: launches of the attention alone in a row, 24 heads over 4).
+// Whole tiles in one slice take 10.5 us + 3.8 a 128-key tile while few pairs of CTAs run (37 tokens, 1 .. 110 tiles), 10 -
+// 11 us + 4.2 with 40 - 64 pairs. A launch with fewer pairs than the device has SM pairs can therefore be shortened by
+// slices of the keys, which fold in one cluster (two cost 3.6 us, four 4.8, eight 7; 301 tokens at 3,001: 32 pairs, 26
+// tiles, 111 us in one and 69 in two), and by smaller query tiles. Those shorten what a pair does before and after its
+// walk, but more pairs slow each other down: two thirds of the size gain ~1 us up to 48 pairs (200 tokens at 0: 17.7 us
+// against 19.0; 301: 21.9, 22.8) and nothing beyond (400, 60 pairs: 26.7, 27.6; 500, 72 pairs: 27.4, 27.2; 672, 96: 45.9,
+// 35.4), so they are for launches that leave a third of the places free; slices also take the size that fills the pairs a
+// whole tile needs (64 tokens at 2,000 in five slices: 31.5 us with tiles of 16, 32.7 of 21; one slice gains nothing from
+// it). This takes the shape that an estimate fitted to 3,350 such times (5 % rms, less what all shapes share) says is
+// shortest, among those whose clusters all start together; a slice stays below the 64 tiles where a pair would move its
+// sums to memory. Launches of more pairs than that keep whole tiles and one slice. Over 196 sizes with 1, 4 and 8 KV heads
+// and groups of four, six and eight the shape it takes is on average 1.0 % behind the best one, 163 times within 2 %; the
+// worst are 130 tokens at 0 (17.4 us, tiles of 16: 15.1) and 500 at 3,001 (128.6, 121.1), where the estimate does not see
+// that the last tiles of a KV head leave a pair half empty.
 struct ChunkShape {
     int qtile, fold;
 };
@@ -1068,9 +1070,9 @@ static ChunkShape chunk_shape(int tokens, int n_kv, int group, int key_tiles) {
         for (int qtile = least > smallest ? least : smallest; qtile <= full; qtile++) {
             const int pairs = pairs_of(qtile) * fold;
             if (qtile < full && pairs > few && (fold == 1 || pairs > pairs_of(full) * fold)) continue;
-            const float step = 3.1f + 0.022f * (float)pairs;
-            const float us = step * (float)((key_tiles + fold - 1) / fold) + 8.0f * (float)(qtile * group) / 126.0f +
-                             (fold > 1 ? 3.0f : 0.0f);
+            const float step = 3.7f + 0.01f * (float)pairs;
+            const float us = step * (float)((key_tiles + fold - 1) / fold) + 4.1f * (float)(qtile * group) / 126.0f +
+                             (fold > 1 ? 2.0f + 0.26f * (float)fold : 0.0f);
             if (us < best_us) {
                 best_us = us;
                 best = {qtile, fold};

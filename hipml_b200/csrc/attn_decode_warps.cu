@@ -24,8 +24,8 @@
 //     8 x 8 tiles, as an exact f16 high + low pair after multiplication with the block's scale; the
 //     codes are the A operand (16 dims x 16 keys), converted exactly (0x6400 | (code + 128) is
 //     1152 + code). 64 accumulators per lane hold all 256 dims x 8 heads.
-// What bounds it: long caches the HBM stream and the issue rate together (100,000 rows: 43 - 45 us a
-// layer in a captured chain = 4.85 - 5.04 TB/s, 33 us of it in the loop; 1,555 warp instructions per 32 rows of K and V, where 64-row
+// What bounds it: long caches the HBM stream and the issue rate together (100,000 rows: 42 - 45 us a
+// layer in a row = 4.85 - 5.15 TB/s, 33 us of it in the loop; 1,555 warp instructions per 32 rows of K and V, where 64-row
 // tiles with CTA barriers and softmax through shared memory took 2,370, 57 us a layer); short ones
 // the chain of dependent latencies (8,192 rows: 10.0 us, before 16).
 //
@@ -677,13 +677,14 @@ int launch_c(cudaStream_t stream, const DecodeParams &p, int slots) {
 // Which form. One stream (or columns of one) has ~37 SMs per KV head: clusters of two, wide (8,192 rows: 11.5 us
 // a layer while partials were still read, against 14.4 with two small CTAs per SM and 13.1 with clusters of four,
 // of which only 33 fit the device); clusters of eight up to the 1,023 rows that the engine's policy gives fewer than
-// 128 splits, where one holds a head and nothing is folded through memory (700 rows, launches in a row: 7.4 us, of four
-// 8.4, of two 8.0), while the device holds those of two launches (15: with eight KV heads the next launch waits for
-// this one, 10.5 us against 8.7 with pairs); of four up to 519 (300 rows: 6.4 us, of eight 7.0, of two 8.0; below ~200
-// rows pairs would be 0.5 us quicker still, but how long a stream is the host does not know from so few splits).
-// Several slots: no clusters, a head has too few CTAs to pair them; wide up to 28 (slot, head) pairs (4 KV
-// heads, 5 slots of 512 .. 3,000 rows: 14.9 us a layer against 16.5), beyond that the twice as fine runs of
-// the small CTAs balance better (8 slots of 512 .. 8,192: 24.6 us against 25.4, 10 slots 32.8 against 34.2).
+// 128 splits, where one holds a head and nothing is folded through memory (672 rows, launches in a row: 6.1 us, of four
+// 7.8, of two 7.8), while the device holds those of two launches (15: with eight KV heads the next launch waits for
+// this one, 11.3 us against 8.1 with pairs; with six, whose next launch finds room for one head in two, 7.3 against 7.8);
+// of four up to 519 (300 rows: 6.2 us, of eight 6.6, of two 7.7; at 100 rows pairs are as quick, 6.2 against 6.1).
+// Several slots: no clusters, a head has too few CTAs to pair them; wide up to 28 (slot, head) pairs (4 KV heads, 5
+// slots of 512 .. 3,000 rows: 14.3 us a layer against 14.6, 7 of 512 .. 8,192: 21.7, 25.7), beyond that the twice as fine
+// runs of the small CTAs balance better where the last fold is not the longer part (8 slots of 512 .. 8,192: 24.1 us
+// against 24.4, 16: 39.8, 41.6; 10: 28.1, 27.4).
 int launch_decode_warps(cudaStream_t stream, const DecodeParams &p, int slots) {
     const bool one_stream = !p.by_stride && p.run_cap >= 4 && p.share_slots == 0;
     if (one_stream)

@@ -323,7 +323,7 @@ __device__ __forceinline__ void load_v_q8(const unsigned *row, int g, VFrag &f) 
 // q4_0: the low (i = 0) and the high nibbles of code bytes 2g and 2g + 1 of each row. Both nibbles of a byte serve the
 // same lane, and its two bytes are a half word, so that a pair of rows is one word and a nibble of it one mask: ten
 // instructions for eight values and none to stitch a word across the scale, where a word a row with one nibble of each
-// byte took 14 and four more (30,000 rows: 19.2 -> 18.8 us a layer; two slots of up to 6,667: 13.9 -> 13.3).
+// byte took 14 and four more (30,000 rows: 19.2 -> 18.8 us a layer; two slots of up to 6,667: 13.5 -> 13.3).
 template <int M>
 __device__ __forceinline__ void load_v_q4(const unsigned *row, int g, VFrag &f) {
     using R = Row<true>;
@@ -578,8 +578,8 @@ __device__ __forceinline__ void fold_cluster(const float4 *cpart, const float2 *
 // Merge of a cluster, one column: every CTA sends each item of its partial to the CTA that folds it (slice r of
 // the items: CTA r) as soon as it has it, and that one waits on its own barrier and reads locally; none has to
 // stay for another's reads. (A barrier of the cluster, remote loads and another barrier were 0.9 us of the 8.3 us
-// that a layer of 672 rows takes, 0.7 of 14.9 with its front end at 8,192 rows, 0.6 of 12.6 over the f32 cache at
-// 2,048; four columns of 8,192 rows took 34.1 us a layer sent this way and 33.3 read.)
+// that a layer of 672 rows took, 0.7 of 14.9 with its front end at 8,192 rows, 0.6 of 12.6 over the f32 cache at
+// 2,048. Several columns, whose partials would need an inbox each, are read: fold_cluster.)
 // inbox: [kC sources][items / kC] float4, inbox_ml: [kC][8 heads]; kC divides 64. The receiver's barrier expects
 // inbox_bytes.
 template <int kC>

@@ -616,14 +616,15 @@ static int check_stage(const void *k_cache, const void *v_cache, int n_kv, int h
     return 0;
 }
 
-// Whether a one-pass chunk goes straight from the cache on the CUDA cores (attn_chunk_small.cu): the
-// tensor-core path has ~17 us of fixed latency and takes 21 - 28 us up to 1,024 keys. The small kernel is bound by
-// the walk of the last token's CTA, 4 us + 5.6 us per 100 keys (6.9 with groups of more than six), and from about a
-// wave of CTAs on by their number (tokens * n_kv: 2 us per 1,000 (query, key) pairs of 4 KV heads). 1 to 37 tokens
-// with 256 keys to see: 18.3 - 19.5 us against 21.2 - 23.2; with 384: 25.3 - 27.2 against 25.5 - 27.2; with 448, two key
-// slices there: 28.8 - 30.7 against 22.4 - 27.5; with 1,000, where pairs alone would let one token in, 59 against 24.
-// Groups of eight, 192 keys: 18.1 against 20.4, 256: 23 against 20.
-// 100 tokens at 0: 17 against 25; 64 at 128 (10,300 pairs): 22.4 against 23.5; 100 at 92: 31 against 23.
+// Whether a one-pass chunk goes straight from the cache on the CUDA cores (attn_chunk_small.cu): staging and attention on
+// the tensor cores take 16 - 19 us up to 128 keys and 20 - 27 up to 512 (q8_0, 24 heads over 4, calls in a row). The small
+// kernel is bound by the walk of the last token's CTA, 4 us + 5.4 us per 100 keys (f32 4.3, q4_0 5.7, groups of eight 7),
+// and from about a wave of CTAs on by their number (tokens * n_kv). 1 / 37 tokens with 256 keys to see: 18.0 / 18.8 us
+// against 19.9 / 22.5; with 384: 25.1 / 26.3 against 24.1 / 26.1; with 448, two key slices there: 28.6 / 29.7 against 22.4 /
+// 25.5. Groups of eight, 192 keys: 18.0 / 18.7 against 20.1 / 22.7, 256: 22.6 / 23.3 against 20.1 / 22.7. 64 tokens at 64:
+// 16.0 against 19.1; at 128 (10,272 pairs): 21.9 against 22.5; 100 at 28: 18.4 against 19.4, at 92: 30.1 against 22.5. The
+// lines are right on average, not everywhere: 37 tokens at 171 would be quicker here (16.2 against 22.6), and of 16, whose
+// launches in a row get in each other's way, 256 keys (23.1 against 22.6) and 384 (33.0, 26.5) there.
 static bool small_chunk(int n_heads, int n_kv, int pos0, int tokens) {
     const long long pairs = (long long)tokens * pos0 + (long long)tokens * (tokens + 1) / 2;
     return pos0 + tokens <= (n_heads > 6 * n_kv ? 208 : 384) && pairs * n_kv <= 26000;

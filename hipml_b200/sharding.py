@@ -96,10 +96,12 @@ def fold_triples(gathered: np.ndarray) -> np.ndarray:
     return out.astype(np.float32)
 
 
-# Cost model of one launch of the tensor-core chunk kernel (B200, measured with a per-CTA time
-# line): a CTA pair spends ~13 us outside its key-tile loop and 4.4 us per 128-key tile in it;
-# slicing the key axis adds a combine pass, the partials' round trip and a launch (~30 us).
-PAIR_FIXED_US, PAIR_STEP_US, SLICED_EXTRA_US = 13.0, 4.4, 30.0
+# Cost model of one launch of the tensor-core chunk kernel (B200): 11 us of a CTA pair's own and 4.5 us per 128-key tile
+# fit launches of 2,048 rows in one slice (1, 2 and 4 KV heads at 0 .. 30,720: 81 us .. 3.8 ms) within 8 % rms; slicing the
+# key axis adds a combine pass, the partials' round trip and a launch, ~30 us with one KV head (more with four, where 108 us
+# were seen). What it picks is on average 1.7 % behind the best of 1 .. 6 slices over these; most, 11 %, with four KV
+# heads at 14,336 (three slices 1.86 ms, one 1.67).
+PAIR_FIXED_US, PAIR_STEP_US, SLICED_EXTRA_US = 11.0, 4.5, 30.0
 
 
 def chunk_launch_estimate_us(chunk_rows: int, group: int, local_n_kv: int, pos0: int, slices: int,
@@ -135,7 +137,8 @@ def prefill_key_splits(chunk_rows: int, group: int, local_n_kv: int, sm_pairs: i
     position given the count comes from the cost model above instead: the first chunk of a
     prefill, whose query tiles see 1 - 16 key tiles, wants fewer slices than the later ones
     (measured, 2048 rows: one KV head 2 / 3 / 3 / 3 slices at positions 0 / 2048 / 4096 / 6144,
-    two KV heads 1 / 1 / 2 - 3 / 3, four KV heads 1 up to 8,192 keys; the model picks the same)."""
+    two KV heads 1 / 1 / 1 / 2, four KV heads 1 up to 8,192 keys; the model picks the same but
+    for two KV heads at 4096, 3 slices at 378 us against 346, and at 6144, 3 at 486 against 479)."""
     qtile = max(128 // group, 1)
     pairs = -(-(-(-chunk_rows // qtile)) // 2) * local_n_kv
     if pos0 is None:
@@ -144,8 +147,9 @@ def prefill_key_splits(chunk_rows: int, group: int, local_n_kv: int, sm_pairs: i
         return max(1, min(8, round(2 * sm_pairs / pairs)))
     # (deep chunks: the jobs are long and alike, so what matters is that jobs / SM pairs comes
     # out just under a whole number - 196, 98 or 49 pairs x 3 slices = 7.9, 4.0, 2.0 rounds;
-    # measured on the 100,000-token prefill: 302 -> 289 ms per layer with all four KV heads,
-    # 150 -> 142 ms with two, 3 the best of 2 .. 8 with one)
+    # measured on the 100,000-token prefill, when a tile's softmax still took longer than its
+    # MMAs: 302 -> 289 ms per layer with all four KV heads, 150 -> 142 ms with two, 3 the best
+    # of 2 .. 8 with one)
     best, best_us = 1, None
     for slices in range(1, 7):
         us = chunk_launch_estimate_us(chunk_rows, group, local_n_kv, pos0, slices, sm_pairs)
