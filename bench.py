@@ -927,7 +927,7 @@ L2_NOTE = "inputs larger than L2 (7.6 GB of Q/K/V per step)"
 # at position 6144 (ncu capture summarised in profiles/attn_chunk_tc_2048_at_6144.md), and the
 # algorithmic bytes of that launch (Q in, out, the staged K/V image once); other chunks are
 # scaled by their algorithmic bytes.
-NCU_CHUNK_TRAFFIC_BYTES = 143.0e6
+NCU_CHUNK_TRAFFIC_BYTES = 146.6e6
 NCU_CHUNK_ALGORITHMIC_BYTES = 2 * CHUNK * QW * 4 + 8192 * 8192
 
 
