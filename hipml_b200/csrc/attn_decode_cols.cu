@@ -56,10 +56,10 @@ __device__ int g_arrive_cols[kArriveRegions * kArriveRegionInts];
 
 // Which columns a cluster takes. Neighbouring columns with the same plan (the same units for every warp), at
 // most `each` of them (as many as fit the tiles, in groups of one size), are a group; a cluster has run `run` of
-// groups `group`, `group` + `hop`, ... Groups go to clusters of their own while a head has clusters to spare for their
-// runs, and columns share conversions beyond (4 columns of 300 rows take 2 runs each: 8 clusters of the head's 18; of 8,192 rows 17: one cluster
-// per run takes all four). `cap`: the clusters of a head; what its groups do not need ends at once, so there is one
-// round of them and they take the groups in turn.
+// groups `group`, `group` + `hop`, ... Groups go to clusters of their own while a head has clusters to spare for
+// their runs, and columns share conversions beyond (4 columns of 300 rows take 2 runs each: 8 clusters of the head's
+// 18; of 8,192 rows 17: one cluster per run takes all four). `cap`: the clusters of a head; what its groups do not
+// need ends at once, so there is one round of them and they take the groups in turn.
 struct Share {
     int each, run, group, hop;
     unsigned starts;   // bit c: column c's plan is not column c - 1's
@@ -233,276 +233,276 @@ __global__ void __launch_bounds__(kThreads, 1) attn_decode_cols(DecodeParams p, 
         checked = true;
         tc_fence_after();
         if (base >= p.n_slots) break;
-        if (live) {
-        // this warp's accumulators of tile a: lanes 32 * (warp % 4), columns 128 a + 64 * (warp / 4)
-        const unsigned tmem = s_tmem + ((unsigned)(warp & 3) << 21) + 64u * (warp >> 2);
-        // live rows of heads 2t, 2t + 1 of every tile (heads past the last: the longest's)
-        int len[kTiles][2];
-#pragma unroll
-        for (int a = 0; a < kTiles; a++)
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int f = 8 * a + 2 * t + h;
-                len[a][h] = f < heads ? s_len[base + f / group] : row1;
-            }
-
-        Running run[kTiles];
-#pragma unroll
-        for (int a = 0; a < kTiles; a++) start(run[a]);
-        auto work = [&](auto row_tiles, int i, int rows) __attribute__((always_inline)) {
-            constexpr int kT = decltype(row_tiles)::value;
-            const int r0 = first + i * w.unit * kWarps;
-            // ---- scores of all tiles
-            wait(0);
-            float s[kTiles][kT][4];
+        if (live) {   // a run of these columns that has rows
+            // this warp's accumulators of tile a: lanes 32 * (warp % 4), columns 128 a + 64 * (warp / 4)
+            const unsigned tmem = s_tmem + ((unsigned)(warp & 3) << 21) + 64u * (warp >> 2);
+            // live rows of heads 2t, 2t + 1 of every tile (heads past the last: the longest's)
+            int len[kTiles][2];
 #pragma unroll
             for (int a = 0; a < kTiles; a++)
 #pragma unroll
-                for (int j = 0; j < kT; j++)
+                for (int h = 0; h < 2; h++) {
+                    const int f = 8 * a + 2 * t + h;
+                    len[a][h] = f < heads ? s_len[base + f / group] : row1;
+                }
+
+            Running run[kTiles];
 #pragma unroll
-                    for (int e = 0; e < 4; e++) s[a][j][e] = 0.0f;
-            const unsigned *const krow = reinterpret_cast<const unsigned *>(ring) + g * Row<false>::kPitch;
-#pragma unroll 1
-            for (int M = 0; M < 4; M++) {   // pairs of blocks
-                KFrag<kT> f;
-                load_k<0, false, kT>(krow + M * Row<false>::kPair, t, f);
+            for (int a = 0; a < kTiles; a++) start(run[a]);
+            auto work = [&](auto row_tiles, int i, int rows) __attribute__((always_inline)) {
+                constexpr int kT = decltype(row_tiles)::value;
+                const int r0 = first + i * w.unit * kWarps;
+                // ---- scores of all tiles
+                wait(0);
+                float s[kTiles][kT][4];
 #pragma unroll
                 for (int a = 0; a < kTiles; a++)
-                    if (a < tiles)
-                        add_scores<0, kT>(f, query_of(a) + lane + 4 * 32 * M,
-                                          reinterpret_cast<const float4 *>(bias_of(a)) + t + 8 * M, s[a]);
-            }
-            __syncwarp();
-            kp += step;
-            if (lane == 0 && i + 1 < nw) fetch(i + 1, kp, 0);
-            // ---- softmax (where the unit begins past a column's end, that column gets nothing from it)
-            __half2 ph[kTiles][kT][2], pl[kTiles][kT][2];
-            auto sight = [&](int a, int h) { return min(w.unit, min(row1, len[a][h]) - r0); };
-            // Heads (a bit each) whose references move: all of a column as soon as one of them is exceeded, no others, as
-            // in the column's own launch.
-            unsigned moving = 0;
 #pragma unroll
-            for (int a = 0; a < kTiles; a++) {
-                if (a >= tiles) break;
-                const int rows_of[2] = {sight(a, 0), sight(a, 1)};
-                float nm[2], x[kT][4];
-                bool over[2];
-                exponents<kT, true>(s[a], rows_of, g, run[a], nm, x, over);
-                // (lane t of each group of four has heads 2t, 2t + 1)
-                if (over[0]) moving |= 1u << (8 * a + 2 * t);
-                if (over[1]) moving |= 2u << (8 * a + 2 * t);
-            }
-            if (__any_sync(0xffffffffu, moving != 0)) {
-                moving = __reduce_or_sync(0xffffffffu, moving);
-                const unsigned one = (1u << group) - 1;
-                for (int c = 0; c < n; c++)
-                    if (moving >> (c * group) & one) moving |= one << (c * group);
-            }
+                    for (int j = 0; j < kT; j++)
 #pragma unroll
-            for (int a = 0; a < kTiles; a++) {
-                if (a >= tiles) break;
-                const int rows_of[2] = {sight(a, 0), sight(a, 1)};
-                const unsigned mine = moving >> (8 * a);
-                auto decide = [&](const bool (&)[2], bool (&move)[2]) {
-                    move[0] = mine >> (2 * t) & 1;
-                    move[1] = mine >> (2 * t + 1) & 1;
-                    return (mine & 0xff) != 0;
-                };
-                float corr[2];
-                if (softmax<kT, true>(s[a], rows_of, g, run[a], ph[a], pl[a], corr, decide) && i > 0) {
+                        for (int e = 0; e < 4; e++) s[a][j][e] = 0.0f;
+                const unsigned *const krow = reinterpret_cast<const unsigned *>(ring) + g * Row<false>::kPitch;
 #pragma unroll 1
-                    for (int b = 0; b < 4; b++) {
-                        float v[16];
-                        tmem_ld16(tmem + 128 * a + 16 * b, v);
+                for (int M = 0; M < 4; M++) {   // pairs of blocks
+                    KFrag<kT> f;
+                    load_k<0, false, kT>(krow + M * Row<false>::kPair, t, f);
 #pragma unroll
-                        for (int e = 0; e < 16; e++) v[e] *= corr[e & 1];
-                        tmem_st16(tmem + 128 * a + 16 * b, v);
-                    }
-                    tmem_wait_st();
+                    for (int a = 0; a < kTiles; a++)
+                        if (a < tiles)
+                            add_scores<0, kT>(f, query_of(a) + lane + 4 * 32 * M,
+                                              reinterpret_cast<const float4 *>(bias_of(a)) + t + 8 * M, s[a]);
                 }
-            }
-            // ---- values
-            wait(1);
-            unsigned char *const vt = ring + C::kSlot;
-            // rows past the end have weight 0, but their scales must not be NaN or infinite
-            auto clear_rows = [&](int from, int to) {
-                for (int j = lane; j < (to - from) * (kRowBytes / 16); j += 32)
-                    reinterpret_cast<uint4 *>(vt + from * kRowBytes)[j] = make_uint4(0, 0, 0, 0);
                 __syncwarp();
-            };
-            if (rows < 16 * kT) clear_rows(rows, 16 * kT);
-            // Where a column ends inside the unit, the rows past its end are other columns': they stay. If one of them
-            // has such a scale, the columns take turns, the longest first, and each clears what it does not see.
-            auto rows_of = [&](int c) { return max(0, min(w.unit, min(row1, s_len[base + c]) - r0)); };
-            int shortest = rows;
-            for (int c = 0; c < n; c++) shortest = min(shortest, rows_of(c));
-            bool apart = false;
-            if (shortest < rows) {
-                bool bad = false;
-                for (int j = lane; j < (rows - shortest) * 8; j += 32) {
-                    const unsigned char *const scale = vt + (shortest + (j >> 3)) * kRowBytes + (j & 7) * kQ8BlockBytes;
-                    bad = bad || (*reinterpret_cast<const unsigned short *>(scale) & 0x7c00u) == 0x7c00u;
-                }
-                apart = __any_sync(0xffffffffu, bad);
-            }
-            const unsigned *const vrow = reinterpret_cast<const unsigned *>(vt) + 2 * t * Row<false>::kPitch;
-            // the values of the unit for all heads, or for those of column `only` (begun: there is something to add to)
-            auto value = [&](int M, auto masked, int only, bool begun) __attribute__((always_inline)) {
-                constexpr bool kMasked = decltype(masked)::value != 0;
-                VFrag f[kT];
-#pragma unroll
-                for (int j = 0; j < kT; j++)
-                    load_v<0, false>(vrow + M * Row<false>::kPair + j * 16 * Row<false>::kPitch, g, f[j]);
+                kp += step;
+                if (lane == 0 && i + 1 < nw) fetch(i + 1, kp, 0);
+                // ---- softmax (where the unit begins past a column's end, that column gets nothing from it)
+                __half2 ph[kTiles][kT][2], pl[kTiles][kT][2];
+                auto sight = [&](int a, int h) { return min(w.unit, min(row1, len[a][h]) - r0); };
+                // Heads (a bit each) whose references move: all of a column as soon as one of them is exceeded, no others, as
+                // in the column's own launch.
+                unsigned moving = 0;
 #pragma unroll
                 for (int a = 0; a < kTiles; a++) {
                     if (a >= tiles) break;
-                    float v[16];
-#pragma unroll
-                    for (int e = 0; e < 16; e++) v[e] = 0.0f;
-                    if (begun) tmem_ld16(tmem + 128 * a + 16 * M, v);
-                    float ve[2][4], vo[2][4];
-#pragma unroll
-                    for (int e = 0; e < 8; e++) {
-                        ve[e >> 2][e & 3] = v[e];
-                        vo[e >> 2][e & 3] = v[8 + e];
-                    }
-                    const bool keep = !kMasked || (8 * a + g) / group == only;
-#pragma unroll
-                    for (int j = 0; j < kT; j++) add_values<kMasked>(f[j], ph[a][j], pl[a][j], ve, vo, keep);
-#pragma unroll
-                    for (int e = 0; e < 8; e++) {
-                        v[e] = ve[e >> 2][e & 3];
-                        v[8 + e] = vo[e >> 2][e & 3];
-                    }
-                    tmem_st16(tmem + 128 * a + 16 * M, v);
+                    const int rows_of[2] = {sight(a, 0), sight(a, 1)};
+                    float nm[2], x[kT][4];
+                    bool over[2];
+                    exponents<kT, true>(s[a], rows_of, g, run[a], nm, x, over);
+                    // (lane t of each group of four has heads 2t, 2t + 1)
+                    if (over[0]) moving |= 1u << (8 * a + 2 * t);
+                    if (over[1]) moving |= 2u << (8 * a + 2 * t);
                 }
-            };
-            if (!apart) {
-#pragma unroll 1
-                for (int M = 0; M < 4; M++) value(M, Int<0>{}, 0, i > 0);
-            } else {
-                int upto = rows;
-                unsigned left = (1u << n) - 1;
-                for (bool begun = i > 0; left != 0; begun = true) {
-                    int c_at = 0, most = -1;
+                if (__any_sync(0xffffffffu, moving != 0)) {
+                    moving = __reduce_or_sync(0xffffffffu, moving);
+                    const unsigned one = (1u << group) - 1;
                     for (int c = 0; c < n; c++)
-                        if ((left >> c & 1) && rows_of(c) > most) {
-                            most = rows_of(c);
-                            c_at = c;
+                        if (moving >> (c * group) & one) moving |= one << (c * group);
+                }
+#pragma unroll
+                for (int a = 0; a < kTiles; a++) {
+                    if (a >= tiles) break;
+                    const int rows_of[2] = {sight(a, 0), sight(a, 1)};
+                    const unsigned mine = moving >> (8 * a);
+                    auto decide = [&](const bool (&)[2], bool (&move)[2]) {
+                        move[0] = mine >> (2 * t) & 1;
+                        move[1] = mine >> (2 * t + 1) & 1;
+                        return (mine & 0xff) != 0;
+                    };
+                    float corr[2];
+                    if (softmax<kT, true>(s[a], rows_of, g, run[a], ph[a], pl[a], corr, decide) && i > 0) {
+#pragma unroll 1
+                        for (int b = 0; b < 4; b++) {
+                            float v[16];
+                            tmem_ld16(tmem + 128 * a + 16 * b, v);
+#pragma unroll
+                            for (int e = 0; e < 16; e++) v[e] *= corr[e & 1];
+                            tmem_st16(tmem + 128 * a + 16 * b, v);
                         }
+                        tmem_wait_st();
+                    }
+                }
+                // ---- values
+                wait(1);
+                unsigned char *const vt = ring + C::kSlot;
+                // rows past the end have weight 0, but their scales must not be NaN or infinite
+                auto clear_rows = [&](int from, int to) {
+                    for (int j = lane; j < (to - from) * (kRowBytes / 16); j += 32)
+                        reinterpret_cast<uint4 *>(vt + from * kRowBytes)[j] = make_uint4(0, 0, 0, 0);
                     __syncwarp();
-                    clear_rows(most, upto);
-                    upto = most;
-                    left &= ~(1u << c_at);
-                    tmem_wait_st();   // what the turn before stored is loaded again
-#pragma unroll 1
-                    for (int M = 0; M < 4; M++) value(M, Int<1>{}, c_at, begun);
+                };
+                if (rows < 16 * kT) clear_rows(rows, 16 * kT);
+                // Where a column ends inside the unit, the rows past its end are other columns': they stay. If one of them
+                // has such a scale, the columns take turns, the longest first, and each clears what it does not see.
+                auto rows_of = [&](int c) { return max(0, min(w.unit, min(row1, s_len[base + c]) - r0)); };
+                int shortest = rows;
+                for (int c = 0; c < n; c++) shortest = min(shortest, rows_of(c));
+                bool apart = false;
+                if (shortest < rows) {
+                    bool bad = false;
+                    for (int j = lane; j < (rows - shortest) * 8; j += 32) {
+                        const unsigned char *const scale = vt + (shortest + (j >> 3)) * kRowBytes + (j & 7) * kQ8BlockBytes;
+                        bad = bad || (*reinterpret_cast<const unsigned short *>(scale) & 0x7c00u) == 0x7c00u;
+                    }
+                    apart = __any_sync(0xffffffffu, bad);
                 }
-            }
-            tmem_wait_st();
-            __syncwarp();
-            vp += step;
-            if (lane == 0 && i + 1 < nw) {
-                if (apart) fence_async_shared();   // generic writes to the slot come before the copy's
-                fetch(i + 1, vp, 1);
-            }
-            phase ^= 1;
-        };
-        for (int i = 0; i < nw; i++) {
-            const int rows = min(w.unit, row1 - (first + i * w.unit * kWarps));
-            if (rows > 16)
-                work(Int<2>{}, i, rows);
-            else
-                work(Int<1>{}, i, rows);
-        }
-
-        // ---- merge: the warps of the CTA, two tiles at a time, then the cluster, then the runs
-        const int items = group * 64;   // of a column
-        const bool one_run = w.runs == 1 && p.out != nullptr;
-        float2 *const wml = reinterpret_cast<float2 *>(smem + C::kOffMl);    // [heads][warps]
-        float4 *const cpart = reinterpret_cast<float4 *>(smem + C::kOffQ);   // [heads][64]: over the query fragments
-        float2 *const cml = reinterpret_cast<float2 *>(smem + C::kOffCml);   // [heads]
+                const unsigned *const vrow = reinterpret_cast<const unsigned *>(vt) + 2 * t * Row<false>::kPitch;
+                // the values of the unit for all heads, or for those of column `only` (begun: there is something to add to)
+                auto value = [&](int M, auto masked, int only, bool begun) __attribute__((always_inline)) {
+                    constexpr bool kMasked = decltype(masked)::value != 0;
+                    VFrag f[kT];
 #pragma unroll
-        for (int a = 0; a < kTiles; a++) {
-            if (a >= tiles) break;
-            sum_rows(run[a]);
-            if (g == 0) {
-                wml[(8 * a + 2 * t) * kWarps + warp] = make_float2(-run[a].nm[0], run[a].l[0]);
-                wml[(8 * a + 2 * t + 1) * kWarps + warp] = make_float2(-run[a].nm[1], run[a].l[1]);
-            }
-        }
-#pragma unroll 1
-        for (int a0 = 0; a0 < tiles; a0 += 2) {
-            const int a1 = min(a0 + 2, tiles);
-#pragma unroll 1
-            for (int a = a0; a < a1; a++) {
-                float v[64];
+                    for (int j = 0; j < kT; j++)
+                        load_v<0, false>(vrow + M * Row<false>::kPair + j * 16 * Row<false>::kPitch, g, f[j]);
 #pragma unroll
-                for (int e = 0; e < 64; e++) v[e] = 0.0f;
-                if (nw > 0) tmem_ld64(tmem + 128 * a, v);
-                float acc[8][2][4];
+                    for (int a = 0; a < kTiles; a++) {
+                        if (a >= tiles) break;
+                        float v[16];
 #pragma unroll
-                for (int e = 0; e < 64; e++) acc[e >> 3][(e >> 2) & 1][e & 3] = v[e];
-                store_warp_partial<false>(reinterpret_cast<float *>(ring + (a - a0) * C::kPartial), acc,
-                                          min(8, heads - 8 * a), g, t);
-            }
-            __syncthreads();
+                        for (int e = 0; e < 16; e++) v[e] = 0.0f;
+                        if (begun) tmem_ld16(tmem + 128 * a + 16 * M, v);
+                        float ve[2][4], vo[2][4];
+#pragma unroll
+                        for (int e = 0; e < 8; e++) {
+                            ve[e >> 2][e & 3] = v[e];
+                            vo[e >> 2][e & 3] = v[8 + e];
+                        }
+                        const bool keep = !kMasked || (8 * a + g) / group == only;
+#pragma unroll
+                        for (int j = 0; j < kT; j++) add_values<kMasked>(f[j], ph[a][j], pl[a][j], ve, vo, keep);
+#pragma unroll
+                        for (int e = 0; e < 8; e++) {
+                            v[e] = ve[e >> 2][e & 3];
+                            v[8 + e] = vo[e >> 2][e & 3];
+                        }
+                        tmem_st16(tmem + 128 * a + 16 * M, v);
+                    }
+                };
+                if (!apart) {
 #pragma unroll 1
-            for (int a = a0; a < a1; a++)
-                fold_warps(smem + (a - a0) * C::kPartial, C::kRing, wml + 8 * a * kWarps, min(8, heads - 8 * a) * 64,
-                           [&](int item, const Part &r) {
-                               cpart[a * 512 + item] = r.a;
-                               if ((item & 63) == 0) cml[a * 8 + (item >> 6)] = make_float2(r.m, r.l);
-                           });
-            if (a1 < tiles) __syncthreads();
-        }
-        cluster_sync_all();
-        // Column after column, beginning with another one in every run. Warps 0 .. group - 1 fold the cluster's partials
-        // of a column; another one (the s-th itself where there is none) announces the run.
-        auto column = [&](int s) { return (s + w.run) % n; };
-        const bool meet = p.out != nullptr && !one_run;
-        for (int s = 0; s < n; s++) {
-            const int c = column(s), announcer = group < 8 ? group + s % (8 - group) : s;
-            if (warp < group)
-                fold_cluster<kC>(cpart + c * items, cml + c * group, items, rank, [&](int item, const Part &r) {
-                    if (one_run) emit_item(p, base + c, kvh, group, item, r);
-                    const size_t row = (size_t)(kvh * group + (item >> 6)) * p.splits + w.run;
-                    reinterpret_cast<float4 *>(p.part_acc + (size_t)(base + c) * p.acc_slot + row * 256)[item & 63] = r.a;
-                    if (writes_pair<kC>(items, rank, item))
-                        *reinterpret_cast<float2 *>(p.part_ml + (size_t)(base + c) * p.ml_slot + row * 2) =
-                            make_float2(r.m, r.l);
-                });
-            if (!meet) continue;
-            const int threads = 32 * (group < 8 ? group + 1 : 8);
-            if (warp == announcer) {
-                named_sync(kArriveBar + s, threads);
-                if (lane == 0) {
-                    int *const ctr = g_arrive_cols + (size_t)p.arrive_region * kArriveRegionInts +
-                                     (size_t)((base + c) * p.n_kv + kvh) * p.arrive_stride + rank;
-                    const int last = arrive_acq_rel(ctr) == w.runs - 1;
-                    if (last) *ctr = 0;
-                    s_last[s] = last;
+                    for (int M = 0; M < 4; M++) value(M, Int<0>{}, 0, i > 0);
+                } else {
+                    int upto = rows;
+                    unsigned left = (1u << n) - 1;
+                    for (bool begun = i > 0; left != 0; begun = true) {
+                        int c_at = 0, most = -1;
+                        for (int c = 0; c < n; c++)
+                            if ((left >> c & 1) && rows_of(c) > most) {
+                                most = rows_of(c);
+                                c_at = c;
+                            }
+                        __syncwarp();
+                        clear_rows(most, upto);
+                        upto = most;
+                        left &= ~(1u << c_at);
+                        tmem_wait_st();   // what the turn before stored is loaded again
+#pragma unroll 1
+                        for (int M = 0; M < 4; M++) value(M, Int<1>{}, c_at, begun);
+                    }
                 }
+                tmem_wait_st();
                 __syncwarp();
-            } else if (warp < group) {
-                named_arrive(kArriveBar + s, threads);
-            }
-        }
-        cluster_arrive();   // no CTA may leave, or start over, while another still reads its partials
-        if (meet) {
-            __syncthreads();
-            for (int s = 0; s < n; s++)
-                if (s_last[s]) {
-                    if constexpr (kC == 2)
-                        fold_runs<kC, 18>(p, base + column(s), kvh, group, w.runs, rank, nullptr);
-                    else
-                        fold_runs<kC, 8>(p, base + column(s), kvh, group, w.runs, rank, nullptr);
+                vp += step;
+                if (lane == 0 && i + 1 < nw) {
+                    if (apart) fence_async_shared();   // generic writes to the slot come before the copy's
+                    fetch(i + 1, vp, 1);
                 }
+                phase ^= 1;
+            };
+            for (int i = 0; i < nw; i++) {
+                const int rows = min(w.unit, row1 - (first + i * w.unit * kWarps));
+                if (rows > 16)
+                    work(Int<2>{}, i, rows);
+                else
+                    work(Int<1>{}, i, rows);
+            }
+
+            // ---- merge: the warps of the CTA, two tiles at a time, then the cluster, then the runs
+            const int items = group * 64;   // of a column
+            const bool one_run = w.runs == 1 && p.out != nullptr;
+            float2 *const wml = reinterpret_cast<float2 *>(smem + C::kOffMl);    // [heads][warps]
+            float4 *const cpart = reinterpret_cast<float4 *>(smem + C::kOffQ);   // [heads][64]: over the query fragments
+            float2 *const cml = reinterpret_cast<float2 *>(smem + C::kOffCml);   // [heads]
+#pragma unroll
+            for (int a = 0; a < kTiles; a++) {
+                if (a >= tiles) break;
+                sum_rows(run[a]);
+                if (g == 0) {
+                    wml[(8 * a + 2 * t) * kWarps + warp] = make_float2(-run[a].nm[0], run[a].l[0]);
+                    wml[(8 * a + 2 * t + 1) * kWarps + warp] = make_float2(-run[a].nm[1], run[a].l[1]);
+                }
+            }
+#pragma unroll 1
+            for (int a0 = 0; a0 < tiles; a0 += 2) {
+                const int a1 = min(a0 + 2, tiles);
+#pragma unroll 1
+                for (int a = a0; a < a1; a++) {
+                    float v[64];
+#pragma unroll
+                    for (int e = 0; e < 64; e++) v[e] = 0.0f;
+                    if (nw > 0) tmem_ld64(tmem + 128 * a, v);
+                    float acc[8][2][4];
+#pragma unroll
+                    for (int e = 0; e < 64; e++) acc[e >> 3][(e >> 2) & 1][e & 3] = v[e];
+                    store_warp_partial<false>(reinterpret_cast<float *>(ring + (a - a0) * C::kPartial), acc,
+                                              min(8, heads - 8 * a), g, t);
+                }
+                __syncthreads();
+#pragma unroll 1
+                for (int a = a0; a < a1; a++)
+                    fold_warps(smem + (a - a0) * C::kPartial, C::kRing, wml + 8 * a * kWarps, min(8, heads - 8 * a) * 64,
+                               [&](int item, const Part &r) {
+                                   cpart[a * 512 + item] = r.a;
+                                   if ((item & 63) == 0) cml[a * 8 + (item >> 6)] = make_float2(r.m, r.l);
+                               });
+                if (a1 < tiles) __syncthreads();
+            }
+            cluster_sync_all();
+            // Column after column, beginning with another one in every run. Warps 0 .. group - 1 fold the cluster's partials
+            // of a column; another one (the s-th itself where there is none) announces the run.
+            auto column = [&](int s) { return (s + w.run) % n; };
+            const bool meet = p.out != nullptr && !one_run;
+            for (int s = 0; s < n; s++) {
+                const int c = column(s), announcer = group < 8 ? group + s % (8 - group) : s;
+                if (warp < group)
+                    fold_cluster<kC>(cpart + c * items, cml + c * group, items, rank, [&](int item, const Part &r) {
+                        if (one_run) emit_item(p, base + c, kvh, group, item, r);
+                        const size_t row = (size_t)(kvh * group + (item >> 6)) * p.splits + w.run;
+                        reinterpret_cast<float4 *>(p.part_acc + (size_t)(base + c) * p.acc_slot + row * 256)[item & 63] = r.a;
+                        if (writes_pair<kC>(items, rank, item))
+                            *reinterpret_cast<float2 *>(p.part_ml + (size_t)(base + c) * p.ml_slot + row * 2) =
+                                make_float2(r.m, r.l);
+                    });
+                if (!meet) continue;
+                const int threads = 32 * (group < 8 ? group + 1 : 8);
+                if (warp == announcer) {
+                    named_sync(kArriveBar + s, threads);
+                    if (lane == 0) {
+                        int *const ctr = g_arrive_cols + (size_t)p.arrive_region * kArriveRegionInts +
+                                         (size_t)((base + c) * p.n_kv + kvh) * p.arrive_stride + rank;
+                        const int last = arrive_acq_rel(ctr) == w.runs - 1;
+                        if (last) *ctr = 0;
+                        s_last[s] = last;
+                    }
+                    __syncwarp();
+                } else if (warp < group) {
+                    named_arrive(kArriveBar + s, threads);
+                }
+            }
+            cluster_arrive();   // no CTA may leave, or start over, while another still reads its partials
+            if (meet) {
+                __syncthreads();
+                for (int s = 0; s < n; s++)
+                    if (s_last[s]) {
+                        if constexpr (kC == 2)
+                            fold_runs<kC, 18>(p, base + column(s), kvh, group, w.runs, rank, nullptr);
+                        else
+                            fold_runs<kC, 8>(p, base + column(s), kvh, group, w.runs, rank, nullptr);
+                    }
+            }
+            cluster_wait();
+            __syncthreads();
+            if (lane == 0) fence_async_shared();   // partials were written over the rings; a next round's copies follow
         }
-        cluster_wait();
-        __syncthreads();
-        if (lane == 0) fence_async_shared();   // partials were written over the rings; a next round's copies follow
-        }   // a live run of these columns
         sh.group += sh.hop;   // the cluster's next group of columns
         if (sh.group >= groups) break;
         find_group(sh, p.n_slots, base, end);
