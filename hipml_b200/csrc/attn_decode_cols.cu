@@ -427,8 +427,8 @@ __global__ void __launch_bounds__(kThreads, 1) attn_decode_cols(DecodeParams p, 
                 if (a >= tiles) break;
                 sum_rows(run[a]);
                 if (g == 0) {
-                    wml[(8 * a + 2 * t) * kWarps + warp] = make_float2(-run[a].nm[0], run[a].l[0]);
-                    wml[(8 * a + 2 * t + 1) * kWarps + warp] = make_float2(-run[a].nm[1], run[a].l[1]);
+                    wml[(8 * a + 2 * t) * kWarps + warp] = make_float2(run[a].m[0], run[a].l[0]);
+                    wml[(8 * a + 2 * t + 1) * kWarps + warp] = make_float2(run[a].m[1], run[a].l[1]);
                 }
             }
 #pragma unroll 1

@@ -442,8 +442,8 @@ __global__ void __launch_bounds__(kThreads, kWide ? 1 : 2) attn_decode_warps(Dec
     sum_rows(run);
     float2 *const wml = reinterpret_cast<float2 *>(smem + C::kOffMl);      // [8 heads][warp]
     if (g == 0) {
-        wml[(2 * t) * kWarps + warp] = make_float2(-run.nm[0], run.l[0]);
-        wml[(2 * t + 1) * kWarps + warp] = make_float2(-run.nm[1], run.l[1]);
+        wml[(2 * t) * kWarps + warp] = make_float2(run.m[0], run.l[0]);
+        wml[(2 * t + 1) * kWarps + warp] = make_float2(run.m[1], run.l[1]);
     }
     store_warp_partial<kQ4>(reinterpret_cast<float *>(ring), acc, group, g, t);
     __syncthreads();
@@ -463,7 +463,7 @@ __global__ void __launch_bounds__(kThreads, kWide ? 1 : 2) attn_decode_warps(Dec
             acc_at[2] = r.a.z;
             acc_at[3] = r.a.w;
             if (with_ml) {
-                ml_at[0] = r.m;
+                ml_at[0] = p.unit_weights ? r.m - kPScaleLog2 : r.m;
                 ml_at[1] = r.l;
             }
         }
@@ -527,7 +527,7 @@ __global__ void __launch_bounds__(kThreads, kWide ? 1 : 2) attn_decode_warps(Dec
                         constexpr float kInv = 1.0f / kPScale;
 #pragma unroll
                         for (int i = 0; i < 8; i++) f.a[i] = staged[warp * 256 + lane * 8 + i] * kInv;
-                        f.big = ml.x + kPScaleLog2;
+                        f.big = ml.x;
                         f.den = ml.y * kInv;
                     }
                     fold_finish(p, status, w.slot, w.kvh, group, f);
@@ -579,7 +579,7 @@ __global__ void __launch_bounds__(kThreads) attn_decode_warps_fold(DecodeParams 
         constexpr float kInv = 1.0f / kPScale;
 #pragma unroll
         for (int i = 0; i < 8; i++) f.a[i] = staged[warp * 256 + lane * 8 + i] * kInv;
-        f.big = ml.x + kPScaleLog2;
+        f.big = ml.x;
         f.den = ml.y * kInv;
     }
     fold_finish(p, status, slot, kvh, group, f);

@@ -204,7 +204,10 @@ static int decode_kv(hipml_stream_t stream, const int *step, int selector, const
         if ((reinterpret_cast<size_t>(part_ml) & 7) != 0)
             return fail(HIPML_ERR_INVALID_ARGUMENT, "part_ml must be 8-byte aligned");
         fold_launch = (reinterpret_cast<size_t>(part_acc) & 15) != 0;
-        if (fold_launch) p.run_cap = 0;   // (every slot is written: that fold reads all `splits`)
+        if (fold_launch) {
+            p.run_cap = 0;        // (every slot is written: that fold reads all `splits`)
+            p.unit_weights = 1;   // (and makes rows of them that are folded with other bodies')
+        }
     }
     if (!fold_launch) {
         p.out = out;

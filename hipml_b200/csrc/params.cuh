@@ -45,6 +45,7 @@ struct DecodeParams {
     float *out = nullptr;            // nullptr: partials only, the caller launches the fold
     long long out_slot = 0, out_head_stride = 0;
     int normalize = 1;               // 0: out row = [acc (unnormalised) | max | sum]
+    int unit_weights = 0;            // partials only: a body that scales its weights leaves the scale out of their maxima
     const float *gate = nullptr;     // optional, normalize only: out *= sigmoid(gate)
     int arrive_region = -1, arrive_stride = 0;
     // Sequence-split decode across GPUs: instead of writing `out` directly the folding CTA

@@ -381,9 +381,10 @@ def _triple(q, k, v, n_kv, scale):
 
 
 # every body of the head_dim-256 kernel: one run, several, a head in one cluster
+@pytest.mark.parametrize("fold_mode", [0, 1], ids=["fold_inside", "fold_launch"])
 @pytest.mark.parametrize("selector", [0, 1, 6, 7, 8])
 @pytest.mark.parametrize("seq", [1, 40, 700, 5000])
-def test_a_shard_s_triple_is_its_sum_of_weights(seq, selector):
+def test_a_shard_s_triple_is_its_sum_of_weights(seq, selector, fold_mode):
     """acc * 2^max and sum * 2^max are the sums over the rows, whichever body made them: a caller folds them with others."""
     from hipml_b200 import api
     heads, n_kv, hd, scale = 24, 4, 256, 0.0625
@@ -394,7 +395,11 @@ def test_a_shard_s_triple_is_its_sum_of_weights(seq, selector):
     acc, ml = (torch.full((heads * splits * n,), float("nan"), device="cuda") for n in (hd, 2))
     got = torch.full((heads, hd + 2), float("nan"), device="cuda")
     step = torch.tensor([seq - 1, seq] + [0] * 6, dtype=torch.int32, device="cuda")
-    api.attn_decode_kv_shard(step, q, kc, vc, acc, ml, got, heads, n_kv, hd, seq + 3, scale, splits, selector=selector)
+    api.set_decode_fold_mode(fold_mode)
+    try:
+        api.attn_decode_kv_shard(step, q, kc, vc, acc, ml, got, heads, n_kv, hd, seq + 3, scale, splits, selector=selector)
+    finally:
+        api.set_decode_fold_mode(0)
     assert api.check_device_status() == 0
     total, out = _triple(q, k, v, n_kv, scale)
     got = got.double()
@@ -423,6 +428,34 @@ def test_shards_of_different_bodies_fold_to_the_whole_cache():
     api.attn_decode_combine(gathered, out, heads, hd, len(parts))
     assert api.check_device_status() == 0
     assert _close(out, _triple(q, torch.cat(keys), torch.cat(values), n_kv, scale)[1])
+
+
+@pytest.mark.parametrize("fold_mode", [0, 1], ids=["fold_inside", "fold_launch"])
+def test_ranks_of_different_bodies_exchange_the_same_sums(fold_mode):
+    """Each rank's workspace on this device, all publish, then all collect."""
+    from hipml_b200 import api
+    heads, n_kv, hd, scale, lens, selectors = 24, 4, 256, 0.0625, (700, 300), (0, 8)
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    q = torch.randn(heads * hd, device="cuda", generator=gen)
+    ws = [torch.zeros(api.decode_exchange_bytes(heads, hd, 2), dtype=torch.uint8, device="cuda") for _ in lens]
+    ranks = [_quantised_cache(gen, n, n, n_kv, 0) for n in lens]
+    outs = torch.full((2, heads, hd), float("nan"), device="cuda")
+    api.set_decode_fold_mode(fold_mode)
+    try:
+        for phase in (1, 2):
+            for r, (n, (kc, vc, _)) in enumerate(zip(lens, ranks)):
+                splits = api.decode_splits(n)
+                acc, ml = (torch.full((heads * splits * m,), float("nan"), device="cuda") for m in (hd, 2))
+                step = torch.tensor([n - 1, n] + [0] * 6, dtype=torch.int32, device="cuda")
+                api.attn_decode_kv_shard_exchange(step, q, kc, vc, acc, ml, outs[r], heads, n_kv, hd, n, scale, splits,
+                                                  [w.data_ptr() for w in ws], r, phases=phase, wait_limit_us=1000,
+                                                  selector=selectors[r])
+    finally:
+        api.set_decode_fold_mode(0)
+    assert api.check_device_status() == 0
+    want = _triple(q, *(torch.cat([c[2][i] for c in ranks]) for i in range(2)), n_kv, scale)[1]
+    for out in outs:
+        assert _close(out, want)
 
 
 # an empty shard, one row, one run, several; a length past the cache, whose rows are followed by others that would be seen
