@@ -1050,8 +1050,8 @@ static int fold_capacity(int slices) {
 // shortest, among those whose clusters all start together; a slice stays below the 64 tiles where a pair would move its
 // sums to memory. Launches of more pairs than that keep whole tiles and one slice. Over 196 sizes with 1, 4 and 8 KV heads
 // and groups of four, six and eight the shape it takes is on average 1.0 % behind the best one, 163 times within 2 %; the
-// worst are 130 tokens at 0 (17.4 us, tiles of 16: 15.1) and 500 at 3,001 (128.6, 121.1), where the estimate does not see
-// that the last tiles of a KV head leave a pair half empty.
+// worst are 130 tokens at 0 (17.4 us in tiles of 14; 15.1 of 16, whose longest pair holds two queries) and 500 at 3,001
+// (128.6 us in whole tiles; 121.1 of 16, which are more pairs than leave a third of the places free).
 struct ChunkShape {
     int qtile, fold;
 };
